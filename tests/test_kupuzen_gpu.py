@@ -169,6 +169,21 @@ def test_prompts_of_more_than_a_thousand_tokens_and_many_heads(dev, dtype):
     m.close()
 
 
+@pytest.mark.parametrize("ff", [48, 5008])
+def test_32bit_products_at_the_edges_of_row_tiles(dev, ff):
+    """Rows around the GEMM's 128-row tiles, inner widths of many 64-wide stages, few and many output tiles (64 and 128
+    columns wide). A sum of K fp32 terms is off by about sqrt(K) 2^-24 of its size, below 1e-5 with a wide margin."""
+    case = U.config([(U.attn(2, 1, 32, 32, 400, 8), ff)], width=1088, vocab=60)
+    W, toks = U.weights(case, 69), U.tokens(case[0], 300, 70)
+    want = D.run(case[0], W, toks)
+    m = load(dev, case, W, 300, "float32")
+    for n in (2, 127, 128, 129, 300):
+        assert U.rel_err(m.forward_rows(toks[:n], 0, np.arange(n)), want[:n]) < 1e-5, n
+    one = m.forward_rows(toks[:1], 0, [0])  # the output layer's GEMM behind a single-token pass
+    assert U.rel_err(one, want[:1]) < 1e-5
+    m.close()
+
+
 def test_a_stream_too_wide_for_the_norm_inside_the_decode_projection(dev):
     case = U.config([(U.attn(2, 1, 32, 32, 9, 8), 24), (U.delta(2, 1, 32, 16, 4, (5, 5)), 16)], width=6016, vocab=40)
     W, toks = U.weights(case, 67), U.tokens(case[0], 30, 68)

@@ -42,7 +42,7 @@ double rotation_frequency(const RotSpec &r, uint32_t i) {
 Decoder::~Decoder() {
   for (DecLayer &l : L)
     for (vkl_tensor *t : {l.norm.w, l.norm.b, l.norm2.w, l.norm2.b, l.qw, l.kw, l.freq, l.sink, l.taps, l.wl, l.biasl, l.rate, l.onorm, l.w1, l.bias1, l.w2, l.bias_o, l.rel, l.we1, l.we2, l.table, l.slot, l.token, l.tile_expert}) vkl_tensor_release(t);
-  for (vkl_tensor *t : {emb, head, step, final_norm.w, final_norm.b, x, h, q, gate, a2, low, dv, dz, dblocks, xe, hp, tp, y, want, hw, logits_rows, trace, attn_scratch, attn_counters}) vkl_tensor_release(t);
+  for (vkl_tensor *t : {emb, head, step, final_norm.w, final_norm.b, x, h, q, gate, a2, low, dv, dz, dblocks, split, xe, hp, tp, y, want, hw, logits_rows, trace, attn_scratch, attn_counters}) vkl_tensor_release(t);
 }
 
 namespace {
@@ -700,6 +700,12 @@ int decoder_ensure_rows(vkl_model *m, uint32_t T) {
       VKL_OKAY(zeros(m, &d->y, 1, rows, d->ldw, VKL_FP32));
     }
   }
+  if (d->f32 && T > 1) {  // the three bf16 parts of a GEMM's input, whichever is the largest
+    size_t most = std::max((size_t)(d->spec.two_norms ? 2 : 1) * T * d->ldw, (size_t)T * d->k2_max);
+    if (d->recurrent) most = std::max(most, (size_t)2 * T * d->low_max);
+    if (d->top_max) most = std::max(most, (size_t)d->hp->h * std::max(d->ldw, d->ffe_max));
+    VKL_OKAY(ensure_tensor(m->dev, &d->split, 3, 1, most, VKL_BF16));
+  }
   // decode: enough cache ranges to spread a few key heads over the SMs; longer calls have rows enough
   m->splits = 1;
   for (size_t i = 0; i < d->L.size(); ++i) {
@@ -913,7 +919,8 @@ int run_delta(vkl_model *m, size_t r, uint32_t T, bool pdl) {
   g.out.scale = 1.f;
   g.error = (uint32_t *)m->state->data() + 6;
   m->gemm_used = true;
-  VKL_LAUNCH(1, f32 ? launch_gemm_rows_f32(g, s) : launch_gemm_rows_bf16(g, s));
+  if (f32) g.split = (bf16 *)d->split->data();
+  VKL_LAUNCH(f32 ? 2 : 1, f32 ? launch_gemm_rows_f32(g, s) : launch_gemm_rows_bf16(g, s));
   p.z = g.out.f32;
   p.z_ld = l.nl;
   p.v = (float *)d->dv->data();
@@ -936,7 +943,8 @@ int decoder_run(vkl_model *m, uint32_t T, bool pdl, Marker *mk) {
   auto gemm = [&](GemmRows &g) -> int {
     g.error = (uint32_t *)m->state->data() + 6;
     m->gemm_used = true;
-    VKL_LAUNCH(1, f32 ? launch_gemm_rows_f32(g, s) : launch_gemm_rows_bf16(g, s));
+    if (f32) g.split = (bf16 *)d->split->data();
+    VKL_LAUNCH(f32 ? 2 : 1, f32 ? launch_gemm_rows_f32(g, s) : launch_gemm_rows_bf16(g, s));
     return VKL_OK;
   };
   MARK(-1);
@@ -1188,6 +1196,7 @@ int decoder_run(vkl_model *m, uint32_t T, bool pdl, Marker *mk) {
     VKL_OKAY(ensure_tensor(m->dev, &d->want, 1, 1, n, VKL_UINT32));
     VKL_OKAY(ensure_tensor(m->dev, &d->hw, 1, n, d->ldw, compute_dtype(d)));
     VKL_OKAY(ensure_tensor(m->dev, &d->logits_rows, 1, n, d->vocab_p, VKL_FP32));
+    if (f32 && (!d->split || d->split->w < (size_t)n * d->ldw)) VKL_OKAY(ensure_tensor(m->dev, &d->split, 3, 1, (size_t)n * d->ldw, VKL_BF16));
     VKL_CUDA(cudaMemcpyAsync(d->want->data(), d->want_rows.data(), (size_t)n * 4, cudaMemcpyHostToDevice, s));
     VKL_LAUNCH(1, launch_gather_rows(d->h->data(), (const int32_t *)d->want->data(), n, (uint32_t)(d->ldw * es), d->hw->data(), s));
     GemmRows g = {};

@@ -121,6 +121,7 @@ struct Decoder {
   // activations for vkl_model::cap_T rows
   vkl_tensor *x = nullptr, *h = nullptr, *q = nullptr, *gate = nullptr, *a2 = nullptr;
   vkl_tensor *low = nullptr, *dv = nullptr, *dz = nullptr, *dblocks = nullptr;  // delta rule
+  vkl_tensor *split = nullptr;  // 32-bit mode: a GEMM's input in three bfloat16 parts
   vkl_tensor *xe = nullptr, *hp = nullptr, *tp = nullptr, *y = nullptr;  // experts: one token; grouped rows
   vkl_tensor *want = nullptr, *hw = nullptr, *logits_rows = nullptr, *trace = nullptr;
   uint32_t low_max = 0, dv_max = 0, dz_max = 0;

@@ -26,11 +26,10 @@
 //             raw fp32 rows with 128-bit stores.
 // Every mbarrier wait is bounded; on a time-out the kernel raises the error word, lets
 // copies in flight land, frees its TMEM and returns.
-#include <cuda.h>
-
 #include "common.cuh"
 #include "kernels.h"
 #include "rows.cuh"
+#include "tcgen05.cuh"
 
 #ifndef VKL_GEMM_TRACE
 #define VKL_GEMM_TRACE 0  // diagnostic build: CTA (0,0) stamps the global timer at fixed points of every K step
@@ -70,9 +69,6 @@ namespace {
 #ifndef VKL_GEMM_MMAONLY
 #define VKL_GEMM_MMAONLY 0  // diagnostic build: the MMA lane runs alone on whatever the shared memory holds
 #endif
-constexpr int BM = 128, BK = 64;
-constexpr uint32_t A_TILE_BYTES = BM * BK * 2;  // 16 KB
-constexpr uint32_t GEMM_WAIT_LIMIT = 1u << 22;
 constexpr int GEMM_THREADS = 192;          // FP16 weights: TMA producer, MMA, four epilogue warps
 #ifndef VKL_GEMM_NDW
 #define VKL_GEMM_NDW 16
@@ -107,78 +103,6 @@ template <int BN, bool Q8 = false> struct Cfg {
   static constexpr int STAGES = (RING_BYTES / (int)STAGE_BYTES) < 8 ? (RING_BYTES / (int)STAGE_BYTES) : 8;
   static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + (Q8 ? Q8_STAGING_BYTES : 0) + 1024;
 };
-
-__device__ __forceinline__ uint32_t sa(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// Bounded wait. `sleep_ns`: pause between polls, for the waits that are long by design (the epilogue warps wait
-// for the whole K loop): a warp that spins takes issue slots from the warps that work on the same sub-partition.
-__device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, uint32_t sleep_ns = 0) {
-  for (uint32_t i = 0; i < GEMM_WAIT_LIMIT; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if (sleep_ns) __nanosleep(sleep_ns);
-  }
-  return false;
-}
-
-// The same with the non-blocking test (mbarrier.test_wait), for the MMA lane: try_wait may suspend the thread.
-__device__ __forceinline__ bool mbar_spin_bounded(uint32_t bar, uint32_t parity) {
-  for (uint32_t i = 0; i < (GEMM_WAIT_LIMIT << 4); ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-
-// Shared-memory matrix descriptor: K-major tile, 128-byte swizzle, 8-row groups 1024 B apart.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr & 0x3FFFFu) >> 4);  // start address, 16-byte units
-  d |= (uint64_t)1 << 16;                   // leading-dimension offset (unused with swizzle)
-  d |= (uint64_t)(1024 >> 4) << 32;         // stride between 8-row groups
-  d |= (uint64_t)1 << 46;                   // descriptor version of this architecture
-  d |= (uint64_t)2 << 61;                   // 128-byte swizzle
-  return d;
-}
-
-// kind::f16 instruction descriptor: fp16 x fp16 or bf16 x bf16 -> fp32, both operands K-major, M x N tile.
-__host__ __device__ constexpr uint32_t instr_desc(uint32_t m, uint32_t n, bool bf) {
-  return (1u << 4) | (bf ? (1u << 7) | (1u << 10) : 0u) | ((n >> 3) << 17) | ((m >> 4) << 24);
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-               "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-               : "memory");
-}
-
-template <int COLS> __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"((uint32_t)COLS) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
-        "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 
 // One Q8_0 unit (16 rows x 32 columns, 512 bytes of codes) -> fp16 values q * d in the swizzled W tile.
 // Lane (g, t) holds 8 codes of row g and 8 codes of row g + 8 at columns 8 t .. 8 t + 7 (common.cuh). 128-byte
@@ -506,32 +430,6 @@ __global__ void swiglu_f32_kernel(const float *__restrict__ gate, const float *_
   out[i] = __float2half_rn(g / (1.0f + expf(-g)) * up[i]);
 }
 
-using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                 const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiled encode_tiled() {
-  static EncodeTiled fn = [] {
-    void *f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = nullptr;
-    return reinterpret_cast<EncodeTiled>(f);
-  }();
-  return fn;
-}
-
-// Tensor map over a row-major fp16 or bf16 matrix [rows, K]: boxes of 64 columns x box_rows rows,
-// 128-byte swizzle, rows beyond the matrix read as zero.
-bool make_map(CUtensorMap *map, const void *base, uint32_t rows, uint32_t K, uint32_t box_rows, bool bf = false) {
-  EncodeTiled enc = encode_tiled();
-  if (!enc) return false;
-  const cuuint64_t dims[2] = {K, rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-  const cuuint32_t box[2] = {BK, box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  return enc(map, bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 template <int BN, int KIND> cudaError_t launch_bn(const typename GemmArgs<KIND>::Type &p, cudaStream_t s, uint32_t w_rows) {
   constexpr bool Q8 = KIND == GK_Q8;
   CUtensorMap ma, mw;
@@ -551,13 +449,6 @@ template <int BN, int KIND> cudaError_t launch_bn(const typename GemmArgs<KIND>:
 }
 
 }  // namespace
-
-// SMs of the current device (the tile shape is chosen so that the grid still fills them).
-static size_t sm_count() {
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
-  return (size_t)n;
-}
 
 bool gemm_tcgen05_supported(uint32_t M, uint32_t N, uint32_t K) { return M >= 1 && K % BK == 0 && K >= BK && (N % 8) == 0; }
 

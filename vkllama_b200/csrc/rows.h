@@ -138,11 +138,12 @@ struct GemmRows {
   const int32_t *tile_expert;  // grouped: expert of every 128-row tile of A (-1: no tokens), or null
   uint32_t w_rows;             // grouped: experts * N
   uint32_t *error;
+  bf16 *split;                 // 32-bit only: room for 3 bf16 matrices of A's size (both inputs, with n2)
   RowsOut out;
 };
 constexpr uint32_t kInputAlign = 256;  // no tile of the GEMMs crosses a multiple of this many weight rows
 cudaError_t launch_gemm_rows_bf16(const GemmRows &p, cudaStream_t s);  // tcgen05
-cudaError_t launch_gemm_rows_f32(const GemmRows &p, cudaStream_t s);   // true 32-bit
+cudaError_t launch_gemm_rows_f32(const GemmRows &p, cudaStream_t s);   // true 32-bit (tcgen05 on A in three parts): two launches
 
 // ---- attention over a cache of keys and values, or of rows that are both (kv_attention.cu) ----
 struct KvAttn {
