@@ -536,6 +536,35 @@ def test_multiheadattention_many_rows(dev, T, offset, maxlen):
     assert_close(got, want, what="mha T=%d offset=%d maxlen=%d" % (T, offset, maxlen))
 
 
+# A cache that is split over CTAs: few rows behind a long history, in tiles (32 rows and more), row by row, the clipped
+# last row, and across the end of the ring; parts that a query row does not see, a last part of one column.
+@pytest.mark.parametrize("T,offset,maxlen,dim,clip", [(33, 700, 1024, 128, False), (70, 450, 512, 64, False), (64, 193, 257, 128, False),
+                                                     (45, 700, 1024, 64, True), (2, 511, 513, 128, False), (31, 300, 512, 64, False),
+                                                     (1, 64, 128, 128, False), (1, 511, 1024, 128, True)])
+def test_multiheadattention_split_cache(dev, T, offset, maxlen, dim, clip):
+    heads = 2
+    Wd = heads * dim
+    ws = [O.synth_q8_0(163, i, Wd, Wd, 0.0, 0.05) for i in range(4)]  # wk, wq, wv, wo
+    att = O.lib().orc_attn_create(heads, dim, maxlen)
+    cmd = vk.Command(dev)
+    cmd.begin()
+    tw = [up(cmd, dev, w, vk.Q8_0, 1, Wd, Wd) for w in ws]
+    op = vk.MultiHeadAttentionV2(dev, cmd, tw[0], tw[1], tw[2], tw[3], maxlen, dim, True, vk.FP16, True, clip).init()
+    cmd.end()
+    cmd.submit_and_wait()
+    for (t, off) in [(offset, 0), (T, offset), (T, offset)]:  # twice: the arrival counters are left at zero
+        x = O.synth_f16(163, 10 + off, t * Wd).reshape(t, Wd)
+        want = np.empty((1 if clip else t) * Wd, np.uint16)
+        O.lib().orc_attn_forward_q8_0(att, x, ws[0], ws[1], ws[2], ws[3], t, off, int(clip), want)
+        cmd.begin()
+        tx = up(cmd, dev, x, vk.FP16, 1, t, Wd)
+        got = cmd.download(op(tx, off))
+        cmd.end()
+        cmd.submit_and_wait()
+        assert_close(got, want, what="mha T=%d offset=%d maxlen=%d clip=%s" % (t, off, maxlen, clip))
+    O.lib().orc_attn_destroy(att)
+
+
 # ---- device memory pool -----------------------------------------------------------------------
 def test_released_block_is_not_reused_while_queued_work_still_writes_it(dev):
     """Ops return without synchronising and every command has its own stream. A tensor released on

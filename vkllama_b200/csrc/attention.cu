@@ -27,21 +27,34 @@ __device__ __forceinline__ void rope_pair(float x0, float x1, float c, float s, 
   o1 = __float2half_rn(x0 * s + x1 * c);
 }
 
-// Multi-token calls: cache[h,(pos+m)%maxlen,:] = rope(k[m,h,:]) and v likewise.
-__global__ void rope_append_kernel(const AttnParams p) {
-  const uint32_t h = blockIdx.x, m = blockIdx.y, i = threadIdx.x;  // i: pair index
-  if (2 * i >= p.dim) return;
+// Eight consecutive dimensions d .. d + 7 of a row at position pos, rotated.
+__device__ __forceinline__ uint4 rope8(uint4 raw, const AttnParams &p, size_t pos, uint32_t d) {
+  union {
+    uint4 u;
+    __half h[8];
+  } x;
+  x.u = raw;
+  const size_t fi = pos * (p.dim / 2) + d / 2;
+  const float4 c = __ldg(reinterpret_cast<const float4 *>(p.freqc + fi)), s = __ldg(reinterpret_cast<const float4 *>(p.freqs + fi));
+  const float cs[4] = {c.x, c.y, c.z, c.w}, sn[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) rope_pair(__half2float(x.h[2 * i]), __half2float(x.h[2 * i + 1]), cs[i], sn[i], x.h[2 * i], x.h[2 * i + 1]);
+  return x.u;
+}
+
+// Multi-token calls: cache[h,(pos+m)%maxlen,:] = rope(k[m,h,:]) and v likewise. A thread moves eight dimensions with
+// 16-byte accesses (the head width is a multiple of 8): bound by memory. 2048 rows of 32 heads x 128: 36 us with a
+// thread per pair and 64 threads per block, 10 this way.
+__global__ void __launch_bounds__(256) rope_append_kernel(const AttnParams p) {
+  const uint32_t vecs = p.dim / 8, row = p.heads * vecs;
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= (size_t)p.T * row) return;
+  const uint32_t m = (uint32_t)(i / row), c = (uint32_t)(i % row), h = c / vecs, d = c % vecs * 8;
   const uint32_t pos = *p.pos_dev + m;
-  const size_t fi = (size_t)pos * (p.dim / 2) + i;
-  const float c = p.freqc[fi], s = p.freqs[fi];
-  const size_t src = (size_t)m * p.heads * p.dim + (size_t)h * p.dim + 2 * i;
-  const size_t dst = ((size_t)h * p.maxlen + pos % p.maxlen) * p.dim + 2 * i;
-  __half k0, k1;
-  rope_pair(__half2float(p.k[src]), __half2float(p.k[src + 1]), c, s, k0, k1);
-  p.kcache[dst] = k0;
-  p.kcache[dst + 1] = k1;
-  p.vcache[dst] = p.v[src];
-  p.vcache[dst + 1] = p.v[src + 1];
+  const size_t src = (size_t)m * p.heads * p.dim + (size_t)c * 8, dst = ((size_t)h * p.maxlen + pos % p.maxlen) * p.dim + d;
+  const uint4 k = __ldg(reinterpret_cast<const uint4 *>(p.k + src)), v = __ldg(reinterpret_cast<const uint4 *>(p.v + src));
+  *reinterpret_cast<uint4 *>(p.kcache + dst) = rope8(k, p, pos, d);
+  *reinterpret_cast<uint4 *>(p.vcache + dst) = v;
 }
 
 // grid (heads, T, splits), 128 threads. FUSED: T == 1, the CTA whose column
@@ -60,8 +73,16 @@ __global__ void __launch_bounds__(kAttnThreads) attention_kernel(const AttnParam
   const uint32_t pos0 = *p.pos_dev;
   const uint32_t L = min(pos0 + p.T, p.maxlen);
   const uint32_t vis = min(L, m + (L - p.T) + 1);  // causal: col <= row + (W - H)
-  uint32_t chunk = (vis + p.splits - 1) / p.splits;
+  // a split holds 64 columns or more: a short cache is not spread over CTAs whose parts cost more to merge (one row,
+  // up to 49 columns: 11.8 us in eight splits of at most 32 columns, 7.5 in one)
+  uint32_t splits = min(p.splits, (vis + 63) / 64);
+  uint32_t chunk = (vis + splits - 1) / splits;
   chunk = (chunk + 31) & ~31u;
+  splits = (vis + chunk - 1) / chunk;
+  if (split >= splits) {
+    if (p.use_pdl) asm volatile("griddepcontrol.launch_dependents;");
+    return;
+  }
   const uint32_t c0 = min(split * chunk, vis), c1 = min(c0 + chunk, vis);
   const uint32_t jn = pos0 % p.maxlen;  // FUSED: physical column of the new token
   const bool owns_new = FUSED && jn >= c0 && jn < c1;
@@ -178,7 +199,7 @@ __global__ void __launch_bounds__(kAttnThreads) attention_kernel(const AttnParam
   if (p.use_pdl) asm volatile("griddepcontrol.launch_dependents;");
 
   __half *orow = p.out + (p.clip ? (size_t)h * D : row_in);
-  if (p.splits == 1) {
+  if (splits == 1) {
     if (grp == 0 && dp < npair) {
       orow[2 * dp] = __float2half_rn(acc.x / lloc);
       orow[2 * dp + 1] = __float2half_rn(acc.y / lloc);
@@ -199,21 +220,21 @@ __global__ void __launch_bounds__(kAttnThreads) attention_kernel(const AttnParam
   __threadfence();
   __syncthreads();
   __shared__ uint32_t s_last;
-  if (tid == 0) s_last = atomicAdd(&p.counters[unit], 1u) == p.splits - 1;
+  if (tid == 0) s_last = atomicAdd(&p.counters[unit], 1u) == splits - 1;
   __syncthreads();
   if (!s_last) return;
   __threadfence();
   const float *base = p.scratch + unit * p.splits * (D + 2);
   float M = -INFINITY;
-  for (uint32_t s = 0; s < p.splits; ++s) M = fmaxf(M, __ldcg(base + s * (D + 2) + D));
+  for (uint32_t s = 0; s < splits; ++s) M = fmaxf(M, __ldcg(base + s * (D + 2) + D));
   float den = 0.f;
-  for (uint32_t s = 0; s < p.splits; ++s) {
+  for (uint32_t s = 0; s < splits; ++s) {
     const float ms = __ldcg(base + s * (D + 2) + D), ls = __ldcg(base + s * (D + 2) + D + 1);
     if (ls > 0.f) den += ls * expf(ms - M);
   }
   for (uint32_t d = tid; d < D; d += kAttnThreads) {
     float num = 0.f;
-    for (uint32_t s = 0; s < p.splits; ++s) {
+    for (uint32_t s = 0; s < splits; ++s) {
       const float ms = __ldcg(base + s * (D + 2) + D), ls = __ldcg(base + s * (D + 2) + D + 1);
       if (ls > 0.f) num += __ldcg(base + s * (D + 2) + d) * expf(ms - M);
     }
@@ -238,6 +259,14 @@ size_t attn_smem(const AttnParams &p) {
 // O += P.V with V fragments transposed by ldmatrix. Columns are physical cache rows 0..L-1 with
 // the reference's mask col <= row + (L - T) (softmax_fp16.comp:52-60), so a wrapped ring behaves
 // as in the per-row kernel.
+//
+// Bound: the mma.sync pipe (a quarter of the tcgen05 rate) beside the softmax's instructions. So all fragments
+// come by ldmatrix, the V tile is on its way (cp.async) during Q.K^T and the next K tile during P.V, only
+// tiles at the causal edge are masked, and one tile of each (52 KB) leaves room for three CTAs per SM that hide each
+// other's softmax. Few query tiles behind a long cache do not fill the SMs: the cache is then split
+// (grid z, at least kSplitTiles tiles each) and the CTA of a query tile that finishes last merges the parts in order.
+// 32 heads x 128, 2048 rows: 255 us with scalar fragment loads and no overlap, 140 now (244 TFLOP/s of the causal half);
+// 40 heads, 45 rows behind 700: 66 -> 19 us, mostly by the splits.
 __device__ __forceinline__ void mma16816_h(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -248,99 +277,127 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
   return *reinterpret_cast<const uint32_t *>(&v);
 }
 
+__device__ __forceinline__ void ldm4(uint32_t (&r)[4], const __half *p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldm4t(uint32_t (&r)[4], const __half *p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+
+constexpr uint32_t kSplitTiles = 2;   // a split of the tile kernel holds at least this many 64-row cache tiles
+constexpr uint32_t kMostSplits = 8;
+constexpr float kLog2e = 1.4426950408889634f;
+
 template <int D>
-__global__ void __launch_bounds__(128) attention_tile_kernel(const AttnParams p) {
+__global__ void __launch_bounds__(128, 3) attention_tile_kernel(const AttnParams p) {
   constexpr int QT = 64, KT = 64, LD = D + 8;  // padded rows: conflict-free fragment loads
   extern __shared__ __align__(16) __half smh[];
   __half *q_s = smh;             // [QT][LD] roped queries
   __half *k_s = q_s + QT * LD;   // [KT][LD]
   __half *v_s = k_s + KT * LD;   // [KT][LD]
-  const uint32_t h = blockIdx.x, m0 = blockIdx.y * QT, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  __shared__ uint32_t last_s;
+  const uint32_t h = blockIdx.x, qt = gridDim.y - 1 - blockIdx.y, m0 = qt * QT;  // longest rows first
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const uint32_t T = p.T, pos0 = *p.pos_dev;
   const uint32_t L = min(pos0 + T, p.maxlen), shift = L - T;
-  for (uint32_t i = tid; i < QT * (D / 2); i += 128) {  // rotate the query tile at positions pos0 + row
-    const uint32_t r = i / (D / 2), pr = i % (D / 2), m = m0 + r;
-    __half r0 = __float2half_rn(0.f), r1 = r0;
-    if (m < T) {
-      const size_t fi = (size_t)(pos0 + m) * (D / 2) + pr, src = (size_t)m * p.heads * D + (size_t)h * D + 2 * pr;
-      rope_pair(__half2float(p.q[src]), __half2float(p.q[src + 1]), p.freqc[fi], p.freqs[fi], r0, r1);
+  const uint32_t jmax = min(L, min(m0 + QT, T) + shift);  // columns any row of this tile can see
+  const uint32_t tiles = (jmax + KT - 1) / KT;
+  const uint32_t most = min(gridDim.z, (tiles + kSplitTiles - 1) / kSplitTiles), per = (tiles + most - 1) / most, splits = (tiles + per - 1) / per;
+  const uint32_t split = blockIdx.z;
+  if (split >= splits) return;
+  const uint32_t j_begin = split * per * KT, j_end = min(jmax, j_begin + per * KT);
+  const __half *kc = p.kcache + (size_t)h * p.maxlen * D, *vc = p.vcache + (size_t)h * p.maxlen * D;
+  auto fetch = [&](__half *dst, const __half *src, uint32_t j0) {  // 64 cache rows; those beyond L become zero
+#pragma unroll
+    for (uint32_t i = tid; i < KT * (D / 8); i += 128) {
+      const uint32_t r = i / (D / 8), c8 = i % (D / 8), j = j0 + r;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * LD + c8 * 8)),
+                   "l"(src + (j < L ? (size_t)j * D + c8 * 8 : 0)), "r"(j < L ? 16u : 0u)
+                   : "memory");
     }
-    q_s[r * LD + 2 * pr] = r0;
-    q_s[r * LD + 2 * pr + 1] = r1;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(k_s, kc, j_begin);
+  for (uint32_t i = tid; i < QT * (D / 8); i += 128) {  // rotate the query tile at positions pos0 + row
+    const uint32_t r = i / (D / 8), d = i % (D / 8) * 8, m = m0 + r;
+    uint4 q = make_uint4(0, 0, 0, 0);
+    if (m < T) q = rope8(__ldg(reinterpret_cast<const uint4 *>(p.q + (size_t)m * p.heads * D + (size_t)h * D + d)), p, (size_t)pos0 + m, d);
+    *reinterpret_cast<uint4 *>(q_s + r * LD + d) = q;
   }
   const uint32_t r_lo = m0 + warp * 16 + g, r_hi = r_lo + 8;
   const uint32_t vis_lo = r_lo < T ? min(L, r_lo + shift + 1) : 0u, vis_hi = r_hi < T ? min(L, r_hi + shift + 1) : 0u;
-  const uint32_t jmax = min(L, min(m0 + QT, T) + shift);  // columns any row of this tile can see
+  const uint32_t vis_all = m0 + warp * 16 + 15 < T ? min(L, m0 + warp * 16 + shift + 1) : 0u;  // columns that all of the warp's rows see
   const float scale = 1.0f / sqrtf((float)D);
   float o[D / 8][4];
 #pragma unroll
   for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-  float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;
-  const __half *kc = p.kcache + (size_t)h * p.maxlen * D, *vc = p.vcache + (size_t)h * p.maxlen * D;
-  const __half *qw = q_s + (warp * 16 + g) * LD + 2 * t;
-  for (uint32_t j0 = 0; j0 < jmax; j0 += KT) {
-    __syncthreads();  // the previous tile is consumed (and, first time, the query tile is written)
-    for (uint32_t i = tid; i < KT * (D / 8); i += 128) {
-      const uint32_t r = i / (D / 8), c8 = i % (D / 8), j = j0 + r;
-      uint4 kv = make_uint4(0, 0, 0, 0), vv = kv;
-      if (j < L) {
-        kv = __ldg(reinterpret_cast<const uint4 *>(kc + (size_t)j * D) + c8);
-        vv = __ldg(reinterpret_cast<const uint4 *>(vc + (size_t)j * D) + c8);
-      }
-      *reinterpret_cast<uint4 *>(k_s + r * LD + c8 * 8) = kv;
-      *reinterpret_cast<uint4 *>(v_s + r * LD + c8 * 8) = vv;
-    }
-    __syncthreads();
+  float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;  // l: this thread's columns, summed over the row's four threads at the end
+  const __half *qf = q_s + (warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LD + (lane >> 4) * 8;
+  const __half *kf = k_s + ((lane & 7) + (lane >> 4) * 8) * LD + ((lane >> 3) & 1) * 8;
+  const __half *vf = v_s + ((lane & 7) + ((lane >> 3) & 1) * 8) * LD + (lane >> 4) * 8;
+  for (uint32_t j0 = j_begin; j0 < j_end; j0 += KT) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // the K tile is here for everyone (first time: the query tile too), the last V tile is consumed
+    fetch(v_s, vc, j0);
     // ---- S = Q.K^T: 16 rows x 64 columns per warp
     float sc[KT / 8][4];
 #pragma unroll
     for (int nt = 0; nt < KT / 8; ++nt) sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f;
 #pragma unroll
     for (int kk = 0; kk < D / 16; ++kk) {
-      const uint32_t a0 = *reinterpret_cast<const uint32_t *>(qw + kk * 16), a1 = *reinterpret_cast<const uint32_t *>(qw + 8 * LD + kk * 16);
-      const uint32_t a2 = *reinterpret_cast<const uint32_t *>(qw + kk * 16 + 8), a3 = *reinterpret_cast<const uint32_t *>(qw + 8 * LD + kk * 16 + 8);
+      uint32_t a[4], b[4];
+      ldm4(a, qf + kk * 16);
 #pragma unroll
-      for (int nt = 0; nt < KT / 8; ++nt) {
-        const __half *kr = k_s + (nt * 8 + g) * LD + kk * 16 + 2 * t;
-        mma16816_h(sc[nt], a0, a1, a2, a3, *reinterpret_cast<const uint32_t *>(kr), *reinterpret_cast<const uint32_t *>(kr + 8));
+      for (int nt = 0; nt < KT / 8; nt += 2) {
+        ldm4(b, kf + nt * 8 * LD + kk * 16);
+        mma16816_h(sc[nt], a[0], a[1], a[2], a[3], b[0], b[1]);
+        mma16816_h(sc[nt + 1], a[0], a[1], a[2], a[3], b[2], b[3]);
       }
     }
     // ---- scaled fp16 scores, mask, running max and sum
     float tmax_lo = -INFINITY, tmax_hi = -INFINITY;
 #pragma unroll
     for (int nt = 0; nt < KT / 8; ++nt) {
-      const uint32_t c = j0 + nt * 8 + 2 * t;
-      sc[nt][0] = c < vis_lo ? round_h(sc[nt][0] * scale) : -INFINITY;
-      sc[nt][1] = c + 1 < vis_lo ? round_h(sc[nt][1] * scale) : -INFINITY;
-      sc[nt][2] = c < vis_hi ? round_h(sc[nt][2] * scale) : -INFINITY;
-      sc[nt][3] = c + 1 < vis_hi ? round_h(sc[nt][3] * scale) : -INFINITY;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sc[nt][i] = round_h(sc[nt][i] * scale);
+    }
+    if (j0 + KT > vis_all) {  // uniform over the warp
+#pragma unroll
+      for (int nt = 0; nt < KT / 8; ++nt) {
+        const uint32_t c = j0 + nt * 8 + 2 * t;
+        if (c >= vis_lo) sc[nt][0] = -INFINITY;
+        if (c + 1 >= vis_lo) sc[nt][1] = -INFINITY;
+        if (c >= vis_hi) sc[nt][2] = -INFINITY;
+        if (c + 1 >= vis_hi) sc[nt][3] = -INFINITY;
+      }
+    }
+#pragma unroll
+    for (int nt = 0; nt < KT / 8; ++nt) {
       tmax_lo = fmaxf(tmax_lo, fmaxf(sc[nt][0], sc[nt][1]));
       tmax_hi = fmaxf(tmax_hi, fmaxf(sc[nt][2], sc[nt][3]));
     }
-    tmax_lo = fmaxf(tmax_lo, __shfl_xor_sync(0xffffffffu, tmax_lo, 1));
-    tmax_lo = fmaxf(tmax_lo, __shfl_xor_sync(0xffffffffu, tmax_lo, 2));
-    tmax_hi = fmaxf(tmax_hi, __shfl_xor_sync(0xffffffffu, tmax_hi, 1));
-    tmax_hi = fmaxf(tmax_hi, __shfl_xor_sync(0xffffffffu, tmax_hi, 2));
+#pragma unroll
+    for (int w = 1; w < 4; w <<= 1) {
+      tmax_lo = fmaxf(tmax_lo, __shfl_xor_sync(0xffffffffu, tmax_lo, w));
+      tmax_hi = fmaxf(tmax_hi, __shfl_xor_sync(0xffffffffu, tmax_hi, w));
+    }
     const float mn_lo = fmaxf(m_lo, tmax_lo), mn_hi = fmaxf(m_hi, tmax_hi);
-    const float corr_lo = m_lo == -INFINITY ? 0.f : expf(m_lo - mn_lo), corr_hi = m_hi == -INFINITY ? 0.f : expf(m_hi - mn_hi);
+    const float ref_lo = mn_lo == -INFINITY ? 0.f : mn_lo, ref_hi = mn_hi == -INFINITY ? 0.f : mn_hi;
+    const float corr_lo = exp2f((m_lo - ref_lo) * kLog2e), corr_hi = exp2f((m_hi - ref_hi) * kLog2e);
+    m_lo = mn_lo;
+    m_hi = mn_hi;
     float rs_lo = 0.f, rs_hi = 0.f;
 #pragma unroll
     for (int nt = 0; nt < KT / 8; ++nt) {
-      sc[nt][0] = sc[nt][0] == -INFINITY ? 0.f : expf(sc[nt][0] - mn_lo);
-      sc[nt][1] = sc[nt][1] == -INFINITY ? 0.f : expf(sc[nt][1] - mn_lo);
-      sc[nt][2] = sc[nt][2] == -INFINITY ? 0.f : expf(sc[nt][2] - mn_hi);
-      sc[nt][3] = sc[nt][3] == -INFINITY ? 0.f : expf(sc[nt][3] - mn_hi);
+      sc[nt][0] = exp2f((sc[nt][0] - ref_lo) * kLog2e);
+      sc[nt][1] = exp2f((sc[nt][1] - ref_lo) * kLog2e);
+      sc[nt][2] = exp2f((sc[nt][2] - ref_hi) * kLog2e);
+      sc[nt][3] = exp2f((sc[nt][3] - ref_hi) * kLog2e);
       rs_lo += sc[nt][0] + sc[nt][1];
       rs_hi += sc[nt][2] + sc[nt][3];
     }
-    rs_lo += __shfl_xor_sync(0xffffffffu, rs_lo, 1);
-    rs_lo += __shfl_xor_sync(0xffffffffu, rs_lo, 2);
-    rs_hi += __shfl_xor_sync(0xffffffffu, rs_hi, 1);
-    rs_hi += __shfl_xor_sync(0xffffffffu, rs_hi, 2);
     l_lo = l_lo * corr_lo + rs_lo;
     l_hi = l_hi * corr_hi + rs_hi;
-    m_lo = mn_lo;
-    m_hi = mn_hi;
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) {
       o[i][0] *= corr_lo;
@@ -348,22 +405,69 @@ __global__ void __launch_bounds__(128) attention_tile_kernel(const AttnParams p)
       o[i][2] *= corr_hi;
       o[i][3] *= corr_hi;
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // the V tile is here for everyone, the K tile is consumed
+    if (j0 + KT < j_end) fetch(k_s, kc, j0 + KT);
     // ---- O += P.V: 16 cache rows per step, V fragments transposed by ldmatrix
 #pragma unroll
     for (int j16 = 0; j16 < KT / 16; ++j16) {
       const uint32_t a0 = pack_h2(sc[2 * j16][0], sc[2 * j16][1]), a1 = pack_h2(sc[2 * j16][2], sc[2 * j16][3]);
       const uint32_t a2 = pack_h2(sc[2 * j16 + 1][0], sc[2 * j16 + 1][1]), a3 = pack_h2(sc[2 * j16 + 1][2], sc[2 * j16 + 1][3]);
-      // lane l gives the address of row l % 8 of matrix l / 8: matrices (rows +0, cols +0), (rows +8, cols +0), (rows +0, cols +8), (rows +8, cols +8)
-      const __half *vrow = v_s + (j16 * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LD + ((lane >> 4) & 1) * 8;
 #pragma unroll
       for (int dt = 0; dt < D / 16; ++dt) {
-        uint32_t b0, b1, b2, b3;
-        const uint32_t addr = (uint32_t)__cvta_generic_to_shared(vrow + dt * 16);
-        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(addr));
-        mma16816_h(o[2 * dt], a0, a1, a2, a3, b0, b1);
-        mma16816_h(o[2 * dt + 1], a0, a1, a2, a3, b2, b3);
+        uint32_t b[4];
+        ldm4t(b, vf + j16 * 16 * LD + dt * 16);
+        mma16816_h(o[2 * dt], a0, a1, a2, a3, b[0], b[1]);
+        mma16816_h(o[2 * dt + 1], a0, a1, a2, a3, b[2], b[3]);
       }
     }
+  }
+#pragma unroll
+  for (int w = 1; w < 4; w <<= 1) {
+    l_lo += __shfl_xor_sync(0xffffffffu, l_lo, w);
+    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, w);
+  }
+  if (splits > 1) {
+    // ---- a part per split, in this kernel's own fragment order: [D / 8 + 1][128 threads] x 16 bytes
+    constexpr uint32_t kPart = (D / 8 + 1) * 128;
+    const uint32_t unit = qt * p.heads + h;
+    float4 *part = reinterpret_cast<float4 *>(p.scratch) + (size_t)unit * gridDim.z * kPart + tid;
+    float4 *mine = part + (size_t)split * kPart;
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i) __stcg(mine + i * 128, make_float4(o[i][0], o[i][1], o[i][2], o[i][3]));
+    __stcg(mine + D / 8 * 128, make_float4(m_lo, m_hi, l_lo, l_hi));
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) last_s = atomicAdd(&p.counters[unit], 1u) == splits - 1;
+    __syncthreads();
+    if (!last_s) return;
+    __threadfence();
+    float M_lo = -INFINITY, M_hi = -INFINITY;
+    for (uint32_t s = 0; s < splits; ++s) {
+      const float4 ml = __ldcg(part + (size_t)s * kPart + D / 8 * 128);
+      M_lo = fmaxf(M_lo, ml.x);
+      M_hi = fmaxf(M_hi, ml.y);
+    }
+    if (M_lo == -INFINITY) M_lo = 0.f;
+    if (M_hi == -INFINITY) M_hi = 0.f;
+    l_lo = l_hi = 0.f;
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    for (uint32_t s = 0; s < splits; ++s) {
+      const float4 ml = __ldcg(part + (size_t)s * kPart + D / 8 * 128);
+      const float c_lo = exp2f((ml.x - M_lo) * kLog2e), c_hi = exp2f((ml.y - M_hi) * kLog2e);
+      l_lo = fmaf(c_lo, ml.z, l_lo);
+      l_hi = fmaf(c_hi, ml.w, l_hi);
+#pragma unroll
+      for (int i = 0; i < D / 8; ++i) {
+        const float4 v = __ldcg(part + (size_t)s * kPart + i * 128);
+        o[i][0] = fmaf(c_lo, v.x, o[i][0]);
+        o[i][1] = fmaf(c_lo, v.y, o[i][1]);
+        o[i][2] = fmaf(c_hi, v.z, o[i][2]);
+        o[i][3] = fmaf(c_hi, v.w, o[i][3]);
+      }
+    }
+    if (tid == 0) p.counters[unit] = 0;
   }
   // ---- out[m, h*D + d] = fp16(O / sum)
   const float inv_lo = l_lo > 0.f ? 1.0f / l_lo : 0.f, inv_hi = l_hi > 0.f ? 1.0f / l_hi : 0.f;
@@ -377,26 +481,48 @@ __global__ void __launch_bounds__(128) attention_tile_kernel(const AttnParams p)
 
 constexpr uint32_t kTileMinRows = 32;  // below this the per-row kernel is used
 
+bool use_tiles(uint32_t T, bool clip, uint32_t dim) {
+  static const bool off = [] { const char *e = getenv("VKLLAMA_PREFILL_ATTENTION"); return e && !strcmp(e, "rows"); }();
+  return !off && T >= kTileMinRows && !clip && (dim == 64 || dim == 128);
+}
+
 }  // namespace
 
-size_t attention_scratch_bytes(uint32_t T, uint32_t heads, uint32_t dim, uint32_t splits) {
-  return (size_t)T * heads * splits * (dim + 2) * sizeof(float);
+// Parts that a cache is split into. The last row of 2048 (32 heads) took 136 us in one part per head and 28 in eight. Tiles: up to three CTAs per SM; rows (128 threads each): four per SM, and eight splits
+// for a single row, as in decode. The kernels use fewer where the cache is short.
+AttnPlan attention_plan(uint32_t T, bool clip, uint32_t heads, uint32_t dim, uint32_t sms) {
+  AttnPlan a = {};
+  const bool tiles = use_tiles(T, clip, dim);
+  const uint32_t rows = tiles ? (T + 63) / 64 : clip ? 1 : T, units = rows * heads, fit = (tiles ? 3 : 4) * sms / units;
+  a.splits = rows == 1 && !tiles ? kMostSplits : fit < 1 ? 1 : fit > kMostSplits ? kMostSplits : fit;
+  a.scratch_bytes = a.splits == 1 ? 0 : (size_t)units * a.splits * (tiles ? 64 * (dim + 8) : dim + 2) * sizeof(float);
+  a.counters = units;
+  return a;
+}
+AttnPlan attention_plan_most(uint32_t T, uint32_t heads, uint32_t dim, uint32_t sms) {
+  AttnPlan a = {};
+  a.splits = kMostSplits;
+  const size_t row_units = (size_t)(kMostSplits * heads > 4 * sms ? kMostSplits * heads : 4 * sms), tile_units = (size_t)3 * sms;
+  a.scratch_bytes = row_units * (dim + 2) * sizeof(float);
+  if (T >= kTileMinRows && a.scratch_bytes < tile_units * 64 * (dim + 8) * sizeof(float)) a.scratch_bytes = tile_units * 64 * (dim + 8) * sizeof(float);
+  a.counters = heads > 4 * sms ? heads : 4 * sms;
+  return a;
 }
 
 cudaError_t launch_attention(const AttnParams &p, cudaStream_t s) {
   if (p.dim > 128 || (p.dim & 7) || p.T == 0) return cudaErrorInvalidValue;
   if (p.T > 1) {
-    rope_append_kernel<<<dim3(p.heads, p.T), 64, 0, s>>>(p);
+    const size_t n = (size_t)p.T * p.heads * (p.dim / 8);
+    rope_append_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  static const bool tile_off = [] { const char *e = getenv("VKLLAMA_PREFILL_ATTENTION"); return e && !strcmp(e, "rows"); }();
-  if (!tile_off && p.T >= kTileMinRows && !p.clip && (p.dim == 64 || p.dim == 128)) {
+  if (use_tiles(p.T, p.clip, p.dim)) {
     const size_t tsmem = (size_t)3 * 64 * (p.dim + 8) * sizeof(__half);
     auto tk = p.dim == 128 ? attention_tile_kernel<128> : attention_tile_kernel<64>;
     cudaError_t e = cudaFuncSetAttribute(tk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem);
     if (e != cudaSuccess) return e;
-    tk<<<dim3(p.heads, (p.T + 63) / 64), 128, tsmem, s>>>(p);
+    tk<<<dim3(p.heads, (p.T + 63) / 64, p.splits), 128, tsmem, s>>>(p);
     return cudaGetLastError();
   }
   const size_t smem = attn_smem(p);

@@ -124,9 +124,9 @@ struct AttnParams {
   __half *out;
   const float *freqc, *freqs;
   const uint32_t *pos_dev;  // position of row 0, read on the device
-  float *scratch;           // splits*T*heads*(dim+2) floats
-  uint32_t *counters;       // T*heads, zero before first use (left zero after)
-  uint32_t T, heads, dim, maxlen, splits;
+  float *scratch;           // of attention_plan's size
+  uint32_t *counters;       // attention_plan's number, zero before first use (left zero after)
+  uint32_t T, heads, dim, maxlen, splits;  // splits: attention_plan's, or fewer
   // clip: only the last row is computed and written to row 0 of `out`; its query is
   // rotated at position pos (row 0), as the reference does after clipping Q
   // (src/ops/multiheadattention_v2.cpp:223-253).
@@ -134,7 +134,13 @@ struct AttnParams {
   int use_pdl;
 };
 cudaError_t launch_attention(const AttnParams &p, cudaStream_t s);
-size_t attention_scratch_bytes(uint32_t T, uint32_t heads, uint32_t dim, uint32_t splits);
+struct AttnPlan {
+  uint32_t splits;
+  size_t scratch_bytes;
+  uint32_t counters;
+};
+AttnPlan attention_plan(uint32_t T, bool clip, uint32_t heads, uint32_t dim, uint32_t sms);
+AttnPlan attention_plan_most(uint32_t T, uint32_t heads, uint32_t dim, uint32_t sms);  // what calls of up to T rows need
 
 // ---- persistent decode step (decode_mega.cu) --------------------------------
 enum MegaKind { MK_EMBED = 0, MK_MATVEC = 1, MK_ATTN_PART = 2, MK_ATTN_COMBINE = 3, MK_ARGMAX = 4, MK_ALLREDUCE = 5 };

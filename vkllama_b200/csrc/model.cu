@@ -66,7 +66,7 @@ int ensure_rows(vkl_model *m, uint32_t T) {
   VKL_OKAY(ensure_tensor(m->dev, &m->t, 1, T, m->ffn_l, VKL_FP16));
   if (T >= gemm_min_rows(q8(m))) VKL_OKAY(ensure_tensor(m->dev, &m->gu32, 2, T, m->ffn_l, VKL_FP32));
   VKL_OKAY(ensure_tensor(m->dev, &m->toks, 1, 1, T, VKL_UINT32));
-  const size_t sc = attention_scratch_bytes(1, m->heads_l, m->head_dim, m->splits);
+  const size_t sc = attention_plan_most(T, m->heads_l, m->head_dim, (uint32_t)m->dev->prop.multiProcessorCount).scratch_bytes;
   VKL_OKAY(ensure_tensor(m->dev, &m->attn_scratch, 1, 1, sc / 4, VKL_FP32));
   m->cap_T = T;
   return VKL_OK;
@@ -194,7 +194,7 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
     a.pos_dev = m->pos_dev();
     a.scratch = (float *)m->attn_scratch->data(); a.counters = (uint32_t *)m->attn_counters->data();
     a.T = T; a.heads = m->heads_l; a.dim = m->head_dim; a.maxlen = m->cfg.maxlen;
-    a.splits = dec ? m->splits : 1;
+    a.splits = attention_plan(T, clip, a.heads, a.dim, (uint32_t)m->dev->prop.multiProcessorCount).splits;
     a.clip = clip;
     a.use_pdl = dec && pdl;
     VKL_LAUNCH(dec ? 1 : 2, launch_attention(a, s));
@@ -815,9 +815,8 @@ int vkl_model_create(vkl_device *dev, const vkl_model_config *cfg, vkl_model **o
   }
   // Positions up to 2*maxlen are valid, the size the reference gives its tables (rope.cpp:73-76).
   if (int st = rope_tables(dev, m->stream, hd, 2 * c.maxlen, &m->fc, &m->fs)) return bail(st);
-  m->splits = 8;
   if ((st = tensor_new(dev, 1, 1, m->vocab_l, VKL_FP16, &m->logits16)) || (st = tensor_new(dev, 1, 1, c.maxlen, VKL_UINT32, &m->forced)) ||
-      (st = tensor_new(dev, 1, 1, m->heads_l, VKL_UINT32, &m->attn_counters)))
+      (st = tensor_new(dev, 1, 1, attention_plan_most(1, m->heads_l, m->head_dim, (uint32_t)dev->prop.multiProcessorCount).counters, VKL_UINT32, &m->attn_counters)))
     return bail(st);
   if (tp > 1) {
     m->tp_flag_off = 4 * tp * c.dim;  // partial sums: [2 parities][tp][dim] words of {fp32 sum, sequence number}
@@ -1298,7 +1297,7 @@ int vkl_model_block_forward(vkl_model *m, uint32_t layer, const void *x_fp16, si
   a.pos_dev = m->pos_dev();
   a.scratch = (float *)m->attn_scratch->data(); a.counters = (uint32_t *)m->attn_counters->data();
   a.T = (uint32_t)T; a.heads = m->heads_l; a.dim = m->head_dim; a.maxlen = m->cfg.maxlen;
-  a.splits = dec ? m->splits : 1;
+  a.splits = attention_plan(a.T, false, a.heads, a.dim, (uint32_t)m->dev->prop.multiProcessorCount).splits;
   VKL_LAUNCH(dec ? 1 : 2, launch_attention(a, s));
   MvParams o = mv(m, y.wo, (__half *)m->ao->data(), x, (uint32_t)T);
   o.residual = x;

@@ -288,7 +288,6 @@ struct MhaOp : vkl_op {
   vkl_tensor *k = nullptr, *q = nullptr, *v = nullptr, *heads_out = nullptr, *out = nullptr;
   vkl_tensor *kcache = nullptr, *vcache = nullptr, *fc = nullptr, *fs = nullptr;
   vkl_tensor *scratch = nullptr, *counters = nullptr, *pos = nullptr;
-  uint32_t splits = 1;
   MhaOp(vkl_device *d, vkl_command *c, vkl_tensor *a, vkl_tensor *b, vkl_tensor *e, vkl_tensor *f, int ml, int dm, int tw, int dt, int kv, int clip)
       : vkl_op(d, c), wk(a), wq(b), wv(e), wo(f), maxlen(ml), dim(dm), transposed_weight(tw), dtype(dt), use_kvcache(kv), clip_output(clip) {
     vkl_tensor_retain(wk); vkl_tensor_retain(wq); vkl_tensor_retain(wv); vkl_tensor_retain(wo);
@@ -318,8 +317,7 @@ struct MhaOp : vkl_op {
     VKL_CUDA(cudaMemsetAsync(kcache->data(), 0, kcache->device_bytes(), cmd->stream));
     VKL_CUDA(cudaMemsetAsync(vcache->data(), 0, vcache->device_bytes(), cmd->stream));
     VKL_OKAY(make_rope_tables(dev, cmd->stream, dim, 2 * maxlen, &fc, &fs));
-    splits = 4;
-    VKL_OKAY(tensor_new(dev, 1, 1, heads * 4, VKL_UINT32, &counters));
+    VKL_OKAY(tensor_new(dev, 1, 1, attention_plan_most(1, (uint32_t)heads, dim, (uint32_t)dev->prop.multiProcessorCount).counters, VKL_UINT32, &counters));
     VKL_CUDA(cudaMemsetAsync(counters->data(), 0, counters->device_bytes(), cmd->stream));
     VKL_OKAY(tensor_new(dev, 1, 1, 1, VKL_UINT32, &pos));
     return VKL_OK;
@@ -354,8 +352,8 @@ struct MhaOp : vkl_op {
     p.x_ld = p.K; p.out_ld = p.N; p.scale = 1.f; p.fp16_weights = !q8;
     VKL_LAUNCH((T + 63) / 64, launch_matvec(p, EPI_PLAIN, false, cmd->stream));
 
-    const uint32_t sp = T == 1 ? splits : 1;
-    const size_t need = attention_scratch_bytes((uint32_t)To, (uint32_t)heads, dim, sp);
+    const AttnPlan plan = attention_plan((uint32_t)T, clip_output && T > 1, (uint32_t)heads, dim, (uint32_t)dev->prop.multiProcessorCount);
+    const size_t need = std::max(plan.scratch_bytes, (size_t)16);
     if (!scratch || scratch->device_bytes() < need) {
       vkl_tensor_release(scratch);
       scratch = nullptr;
@@ -370,7 +368,7 @@ struct MhaOp : vkl_op {
     a.freqc = (const float *)fc->data(); a.freqs = (const float *)fs->data();
     a.pos_dev = (const uint32_t *)pos->data();
     a.scratch = (float *)scratch->data(); a.counters = (uint32_t *)counters->data();
-    a.T = (uint32_t)T; a.heads = (uint32_t)heads; a.dim = dim; a.maxlen = maxlen; a.splits = sp;
+    a.T = (uint32_t)T; a.heads = (uint32_t)heads; a.dim = dim; a.maxlen = maxlen; a.splits = plan.splits;
     a.clip = clip_output ? 1 : 0;
     VKL_LAUNCH(T > 1 ? 2 : 1, launch_attention(a, cmd->stream));
 
