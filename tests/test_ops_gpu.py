@@ -209,6 +209,29 @@ def test_feed_forward_q8_0(dev, M, dim, hidden):
     assert_close(got, want, what="feed_forward")
 
 
+# Many rows: gate and up share a tensor-core tile and meet in its epilogue. Hidden sizes that end inside a half tile, rows
+# around the row tiles of one CTA (128) and of a pair of CTAs (256).
+@pytest.mark.parametrize("wt", ["f16", "q8_0"])
+@pytest.mark.parametrize("M,dim,hidden", [(65, 128, 64), (127, 64, 192), (129, 192, 320), (257, 64, 448), (300, 128, 1088)])
+def test_feed_forward_many_rows(dev, wt, M, dim, hidden):
+    dt = vk.FP16 if wt == "f16" else vk.Q8_0
+    if wt == "f16":
+        ws = [O.synth_f16(57, i, n, 0.0, 0.05) for i, n in ((1, hidden * dim), (2, dim * hidden), (3, hidden * dim))]
+    else:
+        ws = [O.synth_q8_0(57, i, r, c, 0.0, 0.05) for i, (r, c) in ((1, (hidden, dim)), (2, (dim, hidden)), (3, (hidden, dim)))]
+    x = O.synth_f16(57, 4, M * dim).reshape(M, dim)
+    want = np.empty(M * dim, np.uint16)
+    getattr(O.lib(), "orc_feed_forward_" + wt)(x, ws[0], ws[1], ws[2], want, M, dim, hidden)
+    cmd = vk.Command(dev)
+    cmd.begin()
+    w1, w2, w3 = (up(cmd, dev, w, dt, 1, r, c) for w, (r, c) in zip(ws, ((hidden, dim), (dim, hidden), (hidden, dim))))
+    op = vk.FeedForward(dev, cmd, w1, w2, w3, True, dt).init()
+    got = cmd.download(op(up(cmd, dev, x, vk.FP16, 1, M, dim)))
+    cmd.end()
+    cmd.submit_and_wait()
+    assert_close(got, want, what="feed_forward %s M=%d" % (wt, M))
+
+
 # ---- RMSNorm (tests/test_rmsnorm.cpp:100-105: [1,1,128]; 7B rows) -------------
 @pytest.mark.parametrize("rows,W,eps", [(1, 128, 1e-3), (1, 4096, 1e-5), (33, 4096, 1e-5), (5, 100, 1e-6)])
 def test_rms_norm(dev, rows, W, eps):
@@ -534,6 +557,26 @@ def test_multiheadattention_many_rows(dev, T, offset, maxlen):
         cmd.end()
         cmd.submit_and_wait()
     assert_close(got, want, what="mha T=%d offset=%d maxlen=%d" % (T, offset, maxlen))
+
+
+# FP16 weights: 32 rows and more take the tensor-core GEMM (three matrices in one launch), fewer the mat-vec kernel. The
+# same rows in portions of either size agree within the rounding of their fp16 results.
+@pytest.mark.parametrize("T", [32, 129, 300])
+def test_multiheadattention_f16_portions_agree(dev, T):
+    heads, dim, maxlen = 3, 64, 320
+    Wd = heads * dim
+    ws = [O.synth_f16(165, i, Wd * Wd, 0.0, 0.08) for i in range(4)]
+    x = O.synth_f16(165, 9, T * Wd).reshape(T, Wd)
+    cmd = vk.Command(dev)
+    cmd.begin()
+    tw = [up(cmd, dev, w, vk.FP16, 1, Wd, Wd) for w in ws]
+    ops = [vk.MultiHeadAttentionV2(dev, cmd, tw[0], tw[1], tw[2], tw[3], maxlen, dim, True, vk.FP16, True, False).init() for _ in range(2)]
+    whole = cmd.download(ops[0](up(cmd, dev, x, vk.FP16, 1, T, Wd), 0))
+    parts = [cmd.download(ops[1](up(cmd, dev, x[i:i + 20], vk.FP16, 1, len(x[i:i + 20]), Wd), i)) for i in range(0, T, 20)]
+    cmd.end()
+    cmd.submit_and_wait()
+    got = np.concatenate([p.reshape(-1) for p in parts])
+    assert_close(whole, got, tol=4e-3, what="mha fp16 T=%d" % T)
 
 
 # A cache that is split over CTAs: few rows behind a long history, in tiles (32 rows and more), row by row, the clipped

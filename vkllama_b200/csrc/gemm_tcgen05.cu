@@ -26,6 +26,8 @@
 //             raw fp32 rows with 128-bit stores.
 // Every mbarrier wait is bounded; on a time-out the kernel raises the error word, lets
 // copies in flight land, frees its TMEM and returns.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "rows.cuh"
@@ -130,7 +132,7 @@ template <> struct GemmArgs<GK_ROWS> { using Type = GemmRows; };
 
 template <int BN, int KIND>
 __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS, 1)
-    gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const typename GemmArgs<KIND>::Type p) {
+    gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ WeightMaps maps, const typename GemmArgs<KIND>::Type p) {
   constexpr bool Q8 = KIND == GK_Q8;
   using C = Cfg<BN, Q8>;
   extern __shared__ unsigned char smem_raw[];
@@ -146,7 +148,19 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
   __shared__ volatile uint32_t failed_s;
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+  // grid y: one matrix's column tiles behind the other's. SwiGLU: the first half of a W tile is gate rows, the second
+  // the up rows of the same outputs.
+  uint32_t mat = 0, ny = blockIdx.y;
+  bool swiglu = false;
+  if constexpr (KIND != GK_ROWS) {
+    swiglu = p.swiglu;
+    const uint32_t per = (p.N + BN - 1) / BN;
+    if (!swiglu) {
+      mat = ny / per;
+      ny -= mat * per;
+    }
+  }
+  const uint32_t m0 = blockIdx.x * BM, n0 = ny * (swiglu ? BN / 2 : BN);
   const uint32_t nkb = p.K / BK;
   uint32_t w_row = n0, a_row = m0;  // first weight and input row of the tile
   if constexpr (KIND == GK_ROWS) {
@@ -199,7 +213,8 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(Q8 ? A_TILE_BYTES : C::STAGE_BYTES) : "memory");
         unsigned char *st = stages + (size_t)s * C::STAGE_BYTES;
         tma_load_2d(sa(st), &map_a, kb * BK, a_row, bar);
-        if (!Q8) tma_load_2d(sa(st + A_TILE_BYTES), &map_w, kb * BK, w_row, bar);
+        if (!Q8) tma_load_2d(sa(st + A_TILE_BYTES), &maps.w[mat], kb * BK, w_row, bar);
+        if (!Q8 && swiglu) tma_load_2d(sa(st + A_TILE_BYTES + C::B_TILE_BYTES / 2), &maps.w[1], kb * BK, w_row, bar);
       }
     }
   } else if (Q8 && warp >= 6 && (warp & 3u) != 1u && !VKL_GEMM_MMAONLY) {
@@ -226,11 +241,11 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
     bool valid[UPQ];
 #pragma unroll
     for (uint32_t j = 0; j < UPQ; ++j) {
-      const uint32_t u = wi + NDWG * j, tile = n0 / 16 + (u >> 1);
+      const uint32_t u = wi + NDWG * j, up = swiglu && (u >> 1) >= BN / 32 ? 1u : 0u, tile = n0 / 16 + (u >> 1) - up * (BN / 32);
       bl[j] = u & 1u;
       valid[j] = u < UNITS && tile < tiles16;
-      cbase[j] = p.w_codes + (((size_t)tile * groups * 4 + bl[j]) * 32 + lane) * 16;
-      sbase[j] = p.w_scales + ((size_t)tile * groups * 8 + g) * 16;
+      cbase[j] = p.w_codes[mat + up] + (((size_t)tile * groups * 4 + bl[j]) * 32 + lane) * 16;
+      sbase[j] = p.w_scales[mat + up] + ((size_t)tile * groups * 8 + g) * 16;
       const uint32_t ra = (u >> 1) * 16 + g, rb = ra + 8, c = bl[j] * 4 + t;
       off_a[j] = ra * 128 + ((c ^ (ra & 7)) << 4);
       off_b[j] = rb * 128 + ((c ^ (rb & 7)) << 4);
@@ -359,54 +374,38 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
       if (lane == 0) failed_s = 3;
     } else if (!failed_s) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll 1
-      for (uint32_t cc = 0; cc < (uint32_t)BN; cc += 32) {
-        if (n0 + cc >= p.N) break;  // uniform over the warp
+      // 32 fp32 results of this thread's row, from column `col` of the accumulators on
+      auto take = [&](uint32_t col, float (&v)[32]) {
         uint32_t r[32];
-        tmem_ld32(tmem_acc + ((quad * 32u) << 16) + cc, r);
-        if (NACC == 2) {
-          uint32_t r2[32];
-          tmem_ld32(tmem_acc + ((quad * 32u) << 16) + BN + cc, r2);
+        tmem_ld32(tmem_acc + ((quad * 32u) << 16) + col, r);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
+        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+        if (NACC == 2) {
+          tmem_ld32(tmem_acc + ((quad * 32u) << 16) + BN + col, r);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] += __uint_as_float(r[j]);
+        }
+      };
+      const uint32_t cols = swiglu ? BN / 2 : BN;
+#pragma unroll 1
+      for (uint32_t cc = 0; cc < cols; cc += 32) {
+        if (n0 + cc >= p.N) break;  // uniform over the warp
+        float acc[32];
+        take(cc, acc);
+        if constexpr (KIND != GK_ROWS && BN >= 64) {
+          if (swiglu) {
+            float up[32];
+            take(BN / 2 + cc, up);
+            if (row < p.M) swiglu_chunk(acc, up, p.c[0] + (size_t)row * p.N + n0 + cc, p.N - n0 - cc);
+            continue;
+          }
         }
         if constexpr (KIND == GK_ROWS) {
           if (row < p.M) {
-            float v[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-            rows_chunk<bf16>(p.out, row, n0 + cc, v);
+            rows_chunk<bf16>(p.out, row, n0 + cc, acc);
           }
         } else if (row < p.M) {
-          const size_t o = (size_t)row * p.N + n0 + cc;
-#pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            if (n0 + cc + j >= p.N) break;  // N is a multiple of 8
-            float v[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              v[i] = __uint_as_float(r[j + i]) * p.scale + p.bias;
-              if (p.act == 1) v[i] = v[i] / (1.0f + expf(-v[i]));
-            }
-            if (p.c_f32) {
-              *reinterpret_cast<float4 *>(p.c_f32 + o + j) = make_float4(v[0], v[1], v[2], v[3]);
-              *reinterpret_cast<float4 *>(p.c_f32 + o + j + 4) = make_float4(v[4], v[5], v[6], v[7]);
-            } else {
-              union {
-                uint4 u;
-                __half h[8];
-              } out, res;
-              if (p.residual) {
-                res.u = *reinterpret_cast<const uint4 *>(p.residual + o + j);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) out.h[i] = __float2half_rn(round_h(v[i]) + __half2float(res.h[i]));
-              } else {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) out.h[i] = __float2half_rn(v[i]);
-              }
-              *reinterpret_cast<uint4 *>(p.c + o + j) = out.u;
-            }
-          }
+          f16_chunk(p, mat, row, n0 + cc, acc);
         }
       }
     }
@@ -422,29 +421,24 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"((uint32_t)(NACC * BN)) : "memory");
 }
 
-// y <- fp16( silu(gate) * up ) on fp32 inputs: the epilogue of ffn_up_and_gate_fp16.comp.
-__global__ void swiglu_f32_kernel(const float *__restrict__ gate, const float *__restrict__ up, __half *__restrict__ out, size_t n) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float g = gate[i];
-  out[i] = __float2half_rn(g / (1.0f + expf(-g)) * up[i]);
-}
-
 template <int BN, int KIND> cudaError_t launch_bn(const typename GemmArgs<KIND>::Type &p, cudaStream_t s, uint32_t w_rows) {
   constexpr bool Q8 = KIND == GK_Q8;
-  CUtensorMap ma, mw;
-  uint32_t a_rows = p.M;
-  if constexpr (KIND == GK_ROWS) a_rows *= p.n2 ? 2 : 1;
-  if (!make_map(&ma, p.a, a_rows, p.K, BM, KIND == GK_ROWS)) return cudaErrorInvalidValue;
-  if constexpr (Q8) {
-    mw = ma;  // unused: the W tile is written by the dequantising warps
-  } else if (!make_map(&mw, p.w, w_rows, p.K, BN, KIND == GK_ROWS)) {
-    return cudaErrorInvalidValue;
+  CUtensorMap ma;
+  WeightMaps mw = {};  // unused with Q8_0: the W tile is written by the dequantising warps
+  uint32_t a_rows = p.M, ny = (p.N + BN - 1) / BN;
+  if constexpr (KIND == GK_ROWS) {
+    a_rows *= p.n2 ? 2 : 1;
+    if (!make_map(&mw.w[0], p.w, w_rows, p.K, BN, true)) return cudaErrorInvalidValue;
+  } else {
+    for (uint32_t i = 0; i < p.nmat && !Q8; ++i)
+      if (!make_map(&mw.w[i], p.w[i], w_rows, p.K, p.swiglu ? BN / 2 : BN)) return cudaErrorInvalidValue;
+    ny = p.swiglu ? (p.N + BN / 2 - 1) / (BN / 2) : ny * p.nmat;
   }
+  if (!make_map(&ma, p.a, a_rows, p.K, BM, KIND == GK_ROWS)) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<BN, Q8>::SMEM);
   if (e != cudaSuccess) return e;
   // x = row tile, so that the CTAs sharing one tile of W run together and W crosses HBM once
-  gemm_tcgen05_kernel<BN, KIND><<<dim3((p.M + BM - 1) / BM, (p.N + BN - 1) / BN), Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS, Cfg<BN, Q8>::SMEM, s>>>(ma, mw, p);
+  gemm_tcgen05_kernel<BN, KIND><<<dim3((p.M + BM - 1) / BM, ny), Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS, Cfg<BN, Q8>::SMEM, s>>>(ma, mw, p);
   return cudaGetLastError();
 }
 
@@ -460,14 +454,14 @@ static int forced_bn() {
   static const int forced = [] { const char *e = getenv("VKLLAMA_GEMM_BN"); return e ? atoi(e) : 0; }();  // experiments
   return forced == 256 || forced == 128 || forced == 64 || forced == 32 ? forced : 0;
 }
-static int pick_bn(uint32_t M, uint32_t N, bool q8) {
-  if (int f = forced_bn()) return (q8 || f >= 128) ? f : 128;
+static int pick_bn(uint32_t M, uint32_t N, uint32_t nmat, bool swiglu, bool q8) {
+  if (int f = forced_bn()) return std::max(f, q8 ? (swiglu ? 64 : 32) : 128);
   const size_t mt = (M + BM - 1) / BM, sms = sm_count();
   int best = 0;
   double best_cost = 0.0;
   for (int bn : {256, 128, 64, 32}) {
-    if (!q8 && bn < 128) break;
-    const size_t ctas = mt * ((N + bn - 1) / bn), waves = (ctas + sms - 1) / sms;
+    if (bn < (q8 ? (swiglu ? 64 : 32) : 128)) break;
+    const size_t ctas = mt * (swiglu ? (2 * N + bn - 1) / bn : nmat * ((N + bn - 1) / bn)), waves = (ctas + sms - 1) / sms;
     // measured time of one wave at K = 4096, us: Q8_0 30.9 / 31.2 / 43.0 / 73.4 for 32 / 64 / 128 / 256 columns, FP16 27 + 0.022 bn
     const double wave = q8 ? (bn == 32 ? 30.9 : bn == 64 ? 31.2 : bn == 128 ? 43.0 : 73.4) : 27.0 + 0.022 * bn;
     const double cost = (double)waves * wave;
@@ -479,16 +473,24 @@ static int pick_bn(uint32_t M, uint32_t N, bool q8) {
   return best;
 }
 
+static bool gemm_params_ok(const GemmParams &p, bool q8) {
+  if (!gemm_tcgen05_supported(p.M, p.N, p.K) || !p.nmat || p.nmat > 3 || (p.swiglu && p.nmat != 2) || (p.c_f32 && (p.swiglu || p.nmat != 1))) return false;
+  for (uint32_t i = 0; i < p.nmat; ++i)
+    if (q8 ? !p.w_codes[i] || !p.w_scales[i] : !p.w[i]) return false;
+  return true;
+}
+
 cudaError_t launch_gemm_f16_tcgen05(const GemmParams &p, cudaStream_t s) {
-  if (!gemm_tcgen05_supported(p.M, p.N, p.K)) return cudaErrorInvalidValue;
-  if ((reinterpret_cast<uintptr_t>(p.a) | reinterpret_cast<uintptr_t>(p.w)) & 15) return cudaErrorMisalignedAddress;
-  return pick_bn(p.M, p.N, false) == 256 ? launch_bn<256, GK_F16>(p, s, p.N) : launch_bn<128, GK_F16>(p, s, p.N);
+  if (!gemm_params_ok(p, false)) return cudaErrorInvalidValue;
+  for (uint32_t i = 0; i < p.nmat; ++i)
+    if ((reinterpret_cast<uintptr_t>(p.a) | reinterpret_cast<uintptr_t>(p.w[i])) & 15) return cudaErrorMisalignedAddress;
+  return pick_bn(p.M, p.N, p.nmat, p.swiglu, false) == 256 ? launch_bn<256, GK_F16>(p, s, p.N) : launch_bn<128, GK_F16>(p, s, p.N);
 }
 
 cudaError_t launch_gemm_q8_tcgen05(const GemmParams &p, cudaStream_t s) {
-  if (!gemm_tcgen05_supported(p.M, p.N, p.K) || !p.w_codes || !p.w_scales) return cudaErrorInvalidValue;
+  if (!gemm_params_ok(p, true)) return cudaErrorInvalidValue;
   if (reinterpret_cast<uintptr_t>(p.a) & 15) return cudaErrorMisalignedAddress;
-  switch (pick_bn(p.M, p.N, true)) {
+  switch (pick_bn(p.M, p.N, p.nmat, p.swiglu, true)) {
     case 256: return launch_bn<256, GK_Q8>(p, s, p.N);
     case 128: return launch_bn<128, GK_Q8>(p, s, p.N);
     case 64: return launch_bn<64, GK_Q8>(p, s, p.N);
@@ -501,13 +503,7 @@ cudaError_t launch_gemm_rows_bf16(const GemmRows &p, cudaStream_t s) {
   if ((reinterpret_cast<uintptr_t>(p.a) | reinterpret_cast<uintptr_t>(p.w)) & 15) return cudaErrorMisalignedAddress;
   // grouped: a tile's weight rows beyond its expert's N are read (the next expert's, or zeros) and dropped by the epilogue
   const uint32_t w_rows = p.tile_expert ? p.w_rows : p.N;
-  return pick_bn(p.M, p.N, false) == 256 ? launch_bn<256, GK_ROWS>(p, s, w_rows) : launch_bn<128, GK_ROWS>(p, s, w_rows);
-}
-
-cudaError_t launch_swiglu_f32(const float *gate, const float *up, __half *out, size_t n, cudaStream_t s) {
-  if (!n) return cudaSuccess;
-  swiglu_f32_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(gate, up, out, n);
-  return cudaGetLastError();
+  return pick_bn(p.M, p.N, 1, false, false) == 256 ? launch_bn<256, GK_ROWS>(p, s, w_rows) : launch_bn<128, GK_ROWS>(p, s, w_rows);
 }
 
 }  // namespace vkl

@@ -305,18 +305,23 @@ cudaError_t decode_mega_occupancy(size_t smem_bytes, int *blocks_per_sm);
 cudaError_t launch_decode_mega(const MegaParams &p, int grid, cudaStream_t s);
 
 // ---- dense FP16 GEMM on tcgen05 tensor cores: C[M,N] = A[M,K] . W[N,K]^T (gemm_tcgen05.cu) ----
+// One to three weight matrices of the same shape that share the input (queries, keys, values), each with an output of its
+// own, or a gate and an up matrix whose results meet in the epilogue.
 struct GemmParams {
-  const __half *a;         // [M,K] row-major
-  const __half *w;         // [N,K] row-major (a transposed-weight matrix of the reference); FP16 weights
-  const uint8_t *w_codes;  // Q8_0 weights [N,K] as tiled planes (common.cuh): codes ...
-  const uint8_t *w_scales; // ... and scales
-  __half *c;               // [M,N] fp16 output, or nullptr when c_f32 is set
-  float *c_f32;            // raw fp32 output (for the fused SwiGLU step)
-  const __half *residual;  // optional [M,N]: c = fp16(fp16(acc) + residual)
-  uint32_t *error;         // device word raised when a bounded wait ran out
+  const __half *a;            // [M,K] row-major
+  const __half *w[3];         // [N,K] row-major (a transposed-weight matrix of the reference); FP16 weights
+  const uint8_t *w_codes[3];  // Q8_0 weights [N,K] as tiled planes (common.cuh): codes ...
+  const uint8_t *w_scales[3]; // ... and scales
+  __half *c[3];               // [M,N] fp16 output, or nullptr when c_f32 is set
+  uint32_t nmat;
+  int swiglu;                 // c[0] = fp16(silu(gate) * up) of the fp32 products with w[0] (gate) and w[1] (up): the
+                              // rounding of ffn_up_and_gate_fp16.comp; scale, bias, act and residual are not used
+  float *c_f32;               // raw fp32 output of w[0] (partial sums of a sharded projection)
+  const __half *residual;     // optional [M,N]: c = fp16(fp16(acc) + residual)
+  uint32_t *error;            // device word raised when a bounded wait ran out
   uint32_t M, N, K;
-  float scale, bias;       // MatMul's scale and bias (mat_mul.cpp:39-41)
-  int act;                 // 0 none, 1 SiLU
+  float scale, bias;          // MatMul's scale and bias (mat_mul.cpp:39-41)
+  int act;                    // 0 none, 1 SiLU
 };
 constexpr uint32_t GEMM_MIN_ROWS = 32;  // below this the weight-streaming mat-vec kernel is used
 bool gemm_tcgen05_supported(uint32_t M, uint32_t N, uint32_t K);
@@ -326,8 +331,7 @@ constexpr uint32_t GEMM_Q8_MIN_ROWS = 64;  // below this the rows-at-a-time kern
 cudaError_t launch_gemm_q8_tcgen05(const GemmParams &p, cudaStream_t s);
 // Rows from which a weight of this kind goes to the tensor-core GEMM.
 inline uint32_t gemm_min_rows(bool q8) { return q8 ? GEMM_Q8_MIN_ROWS : GEMM_MIN_ROWS; }
-// Dispatch on the weight kind: w set = FP16 weights, else w_codes / w_scales = Q8_0.
-inline cudaError_t launch_gemm_tcgen05(const GemmParams &p, cudaStream_t s) { return p.w ? launch_gemm_f16_tcgen05(p, s) : launch_gemm_q8_tcgen05(p, s); }
-cudaError_t launch_swiglu_f32(const float *gate, const float *up, __half *out, size_t n, cudaStream_t s);
+// Dispatch on the weight kind: w[0] set = FP16 weights, else w_codes / w_scales = Q8_0.
+inline cudaError_t launch_gemm_tcgen05(const GemmParams &p, cudaStream_t s) { return p.w[0] ? launch_gemm_f16_tcgen05(p, s) : launch_gemm_q8_tcgen05(p, s); }
 
 }  // namespace vkl

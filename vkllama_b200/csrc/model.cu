@@ -64,7 +64,6 @@ int ensure_rows(vkl_model *m, uint32_t T) {
   VKL_OKAY(ensure_tensor(m->dev, &m->v, 1, T, m->dim_l, VKL_FP16));
   VKL_OKAY(ensure_tensor(m->dev, &m->ao, 1, T, m->dim_l, VKL_FP16));
   VKL_OKAY(ensure_tensor(m->dev, &m->t, 1, T, m->ffn_l, VKL_FP16));
-  if (T >= gemm_min_rows(q8(m))) VKL_OKAY(ensure_tensor(m->dev, &m->gu32, 2, T, m->ffn_l, VKL_FP32));
   VKL_OKAY(ensure_tensor(m->dev, &m->toks, 1, 1, T, VKL_UINT32));
   const size_t sc = attention_plan_most(T, m->heads_l, m->head_dim, (uint32_t)m->dev->prop.multiProcessorCount).scratch_bytes;
   VKL_OKAY(ensure_tensor(m->dev, &m->attn_scratch, 1, 1, sc / 4, VKL_FP32));
@@ -94,13 +93,7 @@ MvParams mv(const vkl_model *m, const vkl_tensor *w, const __half *x, __half *ou
 GemmParams gemm(vkl_model *m, const vkl_tensor *w, const __half *a, __half *out, uint32_t M) {
   GemmParams g = {};
   g.a = a;
-  if (q8(m)) {
-    g.w_codes = w->codes();
-    g.w_scales = w->scales();
-  } else {
-    g.w = (const __half *)w->data();
-  }
-  g.c = out;
+  add_weight(g, w, out);
   g.M = M;
   g.N = (uint32_t)w->h;
   g.K = (uint32_t)w->w;
@@ -138,7 +131,7 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
   auto reduce_rows = [&](GemmParams g, __half *xio, uint32_t nrows) -> int {
     const uint32_t seq = ++m->tp_pf_seq;
     const size_t region = m->tp_pf_off + (size_t)(seq & 1u) * m->tp_pf_rows * D * 4;
-    g.c = nullptr;
+    g.c[0] = nullptr;
     g.residual = nullptr;
     g.c_f32 = (float *)((char *)m->tp_buf + region);
     VKL_LAUNCH(1, launch_gemm_tcgen05(g, s));
@@ -178,9 +171,10 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
       VKL_LAUNCH(1, launch_matvec(p, EPI_PLAIN, true, s));
     } else if (use_gemm(m, T)) {
       VKL_LAUNCH(1, launch_rms_norm(x, (const float *)y.attn_norm->data(), xn, T, D, m->cfg.eps, s));
-      VKL_LAUNCH(1, launch_gemm_tcgen05(gemm(m, y.wk, xn, kb, T), s));
-      VKL_LAUNCH(1, launch_gemm_tcgen05(gemm(m, y.wq, xn, qb, T), s));
-      VKL_LAUNCH(1, launch_gemm_tcgen05(gemm(m, y.wv, xn, vb, T), s));
+      GemmParams g = gemm(m, y.wk, xn, kb, T);
+      add_weight(g, y.wq, qb);
+      add_weight(g, y.wv, vb);
+      VKL_LAUNCH(1, launch_gemm_tcgen05(g, s));
     } else {
       VKL_LAUNCH(1, launch_rms_norm(x, (const float *)y.attn_norm->data(), xn, T, D, m->cfg.eps, s));
       VKL_LAUNCH((T + 63) / 64, launch_matvec(p, EPI_PLAIN, false, s));
@@ -229,19 +223,10 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
       VKL_LAUNCH(1, launch_matvec(f, EPI_SWIGLU, true, s));
     } else if (use_gemm(m, rows)) {
       VKL_LAUNCH(1, launch_rms_norm(xr, (const float *)y.ffn_norm->data(), xn, rows, D, m->cfg.eps, s));
-      float *g32 = (float *)m->gu32->data(), *u32 = g32 + (size_t)rows * m->ffn_l;
-      GemmParams g = gemm(m, y.gate, xn, nullptr, rows);
-      g.c_f32 = g32;
+      GemmParams g = gemm(m, y.gate, xn, tb, rows);
+      add_weight(g, y.up, nullptr);
+      g.swiglu = 1;
       VKL_LAUNCH(1, launch_gemm_tcgen05(g, s));
-      if (q8(m)) {
-        g.w_codes = y.up->codes();
-        g.w_scales = y.up->scales();
-      } else {
-        g.w = (const __half *)y.up->data();
-      }
-      g.c_f32 = u32;
-      VKL_LAUNCH(1, launch_gemm_tcgen05(g, s));
-      VKL_LAUNCH(1, launch_swiglu_f32(g32, u32, tb, (size_t)rows * m->ffn_l, s));
     } else {
       VKL_LAUNCH(1, launch_rms_norm(xr, (const float *)y.ffn_norm->data(), xn, rows, D, m->cfg.eps, s));
       VKL_LAUNCH((rows + 63) / 64, launch_matvec(f, EPI_SWIGLU, false, s));

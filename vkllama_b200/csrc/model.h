@@ -48,7 +48,6 @@ struct vkl_model {
   // activations, sized for `cap_T` rows
   uint32_t cap_T = 0;
   vkl_tensor *x = nullptr, *xn = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *ao = nullptr, *t = nullptr;
-  vkl_tensor *gu32 = nullptr;  // [2, cap_T, ffn] fp32 gate and up results of the FP16 prefill GEMMs
   bool gemm_used = false;      // a tensor-core GEMM ran since the last check of state[6]
   vkl_tensor *logits16 = nullptr, *logits32 = nullptr;
   vkl_tensor *toks = nullptr;  // [cap_T] device token ids; toks[0] is the decode token
@@ -93,7 +92,7 @@ struct vkl_model {
     for (auto &l : L)
       for (vkl_tensor *p : {l.attn_norm, l.ffn_norm, l.wq, l.wk, l.wv, l.wo, l.gate, l.up, l.down, l.kcache, l.vcache, l.state, l.ring}) vkl_tensor_release(p);
     for (vkl_tensor *p : mega_packed) vkl_tensor_release(p);
-    for (vkl_tensor *p : {tok_embd, output_norm, output, fc, fs, x, xn, q, k, v, ao, t, gu32, logits16, logits32, toks, state, out_ids, forced, argpart, attn_scratch, attn_counters, mega_ops, mega_sync, mega_arg, mega_attn, mega_stages, mega_counts, mega_ll})
+    for (vkl_tensor *p : {tok_embd, output_norm, output, fc, fs, x, xn, q, k, v, ao, t, logits16, logits32, toks, state, out_ids, forced, argpart, attn_scratch, attn_counters, mega_ops, mega_sync, mega_arg, mega_attn, mega_stages, mega_counts, mega_ll})
       vkl_tensor_release(p);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);

@@ -115,13 +115,8 @@ struct MatMulOp : vkl_op {
       if (a->h >= gemm_min_rows(!p.fp16_weights) && gemm_tcgen05_supported((uint32_t)a->h, (uint32_t)N, (uint32_t)K)) {
         // many rows: one pass over the weights on the tcgen05 tensor cores (Q8_0 dequantised on the way in)
         GemmParams g = {};
-        g.a = (const __half *)a->data(); g.c = (__half *)out->data();
-        if (p.fp16_weights) {
-          g.w = (const __half *)weight->data();
-        } else {
-          g.w_codes = weight->codes();
-          g.w_scales = weight->scales();
-        }
+        g.a = (const __half *)a->data();
+        add_weight(g, weight, (__half *)out->data());
         g.M = (uint32_t)a->h; g.N = (uint32_t)N; g.K = (uint32_t)K;
         g.scale = scale; g.bias = bias; g.act = act;
         VKL_OKAY(command_error_word(cmd, &g.error));
@@ -166,14 +161,14 @@ struct MatMulOp : vkl_op {
 struct FeedForwardOp : vkl_op {
   vkl_tensor *w1, *w2, *w3;  // gate, down, up
   int transposed_weight, dtype;
-  vkl_tensor *t0 = nullptr, *out = nullptr, *gu32 = nullptr;
+  vkl_tensor *t0 = nullptr, *out = nullptr;
   FeedForwardOp(vkl_device *d, vkl_command *c, vkl_tensor *a, vkl_tensor *b, vkl_tensor *e, int tw, int dt)
       : vkl_op(d, c), w1(a), w2(b), w3(e), transposed_weight(tw), dtype(dt) {
     vkl_tensor_retain(w1); vkl_tensor_retain(w2); vkl_tensor_retain(w3);
   }
   ~FeedForwardOp() override {
     vkl_tensor_release(w1); vkl_tensor_release(w2); vkl_tensor_release(w3);
-    vkl_tensor_release(t0); vkl_tensor_release(out); vkl_tensor_release(gu32);
+    vkl_tensor_release(t0); vkl_tensor_release(out);
   }
   // src/ops/feed_forward.cpp:24-68
   int init() override {
@@ -201,29 +196,19 @@ struct FeedForwardOp : vkl_op {
     const bool q8 = dtype == VKL_Q8_0;
     if (x->h >= gemm_min_rows(q8) && gemm_tcgen05_supported((uint32_t)x->h, (uint32_t)w1->h, (uint32_t)w1->w) &&
         gemm_tcgen05_supported((uint32_t)x->h, (uint32_t)w2->h, (uint32_t)w2->w)) {
-      // many rows: gate and up as tensor-core GEMMs with raw fp32 results, SwiGLU on those
+      // many rows: gate and up as one tensor-core GEMM with SwiGLU on its fp32 results
       // (the rounding points of ffn_up_and_gate_fp16.comp), then the down GEMM
-      VKL_OKAY(ensure_tensor(dev, &gu32, 2, x->h, w1->h, VKL_FP32));
-      auto weight_of = [q8](GemmParams &gp, const vkl_tensor *w) {
-        gp.w = q8 ? nullptr : (const __half *)w->data();
-        gp.w_codes = q8 ? w->codes() : nullptr;
-        gp.w_scales = q8 ? w->scales() : nullptr;
-      };
       GemmParams g = {};
-      g.a = (const __half *)x->data(); g.c_f32 = (float *)gu32->data();
-      weight_of(g, w1);
+      g.a = (const __half *)x->data();
+      add_weight(g, w1, (__half *)t0->data());
+      add_weight(g, w3, nullptr);
+      g.swiglu = 1;
       g.M = (uint32_t)x->h; g.N = (uint32_t)w1->h; g.K = (uint32_t)w1->w;
-      g.scale = 1.f;
       VKL_OKAY(command_error_word(cmd, &g.error));
       VKL_LAUNCH(1, launch_gemm_tcgen05(g, cmd->stream));
-      weight_of(g, w3);
-      g.c_f32 += (size_t)x->h * w1->h;
-      VKL_LAUNCH(1, launch_gemm_tcgen05(g, cmd->stream));
-      VKL_LAUNCH(1, launch_swiglu_f32((const float *)gu32->data(), (const float *)gu32->data() + (size_t)x->h * w1->h, (__half *)t0->data(),
-                                      (size_t)x->h * w1->h, cmd->stream));
       GemmParams d = {};
-      d.a = (const __half *)t0->data(); d.c = (__half *)out->data();
-      weight_of(d, w2);
+      d.a = (const __half *)t0->data();
+      add_weight(d, w2, (__half *)out->data());
       d.M = (uint32_t)x->h; d.N = (uint32_t)w2->h; d.K = (uint32_t)w2->w;
       d.scale = 1.f; d.error = g.error;
       VKL_LAUNCH(1, launch_gemm_tcgen05(d, cmd->stream));
@@ -350,7 +335,19 @@ struct MhaOp : vkl_op {
     p.nmat = 3;
     p.N = (uint32_t)Wd; p.K = (uint32_t)wk->w; p.M = (uint32_t)T;
     p.x_ld = p.K; p.out_ld = p.N; p.scale = 1.f; p.fp16_weights = !q8;
-    VKL_LAUNCH((T + 63) / 64, launch_matvec(p, EPI_PLAIN, false, cmd->stream));
+    // FP16 weights and many rows: the tensor-core GEMM, as MatMul does (Q8_0 keeps its exact fp32 scaling here)
+    GemmParams g = {};
+    if (!q8 && T >= gemm_min_rows(false) && gemm_tcgen05_supported((uint32_t)T, p.N, p.K)) {
+      g.a = p.x;
+      add_weight(g, wk, (__half *)k->data());
+      add_weight(g, wq, (__half *)q->data());
+      add_weight(g, wv, (__half *)v->data());
+      g.M = (uint32_t)T; g.N = p.N; g.K = p.K; g.scale = 1.f;
+      VKL_OKAY(command_error_word(cmd, &g.error));
+      VKL_LAUNCH(1, launch_gemm_tcgen05(g, cmd->stream));
+    } else {
+      VKL_LAUNCH((T + 63) / 64, launch_matvec(p, EPI_PLAIN, false, cmd->stream));
+    }
 
     const AttnPlan plan = attention_plan((uint32_t)T, clip_output && T > 1, (uint32_t)heads, dim, (uint32_t)dev->prop.multiProcessorCount);
     const size_t need = std::max(plan.scratch_bytes, (size_t)16);
@@ -379,7 +376,16 @@ struct MhaOp : vkl_op {
     w.nmat = 1;
     w.N = (uint32_t)wo->h; w.K = (uint32_t)wo->w; w.M = (uint32_t)To;
     w.x_ld = w.K; w.out_ld = w.N; w.scale = 1.f; w.fp16_weights = !q8;
-    VKL_LAUNCH((To + 63) / 64, launch_matvec(w, EPI_PLAIN, false, cmd->stream));
+    if (!q8 && To >= gemm_min_rows(false) && gemm_tcgen05_supported((uint32_t)To, w.N, w.K)) {
+      g = GemmParams{};
+      g.a = w.x;
+      add_weight(g, wo, (__half *)out->data());
+      g.M = (uint32_t)To; g.N = w.N; g.K = w.K; g.scale = 1.f;
+      VKL_OKAY(command_error_word(cmd, &g.error));
+      VKL_LAUNCH(1, launch_gemm_tcgen05(g, cmd->stream));
+    } else {
+      VKL_LAUNCH((To + 63) / 64, launch_matvec(w, EPI_PLAIN, false, cmd->stream));
+    }
     *o = out;
     return leave();
   }

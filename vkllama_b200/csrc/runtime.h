@@ -123,4 +123,15 @@ int tensor_new(vkl_device *dev, size_t c, size_t h, size_t w, int dtype, vkl_ten
 // Make *slot a dense tensor of this shape, reusing it when it already matches.
 int ensure_tensor(vkl_device *dev, vkl_tensor **slot, size_t c, size_t h, size_t w, int dtype);
 int recording(vkl_command *cmd, const char *who);
+// One more weight of a GEMM, and where its results go (a SwiGLU's up matrix: null).
+inline void add_weight(GemmParams &g, const vkl_tensor *w, __half *out) {
+  const uint32_t i = g.nmat++;
+  if (w->dtype == VKL_Q8_0) {
+    g.w_codes[i] = w->codes();
+    g.w_scales[i] = w->scales();
+  } else {
+    g.w[i] = (const __half *)w->data();
+  }
+  g.c[i] = out;
+}
 }  // namespace vkl

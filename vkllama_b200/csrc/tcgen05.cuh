@@ -1,8 +1,10 @@
-// What the tcgen05 GEMM kernels share: bounded barrier waits, descriptors, TMA and TMEM access, tensor maps.
+// What the tcgen05 GEMM kernels share: bounded barrier waits, descriptors, TMA and TMEM access, epilogues of the Llama
+// path, tensor maps.
 #pragma once
 #include <cuda.h>
 
 #include "common.cuh"
+#include "kernels.h"
 
 namespace vkl {
 namespace {
@@ -81,6 +83,57 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr)
       : "memory");
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+struct WeightMaps {
+  CUtensorMap w[3];
+};
+
+// 32 outputs fp16(silu(gate) * up) of a row, of which n exist (n a multiple of 8).
+__device__ __forceinline__ void swiglu_chunk(const float (&gate)[32], const float (&up)[32], __half *out, uint32_t n) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 8) {
+    if (j >= n) break;
+    union {
+      uint4 u;
+      __half h[8];
+    } y;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) y.h[i] = __float2half_rn(gate[j + i] / (1.0f + expf(-gate[j + i])) * up[j + i]);
+    *reinterpret_cast<uint4 *>(out + j) = y.u;
+  }
+}
+// 32 results of matrix `mat`: this row's columns from n on, rounded as GemmParams says.
+__device__ __forceinline__ void f16_chunk(const GemmParams &p, uint32_t mat, uint32_t row, uint32_t n, const float (&acc)[32]) {
+  const size_t o = (size_t)row * p.N + n;
+#pragma unroll
+  for (int j = 0; j < 32; j += 8) {
+    if (n + j >= p.N) break;  // N is a multiple of 8
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v[i] = acc[j + i] * p.scale + p.bias;
+      if (p.act == 1) v[i] = v[i] / (1.0f + expf(-v[i]));
+    }
+    if (p.c_f32) {
+      *reinterpret_cast<float4 *>(p.c_f32 + o + j) = make_float4(v[0], v[1], v[2], v[3]);
+      *reinterpret_cast<float4 *>(p.c_f32 + o + j + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    } else {
+      union {
+        uint4 u;
+        __half h[8];
+      } out, res;
+      if (p.residual) {
+        res.u = *reinterpret_cast<const uint4 *>(p.residual + o + j);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) out.h[i] = __float2half_rn(round_h(v[i]) + __half2float(res.h[i]));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) out.h[i] = __float2half_rn(v[i]);
+      }
+      *reinterpret_cast<uint4 *>(p.c[mat] + o + j) = out.u;
+    }
+  }
 }
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
