@@ -102,47 +102,40 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tmem_acc = tmem_base_s;
 
   if (warp == 0) {
-    if (lane == 0) {
-      for (uint32_t kb = 0; kb < nkb; ++kb) {
-        const uint32_t s = kb % C::STAGES, use = kb / C::STAGES;
-        if (use > 0 && !mbar_wait_bounded(sa(&empty[s]), (use - 1) & 1u)) {
+    if (elect_one()) {
+      RingPos<C::STAGES> pos;
+      for (uint32_t kb = 0; kb < nkb; ++kb, pos.next()) {
+        if (kb >= C::STAGES && !mbar_wait_bounded(sa(&empty[pos.s]), pos.phase ^ 1u)) {
           failed_s = 1;
           break;
         }
-        if (failed_s) break;
-        const uint32_t bar = sa(&full[s]), st = sa(stages + (size_t)s * C::STAGE_BYTES);
+        const uint32_t bar = sa(&full[pos.s]), st = sa(stages) + pos.s * C::STAGE_BYTES;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(C::STAGE_BYTES) : "memory");
         // rows beyond a part's end are the next part's (or zeros): they make rows that the epilogue drops
+#pragma unroll
         for (uint32_t i = 0; i < kParts; ++i) tma_load_2d(st + i * A_TILE_BYTES, &map_a, kb * BK, i * rows + a_row, bar);
         tma_load_2d(st + kParts * A_TILE_BYTES, &map_w, kb * BK, w_row, bar);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = instr_desc(BM, BN, true);
-      for (uint32_t kb = 0; kb < nkb; ++kb) {
-        const uint32_t s = kb % C::STAGES, use = kb / C::STAGES, b = kb % kBuffers, buse = kb / kBuffers;
-        if ((buse > 0 && !mbar_wait_bounded(sa(&acc_empty[b]), (buse - 1) & 1u)) || !mbar_wait_bounded(sa(&full[s]), use & 1u)) {
+      const uint32_t a0 = desc_lo(sa(stages)), w0 = desc_lo(sa(stages) + kParts * A_TILE_BYTES);
+      RingPos<C::STAGES> pos;
+      RingPos<kBuffers> buf;
+      for (uint32_t kb = 0; kb < nkb; ++kb, pos.next(), buf.next()) {
+        if ((kb >= kBuffers && !mbar_wait_bounded(sa(&acc_empty[buf.s]), buf.phase ^ 1u)) || !mbar_wait_bounded(sa(&full[pos.s]), pos.phase)) {
           failed_s = 2;
           break;
         }
-        if (failed_s) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t st = sa(stages + (size_t)s * C::STAGE_BYTES), w_addr = st + kParts * A_TILE_BYTES;
+        const uint32_t off = pos.s * (C::STAGE_BYTES >> 4), acc = tmem_acc + buf.s * BN;
 #pragma unroll
-        for (int i = kParts - 1; i >= 0; --i) {  // small parts first: little is cut off from their sums
+        for (int i = kParts - 1; i >= 0; --i)  // small parts first: little is cut off from their sums
 #pragma unroll
-          for (uint32_t k = 0; k < BK / 16; ++k) {
-            const uint64_t da = smem_desc(st + i * A_TILE_BYTES + k * 32), db = smem_desc(w_addr + k * 32);
-            const uint32_t accumulate = i < kParts - 1 || k ? 1u : 0u;
-            asm volatile(
-                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_acc + b * BN),
-                "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-                : "memory");
-          }
-        }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sa(&empty[s])) : "memory");
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sa(&acc_full[b])) : "memory");
+          for (uint32_t k = 0; k < BK / 16; ++k) mma_f16<1>(acc, a0 + off + i * (A_TILE_BYTES >> 4) + 2 * k, w0 + off + 2 * k, idesc, i < kParts - 1 || k);
+        mma_commit(sa(&empty[pos.s]));
+        mma_commit(sa(&acc_full[buf.s]));
       }
     }
   } else {

@@ -33,44 +33,9 @@
 #include "rows.cuh"
 #include "tcgen05.cuh"
 
-#ifndef VKL_GEMM_TRACE
-#define VKL_GEMM_TRACE 0  // diagnostic build: CTA (0,0) stamps the global timer at fixed points of every K step
-#endif
-#if VKL_GEMM_TRACE
-__device__ unsigned long long g_gemm_trace[8 * 512];
-extern "C" int vkl_debug_gemm_trace_clear() {
-  static unsigned long long zeros[8 * 512];
-  return (int)cudaMemcpyToSymbol(g_gemm_trace, zeros, sizeof(zeros));
-}
-extern "C" int vkl_debug_gemm_trace(unsigned long long *out, size_t n) {
-  return (int)cudaMemcpyFromSymbol(out, g_gemm_trace, (n < 8 * 512 ? n : 8 * 512) * sizeof(unsigned long long));
-}
-#define GEMM_STAMP(kb, k)                                                                       \
-  do {                                                                                          \
-    if (blockIdx.x == 0 && blockIdx.y == 0 && (kb) < 512) {                                     \
-      unsigned long long t_;                                                                    \
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_));                                    \
-      g_gemm_trace[(kb) * 8 + (k)] = t_;                                                        \
-    }                                                                                           \
-  } while (0)
-#else
-#define GEMM_STAMP(kb, k) \
-  do {                    \
-  } while (0)
-#endif
-
 namespace vkl {
 namespace {
 
-#ifndef VKL_GEMM_NACC2
-#define VKL_GEMM_NACC2 1
-#endif
-#ifndef VKL_GEMM_TESTWAIT
-#define VKL_GEMM_TESTWAIT 0
-#endif
-#ifndef VKL_GEMM_MMAONLY
-#define VKL_GEMM_MMAONLY 0  // diagnostic build: the MMA lane runs alone on whatever the shared memory holds
-#endif
 constexpr int GEMM_THREADS = 192;          // FP16 weights: TMA producer, MMA, four epilogue warps
 #ifndef VKL_GEMM_NDW
 #define VKL_GEMM_NDW 16
@@ -141,9 +106,6 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
   __shared__ __align__(8) uint64_t full[C::STAGES];   // TMA bytes of the stage have landed
   __shared__ __align__(8) uint64_t empty[C::STAGES];  // the MMAs have read the stage
   __shared__ __align__(8) uint64_t acc_ready;
-#if VKL_GEMM_TRACE
-  __shared__ __align__(8) uint64_t full_a[C::STAGES];  // diagnostic build, Q8_0: the A tile's copy completes on a barrier of its own
-#endif
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile uint32_t failed_s;
 
@@ -175,9 +137,6 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
     for (int s = 0; s < C::STAGES; ++s) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sa(&full[s])), "r"(Q8 ? 1u + NDWG : 1u) : "memory");  // the TMA lane (+ one lane per dequantising warp)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sa(&empty[s])) : "memory");
-#if VKL_GEMM_TRACE
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sa(&full_a[s])) : "memory");
-#endif
     }
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sa(&acc_ready)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -186,7 +145,7 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
   // Tiles of up to 128 columns accumulate the even and the odd 16-wide K slices in two TMEM accumulators, added in
   // the epilogue: a tcgen05.mma of so few columns takes about 110 cycles however narrow it is when it has to
   // follow the one before it on the same accumulator; two independent chains hide half of that.
-  constexpr uint32_t NACC = VKL_GEMM_NACC2 && BN <= 128 ? 2 : 1;
+  constexpr uint32_t NACC = BN <= 128 ? 2 : 1;
   if (warp == 1) tmem_alloc<NACC * BN>(sa(&tmem_base_s));
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -195,29 +154,21 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
 
   if (warp == 0) {
     // ---------------------------------------------------------------- producer
-    if (lane == 0 && !VKL_GEMM_MMAONLY) {
-      for (uint32_t kb = 0; kb < nkb; ++kb) {
-        const uint32_t s = kb % C::STAGES, use = kb / C::STAGES;
-        if (use > 0 && !mbar_wait_bounded(sa(&empty[s]), (use - 1) & 1u)) {
+    if (elect_one()) {
+      RingPos<C::STAGES> pos;
+      for (uint32_t kb = 0; kb < nkb; ++kb, pos.next()) {
+        if (kb >= C::STAGES && !mbar_wait_bounded(sa(&empty[pos.s]), pos.phase ^ 1u)) {
           failed_s = 1;
           break;
         }
-        if (failed_s) break;
-        GEMM_STAMP(kb, 0);  // the stage is free: its A tile is requested now
-#if VKL_GEMM_TRACE
-        const uint32_t bar = Q8 ? sa(&full_a[s]) : sa(&full[s]);
-        if (Q8) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sa(&full[s])) : "memory");  // the producer's share of the count
-#else
-        const uint32_t bar = sa(&full[s]);
-#endif
+        const uint32_t bar = sa(&full[pos.s]), st = sa(stages) + pos.s * C::STAGE_BYTES;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(Q8 ? A_TILE_BYTES : C::STAGE_BYTES) : "memory");
-        unsigned char *st = stages + (size_t)s * C::STAGE_BYTES;
-        tma_load_2d(sa(st), &map_a, kb * BK, a_row, bar);
-        if (!Q8) tma_load_2d(sa(st + A_TILE_BYTES), &maps.w[mat], kb * BK, w_row, bar);
-        if (!Q8 && swiglu) tma_load_2d(sa(st + A_TILE_BYTES + C::B_TILE_BYTES / 2), &maps.w[1], kb * BK, w_row, bar);
+        tma_load_2d(st, &map_a, kb * BK, a_row, bar);
+        if (!Q8) tma_load_2d(st + A_TILE_BYTES, &maps.w[mat], kb * BK, w_row, bar);
+        if (!Q8 && swiglu) tma_load_2d(st + A_TILE_BYTES + C::B_TILE_BYTES / 2, &maps.w[1], kb * BK, w_row, bar);
       }
     }
-  } else if (Q8 && warp >= 6 && (warp & 3u) != 1u && !VKL_GEMM_MMAONLY) {
+  } else if (Q8 && warp >= 6 && (warp & 3u) != 1u) {
     if constexpr (Q8) {
     // ------------------------------------------- W tile: Q8_0 -> fp16 in shared memory
     // BN rows x 64 columns = (BN / 16) row tiles x 2 blocks: units of 512 bytes of codes, dealt round robin to
@@ -272,12 +223,8 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
         if (kb >= nkb || stop) continue;
         const uint32_t s = kb % C::STAGES, use = kb / C::STAGES;
         uint32_t ok = 1;
-        if (wi == 0 && lane == 0) GEMM_STAMP(kb, 1);  // a dequantising warp turns to the stage
         if (lane == 0 && use > 0) ok = mbar_wait_bounded(sa(&empty[s]), (use - 1) & 1u, 100) ? 1u : 0u;
         ok = __shfl_sync(0xffffffffu, ok, 0);
-#if !VKL_GEMM_TRACE
-        if (wi == 0 && lane == 0) GEMM_STAMP(kb, 2);  // ... has the stage
-#endif
         if (!ok) {
           if (lane == 0) failed_s = 4;
           stop = true;
@@ -289,7 +236,6 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
         }
         asm volatile("cp.async.wait_group %0;" ::"n"(PF - 1) : "memory");  // this stage's copies (the oldest group) have landed
         __syncwarp();
-        if (wi == 0 && lane == 0) GEMM_STAMP(kb, 3);  // ... has its codes
         unsigned char *wt = stages + (size_t)s * C::STAGE_BYTES + A_TILE_BYTES;
 #pragma unroll
         for (uint32_t j = 0; j < UPQ; ++j) {
@@ -311,14 +257,6 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();          // every lane has fenced, and has read the staging slot
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sa(&full[s])) : "memory");
-        if (wi == 0 && lane == 0) GEMM_STAMP(kb, 4);  // ... has written and published its part of the W tile
-#if VKL_GEMM_TRACE
-        if (lane == 0 && blockIdx.x == 0 && blockIdx.y == 0 && kb < 512) {  // [7]: the last warp of the group to publish
-          unsigned long long t_;
-          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_));
-          atomicMax(&g_gemm_trace[kb * 8 + 7], t_);
-        }
-#endif
         request(kb + NG * PF, i);   // refill the slot for this warp's stage PF steps ahead
       }
       if (stop) break;
@@ -327,40 +265,25 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
     }
   } else if (warp == 1) {
     // --------------------------------------------------------------------- MMA
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = instr_desc(BM, BN, KIND == GK_ROWS);
-      for (uint32_t kb = 0; kb < nkb; ++kb) {
-        const uint32_t s = kb % C::STAGES, use = kb / C::STAGES;
-        if (!VKL_GEMM_MMAONLY && !(VKL_GEMM_TESTWAIT ? mbar_spin_bounded(sa(&full[s]), use & 1u) : mbar_wait_bounded(sa(&full[s]), use & 1u))) {
+      const uint32_t a0 = desc_lo(sa(stages)), b0 = desc_lo(sa(stages) + A_TILE_BYTES);
+      RingPos<C::STAGES> pos;
+      bool ok = true;
+      for (uint32_t kb = 0; kb < nkb; ++kb, pos.next()) {
+        if (!mbar_wait_bounded(sa(&full[pos.s]), pos.phase)) {
           failed_s = 2;
+          ok = false;
           break;
         }
-        if (failed_s) break;
-#if VKL_GEMM_TRACE
-        GEMM_STAMP(kb, 2);  // (diagnostic build: reuses slot 2) the MMA lane has the W tile
-        if (Q8 && !mbar_wait_bounded(sa(&full_a[s]), use & 1u)) {
-          failed_s = 2;
-          break;
-        }
-#endif
-        GEMM_STAMP(kb, 5);  // the MMA lane has the full stage
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a_addr = sa(stages + (size_t)s * C::STAGE_BYTES), b_addr = a_addr + A_TILE_BYTES;
+        const uint32_t off = pos.s * (C::STAGE_BYTES >> 4);
 #pragma unroll
-        for (uint32_t k = 0; k < BK / 16; ++k) {
-          const uint64_t da = smem_desc(a_addr + k * 32), db = smem_desc(b_addr + k * 32);
-          const uint32_t accumulate = NACC == 2 ? ((kb | (k >> 1)) ? 1u : 0u) : ((kb | k) ? 1u : 0u);
-          asm volatile(
-              "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_acc + (NACC == 2 ? (k & 1u) * BN : 0u)),
-              "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-              : "memory");
-        }
-        // arrives once every MMA issued so far has completed (implies fence::before_thread_sync)
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sa(&empty[s])) : "memory");
-        GEMM_STAMP(kb, 6);  // ... has issued the stage's MMAs and the commit
-        if (kb + 1 == nkb)
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sa(&acc_ready)) : "memory");
+        for (uint32_t k = 0; k < BK / 16; ++k)
+          mma_f16<1>(tmem_acc + (NACC == 2 ? (k & 1u) * BN : 0u), a0 + off + 2 * k, b0 + off + 2 * k, idesc, k >= NACC || kb);
+        mma_commit(sa(&empty[pos.s]));
       }
+      if (ok) mma_commit(sa(&acc_ready));
     }
   } else if (warp >= 2 && warp < 6) {
     // ---------------------------------------------------------------- epilogue

@@ -31,29 +31,48 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   return false;
 }
 
-// The same with the non-blocking test (mbarrier.test_wait), for the MMA lane: try_wait may suspend the thread.
-__device__ __forceinline__ bool mbar_spin_bounded(uint32_t bar, uint32_t parity) {
-  for (uint32_t i = 0; i < (GEMM_WAIT_LIMIT << 4); ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
+// The single-lane roles (TMA producer, MMA issuer) run a K step's instructions one after the other at their latencies, and
+// the CTA waits on them: at some 780 cycles per step they, not the 256 ... 512 cycles of the MMAs, set the pace of every
+// GEMM here. Hence: the lane is picked by elect.sync, which tells the compiler that one thread is active (under
+// `lane == 0` every instruction with uniform operands, MMAs, commits and copies, became a loop over lanes); stages are
+// counted, not divided; descriptors differ from stage to stage in their low word only; and the loop polls its one barrier, nothing else.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(one));
+  return one != 0;
 }
+template <int STAGES> struct RingPos {
+  uint32_t s = 0, phase = 0;  // stage, and the parity that its barrier completes next
+  __device__ __forceinline__ void next() {
+    if (++s == STAGES) {
+      s = 0;
+      phase ^= 1u;
+    }
+  }
+};
 
-// Shared-memory matrix descriptor: K-major tile, 128-byte swizzle, 8-row groups 1024 B apart.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr & 0x3FFFFu) >> 4);  // start address, 16-byte units
-  d |= (uint64_t)1 << 16;                   // leading-dimension offset (unused with swizzle)
-  d |= (uint64_t)(1024 >> 4) << 32;         // stride between 8-row groups
-  d |= (uint64_t)1 << 46;                   // descriptor version of this architecture
-  d |= (uint64_t)2 << 61;                   // 128-byte swizzle
-  return d;
+// Shared-memory matrix descriptor: K-major tile, 128-byte swizzle, 8-row groups 1024 B apart. Low word: start address
+// in 16-byte units, leading-dimension offset 1 (unused with swizzle); the high one (mma_f16): stride between the groups,
+// descriptor version of this architecture, 128-byte swizzle.
+__device__ __forceinline__ uint32_t desc_lo(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | 1u << 16; }
+
+// One K slice of 16: descriptors by their low words (the high one is the same for every address).
+template <int CTAS> __device__ __forceinline__ void mma_f16(uint32_t acc, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, bool accumulate) {
+  constexpr uint32_t hi = (1024u >> 4) | 1u << 14 | 2u << 29;
+  if constexpr (CTAS == 1)
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .b64 a, b;\n mov.b64 a, {%1, %3};\n mov.b64 b, {%2, %3};\n setp.ne.b32 p, %5, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n}" ::"r"(acc), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"((uint32_t)accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .b64 a, b;\n mov.b64 a, {%1, %3};\n mov.b64 b, {%2, %3};\n setp.ne.b32 p, %5, 0;\n"
+        " tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %4, p;\n}" ::"r"(acc), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"((uint32_t)accumulate)
+        : "memory");
+}
+// arrives on this CTA's barrier once every MMA issued so far has completed (implies fence::before_thread_sync)
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 // kind::f16 instruction descriptor: fp16 x fp16 or bf16 x bf16 -> fp32, both operands K-major, M x N tile.
