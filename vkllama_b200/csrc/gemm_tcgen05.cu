@@ -13,7 +13,8 @@
 // the reference multiplies in fp32; the rows-at-a-time kernel (matvec.cu) keeps the exact form and is used
 // below GEMM_Q8_MIN_ROWS rows.
 //
-// One CTA computes a 128 x BN output tile (BN = 32 ... 256, picked per launch) with these kinds of warps:
+// Long prompts of 16-bit weights go to pairs of CTAs where pick_tile finds them faster (gemm_pair.cu). Here one CTA computes
+// a 128 x BN output tile (BN = 32 ... 256, picked per launch) with these kinds of warps:
 //   warp 0    producer: one lane issues TMA tensor copies (cp.async.bulk.tensor.2d, 128-byte
 //             swizzle) of the A and W tiles of each 64-wide K block into a ring of shared-
 //             memory stages; the copies complete on the stage's "full" mbarrier.
@@ -369,25 +370,50 @@ template <int BN, int KIND> cudaError_t launch_bn(const typename GemmArgs<KIND>:
 
 bool gemm_tcgen05_supported(uint32_t M, uint32_t N, uint32_t K) { return M >= 1 && K % BK == 0 && K >= BK && (N % 8) == 0; }
 
-// W-tile width. A grid runs in waves of one CTA per SM, and a last wave that fills a fraction of the SMs takes
-// as long as a full one: pick the width with the smallest waves x (time of one tile). A tile's time is a fixed
-// part (the K loop's pipeline latencies, the A tile's copies, the epilogue) plus a part that grows with the
-// width; the fixed part dominates, most of all for FP16 weights.
+// Tile shape. A grid runs in waves of one CTA (or pair) per SM (two SMs), and a last wave that fills a fraction of the
+// SMs takes as long as a full one: pick the shape with the smallest waves x (time of one tile). A tile's time is a K step's
+// times their number, plus what a wave does not overlap (its first copies and, without the pairs' second accumulator, its epilogue).
+struct Tile {
+  bool pair;
+  int bn;
+};
 static int forced_bn() {
   static const int forced = [] { const char *e = getenv("VKLLAMA_GEMM_BN"); return e ? atoi(e) : 0; }();  // experiments
   return forced == 256 || forced == 128 || forced == 64 || forced == 32 ? forced : 0;
 }
-static int pick_bn(uint32_t M, uint32_t N, uint32_t nmat, bool swiglu, bool q8) {
-  if (int f = forced_bn()) return std::max(f, q8 ? (swiglu ? 64 : 32) : 128);
+static Tile pick_tile(uint32_t M, uint32_t N, uint32_t K, uint32_t nmat, bool swiglu, bool pairs) {
+  if (int f = forced_bn()) return {false, std::max(f, 128)};
+  // measured, us, fp16, K = 4096 and 11008 (a step: from the difference): 512 rows x 4096 columns 20.4 / 47.7 for 128 columns of one
+  // CTA, 29.2 / 67.8 for 256, 18.5 / 43.8 and 25.4 / 65.1 for a pair's 128 and 256; 2048 rows 73.9 / 183, 59.5 / 149, 61.0 / 156, 53.2 / 139;
+  // 777 x 17152, K = 2048: 97.6, 79.3, 69.3, 55.8
+  static const struct {
+    Tile tile;
+    double step, wave;
+  } shapes[] = {{{true, 256}, 0.38, 0.5}, {{false, 256}, 0.42, 4.0}, {{true, 128}, 0.235, 0.5}, {{false, 128}, 0.25, 4.0}};
+  Tile best = {false, 0};
+  double best_cost = 0.0;
+  for (const auto &sh : shapes) {
+    if (sh.tile.pair && !pairs) continue;
+    const size_t rows = sh.tile.pair ? 2 * BM : BM, bn = (size_t)sh.tile.bn, slots = sm_count() / (sh.tile.pair ? 2 : 1);
+    const size_t tiles = (M + rows - 1) / rows * (swiglu ? (2 * (size_t)N + bn - 1) / bn : nmat * ((N + bn - 1) / bn));
+    const double cost = (double)((tiles + slots - 1) / slots) * (K / BK * sh.step + sh.wave);
+    if (!best.bn || cost < best_cost) {
+      best = sh.tile;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+// Q8_0: the dequantising warps set the pace, one wave at K = 4096 takes 21.5 / 31.4 / 44.5 / 76.5 us for 32 / 64 / 128 / 256 columns.
+static int pick_bn_q8(uint32_t M, uint32_t N, uint32_t nmat, bool swiglu) {
+  if (int f = forced_bn()) return std::max(f, swiglu ? 64 : 32);
   const size_t mt = (M + BM - 1) / BM, sms = sm_count();
   int best = 0;
   double best_cost = 0.0;
   for (int bn : {256, 128, 64, 32}) {
-    if (bn < (q8 ? (swiglu ? 64 : 32) : 128)) break;
+    if (swiglu && bn < 64) break;
     const size_t ctas = mt * (swiglu ? (2 * N + bn - 1) / bn : nmat * ((N + bn - 1) / bn)), waves = (ctas + sms - 1) / sms;
-    // measured time of one wave at K = 4096, us: Q8_0 30.9 / 31.2 / 43.0 / 73.4 for 32 / 64 / 128 / 256 columns, FP16 27 + 0.022 bn
-    const double wave = q8 ? (bn == 32 ? 30.9 : bn == 64 ? 31.2 : bn == 128 ? 43.0 : 73.4) : 27.0 + 0.022 * bn;
-    const double cost = (double)waves * wave;
+    const double cost = (double)waves * (bn == 32 ? 21.5 : bn == 64 ? 31.4 : bn == 128 ? 44.5 : 76.5);
     if (!best || cost < best_cost) {
       best = bn;
       best_cost = cost;
@@ -407,13 +433,15 @@ cudaError_t launch_gemm_f16_tcgen05(const GemmParams &p, cudaStream_t s) {
   if (!gemm_params_ok(p, false)) return cudaErrorInvalidValue;
   for (uint32_t i = 0; i < p.nmat; ++i)
     if ((reinterpret_cast<uintptr_t>(p.a) | reinterpret_cast<uintptr_t>(p.w[i])) & 15) return cudaErrorMisalignedAddress;
-  return pick_bn(p.M, p.N, p.nmat, p.swiglu, false) == 256 ? launch_bn<256, GK_F16>(p, s, p.N) : launch_bn<128, GK_F16>(p, s, p.N);
+  const Tile t = pick_tile(p.M, p.N, p.K, p.nmat, p.swiglu, true);
+  if (t.pair) return launch_gemm_pair_f16(p, t.bn, s);
+  return t.bn == 256 ? launch_bn<256, GK_F16>(p, s, p.N) : launch_bn<128, GK_F16>(p, s, p.N);
 }
 
 cudaError_t launch_gemm_q8_tcgen05(const GemmParams &p, cudaStream_t s) {
   if (!gemm_params_ok(p, true)) return cudaErrorInvalidValue;
   if (reinterpret_cast<uintptr_t>(p.a) & 15) return cudaErrorMisalignedAddress;
-  switch (pick_bn(p.M, p.N, p.nmat, p.swiglu, true)) {
+  switch (pick_bn_q8(p.M, p.N, p.nmat, p.swiglu)) {
     case 256: return launch_bn<256, GK_Q8>(p, s, p.N);
     case 128: return launch_bn<128, GK_Q8>(p, s, p.N);
     case 64: return launch_bn<64, GK_Q8>(p, s, p.N);
@@ -424,9 +452,11 @@ cudaError_t launch_gemm_q8_tcgen05(const GemmParams &p, cudaStream_t s) {
 cudaError_t launch_gemm_rows_bf16(const GemmRows &p, cudaStream_t s) {
   if (!gemm_tcgen05_supported(p.M, p.N, p.K) || p.N % 32 || (p.tile_expert && (p.M % BM || p.n2)) || p.n2 % kInputAlign) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(p.a) | reinterpret_cast<uintptr_t>(p.w)) & 15) return cudaErrorMisalignedAddress;
+  const Tile t = pick_tile(p.M, p.N, p.K, 1, false, !p.tile_expert);  // the two row tiles of a pair share their weights: not grouped
+  if (t.pair) return launch_gemm_pair_bf16(p, t.bn, s);
   // grouped: a tile's weight rows beyond its expert's N are read (the next expert's, or zeros) and dropped by the epilogue
   const uint32_t w_rows = p.tile_expert ? p.w_rows : p.N;
-  return pick_bn(p.M, p.N, 1, false, false) == 256 ? launch_bn<256, GK_ROWS>(p, s, w_rows) : launch_bn<128, GK_ROWS>(p, s, w_rows);
+  return t.bn == 256 ? launch_bn<256, GK_ROWS>(p, s, w_rows) : launch_bn<128, GK_ROWS>(p, s, w_rows);
 }
 
 }  // namespace vkl

@@ -323,6 +323,8 @@ struct GemmParams {
   float scale, bias;          // MatMul's scale and bias (mat_mul.cpp:39-41)
   int act;                    // 0 none, 1 SiLU
 };
+// The same by pairs of CTAs (gemm_pair.cu); bn: columns of W per tile, 128 or 256. Operands as checked by the caller.
+cudaError_t launch_gemm_pair_f16(const GemmParams &p, int bn, cudaStream_t s);
 constexpr uint32_t GEMM_MIN_ROWS = 32;  // below this the weight-streaming mat-vec kernel is used
 bool gemm_tcgen05_supported(uint32_t M, uint32_t N, uint32_t K);
 cudaError_t launch_gemm_f16_tcgen05(const GemmParams &p, cudaStream_t s);

@@ -143,6 +143,7 @@ struct GemmRows {
 };
 constexpr uint32_t kInputAlign = 256;  // no tile of the GEMMs crosses a multiple of this many weight rows
 cudaError_t launch_gemm_rows_bf16(const GemmRows &p, cudaStream_t s);  // tcgen05
+cudaError_t launch_gemm_pair_bf16(const GemmRows &p, int bn, cudaStream_t s);  // by pairs of CTAs (gemm_pair.cu); not grouped
 cudaError_t launch_gemm_rows_f32(const GemmRows &p, cudaStream_t s);   // true 32-bit (tcgen05 on A in three parts): two launches
 
 // ---- attention over a cache of keys and values, or of rows that are both (kv_attention.cu) ----
