@@ -232,6 +232,27 @@ def test_feed_forward_many_rows(dev, wt, M, dim, hidden):
     assert_close(got, want, what="feed_forward %s M=%d" % (wt, M))
 
 
+# 9 to 64 rows: K chunks that end inside a stage, tiles and rows that end inside a CTA's share, one and several CTAs' worth of
+# rows, inputs that the bulk copies do not take (K not in whole blocks), more than one pass of 64 rows.
+@pytest.mark.parametrize("wt", ["f16", "q8_0"])
+@pytest.mark.parametrize("M,N,K", [(9, 24, 32), (16, 48, 160), (17, 100, 416), (31, 5000, 256), (33, 72, 4128), (48, 130, 96), (63, 264, 1056), (45, 40, 72), (77, 40, 96)])
+def test_matmul_few_rows(dev, wt, M, N, K):
+    dt = vk.FP16 if wt == "f16" else vk.Q8_0
+    x = O.synth_f16(167, 1, M * K).reshape(M, K)
+    w = O.synth_f16(167, 2, N * K, 0.0, 0.05) if wt == "f16" else O.synth_q8_0(167, 2, N, K, 0.0, 0.05)
+    cmd = vk.Command(dev)
+    cmd.begin()
+    op = vk.MatMul(dev, cmd, up(cmd, dev, w, dt, 1, N, K), 1.25, 0.5, 0, 0, True, vk.FP16, dt).init()
+    got = cmd.download(op(up(cmd, dev, x, vk.FP16, 1, M, K)))
+    cmd.end()
+    cmd.submit_and_wait()
+    if wt == "f16":
+        want = (x.view(np.float16).astype(np.float64) @ w.view(np.float16).astype(np.float64).reshape(N, K).T * 1.25 + 0.5).astype(np.float16).view(np.uint16)
+    else:
+        want = O.matmul_q8_0(x, w, M, N, K, 1.25, 0.5)
+    assert_close(got, want, tol=2e-3, what="matmul %s %dx%dx%d" % (wt, M, N, K))
+
+
 # ---- RMSNorm (tests/test_rmsnorm.cpp:100-105: [1,1,128]; 7B rows) -------------
 @pytest.mark.parametrize("rows,W,eps", [(1, 128, 1e-3), (1, 4096, 1e-5), (33, 4096, 1e-5), (5, 100, 1e-6)])
 def test_rms_norm(dev, rows, W, eps):

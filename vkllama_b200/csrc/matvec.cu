@@ -1,4 +1,5 @@
-// Weight-streaming mat-vec / skinny mat-mul: Y[M,N] = epilogue(X[M,K] . W[N,K]^T)
+// Weight-streaming mat-vec: Y[M,N] = epilogue(X[M,K] . W[N,K]^T), one row or few
+// (more than 8 rows go to skinny_gemm.cu where its alignment rules allow)
 // for Q8_0 weights (fused dequantisation) and FP16 weights.
 //
 // Replaces the reference's four weight shaders
@@ -314,22 +315,7 @@ cudaError_t launch_m(const MvParams &p, cudaStream_t s) {
   if (XS) return cudaErrorInvalidValue;
   if (p.M <= 16) return launch_t<2, EPI, false, Q8>(p, s);
   if (p.M <= 32) return launch_t<4, EPI, false, Q8>(p, s);
-  // Wider inputs: passes of 64 rows (the weights are re-streamed per pass).
-  for (uint32_t m0 = 0; m0 < p.M; m0 += 64) {
-    MvParams q = p;
-    q.M = (p.M - m0 < 64) ? p.M - m0 : 64;
-    q.x = p.x + (size_t)m0 * p.x_ld;
-    for (int i = 0; i < 3; ++i)
-      if (p.out[i]) q.out[i] = p.out[i] + (size_t)m0 * p.out_ld;
-    if (p.out_f32) q.out_f32 = p.out_f32 + (size_t)m0 * p.out_ld;
-    if (p.residual) q.residual = p.residual + (size_t)m0 * p.out_ld;
-    cudaError_t e = (q.M <= 8)    ? launch_t<1, EPI, false, Q8>(q, s)
-                    : (q.M <= 16) ? launch_t<2, EPI, false, Q8>(q, s)
-                    : (q.M <= 32) ? launch_t<4, EPI, false, Q8>(q, s)
-                                  : launch_t<8, EPI, false, Q8>(q, s);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  return launch_t<8, EPI, false, Q8>(p, s);
 }
 
 template <bool XS, bool Q8>
@@ -349,7 +335,21 @@ cudaError_t launch_matvec(const MvParams &p, int epilogue, bool fuse_norm_smem, 
   if (p.fp16_weights && (p.K & 7)) return cudaErrorInvalidValue;
   if (fuse_norm_smem)
     return p.fp16_weights ? launch_e<true, false>(p, epilogue, s) : launch_e<true, true>(p, epilogue, s);
-  return p.fp16_weights ? launch_e<false, false>(p, epilogue, s) : launch_e<false, true>(p, epilogue, s);
+  // wider inputs: passes of 64 rows (the weights are re-streamed per pass)
+  for (uint32_t m0 = 0; m0 < p.M; m0 += 64) {
+    MvParams q = p;
+    q.M = std::min(64u, p.M - m0);
+    q.x = p.x + (size_t)m0 * p.x_ld;
+    for (int i = 0; i < 3; ++i)
+      if (p.out[i]) q.out[i] = p.out[i] + (size_t)m0 * p.out_ld;
+    if (p.out_f32) q.out_f32 = p.out_f32 + (size_t)m0 * p.out_ld;
+    if (p.residual) q.residual = p.residual + (size_t)m0 * p.out_ld;
+    cudaError_t e = skinny_gemm_takes(q, epilogue) ? launch_skinny_gemm(q, epilogue, s)
+                    : p.fp16_weights     ? launch_e<false, false>(q, epilogue, s)
+                                         : launch_e<false, true>(q, epilogue, s);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace vkl

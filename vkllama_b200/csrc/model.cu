@@ -71,7 +71,7 @@ int ensure_rows(vkl_model *m, uint32_t T) {
   return VKL_OK;
 }
 
-MvParams mv(const vkl_model *m, const vkl_tensor *w, const __half *x, __half *out, uint32_t M) {
+MvParams mv(vkl_model *m, const vkl_tensor *w, const __half *x, __half *out, uint32_t M) {
   MvParams p = {};
   p.codes[0] = w->data();
   p.scales[0] = q8(m) ? w->scales() : nullptr;
@@ -86,6 +86,10 @@ MvParams mv(const vkl_model *m, const vkl_tensor *w, const __half *x, __half *ou
   p.scale = 1.f;
   p.fp16_weights = !q8(m);
   p.use_pdl = 0;
+  if (M > 8) {  // a kernel with bounded waits
+    p.error = (uint32_t *)m->state->data() + 6;
+    m->gemm_used = true;
+  }
   return p;
 }
 
