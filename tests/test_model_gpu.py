@@ -110,6 +110,22 @@ def test_small_model_logits_prefill_then_decode(dev):
         assert_close(gv[:, :17], om.vcache(l)[:, :17], tol=5e-3, what="vcache layer %d" % l)
 
 
+@pytest.mark.parametrize("P", [128, 129, 300])
+def test_q8_0_prompts_around_the_widened_weights_limit(dev, P):
+    """129 tokens and more: the GEMMs' weights are turned into fp16 first. Row tiles of a matrix that end inside a 128-row half
+    tile, blocks that end inside a group of four."""
+    cfg = dict(dim=192, heads=3, ffn=320, vocab=500, layers=2, maxlen=320)
+    om = O.Model(seed=21, **cfg)
+    dm = vk.Model(dev, cfg["dim"], cfg["heads"], cfg["ffn"], cfg["vocab"], cfg["layers"], cfg["maxlen"])
+    dm.synth_weights(21)
+    prompt = O.synth_tokens(21, 1000 + P, P, cfg["vocab"])
+    assert np.abs(dm(prompt, 0) - om.forward(prompt, 0)).max() <= LOGITS_MAX_ABS
+    for l in range(cfg["layers"]):
+        gk, gv = dm.read_kv(l)
+        assert_close(gk[:, :P], om.kcache(l)[:, :P], tol=5e-3, what="kcache layer %d" % l)
+        assert_close(gv[:, :P], om.vcache(l)[:, :P], tol=5e-3, what="vcache layer %d" % l)
+
+
 @pytest.mark.parametrize("seed,P,n_gen", [(8, 9, 40), (9, 1, 20), (10, 33, 64)])
 def test_small_model_greedy_ids_match_oracle(dev, seed, P, n_gen):
     om, dm, cfg = small_pair(dev, seed=seed)

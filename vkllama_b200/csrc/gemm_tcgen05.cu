@@ -438,9 +438,58 @@ cudaError_t launch_gemm_f16_tcgen05(const GemmParams &p, cudaStream_t s) {
   return t.bn == 256 ? launch_bn<256, GK_F16>(p, s, p.N) : launch_bn<128, GK_F16>(p, s, p.N);
 }
 
+namespace {
+// Tiled planes -> row-major fp16(q * d), the values that the dequantising warps write. A thread turns eight codes each of two
+// rows; bound by memory (4096 x 11008: 24 us, 138 MB).
+__global__ void __launch_bounds__(256) widen_kernel(const uint8_t *__restrict__ codes, const uint8_t *__restrict__ scales, __half *__restrict__ out, Q8Layout L) {
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;  // (row tile, block, lane)
+  const uint32_t lane = i & 31, g = lane >> 2, t = lane & 3, per = L.groups * 4;
+  const uint32_t tile = (uint32_t)((i >> 5) / per), b = (uint32_t)((i >> 5) % per), k = b * 32 + t * 8, row = tile * 16 + g;
+  if (tile >= L.tiles || k >= L.K) return;
+  const uint4 w = ldg_stream(codes + i * 16);
+  const __half *d = reinterpret_cast<const __half *>(scales) + (((size_t)tile * L.groups + (b >> 2)) * 8 + g) * 8 + (b & 3);
+  const uint32_t c[2][4] = {{codes_to_h2(w.x, false), codes_to_h2(w.x, true), codes_to_h2(w.y, false), codes_to_h2(w.y, true)},
+                            {codes_to_h2(w.z, false), codes_to_h2(w.z, true), codes_to_h2(w.w, false), codes_to_h2(w.w, true)}};
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    if (row + 8 * r >= L.N) break;
+    const __half2 s = __half2half2(d[4 * r]);
+    uint32_t v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const __half2 x = __hmul2(*reinterpret_cast<const __half2 *>(&c[r][j]), s);
+      v[j] = *reinterpret_cast<const uint32_t *>(&x);
+    }
+    *reinterpret_cast<uint4 *>(out + (size_t)(row + 8 * r) * L.K + k) = make_uint4(v[0], v[1], v[2], v[3]);
+  }
+}
+}  // namespace
+
+// A 128-row tile dequantises the whole matrix for itself, at the pace of its dequantising warps (0.67 us per K step of 128
+// columns); widened once, the matrix runs on the fp16 GEMM's tiles. A prompt through four 7B blocks, us, dequantised in the tiles /
+// widened: 128 rows 989 / 1139, 129 1361 / 1186, 256 1387 / 1207, 257 1613 / 1302, 509 2046 / 1385, 900 3386 / 1816, 2048 6639 / 3102.
+constexpr uint32_t kWideRows = 129;
+bool gemm_q8_wide(uint32_t M) {
+  static const uint32_t rows = [] { const char *e = getenv("VKLLAMA_Q8_WIDE"); return e ? (uint32_t)atoi(e) : kWideRows; }();  // experiments
+  return M >= rows;
+}
+
 cudaError_t launch_gemm_q8_tcgen05(const GemmParams &p, cudaStream_t s) {
   if (!gemm_params_ok(p, true)) return cudaErrorInvalidValue;
   if (reinterpret_cast<uintptr_t>(p.a) & 15) return cudaErrorMisalignedAddress;
+  if (p.wide && gemm_q8_wide(p.M)) {
+    const Q8Layout L = q8_layout(p.N, p.K);
+    const size_t threads = (size_t)L.tiles * L.groups * 4 * 32;
+    GemmParams h = p;
+    for (uint32_t i = 0; i < p.nmat; ++i) {
+      __half *w = p.wide + (size_t)i * p.N * p.K;
+      widen_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(p.w_codes[i], p.w_scales[i], w, L);
+      cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+      h.w[i] = w;
+    }
+    return launch_gemm_f16_tcgen05(h, s);
+  }
   switch (pick_bn_q8(p.M, p.N, p.nmat, p.swiglu)) {
     case 256: return launch_bn<256, GK_Q8>(p, s, p.N);
     case 128: return launch_bn<128, GK_Q8>(p, s, p.N);

@@ -316,6 +316,7 @@ struct GemmParams {
   const __half *w[3];         // [N,K] row-major (a transposed-weight matrix of the reference); FP16 weights
   const uint8_t *w_codes[3];  // Q8_0 weights [N,K] as tiled planes (common.cuh): codes ...
   const uint8_t *w_scales[3]; // ... and scales
+  __half *wide;               // Q8_0: room for the nmat matrices in fp16 (gemm_q8_wide), or null
   __half *c[3];               // [M,N] fp16 output, or nullptr when c_f32 is set
   uint32_t nmat;
   int swiglu;                 // c[0] = fp16(silu(gate) * up) of the fp32 products with w[0] (gate) and w[1] (up): the
@@ -335,6 +336,9 @@ cudaError_t launch_gemm_f16_tcgen05(const GemmParams &p, cudaStream_t s);
 // The same GEMM with Q8_0 weights (w_codes / w_scales), dequantised into the shared-memory tiles.
 constexpr uint32_t GEMM_Q8_MIN_ROWS = 64;  // below this the rows-at-a-time kernel keeps the exact fp32 scaling
 cudaError_t launch_gemm_q8_tcgen05(const GemmParams &p, cudaStream_t s);
+// Whether the Q8_0 matrices are turned into fp16 once, in GemmParams::wide, and multiplied as such.
+bool gemm_q8_wide(uint32_t M);
+inline uint32_t gemm_launches(const GemmParams &p) { return !p.w[0] && p.wide && gemm_q8_wide(p.M) ? p.nmat + 1 : 1; }
 // Rows from which a weight of this kind goes to the tensor-core GEMM.
 inline uint32_t gemm_min_rows(bool q8) { return q8 ? GEMM_Q8_MIN_ROWS : GEMM_MIN_ROWS; }
 // Dispatch on the weight kind: w[0] set = FP16 weights, else w_codes / w_scales = Q8_0.

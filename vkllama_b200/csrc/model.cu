@@ -44,6 +44,7 @@ namespace {
 
 bool q8(const vkl_model *m) { return m->cfg.weight_dtype == VKL_Q8_0; }
 
+bool use_gemm(const vkl_model *m, uint32_t rows);
 int ensure_rows(vkl_model *m, uint32_t T) {
   if (T <= m->cap_T) return VKL_OK;
   if (m->dec) return decoder_ensure_rows(m, T);
@@ -64,6 +65,8 @@ int ensure_rows(vkl_model *m, uint32_t T) {
   VKL_OKAY(ensure_tensor(m->dev, &m->v, 1, T, m->dim_l, VKL_FP16));
   VKL_OKAY(ensure_tensor(m->dev, &m->ao, 1, T, m->dim_l, VKL_FP16));
   VKL_OKAY(ensure_tensor(m->dev, &m->t, 1, T, m->ffn_l, VKL_FP16));
+  if (q8(m) && use_gemm(m, T) && gemm_q8_wide(T))  // the largest set of matrices that share an input
+    VKL_OKAY(ensure_tensor(m->dev, &m->wide, 1, 1, D * std::max((size_t)2 * m->ffn_l, (size_t)3 * m->dim_l), VKL_FP16));
   VKL_OKAY(ensure_tensor(m->dev, &m->toks, 1, 1, T, VKL_UINT32));
   const size_t sc = attention_plan_most(T, m->heads_l, m->head_dim, (uint32_t)m->dev->prop.multiProcessorCount).scratch_bytes;
   VKL_OKAY(ensure_tensor(m->dev, &m->attn_scratch, 1, 1, sc / 4, VKL_FP32));
@@ -102,6 +105,7 @@ GemmParams gemm(vkl_model *m, const vkl_tensor *w, const __half *a, __half *out,
   g.N = (uint32_t)w->h;
   g.K = (uint32_t)w->w;
   g.scale = 1.f;
+  if (m->wide) g.wide = (__half *)m->wide->data();
   g.error = (uint32_t *)m->state->data() + 6;
   m->gemm_used = true;
   return g;
@@ -138,7 +142,7 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
     g.c[0] = nullptr;
     g.residual = nullptr;
     g.c_f32 = (float *)((char *)m->tp_buf + region);
-    VKL_LAUNCH(1, launch_gemm_tcgen05(g, s));
+    VKL_LAUNCH(gemm_launches(g), launch_gemm_tcgen05(g, s));
     TpRowsParams r = {};
     for (uint32_t i = 0; i < m->cfg.tp_size; ++i) {
       r.part[i] = (const float *)((const char *)m->tp_peer[i] + region);
@@ -178,7 +182,7 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
       GemmParams g = gemm(m, y.wk, xn, kb, T);
       add_weight(g, y.wq, qb);
       add_weight(g, y.wv, vb);
-      VKL_LAUNCH(1, launch_gemm_tcgen05(g, s));
+      VKL_LAUNCH(gemm_launches(g), launch_gemm_tcgen05(g, s));
     } else {
       VKL_LAUNCH(1, launch_rms_norm(x, (const float *)y.attn_norm->data(), xn, T, D, m->cfg.eps, s));
       VKL_LAUNCH((T + 63) / 64, launch_matvec(p, EPI_PLAIN, false, s));
@@ -208,7 +212,7 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
     } else if (use_gemm(m, rows)) {
       GemmParams g = gemm(m, y.wo, ao, xr, rows);
       g.residual = xr;
-      VKL_LAUNCH(1, launch_gemm_tcgen05(g, s));
+      VKL_LAUNCH(gemm_launches(g), launch_gemm_tcgen05(g, s));
     } else {
       MvParams o = mv(m, y.wo, ao, xr, rows);
       o.residual = xr;
@@ -230,7 +234,7 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
       GemmParams g = gemm(m, y.gate, xn, tb, rows);
       add_weight(g, y.up, nullptr);
       g.swiglu = 1;
-      VKL_LAUNCH(1, launch_gemm_tcgen05(g, s));
+      VKL_LAUNCH(gemm_launches(g), launch_gemm_tcgen05(g, s));
     } else {
       VKL_LAUNCH(1, launch_rms_norm(xr, (const float *)y.ffn_norm->data(), xn, rows, D, m->cfg.eps, s));
       VKL_LAUNCH((rows + 63) / 64, launch_matvec(f, EPI_SWIGLU, false, s));
@@ -241,7 +245,7 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
     } else if (use_gemm(m, rows)) {
       GemmParams g = gemm(m, y.down, tb, xr, rows);
       g.residual = xr;
-      VKL_LAUNCH(1, launch_gemm_tcgen05(g, s));
+      VKL_LAUNCH(gemm_launches(g), launch_gemm_tcgen05(g, s));
     } else {
       MvParams d = mv(m, y.down, tb, xr, rows);
       d.residual = xr;

@@ -43,6 +43,7 @@ struct vkl_model {
   uint32_t head_dim = 0, heads_l = 0, dim_l = 0, ffn_l = 0, vocab_l = 0;
   std::vector<vkl::Layer> L;  // Llama-2: blocks; a decoder design: layer runs, of which only caches and states live here
   std::unique_ptr<vkl::Decoder> dec;  // set for the layer-list decoder designs
+  vkl_tensor *wide = nullptr;  // long Q8_0 prompts: the weights of one GEMM in fp16
   vkl_tensor *tok_embd = nullptr, *output_norm = nullptr, *output = nullptr;
   vkl_tensor *fc = nullptr, *fs = nullptr;
   // activations, sized for `cap_T` rows
@@ -92,7 +93,7 @@ struct vkl_model {
     for (auto &l : L)
       for (vkl_tensor *p : {l.attn_norm, l.ffn_norm, l.wq, l.wk, l.wv, l.wo, l.gate, l.up, l.down, l.kcache, l.vcache, l.state, l.ring}) vkl_tensor_release(p);
     for (vkl_tensor *p : mega_packed) vkl_tensor_release(p);
-    for (vkl_tensor *p : {tok_embd, output_norm, output, fc, fs, x, xn, q, k, v, ao, t, logits16, logits32, toks, state, out_ids, forced, argpart, attn_scratch, attn_counters, mega_ops, mega_sync, mega_arg, mega_attn, mega_stages, mega_counts, mega_ll})
+    for (vkl_tensor *p : {wide, tok_embd, output_norm, output, fc, fs, x, xn, q, k, v, ao, t, logits16, logits32, toks, state, out_ids, forced, argpart, attn_scratch, attn_counters, mega_ops, mega_sync, mega_arg, mega_attn, mega_stages, mega_counts, mega_ll})
       vkl_tensor_release(p);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
