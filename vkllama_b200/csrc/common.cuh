@@ -63,6 +63,30 @@ __device__ __forceinline__ float warp_max(float v) {
 // Round to fp16 (nearest even) and back: the reference's op-boundary rounding.
 __device__ __forceinline__ float round_h(float v) { return __half2float(__float2half_rn(v)); }
 
+// Eight elements of an RMS norm: their squares added to s, and fp16(x * w * alpha).
+__device__ __forceinline__ float square_sum8(uint4 x, float s) {
+  const uint32_t in[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 v = __half22float2(*reinterpret_cast<const __half2 *>(&in[j]));
+    s += v.x * v.x;
+    s += v.y * v.y;
+  }
+  return s;
+}
+__device__ __forceinline__ uint4 norm8(uint4 x, float4 wa, float4 wb, float alpha) {
+  const uint32_t in[4] = {x.x, x.y, x.z, x.w};
+  const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+  uint32_t out[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 v = __half22float2(*reinterpret_cast<const __half2 *>(&in[j]));
+    const __half2 y = __halves2half2(__float2half_rn(v.x * w[2 * j] * alpha), __float2half_rn(v.y * w[2 * j + 1] * alpha));
+    out[j] = *reinterpret_cast<const uint32_t *>(&y);
+  }
+  return make_uint4(out[0], out[1], out[2], out[3]);
+}
+
 // 128-bit streaming load that does not pollute L1 (weights are read once).
 __device__ __forceinline__ uint4 ldg_stream(const void *p) {
   uint4 r;

@@ -94,8 +94,8 @@ cudaError_t launch_combine(const float *y, uint32_t y_ld, const int32_t *slot, u
   return cudaGetLastError();
 }
 cudaError_t launch_embed_rows(const bf16 *emb, const uint32_t *toks, uint32_t T, float scale, const Residual &r, bool f32, cudaStream_t s) {
-  if (f32) embed_rows_kernel<float><<<T, 256, 0, s>>>(emb, toks, scale, r);
-  else embed_rows_kernel<bf16><<<T, 256, 0, s>>>(emb, toks, scale, r);
+  if (f32) embed_rows_kernel<float><<<T, 1024, 0, s>>>(emb, toks, scale, r);
+  else embed_rows_kernel<bf16><<<T, 1024, 0, s>>>(emb, toks, scale, r);
   return cudaGetLastError();
 }
 cudaError_t launch_pack_rows(const bf16 *src, uint32_t rows, uint32_t cols, bf16 *dst, uint32_t ld, const PackMap &m, cudaStream_t s) {

@@ -106,14 +106,21 @@ __global__ void __launch_bounds__(kThreads) mv_kernel(const MvParams p) {
   if (XS) {
     if (p.use_pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float ssum[kWarps];
+    // whole 16-byte pieces where the rows have them: every CTA goes through the row before its first product (FP16 decode of the 7B
+    // shape: the norm + projection kernels took 30.1 and 33.2 us element by element, 29.3 and 33.3 this way, the lm head 52.8 and 48.2)
+    const bool vec = !((p.K | p.x_ld) & 7) && !((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.norm_w)) & 15);
     for (uint32_t m = 0; m < p.M; ++m) {
       const __half *xr = p.x + (size_t)m * p.x_ld;
       float alpha = 1.f;
       if (p.norm_w) {
         float s = 0.f;
-        for (uint32_t i = threadIdx.x; i < p.K; i += kThreads) {
-          const float v = __half2float(xr[i]);
-          s += v * v;
+        if (vec) {
+          for (uint32_t i = threadIdx.x * 8; i < p.K; i += kThreads * 8) s = square_sum8(*reinterpret_cast<const uint4 *>(xr + i), s);
+        } else {
+          for (uint32_t i = threadIdx.x; i < p.K; i += kThreads) {
+            const float v = __half2float(xr[i]);
+            s += v * v;
+          }
         }
         s = warp_sum(s);
         if (lane == 0) ssum[warp] = s;
@@ -124,9 +131,17 @@ __global__ void __launch_bounds__(kThreads) mv_kernel(const MvParams p) {
         alpha = 1.0f / sqrtf(tot / (float)p.K + p.eps);
         __syncthreads();
       }
-      for (uint32_t i = threadIdx.x; i < p.K; i += kThreads) {
-        const float v = __half2float(xr[i]);
-        xs[(size_t)m * xs_ld + i] = p.norm_w ? __float2half_rn(v * p.norm_w[i] * alpha) : xr[i];
+      if (vec) {
+        for (uint32_t i = threadIdx.x * 8; i < p.K; i += kThreads * 8) {
+          uint4 u = *reinterpret_cast<const uint4 *>(xr + i);
+          if (p.norm_w) u = norm8(u, *reinterpret_cast<const float4 *>(p.norm_w + i), *reinterpret_cast<const float4 *>(p.norm_w + i + 4), alpha);
+          *reinterpret_cast<uint4 *>(xs + (size_t)m * xs_ld + i) = u;
+        }
+      } else {
+        for (uint32_t i = threadIdx.x; i < p.K; i += kThreads) {
+          const float v = __half2float(xr[i]);
+          xs[(size_t)m * xs_ld + i] = p.norm_w ? __float2half_rn(v * p.norm_w[i] * alpha) : xr[i];
+        }
       }
     }
     __syncthreads();
