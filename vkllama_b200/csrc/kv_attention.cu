@@ -64,22 +64,37 @@ template <class T, int LPR, int NQ, bool SEP> __global__ void __launch_bounds__(
   const uint32_t g = blockIdx.x / groups, hg = blockIdx.x % groups, h0 = g * per + hg * NQ, nh = min((uint32_t)NQ, per - hg * NQ);
   const uint32_t m = blockIdx.y, split = blockIdx.z, tid = threadIdx.x, sub = tid / LPR, l = tid % LPR, e0 = l * 8, warp = tid >> 5;
   const bool ev = e0 < p.dp, vv = SEP && e0 < p.vp;
-  if (p.use_pdl) {
-    asm volatile("griddepcontrol.launch_dependents;");  // the out-projection asks for its weights meanwhile
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-  }
+  if (p.use_pdl) asm volatile("griddepcontrol.launch_dependents;");  // the out-projection asks for its weights meanwhile
+  // The kernel before this one writes the newest row and the queries; the position and the older rows are from kernels that
+  // had completed before it began, so the first of them are requested before waiting for it.
   const uint32_t pos = *p.pos + m, vis = pos + 1, lo = first_seen(p, pos);
   const uint32_t splits = min(p.splits, (vis - lo + kSplitRows - 1) / kSplitRows);
   if (split >= splits) return;
   uint32_t chunk = (vis - lo + splits - 1) / splits;
   chunk = (chunk + 31) & ~31u;
   const uint32_t c0 = min(lo + split * chunk, vis), c1 = min(c0 + chunk, vis);
+  const T *base = static_cast<const T *>(p.cache) + (size_t)g * p.maxlen * p.dp + e0;
+  const T *vbase = SEP ? static_cast<const T *>(p.vcache) + (size_t)g * p.maxlen * p.vp + e0 : nullptr;
+  constexpr bool AHEAD = sizeof(T) == 2;  // the next step's rows are requested during this one's arithmetic
+  Raw8<T> kr[U], vr[SEP ? U : 1], kn[AHEAD ? U : 1], vn[AHEAD && SEP ? U : 1];
+  auto request = [&](Raw8<T> *k, Raw8<T> *v, uint32_t jb, uint32_t from, uint32_t to) {  // of the rows of step jb those in [from, to)
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t j = jb + u * NS + sub;
+      if (ev && j >= from && j < to) k[u].load(base + (size_t)j * p.dp);
+      if constexpr (SEP) {
+        if (vv && j >= from && j < to) v[u].load(vbase + (size_t)j * p.vp);
+      }
+    }
+  };
+  request(kr, vr, c0, c0, min(c1, pos));
+  if (p.qk.q && tid < p.qk.pairs) turn_s[tid] = turn_of(pos, p.qk.freq[tid]);
+  if (p.use_pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
   const float qs = query_scale(p, pos);
   float rq = 1.f;
   if (p.qk.q) {  // one raw token: every CTA norms and turns its queries, the ones that see the token itself its key
     const bool newest = c0 < vis && c1 == vis && p.qk.kcache;
     const T *qr = static_cast<const T *>(p.qk.q), *kr = qr + p.qk.k_col;
-    if (tid < p.qk.pairs) turn_s[tid] = turn_of(pos, p.qk.freq[tid]);
     float sq = 0.f, sk = 0.f, v[8];
     for (uint32_t n = tid * 8; n < p.heads * p.dp; n += kRowThreads * 8) {
       load8(qr + n, v);
@@ -115,18 +130,17 @@ template <class T, int LPR, int NQ, bool SEP> __global__ void __launch_bounds__(
     mx[i] = -INFINITY;
     sum[i] = 0.f;
   }
-  const T *base = static_cast<const T *>(p.cache) + (size_t)g * p.maxlen * p.dp + e0;
-  const T *vbase = SEP ? static_cast<const T *>(p.vcache) + (size_t)g * p.maxlen * p.vp + e0 : nullptr;
+  request(kr, vr, c0, pos, c1);  // the newest row, if it is in the first step
   for (uint32_t jb = c0; jb < c1; jb += NS * U) {  // the same trip count for every thread
-    Raw8<T> kr[U], vr[SEP ? U : 1];
+    if constexpr (AHEAD) {
+      request(kn, vn, jb + NS * U, c0, c1);
+    } else {
+      if (jb != c0) request(kr, vr, jb, c0, c1);
+    }
     float s[U][NQ];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const uint32_t j = jb + u * NS + sub;
-      if (ev && j < c1) kr[u].load(base + (size_t)j * p.dp);
-      if constexpr (SEP) {
-        if (vv && j < c1) vr[u].load(vbase + (size_t)j * p.vp);
-      }
 #pragma unroll
       for (int i = 0; i < NQ; ++i) s[u][i] = (j < c1 && i < nh) ? bias_at(p, h0 + i, pos - j) : -INFINITY;
     }
@@ -169,6 +183,13 @@ template <class T, int LPR, int NQ, bool SEP> __global__ void __launch_bounds__(
       for (int i = 0; i < NQ; ++i)
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[i][e] = fmaf(s[u][i], v[e], acc[i][e]);
+    }
+    if constexpr (AHEAD) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        kr[u] = kn[u];
+        if constexpr (SEP) vr[u] = vn[u];
+      }
     }
   }
   // merge the warp's row streams, then the warps, in a fixed order
