@@ -10,6 +10,7 @@
 // Rounding points kept: roped q and k are fp16, the scaled score is rounded to
 // fp16 before the softmax, the head output is fp16. The probabilities are kept
 // in fp32 here (the reference stores them as fp16 between two dispatches).
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 
@@ -502,7 +503,8 @@ AttnPlan attention_plan(uint32_t T, bool clip, uint32_t heads, uint32_t dim, uin
 AttnPlan attention_plan_most(uint32_t T, uint32_t heads, uint32_t dim, uint32_t sms) {
   AttnPlan a = {};
   a.splits = kMostSplits;
-  const size_t row_units = (size_t)(kMostSplits * heads > 4 * sms ? kMostSplits * heads : 4 * sms), tile_units = (size_t)3 * sms;
+  const size_t row_units = (size_t)(kMostSplits * heads > 4 * sms ? kMostSplits * heads : 4 * sms);
+  const size_t tile_units = std::min((size_t)3 * sms, (size_t)kMostSplits * heads * ((T + 63) / 64));
   a.scratch_bytes = row_units * (dim + 2) * sizeof(float);
   if (T >= kTileMinRows && a.scratch_bytes < tile_units * 64 * (dim + 8) * sizeof(float)) a.scratch_bytes = tile_units * 64 * (dim + 8) * sizeof(float);
   a.counters = heads > 4 * sms ? heads : 4 * sms;
