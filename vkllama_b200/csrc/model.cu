@@ -632,6 +632,33 @@ int check_gemm(vkl_model *m) {
   return VKL_OK;
 }
 
+// The error words of the decode kernel and of the bounded waits in prompt kernels come back through pinned memory behind the
+// synchronisation that the caller's results need anyway; each took a copy and a synchronisation of its own (8 us).
+int queue_errors(vkl_model *m, bool decoded) {
+  const size_t lb = (size_t)m->vocab_l * 4;
+  if (!m->pin) VKL_CUDA(cudaHostAlloc((void **)&m->pin, lb + 16, cudaHostAllocDefault));
+  uint32_t *w = (uint32_t *)(m->pin + lb);
+  w[0] = w[1] = 0;
+  if (decoded && m->mega_ready) VKL_CUDA(cudaMemcpyAsync(w, m->mp.error, 4, cudaMemcpyDeviceToHost, m->stream));
+  if (m->gemm_used) VKL_CUDA(cudaMemcpyAsync(w + 1, (uint32_t *)m->state->data() + 6, 4, cudaMemcpyDeviceToHost, m->stream));
+  return VKL_OK;
+}
+int check_errors(vkl_model *m) {  // the stream has been synchronised since; a word that is set is read again, reset and reported
+  const uint32_t *w = (const uint32_t *)(m->pin + (size_t)m->vocab_l * 4);
+  if (w[1]) VKL_OKAY(check_gemm(m));
+  m->gemm_used = false;
+  return w[0] ? check_mega(m) : VKL_OK;
+}
+// The pass's logits, behind one synchronisation.
+int fetch_logits(vkl_model *m, float *logits_out, bool decoded) {
+  VKL_OKAY(queue_errors(m, decoded));
+  const size_t lb = (size_t)m->vocab_l * 4;
+  VKL_CUDA(cudaMemcpyAsync(m->pin, m->logits32->data(), lb, cudaMemcpyDeviceToHost, m->stream));
+  VKL_CUDA(cudaStreamSynchronize(m->stream));
+  memcpy(logits_out, m->pin, lb);
+  return check_errors(m);
+}
+
 int build_decode_graph(vkl_model *m);
 
 // Enqueue one decode step: the persistent kernel when available, else the graph.
@@ -990,19 +1017,10 @@ int vkl_model_forward(vkl_model *m, const uint32_t *toks, size_t n, size_t offse
   if (n == 1) {
     // The per-token call of a host-driven loop: one small launch sets the step up, the logits and the decode
     // kernel's error word come back through pinned memory behind one synchronisation.
-    const size_t lb = (size_t)m->vocab_l * 4;
-    if (!m->pin) VKL_CUDA(cudaHostAlloc((void **)&m->pin, lb + 16, cudaHostAllocDefault));
     begin_token_kernel<<<1, 1, 0, m->stream>>>((uint32_t *)m->state->data(), (uint32_t *)m->toks->data(), (uint32_t)offset, toks[0]);
     VKL_LAUNCH(1, cudaGetLastError());
     VKL_OKAY(decode_step(m));
-    VKL_CUDA(cudaMemcpyAsync(m->pin, m->logits32->data(), lb, cudaMemcpyDeviceToHost, m->stream));
-    uint32_t *errw = (uint32_t *)(m->pin + lb);
-    *errw = 0;
-    if (m->mega_ready) VKL_CUDA(cudaMemcpyAsync(errw, m->mp.error, 4, cudaMemcpyDeviceToHost, m->stream));
-    VKL_CUDA(cudaStreamSynchronize(m->stream));
-    memcpy(logits_out, m->pin, lb);
-    if (*errw) VKL_OKAY(check_mega(m));  // (reads the word again, resets the kernel's state, reports)
-    VKL_OKAY(check_gemm(m));
+    VKL_OKAY(fetch_logits(m, logits_out, true));
     if (m->dec) decoder_end(m, offset + 1);
     return VKL_OK;
   }
@@ -1010,15 +1028,8 @@ int vkl_model_forward(vkl_model *m, const uint32_t *toks, size_t n, size_t offse
   const uint32_t st[2] = {(uint32_t)offset, 0};
   VKL_CUDA(cudaMemcpyAsync(m->state->data(), st, 8, cudaMemcpyHostToDevice, m->stream));
   VKL_CUDA(cudaMemcpyAsync(m->toks->data(), toks, n * 4, cudaMemcpyHostToDevice, m->stream));
-  if (n == 1) {
-    VKL_OKAY(decode_step(m));
-  } else {
-    VKL_OKAY(run_tokens(m, (uint32_t)n, false));
-  }
-  VKL_CUDA(cudaMemcpyAsync(logits_out, m->logits32->data(), (size_t)m->vocab_l * 4, cudaMemcpyDeviceToHost, m->stream));
-  VKL_CUDA(cudaStreamSynchronize(m->stream));
-  if (n == 1) VKL_OKAY(check_mega(m));
-  VKL_OKAY(check_gemm(m));
+  VKL_OKAY(run_tokens(m, (uint32_t)n, false));
+  VKL_OKAY(fetch_logits(m, logits_out, false));
   if (m->dec) decoder_end(m, offset + n);
   return VKL_OK;
 }
@@ -1188,6 +1199,7 @@ int vkl_model_generate(vkl_model *m, const uint32_t *prompt, size_t n_prompt, si
   VKL_CUDA(cudaEventRecord(m->ev1, m->stream));
   for (size_t i = 1; i < n_gen; ++i) VKL_OKAY(decode_step(m));
   VKL_CUDA(cudaEventRecord(m->ev2, m->stream));
+  VKL_OKAY(queue_errors(m, true));
   VKL_CUDA(cudaMemcpyAsync(out_ids, m->out_ids->data(), n_gen * 4, cudaMemcpyDeviceToHost, m->stream));
   VKL_CUDA(cudaStreamSynchronize(m->stream));
   float ms = 0.f;
@@ -1199,9 +1211,9 @@ int vkl_model_generate(vkl_model *m, const uint32_t *prompt, size_t n_prompt, si
     VKL_CUDA(cudaEventElapsedTime(&ms, m->ev1, m->ev2));
     *decode_ms = ms;
   }
-  VKL_OKAY(check_gemm(m));
+  VKL_OKAY(check_errors(m));
   if (m->dec) decoder_end(m, n_prompt + n_gen - 1);
-  return check_mega(m);
+  return VKL_OK;
 }
 
 int vkl_model_last_token(vkl_model *m, uint32_t *id) {
