@@ -2,8 +2,9 @@
 // arithmetic and the epilogues of the mat-vec kernel (matvec.cu): products of codes and inputs on mma.sync with fp32
 // accumulators, the block scale applied in fp32 per 32 columns.
 //
-// Bound: the weights' bytes up to some 24 rows, the mma.sync pipe beyond (a scale per 32 columns and row keeps Q8_0 off
-// tcgen05, whose accumulators cannot be scaled on the way without rounding the weights). What held the mat-vec kernel back at a
+// The roofs are the weights' bytes up to some 24 rows and the mma.sync pipe beyond (a scale per 32 columns and row keeps Q8_0 off
+// tcgen05, whose accumulators cannot be scaled on the way without rounding the weights); at 45 rows the pipe is a third busy, the
+// rest is what one CTA per SM does not overlap: its first copies and its reduction. What held the mat-vec kernel back at a
 // fifth of that was X: every 16-row tile fetched all of it from L2, 0.8 GB for 45 rows of the 13B gate/up. Here a
 // CTA takes 64 weight rows (or 32), and both operands arrive K chunk by K chunk in a ring of shared-memory stages: X (and FP16
 // weights) by TMA tensor copies, Q8_0 planes by bulk copies, a few large ones per chunk, since issuing a copy takes a
