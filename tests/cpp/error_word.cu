@@ -1,0 +1,7 @@
+// Reaches the private error words that kernels raise when a bounded wait runs out, so that a test can raise one from the host.
+#include "model.h"
+
+extern "C" int raise_model_word(vkl_model *m) {
+  const uint32_t one = 1;
+  return (int)cudaMemcpy((uint32_t *)m->state->data() + 6, &one, 4, cudaMemcpyHostToDevice);
+}

@@ -1321,9 +1321,10 @@ int vkl_model_block_forward(vkl_model *m, uint32_t layer, const void *x_fp16, si
   MvParams d = mv(m, y.down, (__half *)m->t->data(), x, (uint32_t)T);
   d.residual = x;
   VKL_LAUNCH((T + 63) / 64, launch_matvec(d, EPI_ADD, false, s));
+  VKL_OKAY(queue_errors(m, false));  // more than 8 rows: the projections' kernels have bounded waits
   VKL_CUDA(cudaMemcpyAsync(out_fp16, x, T * D * 2, cudaMemcpyDeviceToHost, s));
   VKL_CUDA(cudaStreamSynchronize(s));
-  return VKL_OK;
+  return check_errors(m);
 }
 
 int vkl_model_decode_profile(vkl_model *m, uint32_t token, size_t offset, float out_us[20]) {
