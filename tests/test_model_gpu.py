@@ -126,6 +126,33 @@ def test_q8_0_prompts_around_the_widened_weights_limit(dev, P):
         assert_close(gv[:, :P], om.vcache(l)[:, :P], tol=5e-3, what="vcache layer %d" % l)
 
 
+def test_q8_0_prompts_without_room_for_the_widened_weights(dev):
+    """The fp16 copy of the weights (256 MiB here) is for speed: on a device that is full up to 160 MiB the prompt runs in the
+    dequantising tiles, which write the same fp16 values. fp32 sums in another order: the logits differ by fp16 rounding."""
+    import torch
+    dims = (4096, 32, 16384, 500, 1, 256)
+    prompt = O.synth_tokens(22, 1000, 140, 500)
+    roomy = vk.Model(dev, *dims)
+    roomy.synth_weights(22)
+    want = roomy(prompt, 0)
+    roomy.close()
+    dm = vk.Model(dev, *dims)
+    dm.synth_weights(22)
+    dm(prompt[:70], 0)  # everything that a prompt launches is loaded
+    with pytest.raises(vk.VklError):
+        vk.Tensor(1, 1 << 20, 1 << 18, dev, vk.FP32)  # 1 TiB: refused, after the pool's free blocks went back to the driver
+    filler = []
+    try:
+        for mib in (4096, 512, 64, 16, 4):
+            while torch.cuda.mem_get_info()[0] - (mib << 20) > 160 << 20:
+                filler.append(vk.Tensor(1, mib, 1 << 18, dev, vk.FP32))
+        got = dm(prompt, 0)
+    finally:
+        del filler
+    assert np.abs(got - want).max() <= LOGITS_MAX_ABS
+    dm.close()
+
+
 @pytest.mark.parametrize("seed,P,n_gen", [(8, 9, 40), (9, 1, 20), (10, 33, 64)])
 def test_small_model_greedy_ids_match_oracle(dev, seed, P, n_gen):
     om, dm, cfg = small_pair(dev, seed=seed)

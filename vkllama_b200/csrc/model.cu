@@ -65,11 +65,15 @@ int ensure_rows(vkl_model *m, uint32_t T) {
   VKL_OKAY(ensure_tensor(m->dev, &m->v, 1, T, m->dim_l, VKL_FP16));
   VKL_OKAY(ensure_tensor(m->dev, &m->ao, 1, T, m->dim_l, VKL_FP16));
   VKL_OKAY(ensure_tensor(m->dev, &m->t, 1, T, m->ffn_l, VKL_FP16));
-  if (q8(m) && use_gemm(m, T) && gemm_q8_wide(T))  // the largest set of matrices that share an input
-    VKL_OKAY(ensure_tensor(m->dev, &m->wide, 1, 1, D * std::max((size_t)2 * m->ffn_l, (size_t)3 * m->dim_l), VKL_FP16));
   VKL_OKAY(ensure_tensor(m->dev, &m->toks, 1, 1, T, VKL_UINT32));
   const size_t sc = attention_plan_most(T, m->heads_l, m->head_dim, (uint32_t)m->dev->prop.multiProcessorCount).scratch_bytes;
   VKL_OKAY(ensure_tensor(m->dev, &m->attn_scratch, 1, 1, sc / 4, VKL_FP32));
+  // Room for the largest set of matrices that share an input (180 MB at 7B). For speed only: without it the GEMMs dequantise
+  // in their tiles. So it comes last, and where the device has no room for it the model runs without, until its rows grow again.
+  if (q8(m) && use_gemm(m, T) && gemm_q8_wide(T)) {
+    const int st = ensure_tensor(m->dev, &m->wide, 1, 1, D * std::max((size_t)2 * m->ffn_l, (size_t)3 * m->dim_l), VKL_FP16);
+    if (st != VKL_OK && st != VKL_RESOURCE_EXHAUSTED) return st;
+  }
   m->cap_T = T;
   return VKL_OK;
 }
