@@ -6,8 +6,11 @@ import os
 
 import numpy as np
 import pytest
+import torch
 
+from oracle import decoder as D
 from oracle import oracle as O
+import kupuzen_util as U
 import vkllama_b200 as vk
 from util import LOGITS_MAX_ABS, assert_close, decided_prompt, load_from_oracle
 
@@ -126,10 +129,20 @@ def test_q8_0_prompts_around_the_widened_weights_limit(dev, P):
         assert_close(gv[:, :P], om.vcache(l)[:, :P], tol=5e-3, what="vcache layer %d" % l)
 
 
+def fill(dev, mib_left):
+    """Tensors that leave less than mib_left + 4 MiB of the device's memory free, outside the pool too."""
+    with pytest.raises(vk.VklError):
+        vk.Tensor(1, 1 << 20, 1 << 18, dev, vk.FP32)  # 1 TiB: refused, after the pool's free blocks went back to the driver
+    filler = []
+    for mib in (4096, 512, 64, 16, 4):
+        while torch.cuda.mem_get_info()[0] - (mib << 20) > mib_left << 20:
+            filler.append(vk.Tensor(1, mib, 1 << 18, dev, vk.FP32))
+    return filler
+
+
 def test_q8_0_prompts_without_room_for_the_widened_weights(dev):
     """The fp16 copy of the weights (256 MiB here) is for speed: on a device that is full up to 160 MiB the prompt runs in the
     dequantising tiles, which write the same fp16 values. fp32 sums in another order: the logits differ by fp16 rounding."""
-    import torch
     dims = (4096, 32, 16384, 500, 1, 256)
     prompt = O.synth_tokens(22, 1000, 140, 500)
     roomy = vk.Model(dev, *dims)
@@ -139,17 +152,38 @@ def test_q8_0_prompts_without_room_for_the_widened_weights(dev):
     dm = vk.Model(dev, *dims)
     dm.synth_weights(22)
     dm(prompt[:70], 0)  # everything that a prompt launches is loaded
-    with pytest.raises(vk.VklError):
-        vk.Tensor(1, 1 << 20, 1 << 18, dev, vk.FP32)  # 1 TiB: refused, after the pool's free blocks went back to the driver
-    filler = []
+    filler = fill(dev, 160)
     try:
-        for mib in (4096, 512, 64, 16, 4):
-            while torch.cuda.mem_get_info()[0] - (mib << 20) > 160 << 20:
-                filler.append(vk.Tensor(1, mib, 1 << 18, dev, vk.FP32))
         got = dm(prompt, 0)
     finally:
         del filler
     assert np.abs(got - want).max() <= LOGITS_MAX_ABS
+    dm.close()
+
+
+@pytest.mark.parametrize("design", ["llama", "layer list"])
+def test_a_call_without_memory_for_its_rows_leaves_the_model_usable(dev, design):
+    """Growing the activations fails half way; shorter calls after it must not meet the buffers that are missing."""
+    if design == "llama":
+        dm = vk.Model(dev, 4096, 32, 16384, 500, 1, 4096)
+        dm.synth_weights(23)
+    else:
+        case = U.config([(U.attn(2, 1, 32, 32, 400, 8), 4096)], width=1088, vocab=500)
+        W = U.weights(case, 23)
+        dm = vk.Model.from_config(dev, case[0], 4096, vk.BF16, shapes=U.shapes(W))
+        for k, v in W.items():
+            dm.set_weight(k, vk.BF16, D.f32_to_bf16(v.reshape(-1)))
+    prompt = O.synth_tokens(23, 1000, 4000, 500)
+    want, one = dm(prompt[:20], 0), dm(prompt[20:21], 20)
+    filler = fill(dev, 8)
+    try:
+        with pytest.raises(vk.VklError) as e:
+            dm(prompt, 0)
+        assert e.value.code == 8
+    finally:
+        del filler
+    assert (dm(prompt[:20], 0) == want).all()
+    assert (dm(prompt[20:21], 20) == one).all()
     dm.close()
 
 

@@ -664,6 +664,7 @@ int decoder_ensure_rows(vkl_model *m, uint32_t T) {
   Decoder *d = m->dec.get();
   model_drop_graph(m);
   VKL_CUDA(cudaStreamSynchronize(m->stream));
+  m->cap_T = 0;  // an allocation that fails below leaves buffers missing: the next call makes them anew
   const int ct = compute_dtype(d);
   VKL_OKAY(zeros(m, &d->x, 1, T, d->ldw, VKL_FP32));
   VKL_OKAY(zeros(m, &d->h, d->spec.two_norms ? 2 : 1, T, d->ldw, ct));

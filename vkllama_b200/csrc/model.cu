@@ -50,6 +50,7 @@ int ensure_rows(vkl_model *m, uint32_t T) {
   if (m->dec) return decoder_ensure_rows(m, T);
   model_drop_graph(m);  // the graph holds the old buffers
   VKL_CUDA(cudaStreamSynchronize(m->stream));
+  m->cap_T = 0;  // an allocation that fails below leaves buffers missing: the next call makes them anew
   if (m->mega_tried) {  // the op table of the persistent kernel holds the old buffers too
     for (vkl_tensor **t : {&m->mega_ops, &m->mega_sync, &m->mega_arg, &m->mega_attn, &m->mega_stages, &m->mega_counts, &m->mega_ll}) {
       vkl_tensor_release(*t);
