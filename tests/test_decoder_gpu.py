@@ -249,3 +249,46 @@ def test_synthetic_weights_run_and_use_a_cache_of_keys_only(dev):
     k, _ = m.read_kv(0)
     assert (k[:, :20] != 0).any() and not k[:, 20:].any()
     m.close()
+
+
+def test_32bit_products_with_infinities(dev):
+    """An infinite weight times a finite input is an infinity, whatever parts the input is cut into (one in 256 numbers has a
+    middle or a low part of zero: 600 rows meet some); so is an infinite input times a weight other than zero."""
+    cfg = U.config([(U.attn(2, 1, 32), None)], width=192, vocab=70)
+    W, toks = U.weights(cfg, 61), U.tokens(cfg, 600, 62)
+    W["head"][7] = 0
+    W["head"][7, 3] = 1
+    col = D.run(cfg, W, toks)[:, 7]  # the sign of column 3 of the output layer's input
+    assert np.abs(col).min() > 1e-6
+    want = D.run(cfg, W, toks)
+    W["head"][7, 3] = -np.inf
+    m = load(dev, cfg, W, 600, "float32")
+    got = m.forward_rows(toks, 0, np.arange(600))
+    m.close()
+    assert (got[:, 7] == np.where(col > 0, -np.inf, np.inf)).all()
+    rest = np.arange(70) != 7
+    assert U.rel_err(got[:, rest], want[:, rest]) < U.REL["float32"]
+    W["head"][7, 3], W["head"][5, 3], W["final.norm"][3] = 1, 0, np.inf
+    m = load(dev, cfg, W, 600, "float32")
+    got = m.forward_rows(toks, 0, np.arange(600))
+    m.close()
+    sign = np.sign(got[:, 7])
+    assert np.isinf(got[:, 7]).all() and np.isnan(got[:, 5]).all()
+    rest = np.flatnonzero(W["head"][:, 3])
+    assert (got[:, rest] == sign[:, None] * np.sign(W["head"][rest, 3])[None] * np.inf).all()
+
+
+# Inputs of the output layer near both ends of the exponents, its weights scaled the other way. Sums of K = 192 fp32 terms: below
+# 1e-5. At 2^-115 the parts lose what lies below 2^-133: 2^-18 of the largest inputs and more of small ones, 2^-16 with a margin.
+@pytest.mark.parametrize("scale,tol", [(116, 1e-5), (60, 1e-5), (-78, 1e-5), (-82, 1e-5), (-100, 1e-5), (-115, 1.6e-5)])
+def test_32bit_products_over_the_exponent_range(dev, scale, tol):
+    cfg = U.config([(U.attn(2, 1, 32), None)], width=192, vocab=70)
+    W, toks = U.weights(cfg, 63), U.tokens(cfg, 40, 64)
+    want = D.run(cfg, W, toks)
+    for k in ("final.norm", "final.norm.b"):
+        W[k] = W[k] * np.float32(2.0 ** scale)
+    W["head"] = W["head"] * np.float32(2.0 ** -scale)
+    m = load(dev, cfg, W, 64, "float32")
+    err = U.rel_err(m.forward_rows(toks, 0, np.arange(40)), want)
+    m.close()
+    assert err < tol, err

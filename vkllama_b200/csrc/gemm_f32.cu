@@ -3,12 +3,12 @@
 // epilogues are those of the bfloat16 GEMM.
 //
 // Nothing is rounded on the way in: a float's 24 significant bits are cut into three bfloat16 numbers of 8 bits each
-// (high + middle + low = a, exactly, where the low part is not below the smallest subnormal), each product of one of
+// (high + middle + low = a, exactly from 2^-110 on; what lies below 2^-133, bfloat16's smallest step, is cut off), each product of one of
 // them with a bfloat16 weight has 16 bits, and the three products go into the same fp32 sum. What can lose precision is
 // the sum: the tensor core cuts off where an FMA rounds. So the accumulator in TMEM holds 64 products per output
 // only (one stage, the small parts first) and every stage's sum is added to a register in fp32. Against 64 bits (300 tokens,
-// K = 2048 ... 7680) the result is closer than the serial FMA sum that this replaced. An infinity or a NaN of A stays
-// in the high part alone. (Only an infinite WEIGHT shows a difference: it meets the zeros of the lower parts and gives NaN.)
+// K = 2048 ... 7680) the result is closer than the serial FMA sum that this replaced. Infinities and NaN, of A or of W, come out as
+// in that sum (but for numbers below 2^-80 times an infinite weight: NaN).
 //
 // Measured: the 10 GEMMs of a 300-token prompt at width 2048, feed-forward 5632, four layers: 8.26 ms with the FMA kernel
 // (64 x 64 tiles, 15 TFLOP/s), the whole call of 9.31 ms now takes 2.14; error of the logits against 64 bits 7.5e-7 -> 4.7e-7.
@@ -42,14 +42,21 @@ __global__ void __launch_bounds__(256) split_kernel(const float *__restrict__ a,
   uint32_t part[kParts][8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const uint32_t u = __float_as_uint(v[j]);
+    const uint32_t u = __float_as_uint(v[j]), sign = u >> 16 & 0x8000u;
     const bool finite = (u & 0x7f800000u) != 0x7f800000u;
     // cut, not rounded: no overflow at the top of the range, and every remainder is exact
-    part[0][j] = (u >> 16) | (!finite && (u & 0x007fffffu) ? 0x40u : 0u);  // a NaN stays one
     const float r = finite ? v[j] - __uint_as_float(u & 0xffff0000u) : 0.f;
     const uint32_t ur = __float_as_uint(r);
+    part[0][j] = (u >> 16) | (!finite && (u & 0x007fffffu) ? 0x40u : 0u);  // a NaN stays one
     part[1][j] = ur >> 16;
     part[2][j] = __float_as_uint(r - __uint_as_float(ur & 0xffff0000u)) >> 16;
+    // Times an infinite weight a zero part would give NaN where a * w is infinite, so a part of a number from 2^-80 on is never
+    // zero: 2^-126 with its sign takes the place, 2^-46 of the number at most.
+    if ((u & 0x7fffffffu) >= 0x17800000u) {
+#pragma unroll
+      for (int s = 1; s < kParts; ++s)
+        if (!(part[s][j] & 0x7fffu)) part[s][j] = sign | 0x0080u;
+    }
   }
 #pragma unroll
   for (int s = 0; s < kParts; ++s) {
