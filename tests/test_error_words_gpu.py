@@ -20,7 +20,8 @@ def words(tmp_path_factory):
     so = str(tmp_path_factory.mktemp("words") / "error_word.so")
     subprocess.check_call([B.NVCC] + B.FLAGS + ["-shared", "-I", B.CSRC, os.path.join(ROOT, "tests", "cpp", "error_word.cu"), "-o", so])
     L = C.CDLL(so)
-    L.raise_model_word.argtypes = [C.c_void_p]
+    for f in (L.raise_model_word, L.command_is_watched, L.raise_command_word):
+        f.argtypes = [C.c_void_p]
     return L
 
 
@@ -37,3 +38,37 @@ def test_block_forward_reports_its_own_waits(dev, words):
     assert (dm.block_forward(0, x, 0) == want).all()
     dm(np.arange(12, dtype=np.uint32), 0)
     dm.close()
+
+
+# Kernels with bounded waits: more than 8 rows in whole 32-column blocks, but for 9 to 16 rows of a Q8_0 matrix that gives every
+# SM 64 rows (9472 rows on 148 SMs), and the tensor-core GEMM.
+@pytest.mark.parametrize("wt,M,N,K,watched", [("q8_0", 1, 48, 96, False), ("q8_0", 8, 48, 96, False), ("q8_0", 20, 48, 72, False), ("q8_0", 12, 9600, 96, False),
+                                              ("q8_0", 9, 48, 96, True), ("q8_0", 17, 9600, 96, True), ("q8_0", 73, 48, 96, True), ("f16", 12, 9600, 96, True), ("q8_0", 64, 64, 64, True)])
+def test_a_command_asks_for_the_word_only_where_a_kernel_has_waits(dev, words, wt, M, N, K, watched):
+    dt = vk.Q8_0 if wt == "q8_0" else vk.FP16
+    w = O.synth_q8_0(72, 1, N, K, 0.0, 0.05) if wt == "q8_0" else O.synth_f16(72, 1, N * K, 0.0, 0.05)
+    cmd = vk.Command(dev)
+    cmd.begin()
+    tw, tx = vk.Tensor(1, N, K, dev, dt), vk.Tensor(1, M, K, dev, vk.FP16)
+    cmd.upload(w, tw)
+    cmd.upload(O.synth_f16(72, 2, M * K), tx)
+    op = vk.MatMul(dev, cmd, tw, 1.0, 0.0, 0, 0, True, vk.FP16, dt).init()
+    want = cmd.download(op(tx))
+    assert bool(words.command_is_watched(cmd.h)) == watched
+    cmd.end()
+    cmd.submit_and_wait()
+    assert not words.command_is_watched(cmd.h)
+    if not watched:
+        return
+    cmd.begin()
+    op(tx)
+    cmd.end()
+    assert words.raise_command_word(cmd.h) == 0
+    with pytest.raises(vk.VklError) as e:
+        cmd.submit_and_wait()
+    assert e.value.code == 13 and "code 1" in e.value.message
+    cmd.begin()
+    got = cmd.download(op(tx))
+    cmd.end()
+    cmd.submit_and_wait()
+    assert (got == want).all()

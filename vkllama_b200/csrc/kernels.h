@@ -33,12 +33,13 @@ struct MvParams {
   int act;                   // 1 = SiLU on the PLAIN epilogue
   int fp16_weights;          // 0 = Q8_0 tiled planes, 1 = FP16 row-major
   int use_pdl;               // programmatic dependent launch: prefetch weights before waiting
-  uint32_t *error;           // device word raised when a bounded wait ran out (more than 8 rows), or null
+  uint32_t *error;           // device word raised when a bounded wait ran out (where matvec_waits), or null
 };
 cudaError_t launch_matvec(const MvParams &p, int epilogue, bool fuse_norm_smem, cudaStream_t s);
 // 9 to 64 rows (skinny_gemm.cu); launch_matvec sends what it takes there
 bool skinny_gemm_takes(const MvParams &p, int epilogue);
 cudaError_t launch_skinny_gemm(const MvParams &p, int epilogue, cudaStream_t s);
+bool matvec_waits(const MvParams &p, int epilogue);  // whether launch_matvec runs a kernel with bounded waits (p.error)
 
 // 34-byte GGUF blocks <-> tiled planes (codes at dst, scales at dst + codes_bytes).
 cudaError_t launch_q8_repack(const uint8_t *blocks34, uint8_t *planes, uint32_t N, uint32_t K,

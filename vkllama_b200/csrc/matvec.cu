@@ -343,22 +343,33 @@ cudaError_t launch_e(const MvParams &p, int epi, cudaStream_t s) {
   return cudaErrorInvalidValue;
 }
 
+// Wider inputs: passes of 64 rows (the weights are re-streamed per pass). The pass of rows m0, m0 + 1, ...
+constexpr uint32_t kPassRows = 64;
+MvParams pass_at(const MvParams &p, uint32_t m0) {
+  MvParams q = p;
+  q.M = std::min(kPassRows, p.M - m0);
+  q.x = p.x + (size_t)m0 * p.x_ld;
+  for (int i = 0; i < 3; ++i)
+    if (p.out[i]) q.out[i] = p.out[i] + (size_t)m0 * p.out_ld;
+  if (p.out_f32) q.out_f32 = p.out_f32 + (size_t)m0 * p.out_ld;
+  if (p.residual) q.residual = p.residual + (size_t)m0 * p.out_ld;
+  return q;
+}
+
 }  // namespace
 
+bool matvec_waits(const MvParams &p, int epilogue) {
+  for (uint32_t m0 = 0; m0 < p.M; m0 += kPassRows)
+    if (skinny_gemm_takes(pass_at(p, m0), epilogue)) return true;
+  return false;
+}
 cudaError_t launch_matvec(const MvParams &p, int epilogue, bool fuse_norm_smem, cudaStream_t s) {
   if (p.M == 0 || p.N == 0) return cudaSuccess;
   if (p.fp16_weights && (p.K & 7)) return cudaErrorInvalidValue;
   if (fuse_norm_smem)
     return p.fp16_weights ? launch_e<true, false>(p, epilogue, s) : launch_e<true, true>(p, epilogue, s);
-  // wider inputs: passes of 64 rows (the weights are re-streamed per pass)
-  for (uint32_t m0 = 0; m0 < p.M; m0 += 64) {
-    MvParams q = p;
-    q.M = std::min(64u, p.M - m0);
-    q.x = p.x + (size_t)m0 * p.x_ld;
-    for (int i = 0; i < 3; ++i)
-      if (p.out[i]) q.out[i] = p.out[i] + (size_t)m0 * p.out_ld;
-    if (p.out_f32) q.out_f32 = p.out_f32 + (size_t)m0 * p.out_ld;
-    if (p.residual) q.residual = p.residual + (size_t)m0 * p.out_ld;
+  for (uint32_t m0 = 0; m0 < p.M; m0 += kPassRows) {
+    const MvParams q = pass_at(p, m0);
     cudaError_t e = skinny_gemm_takes(q, epilogue) ? launch_skinny_gemm(q, epilogue, s)
                     : p.fp16_weights     ? launch_e<false, false>(q, epilogue, s)
                                          : launch_e<false, true>(q, epilogue, s);

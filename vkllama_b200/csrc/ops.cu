@@ -125,7 +125,7 @@ struct MatMulOp : vkl_op {
         VKL_LAUNCH(1, launch_bmm_f16((const __half *)a->data(), (const __half *)weight->data(), (__half *)out->data(), 1,
                                      (uint32_t)a->h, (uint32_t)N, (uint32_t)K, 0, K, 0, K, 0, N, 1, scale, bias, act, cmd->stream));
       } else {
-        if (p.M > 8) VKL_OKAY(command_error_word(cmd, &p.error));
+        if (matvec_waits(p, EPI_PLAIN)) VKL_OKAY(command_error_word(cmd, &p.error));
         VKL_LAUNCH((a->h + 63) / 64, launch_matvec(p, EPI_PLAIN, false, cmd->stream));
       }
     } else {
@@ -225,7 +225,7 @@ struct FeedForwardOp : vkl_op {
     p.N = (uint32_t)w1->h; p.K = (uint32_t)w1->w; p.M = (uint32_t)x->h;
     p.x_ld = p.K; p.out_ld = p.N;
     p.scale = 1.f; p.fp16_weights = !q8;
-    if (p.M > 8) VKL_OKAY(command_error_word(cmd, &p.error));
+    if (matvec_waits(p, EPI_SWIGLU)) VKL_OKAY(command_error_word(cmd, &p.error));
     VKL_LAUNCH((x->h + 63) / 64, launch_matvec(p, EPI_SWIGLU, false, cmd->stream));
     MvParams d = {};
     d.codes[0] = w2->data(); d.scales[0] = q8 ? w2->scales() : nullptr;
@@ -234,7 +234,8 @@ struct FeedForwardOp : vkl_op {
     d.nmat = 1;
     d.N = (uint32_t)w2->h; d.K = (uint32_t)w2->w; d.M = (uint32_t)x->h;
     d.x_ld = d.K; d.out_ld = d.N;
-    d.scale = 1.f; d.fp16_weights = !q8; d.error = p.error;
+    d.scale = 1.f; d.fp16_weights = !q8;
+    if (matvec_waits(d, EPI_PLAIN)) VKL_OKAY(command_error_word(cmd, &d.error));
     VKL_LAUNCH((x->h + 63) / 64, launch_matvec(d, EPI_PLAIN, false, cmd->stream));
     *o = out;
     return leave();
@@ -348,7 +349,7 @@ struct MhaOp : vkl_op {
       VKL_OKAY(command_error_word(cmd, &g.error));
       VKL_LAUNCH(1, launch_gemm_tcgen05(g, cmd->stream));
     } else {
-      if (T > 8) VKL_OKAY(command_error_word(cmd, &p.error));
+      if (matvec_waits(p, EPI_PLAIN)) VKL_OKAY(command_error_word(cmd, &p.error));
       VKL_LAUNCH((T + 63) / 64, launch_matvec(p, EPI_PLAIN, false, cmd->stream));
     }
 
@@ -387,7 +388,7 @@ struct MhaOp : vkl_op {
       VKL_OKAY(command_error_word(cmd, &g.error));
       VKL_LAUNCH(1, launch_gemm_tcgen05(g, cmd->stream));
     } else {
-      if (To > 8) VKL_OKAY(command_error_word(cmd, &w.error));
+      if (matvec_waits(w, EPI_PLAIN)) VKL_OKAY(command_error_word(cmd, &w.error));
       VKL_LAUNCH((To + 63) / 64, launch_matvec(w, EPI_PLAIN, false, cmd->stream));
     }
     *o = out;

@@ -115,6 +115,7 @@ struct vkl_command {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // recorded by begin() and end()
   std::vector<std::function<void()>> deferred;  // run by wait()
   uint32_t *err_word = nullptr;  // device word raised by a kernel whose bounded wait ran out; read by wait()
+  uint32_t *err_host = nullptr;  // pinned: where it is read to
   bool err_used = false;
 };
 
