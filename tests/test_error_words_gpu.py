@@ -40,10 +40,11 @@ def test_block_forward_reports_its_own_waits(dev, words):
     dm.close()
 
 
-# Kernels with bounded waits: more than 8 rows in whole 32-column blocks, but for 9 to 16 rows of a Q8_0 matrix that gives every
-# SM 64 rows (9472 rows on 148 SMs), and the tensor-core GEMM.
-@pytest.mark.parametrize("wt,M,N,K,watched", [("q8_0", 1, 48, 96, False), ("q8_0", 8, 48, 96, False), ("q8_0", 20, 48, 72, False), ("q8_0", 12, 9600, 96, False),
-                                              ("q8_0", 9, 48, 96, True), ("q8_0", 17, 9600, 96, True), ("q8_0", 73, 48, 96, True), ("f16", 12, 9600, 96, True), ("q8_0", 64, 64, 64, True)])
+# Kernels with bounded waits: the few-row kernel (more than 8 rows, whole 32-column blocks, 5 million weights, 1.6 million from 33
+# rows on; for 9 to 16 rows of Q8_0 at most 370 row tiles of 16 on 148 SMs), and the tensor-core GEMM.
+@pytest.mark.parametrize("wt,M,N,K,watched", [("q8_0", 1, 1300, 3936, False), ("q8_0", 8, 1300, 3936, False), ("q8_0", 20, 1300, 3928, False), ("q8_0", 12, 6000, 864, False),
+                                              ("q8_0", 20, 1300, 3808, False), ("q8_0", 9, 1300, 3936, True), ("q8_0", 17, 1300, 3936, True), ("q8_0", 33, 417, 3936, True),
+                                              ("q8_0", 77, 417, 3936, True), ("f16", 12, 12000, 480, True), ("q8_0", 64, 64, 64, True)])
 def test_a_command_asks_for_the_word_only_where_a_kernel_has_waits(dev, words, wt, M, N, K, watched):
     dt = vk.Q8_0 if wt == "q8_0" else vk.FP16
     w = O.synth_q8_0(72, 1, N, K, 0.0, 0.05) if wt == "q8_0" else O.synth_f16(72, 1, N * K, 0.0, 0.05)

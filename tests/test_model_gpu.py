@@ -113,6 +113,22 @@ def test_small_model_logits_prefill_then_decode(dev):
         assert_close(gv[:, :17], om.vcache(l)[:, :17], tol=5e-3, what="vcache layer %d" % l)
 
 
+@pytest.mark.parametrize("weights", ["q8_0", "fp16"])
+@pytest.mark.parametrize("P", [24, 47, 57])
+def test_few_row_projections_in_a_block(dev, weights, P):
+    """9 to 64 rows through a whole model that is wide enough for the few-row kernel (1.6 million weights in the smallest
+    projection, 5 below 33 rows): three matrices, gate and up, and both projections that add to the stream. FP16: widths that the
+    tensor-core GEMM does not take."""
+    dims = dict(dim=2336, heads=73) if weights == "fp16" else dict(dim=2304, heads=18)
+    om, dm, cfg = (fp16_pair if weights == "fp16" else small_pair)(dev, seed=24, ffn=2400, vocab=100, layers=2, maxlen=64, **dims)
+    prompt = O.synth_tokens(24, 1000 + P, P, cfg["vocab"])
+    assert np.abs(dm(prompt, 0) - om.forward(prompt, 0)).max() <= LOGITS_MAX_ABS
+    for l in range(2):  # the second block's keys and values hold what the first one's projections added
+        gk, gv = dm.read_kv(l)
+        assert_close(gk[:, :P], om.kcache(l)[:, :P], tol=5e-3, what="kcache layer %d" % l)
+        assert_close(gv[:, :P], om.vcache(l)[:, :P], tol=5e-3, what="vcache layer %d" % l)
+
+
 @pytest.mark.parametrize("P", [128, 129, 300])
 def test_q8_0_prompts_around_the_widened_weights_limit(dev, P):
     """129 tokens and more: the GEMMs' weights are turned into fp16 first. Row tiles of a matrix that end inside a 128-row half

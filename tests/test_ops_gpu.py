@@ -209,11 +209,7 @@ def test_feed_forward_q8_0(dev, M, dim, hidden):
     assert_close(got, want, what="feed_forward")
 
 
-# Many rows: gate and up share a tensor-core tile and meet in its epilogue. Hidden sizes that end inside a half tile, rows
-# around the row tiles of one CTA (128) and of a pair of CTAs (256).
-@pytest.mark.parametrize("wt", ["f16", "q8_0"])
-@pytest.mark.parametrize("M,dim,hidden", [(65, 128, 64), (127, 64, 192), (129, 192, 320), (257, 64, 448), (300, 128, 1088)])
-def test_feed_forward_many_rows(dev, wt, M, dim, hidden):
+def feed_forward_check(dev, wt, M, dim, hidden):
     dt = vk.FP16 if wt == "f16" else vk.Q8_0
     if wt == "f16":
         ws = [O.synth_f16(57, i, n, 0.0, 0.05) for i, n in ((1, hidden * dim), (2, dim * hidden), (3, hidden * dim))]
@@ -232,10 +228,22 @@ def test_feed_forward_many_rows(dev, wt, M, dim, hidden):
     assert_close(got, want, what="feed_forward %s M=%d" % (wt, M))
 
 
-# 9 to 64 rows: K chunks that end inside a stage, tiles and rows that end inside a CTA's share, one and several CTAs' worth of
-# rows, inputs that the bulk copies do not take (K not in whole blocks), more than one pass of 64 rows.
+# Many rows: gate and up share a tensor-core tile and meet in its epilogue. Hidden sizes that end inside a half tile, rows
+# around the row tiles of one CTA (128) and of a pair of CTAs (256).
 @pytest.mark.parametrize("wt", ["f16", "q8_0"])
-@pytest.mark.parametrize("M,N,K", [(9, 24, 32), (16, 48, 160), (17, 100, 416), (31, 5000, 256), (33, 72, 4128), (48, 130, 96), (63, 264, 1056), (45, 40, 72), (77, 40, 96)])
+@pytest.mark.parametrize("M,dim,hidden", [(65, 128, 64), (127, 64, 192), (129, 192, 320), (257, 64, 448), (300, 128, 1088)])
+def test_feed_forward_many_rows(dev, wt, M, dim, hidden):
+    feed_forward_check(dev, wt, M, dim, hidden)
+
+
+# 9 to 64 rows. Small matrices, and inputs not in whole 32-column blocks (K = 72): the mat-vec kernel. From 5 million weights on (1.6
+# from 33 rows on): the few-row kernel, with both CTA shapes (64 weight rows where that gives every SM a CTA: N of 9500 and more; else
+# 32) and every number of 8-row fragments; K chunks (256 and 512 columns) that end inside a stage, tiles and rows that
+# end inside a CTA's share, more than one pass of 64 rows.
+@pytest.mark.parametrize("wt", ["f16", "q8_0"])
+@pytest.mark.parametrize("M,N,K", [(9, 24, 32), (16, 48, 160), (17, 100, 416), (31, 5000, 256), (33, 72, 4128), (48, 130, 96), (63, 264, 1056), (45, 40, 72), (77, 40, 96),
+                                   (9, 5000, 1056), (16, 1203, 4192), (17, 312, 16160), (33, 72, 22560), (48, 1650, 992), (63, 264, 6176), (77, 1650, 992),
+                                   (9, 9620, 544), (31, 9620, 544), (40, 9620, 288), (64, 9500, 288)])
 def test_matmul_few_rows(dev, wt, M, N, K):
     dt = vk.FP16 if wt == "f16" else vk.Q8_0
     x = O.synth_f16(167, 1, M * K).reshape(M, K)
@@ -251,6 +259,13 @@ def test_matmul_few_rows(dev, wt, M, N, K):
     else:
         want = O.matmul_q8_0(x, w, M, N, K, 1.25, 0.5)
     assert_close(got, want, tol=2e-3, what="matmul %s %dx%dx%d" % (wt, M, N, K))
+
+
+# Gate and up by the few-row kernel: a pair of tiles per warp, both CTA shapes, hidden sizes that end inside a tile.
+@pytest.mark.parametrize("wt,M,dim,hidden", [("q8_0", 17, 96, 100), ("q8_0", 40, 288, 4744), ("q8_0", 63, 1056, 72), ("q8_0", 20, 96, 4740), ("q8_0", 57, 96, 4740),
+                                             ("f16", 17, 96, 104), ("f16", 33, 544, 72), ("f16", 9, 2080, 4840), ("f16", 63, 96, 4744)])
+def test_feed_forward_few_rows(dev, wt, M, dim, hidden):
+    feed_forward_check(dev, wt, M, dim, hidden)
 
 
 # ---- RMSNorm (tests/test_rmsnorm.cpp:100-105: [1,1,128]; 7B rows) -------------
@@ -578,6 +593,26 @@ def test_multiheadattention_many_rows(dev, T, offset, maxlen):
         cmd.end()
         cmd.submit_and_wait()
     assert_close(got, want, what="mha T=%d offset=%d maxlen=%d" % (T, offset, maxlen))
+
+
+# Q8_0 weights: keys, queries and values as one launch of three matrices of the few-row kernel (832 x 832: 2 million weights).
+@pytest.mark.parametrize("T", [33, 57])
+def test_multiheadattention_few_rows(dev, T):
+    heads, dim, maxlen = 13, 64, 64
+    Wd = heads * dim
+    ws = [O.synth_q8_0(168, i, Wd, Wd, 0.0, 0.05) for i in range(4)]
+    att = O.lib().orc_attn_create(heads, dim, maxlen)
+    x, want = O.synth_f16(168, 9, T * Wd).reshape(T, Wd), np.empty(T * Wd, np.uint16)
+    O.lib().orc_attn_forward_q8_0(att, x, ws[0], ws[1], ws[2], ws[3], T, 0, 0, want)
+    O.lib().orc_attn_destroy(att)
+    cmd = vk.Command(dev)
+    cmd.begin()
+    tw = [up(cmd, dev, w, vk.Q8_0, 1, Wd, Wd) for w in ws]
+    op = vk.MultiHeadAttentionV2(dev, cmd, tw[0], tw[1], tw[2], tw[3], maxlen, dim, True, vk.FP16, True, False).init()
+    got = cmd.download(op(up(cmd, dev, x, vk.FP16, 1, T, Wd), 0))
+    cmd.end()
+    cmd.submit_and_wait()
+    assert_close(got, want, what="mha T=%d" % T)
 
 
 # FP16 weights: 32 rows and more take the tensor-core GEMM (three matrices in one launch), fewer the mat-vec kernel. The
