@@ -10,7 +10,7 @@
 // ordered asynchronous copies, turn every code into the fp16 value fp16(q * d) and store it where a
 // 128-byte-swizzled tensor copy would have put it, so the MMA loop is the same as for FP16 weights.
 // q * d has up to 19 significant bits: this path rounds every weight once to fp16 (relative 2^-12), where
-// the reference multiplies in fp32; the rows-at-a-time kernel (matvec.cu) keeps the exact form and is used
+// the reference multiplies in fp32; the mma.sync kernels (skinny_gemm.cuh, matvec.cu) keep the exact form and run
 // below GEMM_Q8_MIN_ROWS rows.
 //
 // Long prompts of 16-bit weights go to pairs of CTAs where pick_tile finds them faster (gemm_pair.cu). Here one CTA computes
@@ -468,6 +468,7 @@ __global__ void __launch_bounds__(256) widen_kernel(const uint8_t *__restrict__ 
 // A 128-row tile dequantises the whole matrix for itself, at the pace of its dequantising warps (0.67 us per K step of 128
 // columns); widened once, the matrix runs on the fp16 GEMM's tiles. A prompt through four 7B blocks, us, dequantised in the tiles /
 // widened: 128 rows 989 / 1139, 129 1361 / 1186, 256 1387 / 1207, 257 1613 / 1302, 509 2046 / 1385, 900 3386 / 1816, 2048 6639 / 3102.
+// Only vkl_model keeps the room (GemmParams::wide); the operator classes dequantise in the tiles at any number of rows.
 constexpr uint32_t kWideRows = 129;
 bool gemm_q8_wide(uint32_t M) {
   static const uint32_t rows = [] { const char *e = getenv("VKLLAMA_Q8_WIDE"); return e ? (uint32_t)atoi(e) : kWideRows; }();  // experiments

@@ -317,7 +317,7 @@ struct GemmParams {
   const __half *w[3];         // [N,K] row-major (a transposed-weight matrix of the reference); FP16 weights
   const uint8_t *w_codes[3];  // Q8_0 weights [N,K] as tiled planes (common.cuh): codes ...
   const uint8_t *w_scales[3]; // ... and scales
-  __half *wide;               // Q8_0: room for the nmat matrices in fp16 (gemm_q8_wide), or null
+  __half *wide;               // Q8_0: room for the nmat matrices in fp16 (gemm_q8_wide), or null (operators; a device without room)
   __half *c[3];               // [M,N] fp16 output, or nullptr when c_f32 is set
   uint32_t nmat;
   int swiglu;                 // c[0] = fp16(silu(gate) * up) of the fp32 products with w[0] (gate) and w[1] (up): the
@@ -331,11 +331,11 @@ struct GemmParams {
 };
 // The same by pairs of CTAs (gemm_pair.cu); bn: columns of W per tile, 128 or 256. Operands as checked by the caller.
 cudaError_t launch_gemm_pair_f16(const GemmParams &p, int bn, cudaStream_t s);
-constexpr uint32_t GEMM_MIN_ROWS = 32;  // below this the weight-streaming mat-vec kernel is used
+constexpr uint32_t GEMM_MIN_ROWS = 32;  // below this launch_matvec (skinny_gemm.cuh or the mat-vec kernel)
 bool gemm_tcgen05_supported(uint32_t M, uint32_t N, uint32_t K);
 cudaError_t launch_gemm_f16_tcgen05(const GemmParams &p, cudaStream_t s);
 // The same GEMM with Q8_0 weights (w_codes / w_scales), dequantised into the shared-memory tiles.
-constexpr uint32_t GEMM_Q8_MIN_ROWS = 64;  // below this the rows-at-a-time kernel keeps the exact fp32 scaling
+constexpr uint32_t GEMM_Q8_MIN_ROWS = 64;  // below this launch_matvec, whose kernels keep the exact fp32 scaling
 cudaError_t launch_gemm_q8_tcgen05(const GemmParams &p, cudaStream_t s);
 // Whether the Q8_0 matrices are turned into fp16 once, in GemmParams::wide, and multiplied as such.
 bool gemm_q8_wide(uint32_t M);

@@ -1,5 +1,5 @@
 // Weight-streaming mat-vec: Y[M,N] = epilogue(X[M,K] . W[N,K]^T), one row or few
-// (more than 8 rows go to skinny_gemm.cu where its alignment rules allow)
+// (more than 8 rows of larger matrices go to skinny_gemm.cu: skinny_gemm_takes)
 // for Q8_0 weights (fused dequantisation) and FP16 weights.
 //
 // Replaces the reference's four weight shaders
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kThreads) mv_kernel(const MvParams p) {
     if (p.use_pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float ssum[kWarps];
     // whole 16-byte pieces where the rows have them: every CTA goes through the row before its first product (FP16 decode of the 7B
-    // shape: the norm + projection kernels took 30.1 and 33.2 us element by element, 29.3 and 33.3 this way, the lm head 52.8 and 48.2)
+    // shape, us, element by element / this way: the lm head 52.8 / 48.2, norm + QKV 30.1 / 29.3; norm + gate and up, 33.2 / 33.3, does not gain)
     const bool vec = !((p.K | p.x_ld) & 7) && !((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.norm_w)) & 15);
     for (uint32_t m = 0; m < p.M; ++m) {
       const __half *xr = p.x + (size_t)m * p.x_ld;

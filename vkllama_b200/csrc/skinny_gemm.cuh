@@ -10,7 +10,8 @@
 // weights) by TMA tensor copies, Q8_0 planes by bulk copies, a few large ones per chunk, since issuing a copy takes a
 // warp some 60 cycles (a copy per row of X was twice as slow as the mat-vec kernel). Sixteen warps: each takes a pair of 16-row
 // tiles (with SwiGLU a gate and an up tile) and one 32-column block of the chunk, so that an X fragment serves two
-// tiles. The warps' K shares are added in a fixed order at the end.
+// tiles. The warps' K shares are added in a fixed order at the end. 64 to 128 registers; at the cap of 128 (one CTA per SM) some of those of 33 rows and more
+// spill 8 to 52 bytes.
 //
 // Included by skinny_gemm.cu (Q8_0, and the rule) and skinny_gemm_f16.cu. In one file the 48 kernels with their line tables were 10 MB, from which
 // size on nvcc compresses device code: a process's first launch took 9.3 ms to unpack and load them, 3.2 (Q8_0) and 3.6 ms (FP16) now.
