@@ -673,13 +673,7 @@ def test_multiheadattention_f16_portions_agree(dev, T):
     assert_close(whole, got, tol=4e-3, what="mha fp16 T=%d" % T)
 
 
-# A cache that is split over CTAs: few rows behind a long history, in tiles (32 rows and more), row by row, the clipped
-# last row, and across the end of the ring; parts that a query row does not see, a last part of one column.
-@pytest.mark.parametrize("T,offset,maxlen,dim,clip", [(33, 700, 1024, 128, False), (70, 450, 512, 64, False), (64, 193, 257, 128, False),
-                                                     (45, 700, 1024, 64, True), (2, 511, 513, 128, False), (31, 300, 512, 64, False),
-                                                     (1, 64, 128, 128, False), (1, 511, 1024, 128, True)])
-def test_multiheadattention_split_cache(dev, T, offset, maxlen, dim, clip):
-    heads = 2
+def split_cache_check(dev, heads, T, offset, maxlen, dim, clip):
     Wd = heads * dim
     ws = [O.synth_q8_0(163, i, Wd, Wd, 0.0, 0.05) for i in range(4)]  # wk, wq, wv, wo
     att = O.lib().orc_attn_create(heads, dim, maxlen)
@@ -700,6 +694,23 @@ def test_multiheadattention_split_cache(dev, T, offset, maxlen, dim, clip):
         cmd.submit_and_wait()
         assert_close(got, want, what="mha T=%d offset=%d maxlen=%d clip=%s" % (t, off, maxlen, clip))
     O.lib().orc_attn_destroy(att)
+
+
+# A cache that is split over CTAs: few rows behind a long history, in tiles (32 rows and more), row by row, the clipped
+# last row, and across the end of the ring; parts that a query row does not see, a last part of one column.
+@pytest.mark.parametrize("T,offset,maxlen,dim,clip", [(33, 700, 1024, 128, False), (70, 450, 512, 64, False), (64, 193, 257, 128, False),
+                                                     (45, 700, 1024, 64, True), (2, 511, 513, 128, False), (31, 300, 512, 64, False),
+                                                     (1, 64, 128, 128, False), (1, 511, 1024, 128, True)])
+def test_multiheadattention_split_cache(dev, T, offset, maxlen, dim, clip):
+    split_cache_check(dev, 2, T, offset, maxlen, dim, clip)
+
+
+# Row by row: up to 128 columns are one part (in a cache that is no longer than that, too), then parts of 64 and more; a last
+# part of one column, rows on both sides of the limit; from 2 rows x heads per SM on (310 on 148) one part up to 512 columns, then four.
+@pytest.mark.parametrize("heads,T,offset,maxlen,dim,clip", [(2, 1, 127, 128, 64, False), (2, 1, 128, 129, 128, False), (3, 1, 192, 256, 32, False), (3, 7, 124, 300, 40, False),
+                                                           (2, 20, 107, 128, 128, False), (10, 31, 700, 736, 64, False), (10, 31, 497, 640, 32, False), (2, 40, 100, 160, 64, True), (2, 31, 250, 257, 128, False)])
+def test_multiheadattention_parts_of_a_row(dev, heads, T, offset, maxlen, dim, clip):
+    split_cache_check(dev, heads, T, offset, maxlen, dim, clip)
 
 
 # ---- device memory pool -----------------------------------------------------------------------

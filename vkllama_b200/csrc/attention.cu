@@ -21,6 +21,7 @@ namespace vkl {
 namespace {
 
 constexpr int kAttnThreads = 128;
+constexpr uint32_t kMostSplits = 8;  // parts of a cache
 
 __device__ __forceinline__ void rope_pair(float x0, float x1, float c, float s, __half &o0,
                                           __half &o1) {
@@ -58,6 +59,17 @@ __global__ void __launch_bounds__(256) rope_append_kernel(const AttnParams p) {
   *reinterpret_cast<uint4 *>(p.vcache + dst) = v;
 }
 
+// Columns of a part of a cache of which a row sees `vis`. A short cache is one part, since the parts' merge costs 2 us (32 heads, one row of
+// 65 columns, us: one part 6.7, two 9.5; of 101 8.5, 9.7), up to 128 columns where CTAs are few and up to 512 where they fill the SMs without
+// parts (31 rows of up to 231: 33.5, four parts 35.2; 40 heads x 64 24.6, 33.3). Beyond, a part has 64 columns at least (12 rows, 16 heads,
+// 212 columns: four of 64 13.2, seven of 32 16.7).
+__host__ __device__ __forceinline__ uint32_t whole_columns(uint32_t splits) { return splits == kMostSplits ? 128 : 512; }
+__device__ __forceinline__ uint32_t part_columns(uint32_t vis, uint32_t splits) {
+  const uint32_t whole = whole_columns(splits);
+  if (vis <= whole) return whole;
+  return max(((vis + splits - 1) / splits + 31) & ~31u, 64u);
+}
+
 // grid (heads, T, splits), 128 threads. FUSED: T == 1, the CTA whose column
 // range holds the new position rotates k, uses it and writes both cache rows.
 template <bool FUSED>
@@ -74,13 +86,8 @@ __global__ void __launch_bounds__(kAttnThreads) attention_kernel(const AttnParam
   const uint32_t pos0 = *p.pos_dev;
   const uint32_t L = min(pos0 + p.T, p.maxlen);
   const uint32_t vis = min(L, m + (L - p.T) + 1);  // causal: col <= row + (W - H)
-  // a split holds 64 columns or more: a short cache is not spread over CTAs whose parts cost more to merge (one row,
-  // up to 49 columns: 11.8 us in eight splits of at most 32 columns, 7.5 in one)
-  uint32_t splits = min(p.splits, (vis + 63) / 64);
-  uint32_t chunk = (vis + splits - 1) / splits;
-  chunk = (chunk + 31) & ~31u;
-  splits = (vis + chunk - 1) / chunk;
-  if (split >= splits) {
+  const uint32_t chunk = part_columns(vis, p.splits);
+  if (split * chunk >= vis) {
     if (p.use_pdl) asm volatile("griddepcontrol.launch_dependents;");
     return;
   }
@@ -200,7 +207,7 @@ __global__ void __launch_bounds__(kAttnThreads) attention_kernel(const AttnParam
   if (p.use_pdl) asm volatile("griddepcontrol.launch_dependents;");
 
   __half *orow = p.out + (p.clip ? (size_t)h * D : row_in);
-  if (splits == 1) {
+  if (chunk >= vis) {
     if (grp == 0 && dp < npair) {
       orow[2 * dp] = __float2half_rn(acc.x / lloc);
       orow[2 * dp + 1] = __float2half_rn(acc.y / lloc);
@@ -218,38 +225,52 @@ __global__ void __launch_bounds__(kAttnThreads) attention_kernel(const AttnParam
     part[D] = mloc;
     part[D + 1] = lloc;
   }
+  const uint32_t parts = (vis + chunk - 1) / chunk;
   __threadfence();
   __syncthreads();
   __shared__ uint32_t s_last;
-  if (tid == 0) s_last = atomicAdd(&p.counters[unit], 1u) == splits - 1;
+  if (tid == 0) s_last = atomicAdd(&p.counters[unit], 1u) == parts - 1;
   __syncthreads();
   if (!s_last) return;
   __threadfence();
   const float *base = p.scratch + unit * p.splits * (D + 2);
-  float M = -INFINITY;
-  for (uint32_t s = 0; s < splits; ++s) M = fmaxf(M, __ldcg(base + s * (D + 2) + D));
-  float den = 0.f;
-  for (uint32_t s = 0; s < splits; ++s) {
-    const float ms = __ldcg(base + s * (D + 2) + D), ls = __ldcg(base + s * (D + 2) + D + 1);
-    if (ls > 0.f) den += ls * expf(ms - M);
-  }
   for (uint32_t d = tid; d < D; d += kAttnThreads) {
-    float num = 0.f;
-    for (uint32_t s = 0; s < splits; ++s) {
-      const float ms = __ldcg(base + s * (D + 2) + D), ls = __ldcg(base + s * (D + 2) + D + 1);
-      if (ls > 0.f) num += __ldcg(base + s * (D + 2) + d) * expf(ms - M);
+    float M = -INFINITY, den = 0.f, num = 0.f;
+#pragma unroll 1
+    for (uint32_t s0 = 0; s0 < parts; s0 += 4) {  // four parts' loads in flight together
+      float ms[4], ls[4], v[4], m = M;
+#pragma unroll
+      for (uint32_t s = 0; s < 4; ++s) {
+        const float *part = base + (s0 + s) * (D + 2);
+        const bool here = s0 + s < parts;
+        ms[s] = here ? __ldcg(part + D) : -INFINITY;
+        ls[s] = here ? __ldcg(part + D + 1) : 0.f;
+        v[s] = here ? __ldcg(part + d) : 0.f;
+      }
+#pragma unroll
+      for (uint32_t s = 0; s < 4; ++s) m = fmaxf(m, ms[s]);
+      const float keep = M == m ? 1.f : expf(M - m);
+      den *= keep;
+      num *= keep;
+      M = m;
+#pragma unroll
+      for (uint32_t s = 0; s < 4; ++s) {
+        if (ls[s] > 0.f) {
+          const float w = expf(ms[s] - M);
+          den += ls[s] * w;
+          num += v[s] * w;
+        }
+      }
     }
     orow[d] = __float2half_rn(num / den);
   }
   if (tid == 0) p.counters[unit] = 0;
 }
 
-size_t attn_smem(const AttnParams &p) {
-  uint32_t chunk = (p.maxlen + p.splits - 1) / p.splits;
-  chunk = ((chunk + 31) & ~31u) + 32;
+size_t attn_smem(const AttnParams &p) {  // scores of the longest part
+  const uint32_t chunk = std::max(((p.maxlen + p.splits - 1) / p.splits + 31) & ~31u, std::min(whole_columns(p.splits), p.maxlen));
   return (size_t)(4 * p.dim + 8 + chunk) * sizeof(float);
 }
-
 
 // ---- multi-token calls with many rows: 64 query rows of one head per CTA ----------------------
 // The per-row kernel above re-reads the head's K and V rows for every query row. This one stages
@@ -286,7 +307,6 @@ __device__ __forceinline__ void ldm4t(uint32_t (&r)[4], const __half *p) {
 }
 
 constexpr uint32_t kSplitTiles = 2;   // a split of the tile kernel holds at least this many 64-row cache tiles
-constexpr uint32_t kMostSplits = 8;
 constexpr float kLog2e = 1.4426950408889634f;
 
 template <int D>
@@ -481,6 +501,7 @@ __global__ void __launch_bounds__(128, 3) attention_tile_kernel(const AttnParams
 }
 
 constexpr uint32_t kTileMinRows = 32;  // below this the per-row kernel is used
+constexpr uint32_t kMostUnits = 16;    // rows x heads per SM up to which a row's cache is split
 
 bool use_tiles(uint32_t T, bool clip, uint32_t dim) {
   static const bool off = [] { const char *e = getenv("VKLLAMA_PREFILL_ATTENTION"); return e && !strcmp(e, "rows"); }();
@@ -489,13 +510,16 @@ bool use_tiles(uint32_t T, bool clip, uint32_t dim) {
 
 }  // namespace
 
-// Parts that a cache is split into. The last row of 2048 (32 heads) took 136 us in one part per head and 28 in eight. Tiles: up to three CTAs per SM; rows (128 threads each): four per SM, and eight splits
-// for a single row, as in decode. The kernels use fewer where the cache is short.
+// Parts that a cache is split into at most; a kernel uses fewer where the cache is short. Tiles: up to three CTAs per SM. Rows (128
+// threads each, a serial walk over the part): eight, as in decode, while that is up to 16 CTAs per SM, else four, whose idle CTAs cost less
+// on short caches. us in one / four / eight parts: 32 heads x 128, the last row of 2048 129 / 46 / 33; 3 rows behind 2000 96 / 40 / 36;
+// 31 rows behind 700 97 / 83 / 83, behind nothing 7.9 / 8.1 / 8.3; 40 heads, 31 rows behind nothing 8.5 / 8.8 / 10.3.
 AttnPlan attention_plan(uint32_t T, bool clip, uint32_t heads, uint32_t dim, uint32_t sms) {
   AttnPlan a = {};
   const bool tiles = use_tiles(T, clip, dim);
-  const uint32_t rows = tiles ? (T + 63) / 64 : clip ? 1 : T, units = rows * heads, fit = (tiles ? 3 : 4) * sms / units;
-  a.splits = rows == 1 && !tiles ? kMostSplits : fit < 1 ? 1 : fit > kMostSplits ? kMostSplits : fit;
+  const uint32_t rows = tiles ? (T + 63) / 64 : clip ? 1 : T, units = rows * heads;
+  if (tiles) a.splits = std::min(std::max(3 * sms / units, 1u), kMostSplits);
+  else a.splits = rows == 1 || units <= 2 * sms ? kMostSplits : units <= kMostUnits * sms ? 4 : 1;
   a.scratch_bytes = a.splits == 1 ? 0 : (size_t)units * a.splits * (tiles ? 64 * (dim + 8) : dim + 2) * sizeof(float);
   a.counters = units;
   return a;
@@ -503,11 +527,12 @@ AttnPlan attention_plan(uint32_t T, bool clip, uint32_t heads, uint32_t dim, uin
 AttnPlan attention_plan_most(uint32_t T, uint32_t heads, uint32_t dim, uint32_t sms) {
   AttnPlan a = {};
   a.splits = kMostSplits;
-  const size_t row_units = (size_t)(kMostSplits * heads > 4 * sms ? kMostSplits * heads : 4 * sms);
+  // rows: eight parts of a single one or of up to 2 * sms, four of up to kMostUnits * sms
+  const size_t row_parts = std::max({(size_t)kMostSplits * heads, (size_t)kMostSplits * 2 * sms, T > 1 ? (size_t)4 * kMostUnits * sms : 0});
   const size_t tile_units = std::min((size_t)3 * sms, (size_t)kMostSplits * heads * ((T + 63) / 64));
-  a.scratch_bytes = row_units * (dim + 2) * sizeof(float);
+  a.scratch_bytes = row_parts * (dim + 2) * sizeof(float);
   if (T >= kTileMinRows && a.scratch_bytes < tile_units * 64 * (dim + 8) * sizeof(float)) a.scratch_bytes = tile_units * 64 * (dim + 8) * sizeof(float);
-  a.counters = heads > 4 * sms ? heads : 4 * sms;
+  a.counters = std::max(heads, kMostUnits * sms);
   return a;
 }
 
