@@ -79,7 +79,7 @@ int ensure_rows(vkl_model *m, uint32_t T) {
   return VKL_OK;
 }
 
-MvParams mv(vkl_model *m, const vkl_tensor *w, const __half *x, __half *out, uint32_t M) {
+MvParams mv(const vkl_model *m, const vkl_tensor *w, const __half *x, __half *out, uint32_t M) {
   MvParams p = {};
   p.codes[0] = w->data();
   p.scales[0] = q8(m) ? w->scales() : nullptr;
@@ -94,11 +94,15 @@ MvParams mv(vkl_model *m, const vkl_tensor *w, const __half *x, __half *out, uin
   p.scale = 1.f;
   p.fp16_weights = !q8(m);
   p.use_pdl = 0;
-  if (M > 8) {  // a kernel with bounded waits
+  return p;
+}
+// With the error word where the launch has bounded waits: reading it back costs a call 4 us.
+cudaError_t run_mv(vkl_model *m, MvParams &p, int epilogue, bool fuse_norm, cudaStream_t s) {
+  if (!fuse_norm && matvec_waits(p, epilogue)) {
     p.error = (uint32_t *)m->state->data() + 6;
     m->gemm_used = true;
   }
-  return p;
+  return launch_matvec(p, epilogue, fuse_norm, s);
 }
 
 // Many-row projection on the tcgen05 tensor cores (Q8_0 weights are dequantised into the shared-memory tiles).
@@ -181,7 +185,7 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
       p.norm_w = (const float *)y.attn_norm->data();
       p.eps = m->cfg.eps;
       p.use_pdl = pdl;
-      VKL_LAUNCH(1, launch_matvec(p, EPI_PLAIN, true, s));
+      VKL_LAUNCH(1, run_mv(m, p, EPI_PLAIN, true, s));
     } else if (use_gemm(m, T)) {
       VKL_LAUNCH(1, launch_rms_norm(x, (const float *)y.attn_norm->data(), xn, T, D, m->cfg.eps, s));
       GemmParams g = gemm(m, y.wk, xn, kb, T);
@@ -190,7 +194,7 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
       VKL_LAUNCH(gemm_launches(g), launch_gemm_tcgen05(g, s));
     } else {
       VKL_LAUNCH(1, launch_rms_norm(x, (const float *)y.attn_norm->data(), xn, T, D, m->cfg.eps, s));
-      VKL_LAUNCH((T + 63) / 64, launch_matvec(p, EPI_PLAIN, false, s));
+      VKL_LAUNCH((T + 63) / 64, run_mv(m, p, EPI_PLAIN, false, s));
     }
     MARK(1);
     AttnParams a = {};
@@ -222,7 +226,7 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
       MvParams o = mv(m, y.wo, ao, xr, rows);
       o.residual = xr;
       o.use_pdl = dec && pdl;
-      VKL_LAUNCH((rows + 63) / 64, launch_matvec(o, EPI_ADD, false, s));
+      VKL_LAUNCH((rows + 63) / 64, run_mv(m, o, EPI_ADD, false, s));
     }
     MARK(3);
     // --- feed forward --------------------------------------------------------
@@ -233,7 +237,7 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
       f.norm_w = (const float *)y.ffn_norm->data();
       f.eps = m->cfg.eps;
       f.use_pdl = dec && pdl;
-      VKL_LAUNCH(1, launch_matvec(f, EPI_SWIGLU, true, s));
+      VKL_LAUNCH(1, run_mv(m, f, EPI_SWIGLU, true, s));
     } else if (use_gemm(m, rows)) {
       VKL_LAUNCH(1, launch_rms_norm(xr, (const float *)y.ffn_norm->data(), xn, rows, D, m->cfg.eps, s));
       GemmParams g = gemm(m, y.gate, xn, tb, rows);
@@ -242,7 +246,7 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
       VKL_LAUNCH(gemm_launches(g), launch_gemm_tcgen05(g, s));
     } else {
       VKL_LAUNCH(1, launch_rms_norm(xr, (const float *)y.ffn_norm->data(), xn, rows, D, m->cfg.eps, s));
-      VKL_LAUNCH((rows + 63) / 64, launch_matvec(f, EPI_SWIGLU, false, s));
+      VKL_LAUNCH((rows + 63) / 64, run_mv(m, f, EPI_SWIGLU, false, s));
     }
     MARK(4);
     if (sharded) {
@@ -255,7 +259,7 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
       MvParams d = mv(m, y.down, tb, xr, rows);
       d.residual = xr;
       d.use_pdl = dec && pdl;
-      VKL_LAUNCH((rows + 63) / 64, launch_matvec(d, EPI_ADD, false, s));
+      VKL_LAUNCH((rows + 63) / 64, run_mv(m, d, EPI_ADD, false, s));
     }
     MARK(5);
   }
@@ -267,7 +271,7 @@ int run_tokens(vkl_model *m, uint32_t T, bool pdl, Marker *mk = nullptr, bool fi
   h.eps = m->cfg.final_eps;
   h.out_f32 = (float *)m->logits32->data();
   h.use_pdl = dec && pdl;
-  VKL_LAUNCH(1, launch_matvec(h, EPI_PLAIN, true, s));
+  VKL_LAUNCH(1, run_mv(m, h, EPI_PLAIN, true, s));
   MARK(6);
   VKL_LAUNCH(2, launch_argop((const __half *)m->logits16->data(), m->next_dev(), m->argpart->data(), 1, m->vocab_l, 0, s));
   MARK(7);
@@ -1294,10 +1298,10 @@ int vkl_model_block_forward(vkl_model *m, uint32_t layer, const void *x_fp16, si
   if (dec) {
     p.norm_w = (const float *)y.attn_norm->data();
     p.eps = m->cfg.eps;
-    VKL_LAUNCH(1, launch_matvec(p, EPI_PLAIN, true, s));
+    VKL_LAUNCH(1, run_mv(m, p, EPI_PLAIN, true, s));
   } else {
     VKL_LAUNCH(1, launch_rms_norm(x, (const float *)y.attn_norm->data(), xn, (uint32_t)T, (uint32_t)D, m->cfg.eps, s));
-    VKL_LAUNCH((T + 63) / 64, launch_matvec(p, EPI_PLAIN, false, s));
+    VKL_LAUNCH((T + 63) / 64, run_mv(m, p, EPI_PLAIN, false, s));
   }
   AttnParams a = {};
   a.q = (__half *)m->q->data(); a.k = (const __half *)m->k->data(); a.v = (const __half *)m->v->data();
@@ -1311,21 +1315,21 @@ int vkl_model_block_forward(vkl_model *m, uint32_t layer, const void *x_fp16, si
   VKL_LAUNCH(dec ? 1 : 2, launch_attention(a, s));
   MvParams o = mv(m, y.wo, (__half *)m->ao->data(), x, (uint32_t)T);
   o.residual = x;
-  VKL_LAUNCH((T + 63) / 64, launch_matvec(o, EPI_ADD, false, s));
+  VKL_LAUNCH((T + 63) / 64, run_mv(m, o, EPI_ADD, false, s));
   MvParams f = mv(m, y.gate, dec ? x : xn, (__half *)m->t->data(), (uint32_t)T);
   f.codes[1] = y.up->data();
   if (q8(m)) f.scales[1] = y.up->scales();
   if (dec) {
     f.norm_w = (const float *)y.ffn_norm->data();
     f.eps = m->cfg.eps;
-    VKL_LAUNCH(1, launch_matvec(f, EPI_SWIGLU, true, s));
+    VKL_LAUNCH(1, run_mv(m, f, EPI_SWIGLU, true, s));
   } else {
     VKL_LAUNCH(1, launch_rms_norm(x, (const float *)y.ffn_norm->data(), xn, (uint32_t)T, (uint32_t)D, m->cfg.eps, s));
-    VKL_LAUNCH((T + 63) / 64, launch_matvec(f, EPI_SWIGLU, false, s));
+    VKL_LAUNCH((T + 63) / 64, run_mv(m, f, EPI_SWIGLU, false, s));
   }
   MvParams d = mv(m, y.down, (__half *)m->t->data(), x, (uint32_t)T);
   d.residual = x;
-  VKL_LAUNCH((T + 63) / 64, launch_matvec(d, EPI_ADD, false, s));
+  VKL_LAUNCH((T + 63) / 64, run_mv(m, d, EPI_ADD, false, s));
   VKL_OKAY(queue_errors(m, false));  // more than 8 rows: the projections' kernels have bounded waits
   VKL_CUDA(cudaMemcpyAsync(out_fp16, x, T * D * 2, cudaMemcpyDeviceToHost, s));
   VKL_CUDA(cudaStreamSynchronize(s));
