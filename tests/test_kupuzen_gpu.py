@@ -184,6 +184,17 @@ def test_32bit_products_at_the_edges_of_row_tiles(dev, ff):
     m.close()
 
 
+def test_bf16_products_in_several_tiles_per_pair_of_ctas(dev):
+    """1090 rows x 12032 gate and up columns: 235 tiles of 256 x 256 for 74 pairs of CTAs, 7 K steps in a ring of 6 stages."""
+    case = U.config([(U.attn(2, 1, 32, 32, 400, 8), 6016)], width=448, vocab=60)
+    W, toks = U.weights(case, 71), U.tokens(case[0], 1090, 72)
+    want = D.run(case[0], W, toks)
+    m = load(dev, case, W, 1100, "bfloat16")
+    got = m.forward_rows(toks, 0, np.arange(1090))
+    m.close()
+    assert U.rel_err(got, want) < U.REL["bfloat16"]  # of the worst row
+
+
 def test_a_stream_too_wide_for_the_norm_inside_the_decode_projection(dev):
     case = U.config([(U.attn(2, 1, 32, 32, 9, 8), 24), (U.delta(2, 1, 32, 16, 4, (5, 5)), 16)], width=6016, vocab=40)
     W, toks = U.weights(case, 67), U.tokens(case[0], 30, 68)

@@ -240,6 +240,28 @@ def test_feed_forward_many_rows(dev, wt, M, dim, hidden):
     feed_forward_check(dev, wt, M, dim, hidden)
 
 
+# Pairs of CTAs that run several tiles each (74 pairs on 148 SMs): 240 tiles of 256 x 256 with 7 K steps in a ring of 6 stages, 150 of
+# 256 x 128 with 17 in a ring of 8; so an accumulator is given back and filled again, and the ring's phases carry over from tile to
+# tile. Rows and columns that end inside a tile.
+@pytest.mark.parametrize("M,N,K", [(1090, 12040, 448), (500, 9592, 1088)])
+def test_matmul_f16_several_tiles_per_pair(dev, M, N, K):
+    x, w = O.synth_f16(169, 1, M * K).reshape(M, K), O.synth_f16(169, 2, N * K, 0.0, 0.05)
+    cmd = vk.Command(dev)
+    cmd.begin()
+    op = vk.MatMul(dev, cmd, up(cmd, dev, w, vk.FP16, 1, N, K), 1.25, 0.5, 0, 0, True, vk.FP16, vk.FP16).init()
+    got = cmd.download(op(up(cmd, dev, x, vk.FP16, 1, M, K)))
+    cmd.end()
+    cmd.submit_and_wait()
+    want = O.f16(x).astype(np.float64) @ O.f16(w).astype(np.float64).reshape(N, K).T * 1.25 + 0.5
+    err = np.abs(O.f16(got).reshape(M, N) - want).max(1) / np.abs(want).max()  # every row: a wrong tile is wrong in some
+    assert err.max() <= 1e-3, err.max()  # half a step of fp16 at the largest values is 2.4e-4 to 4.9e-4 of them
+
+
+def test_feed_forward_several_tiles_per_pair(dev):
+    """Gate and up by pairs: 240 tiles of 256 rows x 128 gate and 128 up columns."""
+    feed_forward_check(dev, "f16", 1090, 448, 6016)
+
+
 # 9 to 64 rows. Small matrices, and inputs not in whole 32-column blocks (K = 72): the mat-vec kernel. From 5 million weights on (1.6
 # from 33 rows on): the few-row kernel, with both CTA shapes (64 weight rows where that gives every SM a CTA: N of 9500 and more; else
 # 32) and every number of 8-row fragments; K chunks (256 and 512 columns) that end inside a stage, tiles and rows that
@@ -402,6 +424,28 @@ def test_argmax_ties_pick_lowest_index(dev):
     cmd.end()
     cmd.submit_and_wait()
     assert got.ravel().tolist() == [77, 0, 1023]
+
+
+@pytest.mark.parametrize("op_type", [0, 1])
+def test_argop_chunks_of_nan_and_ties_between_chunks(dev, op_type):
+    """40 chunks of 1024, more than a warp has lanes. A chunk of nothing but NaN wins if it is the first one, as in a serial scan
+    with strict compares, and loses anywhere else; equal winners of two chunks: the lower index."""
+    sign, W = 1.0 if op_type == 0 else -1.0, 40 * 1024
+    x = np.zeros((1, 4, W), np.float32)
+    x[0, 0, :1024] = np.nan
+    x[0, 0, 30000] = 5 * sign
+    x[0, 1, 3 * 1024:4 * 1024] = np.nan
+    x[0, 1, 35 * 1024:36 * 1024] = np.nan
+    x[0, 1, 38000] = 7 * sign
+    x[0, 2, [2500, 36000]] = 2 * sign
+    x[0, 3, [39 * 1024, 33 * 1024 + 5]] = 2 * sign
+    cmd = vk.Command(dev)
+    cmd.begin()
+    tx = up(cmd, dev, O.bits(x), vk.FP16, 1, 4, W)
+    got = cmd.download(vk.ArgOp(dev, cmd, op_type, vk.FP16).init()(tx))
+    cmd.end()
+    cmd.submit_and_wait()
+    assert got.ravel().tolist() == [0, 38000, 2500, 33 * 1024 + 5]
 
 
 # ---- Embedding (tests/test_embedding.cpp: ids [55x19],[123x128], vocab 20000x64) --
