@@ -28,9 +28,9 @@ def words(tmp_path_factory):
 def test_model_calls_report_their_own_waits(dev, words):
     """Rows of a block whose projections gave up are not handed out as a success, and the next call is not blamed; calls whose
     kernels have no waits do not ask."""
-    dm = vk.Model(dev, 128, 2, 256, 100, 2, 64)
+    dm = vk.Model(dev, 512, 8, 1600, 100, 2, 64)
     dm.synth_weights(71)
-    x = O.synth_f16(71, 5, 40 * 128).reshape(40, 128)  # gate and up of 17 rows and more: a kernel with bounded waits
+    x = O.synth_f16(71, 5, 40 * 512).reshape(40, 512)  # gate and up of 33 rows and more, 1.6 million weights: a kernel with bounded waits
     want = dm.block_forward(0, x, 0)
     assert words.raise_model_word(dm.h) == 0
     with pytest.raises(vk.VklError) as e:
@@ -38,7 +38,7 @@ def test_model_calls_report_their_own_waits(dev, words):
     assert e.value.code == 13
     assert (dm.block_forward(0, x, 0) == want).all()
     words.raise_model_word(dm.h)
-    for T in (1, 8, 12, 16):  # no such kernel runs: the word is not asked for
+    for T in (1, 8, 12, 32):  # no such kernel runs: the word is not asked for
         dm(np.arange(T, dtype=np.uint32), 0)
     with pytest.raises(vk.VklError) as e:
         dm(np.arange(33, dtype=np.uint32), 0)

@@ -393,7 +393,7 @@ def test_chat_session_multi_token_turns_on_top_of_history(dev):
     one-token calls must interleave on one cache."""
     om, dm, cfg = small_pair(dev, seed=15)
     pos = 0
-    for turn, T in enumerate((7, 40, 3, 33)):  # 8 rows and fewer, and more (gate and up of 33 and 40: the few-row kernel)
+    for turn, T in enumerate((7, 40, 3, 33)):  # 8 rows and fewer, and more
         toks = O.synth_tokens(15, 1100 + turn, T, cfg["vocab"])
         want, got = om.forward(toks, pos), dm(toks, pos)
         assert np.abs(got - want).max() <= LOGITS_MAX_ABS, "turn %d" % turn

@@ -321,9 +321,11 @@ def test_first_few_row_call_of_a_process_is_not_held_up_by_loading(wt):
     assert min(times) < 6e-3, times
 
 
-# Gate and up by the few-row kernel: a pair of tiles per warp, both CTA shapes, hidden sizes that end inside a tile.
-@pytest.mark.parametrize("wt,M,dim,hidden", [("q8_0", 17, 96, 100), ("q8_0", 40, 288, 4744), ("q8_0", 63, 1056, 72), ("q8_0", 20, 96, 4740), ("q8_0", 57, 96, 4740),
-                                             ("f16", 17, 96, 104), ("f16", 33, 544, 72), ("f16", 9, 2080, 4840), ("f16", 63, 96, 4744)])
+# Gate and up by the few-row kernel (1.6 million weights and more from 33 rows on, 6 from 17, 20 below with FP16): a pair of tiles per warp,
+# both CTA shapes (hidden sizes of 4736 and more: 64 weight rows), hidden sizes that end inside a tile. Then small ones by the mat-vec kernel.
+@pytest.mark.parametrize("wt,M,dim,hidden", [("q8_0", 17, 4128, 740), ("q8_0", 40, 288, 4744), ("q8_0", 63, 1056, 776), ("q8_0", 20, 640, 4740), ("q8_0", 57, 192, 4740),
+                                             ("f16", 17, 4128, 744), ("f16", 33, 1056, 776), ("f16", 9, 2080, 4840), ("f16", 63, 224, 4744),
+                                             ("q8_0", 17, 96, 100), ("q8_0", 63, 1056, 72), ("f16", 17, 96, 104)])
 def test_feed_forward_few_rows(dev, wt, M, dim, hidden):
     feed_forward_check(dev, wt, M, dim, hidden)
 

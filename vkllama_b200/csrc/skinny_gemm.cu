@@ -14,6 +14,8 @@ cudaError_t launch_skinny_gemm_f16(const MvParams &p, int epilogue, cudaStream_t
 //   o   D = 512 3.4 / 4.3   1024 3.7 / 5.4   2048 5.6 / 6.9    2304 7.8 / 7.5    4096 11.6 / 10.5;  33 rows: 1024 5.6 / 6.7, 1408 8.5 / 7.4
 //   q   D = 1024 4.2 / 5.5  2048 11.0 / 12.5  2304 14.9 / 13.7  5120 47.9 / 38.0;  33 rows: 704 5.3 / 6.4, 1024 9.7 / 6.9;  FP16: 1024 4.9 / 5.7, 1408 7.0 / 6.7
 //   g   D = 704 4.9 / 5.2, 1024 8.3 / 9.3, any other 0.70 ... 0.95 of the time, 33 rows 0.44 ... 0.85;  up to 16 rows: Q8_0 up to 1.27, FP16 1664 9.5 / 11.5, 2048 16.8 / 14.9
+// Gate and up of less than 6 million weights gain 1 us here (2 from 33 rows on, to 1.6 million), and the error word, which only this kernel needs, costs
+// a call 4 us.
 // So a launch needs as many weights as the lines below say. Over the four launches of a block, widths 128 to 5120, 9 to 63 rows, that is
 // 0.38 to 1.00 of the mat-vec kernel's time (a rule by rows alone: up to 1.29 at widths 512 to 1024).
 bool skinny_gemm_takes(const MvParams &p, int epilogue) {
@@ -25,7 +27,7 @@ bool skinny_gemm_takes(const MvParams &p, int epilogue) {
   const size_t tiles = (swiglu ? 2 : p.nmat) * (size_t)((p.N + 15) / 16), weights = tiles * 16 * p.K;
   // 16 rows of Q8_0: a second wave of CTAs that is a third full is too much already (us: 402 tiles of K = 2304 9.4 / 10.2, 320 of 5120 20.9 / 16.9)
   if (!p.fp16_weights && few && (swiglu || p.nmat > 1 || 2 * tiles > 5 * sm_count())) return false;
-  if (swiglu) return few ? weights >= 20000000 : p.fp16_weights || !half || weights <= 2000000 || weights >= 6000000;
+  if (swiglu) return weights >= (few ? 20000000u : half ? 6000000u : 1600000u);
   if (p.nmat > 1) return weights >= (!half ? 2000000u : !p.fp16_weights ? 15000000u : few ? 25000000u : 5000000u);
   return weights >= (half ? 5000000u : 1600000u);
 }
