@@ -5,33 +5,38 @@
 // the weight stream at every one of them. Here the whole token is one
 // cooperative launch of one CTA per SM:
 //
-//   * a producer warp walks the static schedule of this CTA's weight tiles for
-//     ALL mat-vec ops of the token and streams them with bulk-copy TMA
-//     (cp.async.bulk + mbarrier) into a shared-memory ring, one copy per stage: what a
-//     CTA reads of an op is one consecutive range of the op's packed stream. Weights never
-//     depend on activations, so the producer runs ahead across op boundaries and HBM
-//     stays busy while the consumers sit in a norm, an attention op or a wait;
-//   * eleven consumer warps take their units (one Q8_0 block x 32 rows) of every ring
-//     stage, put the codes into the tensor cores as fp16 subnormals (exact, one byte permute
-//     per pair), multiply (m16n8k16, fp32 accumulate), apply block scales in fp32, reduce
-//     across warps in fixed order and run the fused epilogue (RMSNorm prologue, residual add,
-//     SwiGLU, fp32 logits, running arg-max). What they cost is instruction issue, not the
-//     tensor pipe (12 % busy; mma.sync m16n8k16 (f16) and m16n8k32 (s8) both issue every 8
-//     cycles per scheduler on this GPU). A warp's scheduler is warp % 4: eleven or fifteen
-//     consumer warps (+ the producer) load the four schedulers evenly, every other count is
-//     15-25 % slower; eleven (24 KB stages, seven of them, 168 registers) measured 1.5 %
-//     faster than fifteen (32 KB stages, five, 128 registers). An int8 variant on three exact
-//     byte slices of the input was 30 % slower for its integer-to-float conversions;
+//   * what a CTA reads of an op is one consecutive range of the op's packed stream, cut into equal shares, one per
+//     warp. Every warp streams its share through a ring of its own in shared memory with bulk-copy TMA
+//     (cp.async.bulk + mbarrier): as soon as it has used a piece (MEGA_SU units), its lane 0 requests the piece
+//     that takes its place, across op boundaries. Weights never depend on activations, so HBM stays busy while
+//     the warps sit in a norm, an attention op or a wait;
+//   * a unit is one Q8_0 block x 32 rows: the codes go into the tensor cores as fp16 subnormals (exact, one
+//     byte permute per pair; m16n8k16, fp32 accumulate), block scales are applied in fp32, the warps' sums of
+//     a tile are added in fixed order and the fused epilogue runs (RMSNorm prologue, residual add, SwiGLU, fp32
+//     logits, running arg-max);
 //   * activations cross CTAs as tagged words (value + sequence tag in one 32-bit word) that
 //     the readers poll; only the output layer's arg-max needs a grid barrier.
 //
 // Tiles of op i go to CTA (tile + rot_i) mod grid; rot_i advances by the op's
 // tile count so the uneven remainder rotates over the SMs.
+//
+// What bounds it: not HBM (7B: 1.45 ms per token against 1.07 at the measured copy rate) and not the tensor pipe (12 %), but
+// what a warp executes one instruction after the other: with three warps per scheduler and dependent instructions four to six
+// cycles apart, a branch costs 50 to 100 cycles of a warp's time and even an empty turn of the stream loop took 400. With no
+// weight copies at all a 7B token of the version before took 1.49 of its 1.53 ms. Hence: no producer warp and no barrier pair
+// per stage between warps (its handshake, table entry and two units per stage and warp bounded the earlier form: 1.60 ms);
+// straight-line code for whole pieces; divisions, addresses and residuals worked out before the input arrives; and little code
+// and no spills, because both come from memory behind the weight stream when they miss (150 KB of code 1.68 ms, 123 KB
+// 1.60, 80 KB 1.53 for like loops; 16 warps of 128 registers with 200 bytes of spills 1.9 to 2.0 ms).
+// Warps x units per piece, ms per token (7B) / us per call (13B shape, four blocks): 11 x 4 1.453 / 399, 11 x 5 1.482 / 399,
+// 12 x 3 1.464 / 397, 12 x 4 1.497 / 386, 12 x 5 1.477 / 385, 16 x 2 1.501 / 431, 16 x 3 1.520 / 405: 11 x 4 has the deepest
+// rings at 7B (four pieces, 191 KB).
 // Every wait is bounded; on a time-out the kernel raises *error, stops issuing
 // copies, drains the copies in flight and leaves through the normal path.
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -39,18 +44,16 @@
 namespace vkl {
 namespace {
 
-constexpr int NCW = (int)MEGA_NCW;     // consumer warps (11 + 1 producer warp = 384 threads of 168 registers)
-constexpr int CT = NCW * 32;           // consumer threads
-constexpr int THREADS = CT + 32;       // + producer warp
-constexpr int UPW = (int)MEGA_UPW;     // units (one Q8_0 block x 32 rows) per consumer warp and ring stage
-constexpr int SU = NCW * UPW;          // units per ring stage
-static_assert(SU == (int)MEGA_SU, "host and device agree on the stage size");
+constexpr int NCW = (int)MEGA_NCW;     // warps, 184 registers each
+constexpr int CT = NCW * 32;
+constexpr int THREADS = CT;
+constexpr int SU = (int)MEGA_SU;       // units per piece, the step of a warp's ring
 constexpr uint32_t UNIT_CODES = MEGA_UNIT_CODES, UNIT_SCALES = MEGA_UNIT_SCALES;
 constexpr uint32_t UNIT_BYTES = UNIT_CODES + UNIT_SCALES;  // a unit's codes, then its 32 scales
-constexpr uint32_t STAGE_BYTES = SU * UNIT_BYTES;          // 32640
-static_assert(STAGE_BYTES == MEGA_STAGE_BYTES, "host and device agree on the stage size");
+constexpr uint32_t PIECE_BYTES = SU * UNIT_BYTES;
+static_assert(PIECE_BYTES == MEGA_PIECE_BYTES, "host and device agree on the size of a piece");
 constexpr uint32_t XB_BYTES = 64;      // the input vector in shared memory: fp16, 64 bytes per block of 32 inputs
-constexpr int MAX_NST = 12;            // ring stages are a launch parameter (whatever fits), at most this many
+constexpr int MAX_NST = (int)MEGA_MAX_NST;  // a ring's pieces are a launch parameter (whatever fits), at most this many
 // Every wait of the kernel is bounded by MegaParams::wait_limit polls (about half a microsecond each): the host
 // picks the bound, the same for all waits, so that no wait gives up while another one it depends on is still
 // legitimately waiting (for a slower tensor-parallel rank, say).
@@ -89,6 +92,16 @@ __device__ __forceinline__ void st_rel_sys_u32(uint32_t *p, uint32_t v) {
   asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// Eight halves as floats.
+__device__ __forceinline__ void unpack8(const uint4 &v, float *f) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&w[e]));
+    f[2 * e] = a.x;
+    f[2 * e + 1] = a.y;
+  }
+}
 // ---- tagged activation words: fp16 value | (low 16 bits of the producing op's sequence number) << 16
 __device__ __forceinline__ uint32_t ll_pack(__half v, uint32_t tag) { return (uint32_t)__half_as_ushort(v) | (tag << 16); }
 __device__ __forceinline__ __half ll_half(uint32_t w) { return __ushort_as_half((unsigned short)(w & 0xffffu)); }
@@ -171,24 +184,12 @@ __device__ VKL_SLOW uint32_t slow_ll_wait1(volatile uint32_t *abort_s, uint32_t 
   atomicCAS(error, 0u, 6u);
   return w;
 }
-__device__ VKL_SLOW uint2 slow_ll_wait2(volatile uint32_t *abort_s, uint32_t *error, uint32_t limit, const uint32_t *src, uint32_t tag) {
-  uint2 w = make_uint2(0, 0);
-#pragma unroll 1
-  for (uint32_t i = 0; i < limit; ++i) {
-    w = ld_vol_v2(src);
-    if (((w.x >> 16) == tag) & ((w.y >> 16) == tag)) return w;
-    if ((i & 255u) == 255u && (*(volatile uint32_t *)error != 0u || *abort_s != 0)) {
-      *abort_s = 1;
-      return w;
-    }
-  }
-  *abort_s = 1;
-  atomicCAS(error, 0u, 6u);
-  return w;
-}
 __device__ __forceinline__ bool ll_ready8(const uint4 &a, const uint4 &b, uint32_t tag) {
-  return ((a.x >> 16) == tag) & ((a.y >> 16) == tag) & ((a.z >> 16) == tag) & ((a.w >> 16) == tag) & ((b.x >> 16) == tag) &
-         ((b.y >> 16) == tag) & ((b.z >> 16) == tag) & ((b.w >> 16) == tag);
+  const uint32_t t = tag << 16;
+  return (((a.x ^ t) | (a.y ^ t) | (a.z ^ t) | (a.w ^ t) | (b.x ^ t) | (b.y ^ t) | (b.z ^ t) | (b.w ^ t)) & 0xffff0000u) == 0;
+}
+__device__ __forceinline__ uint4 ll_pack8(const uint4 &a, const uint4 &b) {
+  return make_uint4(__byte_perm(a.x, a.y, 0x5410), __byte_perm(a.z, a.w, 0x5410), __byte_perm(b.x, b.y, 0x5410), __byte_perm(b.z, b.w, 0x5410));
 }
 // polls eight consecutive tagged words until all carry `tag`; the words come back through a, b
 __device__ VKL_SLOW void slow_ll_wait8(volatile uint32_t *abort_s, uint32_t *error, uint32_t limit, const uint32_t *src, uint32_t tag, uint4 &a, uint4 &b) {
@@ -217,12 +218,6 @@ struct Ctx {
     *abort_s = 1;
     atomicCAS(p.error, 0u, code);
   }
-  // Bounded mbarrier wait; false (and the abort flag set) on time-out.
-  __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, uint32_t code, uint32_t sleep_ns = 0) const {
-    if (mbar_try(bar, parity)) return true;  // fast path: the phase is already complete
-    if (aborted()) return false;
-    return slow_mbar_wait(abort_s, p.error, p.wait_limit, bar, parity, code, sleep_ns);
-  }
   // One tagged word, polled (bounded) until its tag is `tag`. Returns the word; on a time-out
   // or an abort returns what it last read (the caller's results are discarded on abort).
   __device__ __forceinline__ uint32_t ll_wait1(const uint32_t *src, uint32_t tag) const {
@@ -230,113 +225,201 @@ struct Ctx {
     if ((w >> 16) == tag) return w;
     return slow_ll_wait1(abort_s, p.error, ll_limit(), src, tag);
   }
-  // Two consecutive tagged words (8-byte aligned), already requested once.
-  __device__ __forceinline__ uint2 ll_wait2(const uint32_t *src, uint2 w, uint32_t tag) const {
-    if (((w.x >> 16) == tag) & ((w.y >> 16) == tag)) return w;
-    return slow_ll_wait2(abort_s, p.error, ll_limit(), src, tag);
-  }
-  // Eight consecutive tagged words (32-byte aligned) -> eight packed halves, polled the same way.
+  // Eight consecutive tagged words (32-byte aligned), already requested once -> eight packed halves, polled the same way.
   __device__ __forceinline__ uint4 ll_wait8(const uint32_t *src, uint4 a, uint4 b, uint32_t tag) const {
     if (!ll_ready8(a, b, tag)) slow_ll_wait8(abort_s, p.error, ll_limit(), src, tag, a, b);
-    return make_uint4((a.x & 0xffffu) | (a.y << 16), (a.z & 0xffffu) | (a.w << 16), (b.x & 0xffffu) | (b.y << 16), (b.z & 0xffffu) | (b.w << 16));
+    return ll_pack8(a, b);
+  }
+  // Up to N vectors of eight tagged words, `stride` words apart: all requested together, then those that were not there.
+  template <int N> __device__ __forceinline__ void ll_gather(const uint32_t *src, uint32_t stride, uint32_t n, uint32_t tag, uint4 (&a)[N], uint4 (&b)[N]) const {
+    uint32_t missing = n >= N ? (1u << N) - 1u : (1u << n) - 1u;
+    const uint32_t limit = ll_limit();
+#pragma unroll 1
+    for (uint32_t i = 0;; ++i) {
+#pragma unroll
+      for (int j = 0; j < N; ++j)
+        if (missing & (1u << j)) {
+          a[j] = ld_vol_v4(src + j * stride);
+          b[j] = ld_vol_v4(src + j * stride + 4);
+        }
+#pragma unroll
+      for (int j = 0; j < N; ++j)
+        if ((missing & (1u << j)) && ll_ready8(a[j], b[j], tag)) missing &= ~(1u << j);
+      if (!missing) return;
+      if (i >= limit) break;
+      if ((i & 255u) == 255u && (*(volatile uint32_t *)p.error != 0u || *abort_s != 0)) {
+        *abort_s = 1;  // give up quietly: another wait has already raised the error
+        return;
+      }
+    }
+    *abort_s = 1;
+    atomicCAS(p.error, 0u, 6u);
   }
 };
 
-// ------------------------------------------------------------------ producer
-// The producer warp walks this CTA's precomputed stage table (one entry per ring
-// stage of the whole token, in consumer order). Lane 0 keeps the shared-memory ring
-// full with bulk copies; the other lanes only fetch table chunks.
-__device__ __forceinline__ void producer(const Ctx &c, unsigned char *ring, uint64_t *full, uint64_t *empty,
-                                         MegaStage *tabs /* [128] in shared memory */) {
-  const MegaParams &p = c.p;
-  const uint32_t lane = threadIdx.x & 31;
-  const MegaStage *table = p.stages + (size_t)blockIdx.x * p.stage_stride;
-  const uint32_t n = p.stage_count[blockIdx.x];
-  const uint32_t NST = p.nst;
-  if (lane < min(n, 32u)) tabs[lane] = table[lane];
-  __syncwarp();
-  uint32_t it = 0, slot = 0, ph = 0;
-  uint32_t issued = 0;  // ring stages issued so far (table entries and stages differ: a KV entry is 0..n stages)
-  bool stop = false;
-  // this CTA's (head, split) and row range of the attention ops: the same for every layer of the token
-  const uint32_t pos0 = p.state[0];
-  const uint32_t Lnow = min(pos0 + 1, p.maxlen);
-  const uint32_t S_eff = mega_splits(Lnow, p.splits, p.split_rows);
-  uint32_t kv_c0 = 0, kv_c1 = 0;
-  if (blockIdx.x < p.heads * S_eff) mega_kv_range(Lnow, S_eff, blockIdx.x % S_eff, kv_c0, kv_c1);
-  const uint32_t kv_head = blockIdx.x / S_eff, kv_rps = mega_kv_rows_per_stage(p.head_dim);
-  for (uint32_t base = 0; base < n && !stop; base += 32) {
-    // chunk base/32 is in tabs[(base/32 % 4)*32 ..]; fetch the next one behind it. The table is a
-    // ring of four chunks because the consumers, up to a ring depth of stages behind, still read
-    // their stages' entries.
-    if (base + 32 + lane < n) tabs[((base / 32 + 1) & 3) * 32 + lane] = table[base + 32 + lane];
-    __syncwarp();
-    if (lane == 0) {
-      const uint32_t end = min(base + 32, n);
-      for (; it < end; ++it) {
-        const MegaStage &e = tabs[it & 127];
-        if (e.n0 == MEGA_KV_MARK) {
-          // K rows, then V rows, of this CTA's split of an attention op: whole cache rows,
-          // contiguous in [heads, maxlen, head_dim], up to kv_rps rows per stage
-          const uint32_t rowb = p.head_dim * 2u;
-          for (uint32_t kv = 0; kv < 2 && !stop; ++kv) {
-            const uint8_t *src = (kv ? e.src2 : e.src) + ((size_t)kv_head * p.maxlen + kv_c0) * rowb;
-            for (uint32_t r0 = kv_c0; r0 < kv_c1; r0 += kv_rps) {
-              if (issued >= NST && !(p.timing_mode & 128u) && !c.wait(s32(&empty[slot]), ph ^ 1u, 2, 0)) {
-                stop = true;
-                break;
-              }
-              const uint32_t fb = s32(&full[slot]), bytes = min(kv_rps, kv_c1 - r0) * rowb;
-              if (p.timing_mode & 2u) {
-                mbar_arrive(fb);
-              } else {
-                mbar_expect(fb, bytes);
-                bulk_g2s(s32(ring + (size_t)slot * STAGE_BYTES), src + (size_t)(r0 - kv_c0) * rowb, bytes, fb);
-              }
-              ++issued;
-              if (++slot == NST) {
-                slot = 0;
-                ph ^= 1u;
-              }
-            }
-          }
-          if (stop) break;
-          continue;
-        }
-        if (issued >= NST && !(p.timing_mode & 128u) && !c.wait(s32(&empty[slot]), ph ^ 1u, 2, 0)) {
-          stop = true;
-          break;
-        }
-        const uint32_t fb = s32(&full[slot]);
-        ++issued;
-        if (p.timing_mode & 2u) {  // diagnostic: consumer speed without the weight stream
-          mbar_arrive(fb);
-        } else {
-          // a CTA's units of an op are consecutive in memory, across its tiles: one copy per stage
-          const uint32_t bytes = (e.n0 + e.n1) * UNIT_BYTES;
-          mbar_expect(fb, bytes);
-          bulk_g2s(s32(ring + (size_t)slot * STAGE_BYTES), e.src, bytes, fb);
-        }
-        if (++slot == NST) {
-          slot = 0;
-          ph ^= 1u;
-        }
+// ------------------------------------------------------------------ weight and cache streams
+// A warp's ring: nst pieces of PIECE_BYTES, each with an mbarrier. Lane 0 walks the CTA's table of runs (MegaRun: what the CTA
+// reads of one op) and requests this warp's share of each, piece by piece; the warp takes them in the same order. A piece is
+// requested into the place of the one that the warp has just taken, so nothing but the copy's own barrier is needed: the
+// reads of the old bytes come before the request in program order (__syncwarp between them). The requests sit between a
+// warp's loads and its arithmetic, so what they need is worked out beforehand: no divisions, nothing from global memory.
+__device__ __forceinline__ uint32_t share_begin(uint32_t units, uint32_t w) { return units * w / NCW; }
+// The cached rows that a warp takes of every attention op of the token.
+struct alignas(16) KvShare {
+  unsigned long long off;  // bytes from the start of a cache to the first of them
+  uint32_t r0, rows;       // the first row's position in the cache, and their number
+};
+struct KvPlan {            // in shared memory, the same for every attention op of the token
+  KvShare share[NCW];
+  uint32_t L, S;           // cached rows, splits per head
+  uint32_t head, split;    // this CTA's; head >= heads: none
+  uint32_t per_piece;      // rows of a piece: at most 16, those of one m16n8k16
+};
+// 4, 8 or 16 lanes hold a cache row's 16-byte parts: log2 of that.
+__device__ __forceinline__ uint32_t kv_lanes_log(uint32_t head_dim) { return head_dim > 64 ? 4u : head_dim > 32 ? 3u : 2u; }
+__device__ __forceinline__ void kv_plan(const MegaParams &p, KvPlan &k, uint32_t pos0, uint32_t warp) {  // one thread per warp
+  const uint32_t L = min(pos0 + 1, p.maxlen), S = mega_splits(L, p.splits, p.split_rows), head = blockIdx.x / S, split = blockIdx.x % S;
+  const uint32_t rowb = p.head_dim * 2u;
+  KvShare sh = {0, 0, 0};
+  if (head < p.heads) {
+    uint32_t c0, c1;
+    mega_kv_range(L, S, split, c0, c1);
+    const uint32_t each = (c1 - c0 + NCW - 1) / NCW;
+    sh.r0 = min(c0 + warp * each, c1);
+    sh.rows = min(each, c1 - sh.r0);
+    sh.off = ((unsigned long long)head * p.maxlen + sh.r0) * rowb;
+  }
+  k.share[warp] = sh;
+  if (warp == 0) {
+    k.L = L;
+    k.S = S;
+    k.head = head;
+    k.split = split;
+    k.per_piece = min(PIECE_BYTES / rowb, 16u);
+  }
+}
+struct RunTable {  // in shared memory
+  const MegaRun *runs;
+  uint32_t n;
+  const KvPlan *kv;
+};
+struct Ring {
+  uint32_t piece, bar;  // shared addresses of the next piece and of its barrier
+  uint32_t ph;          // the barrier's parity
+  uint32_t last;        // the last barrier of the ring
+  bool lead;            // lane 0, until a wait fails: requests
+  // requesting side, lane 0 only
+  const uint8_t *src;
+  uint32_t whole;       // whole pieces of weights that follow at src
+  uint32_t rest;        // bytes of the run behind them (cache run: of one of the caches, all of it)
+  uint32_t next;        // runs of the table that have been begun
+  uint32_t asked;       // pieces requested so far
+  int32_t to_v;         // cache run: V cache minus K cache, / 256; a run of weights: 0
+  bool second;          // cache run: the K piece has been requested, its V piece comes next
+};
+// Lane 0: requests the next piece into the place `piece`.
+template <bool DBG>
+__device__ __forceinline__ void ring_request(const MegaParams &p, const RunTable &tab, Ring &r, uint32_t piece, uint32_t bar, uint32_t warp) {
+  uint32_t bytes = PIECE_BYTES;
+  const uint8_t *src = r.src;
+  if (r.whole) {  // most requests
+    --r.whole;
+    r.src += PIECE_BYTES;
+  } else {
+#pragma unroll 1
+    while (r.rest == 0) {  // on to the next run that has something for this warp
+      if (r.next == tab.n) return;
+      const MegaRun e = tab.runs[r.next++];
+      r.to_v = e.to_v;
+      if (e.units == MEGA_KV_MARK) {
+        const KvShare &sh = tab.kv->share[warp];
+        r.src = e.src + sh.off;
+        r.rest = sh.rows * p.head_dim * 2u;
+      } else {
+        const uint32_t u0 = share_begin(e.units, warp), n = share_begin(e.units, warp + 1) - u0;
+        r.src = e.src + (size_t)u0 * UNIT_BYTES;
+        r.whole = n / SU;
+        r.rest = n % SU * UNIT_BYTES;
+        if (r.whole) break;
       }
     }
-    stop = __shfl_sync(0xffffffffu, stop ? 1 : 0, 0) != 0;
-  }
-  // Nothing may still be landing in this CTA's shared memory when it exits.
-  if (lane == 0) {
-    const uint32_t lo = issued > NST ? issued - NST : 0;
-    for (uint32_t j = lo; j < issued; ++j) {
-      const uint32_t fb = s32(&full[j % NST]), ph2 = (j / NST) & 1u;
-    #pragma unroll 1
-      // (not the caller's bound, which a test may have made very short: a copy in flight lands within microseconds)
-      for (uint32_t i = 0; i < max(p.wait_limit, 1u << 20) && !mbar_try(fb, ph2); ++i) {
+    src = r.src;
+    if (r.to_v != 0) {
+      bytes = min(tab.kv->per_piece * p.head_dim * 2u, r.rest);
+      if (r.second) {
+        src += (long long)r.to_v * 256;
+        r.src += bytes;
+        r.rest -= bytes;
       }
+      r.second = !r.second;
+    } else if (r.whole) {
+      --r.whole;
+      r.src += PIECE_BYTES;
+    } else {
+      bytes = r.rest;
+      r.rest = 0;
+    }
+  }
+  ++r.asked;
+  if (DBG && (p.timing_mode & 2u)) {  // diagnostic: no copies
+    mbar_arrive(bar);
+  } else {
+    mbar_expect(bar, bytes);
+    bulk_g2s(piece, src, bytes, bar);
+  }
+}
+// Waits for the next piece, or until the wait has run out: the warp then goes on with whatever lies there and requests nothing more.
+template <bool DBG>
+__device__ __forceinline__ void ring_take(const Ctx &c, Ring &r) {
+  if (DBG && (c.p.timing_mode & 128u)) return;
+  if (mbar_try(r.bar, r.ph)) return;
+  if (c.aborted() || !slow_mbar_wait(c.abort_s, c.p.error, c.p.wait_limit, r.bar, r.ph, 1, 0)) r.lead = false;
+}
+// The warp has read what it needs of the piece: request the one that takes its place, and on to the next.
+template <bool DBG>
+__device__ __forceinline__ void ring_give(const Ctx &c, const RunTable &tab, Ring &r, uint32_t warp) {
+  __syncwarp();
+  if (r.lead) ring_request<DBG>(c.p, tab, r, r.piece, r.bar, warp);
+  r.piece += PIECE_BYTES;
+  r.bar += 8;
+  if (r.bar > r.last) {
+    const uint32_t nst = c.p.nst;
+    r.bar -= nst * 8;
+    r.piece -= nst * PIECE_BYTES;
+    r.ph ^= 1u;
+  }
+}
+// After a wait that ran out: nothing may still be landing in this CTA's shared memory when it exits.
+__device__ __forceinline__ void ring_drain(const MegaParams &p, const Ring &r) {
+  const uint32_t n = min(r.asked, p.nst), bar0 = r.last - (p.nst - 1) * 8;
+#pragma unroll 1
+  for (uint32_t j = r.asked - n; j < r.asked; ++j) {
+    const uint32_t bar = bar0 + j % p.nst * 8, ph = j / p.nst & 1u;
+    // (not the caller's bound, which a test may have made very short: a copy in flight lands within microseconds)
+#pragma unroll 1
+    for (uint32_t i = 0; i < max(p.wait_limit, 1u << 20) && !mbar_try(bar, ph); ++i) {
     }
   }
 }
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ldsf(uint32_t a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts128(uint32_t a, const uint4 &v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void stsf(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
 
 // ------------------------------------------------------------ grid barrier
 __device__ VKL_SLOW bool grid_barrier(const Ctx &c, uint64_t target, uint32_t round, volatile uint32_t *seen_s) {
@@ -357,10 +440,10 @@ __device__ VKL_SLOW bool grid_barrier(const Ctx &c, uint64_t target, uint32_t ro
     }
     const uint32_t tgt = round;
     bool ok = false;
-  #pragma unroll 1
     // (under tensor parallelism a CTA without a tile of the projections runs ahead to this barrier while others
     // wait for another rank's partial sums: the barrier's wait outlasts theirs, so that the error names theirs)
     const uint32_t limit = c.p.tp_size > 1 ? (c.p.wait_limit < 0x10000000u ? 16u * c.p.wait_limit : 0xffffffffu) : c.p.wait_limit;
+#pragma unroll 1
     for (uint32_t i = 0; i < limit; ++i) {
       if (*seen_s == tgt || ld_acq_u64(c.p.bar) >= target) {
         ok = true;
@@ -379,10 +462,6 @@ __device__ VKL_SLOW bool grid_barrier(const Ctx &c, uint64_t target, uint32_t ro
   return !c.aborted();
 }
 
-__device__ __forceinline__ float ldcg_h(const __half *p) {
-  return __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short *>(p))));
-}
-
 // ------------------------------------------------------------------ mat-vec
 struct Best {
   float v;
@@ -395,6 +474,24 @@ __device__ __forceinline__ bool better(float v, uint32_t i, const Best &b) {
 // Two stored codes (bytes 0 and 2, or 1 and 3, of a plane word) as a pair of fp16 subnormals u * 2^-24.
 __device__ __forceinline__ uint32_t codes_sub_h2(uint32_t w, bool hi) { return __byte_perm(w, 0u, hi ? 0x4341u : 0x4240u); }
 
+// m16n8k16 from a zero accumulator and onto one. (Not volatile: the order is the scheduler's to choose.)
+__device__ __forceinline__ void mma_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ void mma_next(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void lds_if(uint4 &v, uint32_t addr, bool take) {  // other lanes keep what they have
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %5, 0;\n @p ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n}"
+               : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+               : "r"(addr), "r"((uint32_t)take)
+               : "memory");
+}
+
 // One mat-vec op of the token: y = W . x for the op's packed weight stream (MegaOp).
 //
 // Arithmetic. The stored codes u = q + 128 go into the tensor core as fp16 subnormals u * 2^-24
@@ -404,36 +501,64 @@ __device__ __forceinline__ uint32_t codes_sub_h2(uint32_t w, bool hi) { return _
 // the reference does (matmul_b0_fp16_x_q8_0.comp:99-133). The input is column 0 of the B operand,
 // the other columns read zeros. (An integer path, dp4a on three byte planes of the input, was
 // measured 30 % slower: dp4a issues at about 16 lanes per clock and SM on this GPU.)
-template <bool TIMED, bool DBG>
-__device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global, uint32_t &it, uint32_t &slot, uint32_t &ph,
-                                          unsigned char *ring, uint64_t *full, uint64_t *empty, const MegaStage *tabs, __half *xs, float *xbias,
-                                          const __half *zero16, float *red, float *ssum, Best &best, unsigned long long *tw, uint32_t ar_seq,
+template <bool TIMED, bool DBG, bool TP>
+__device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global, const RunTable &tab, Ring &ring, __half *xs, float *xbias,
+                                          float *red, float *ssum, Best &best, unsigned long long *tw, uint32_t ar_seq,
                                           uint32_t tag_in, uint32_t tag_out, uint32_t tag_res, unsigned long long *trace) {
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const uint32_t G = gridDim.x, cta = blockIdx.x;
   // The op's entry sits in shared memory: fields are read where they are used (the prologue, then again
   // in the epilogue) instead of being carried in registers through the streaming loop, which needs them all.
   const MegaOp &op = op_global;
-  const uint32_t K = op.K, tiles = op.tiles, NST = c.p.nst;
+  const uint32_t K = op.K, tiles = op.tiles, blocks = op.blocks;
   const uint32_t tile0 = (cta + G - (op.rot % G)) % G;
   const uint32_t tl = tile0 < tiles ? (tiles - tile0 + G - 1) / G : 0u;  // this CTA's tiles
   // No tile here: nothing to read either. (It must not wait for the input: nobody waits for this
   // CTA's results, so by the time it looked the producers of a later op may have re-tagged the words.)
   if (tl == 0) return;
-  const uint32_t nstages = op_global.stages_per_cta[cta];  // requested here, together with the input: needed when the stream starts
-  // ---- input vector -> shared memory (RMSNorm fused, rounded to fp16 where the
-  // reference's RMSNorm op rounds: rms_norm_fp16.comp:70-77). Norm weights and input are
-  // requested together: one memory round trip.
+  // This warp's share of the CTA's units, and, for the reduction, the warps w0..w1 whose shares touch this thread's tile: their
+  // sums of it lie in the first of their places, but for w0, whose share may have begun tiles before.
+  const uint32_t units = tl * blocks, rspan = c.p.red_slots;
+  uint32_t u = share_begin(units, warp), b = u % blocks;
+  const uint32_t u1 = share_begin(units, warp + 1);
+  auto touching = [&](uint32_t lt, uint32_t &at, uint32_t &n) {
+    const uint32_t ub = lt * blocks, w0 = (NCW * (ub + 1) - 1) / units;
+    n = (NCW * (ub + blocks) - 1) / units - w0;
+    at = (w0 * rspan + lt - share_begin(units, w0) / blocks) * 32;
+    n |= w0 << 16;
+  };
+  // row r of tile lt: which matrix and which of its rows
+  auto row_of = [&](uint32_t lt, uint32_t r, uint32_t &m, uint32_t &n) {
+    const uint32_t gt = tile0 + lt * G;
+    m = 0;
+    if (op.epi == EPI_SWIGLU) {
+      n = gt * 16 + r;
+    } else if (op.nmat == 3) {
+      const uint32_t tpm = (op.N + 31) / 32;
+      m = (gt >= tpm) + (gt >= 2 * tpm);
+      n = (gt - m * tpm) * 32 + r;
+    } else {
+      n = gt * 32 + r;
+    }
+  };
+  // worked out here, not between the end of the stream and the publication of the results
+  uint32_t t_at = 0, t_n = 0, t_m = 0, t_row = 0xffffffffu;
+  if (tid < tl * 32) {
+    touching(tid >> 5, t_at, t_n);
+    row_of(tid >> 5, lane, t_m, t_row);
+  }
+  asm volatile("" : "+r"(t_at), "+r"(t_n), "+r"(t_m), "+r"(t_row));  // (and stays worked out)
+  // ---- input vector -> shared memory (RMSNorm fused, rounded to fp16 where the reference's RMSNorm op rounds:
+  // rms_norm_fp16.comp:70-77). A thread's words are requested together, then only those that were not there yet.
+  uint32_t rw = 0;
   {
-    constexpr int MAXV = (2048 + CT - 1) / CT;  // 8-half vectors per thread: K <= 16384
-    uint4 v[MAXV];
+    constexpr int NV = (11008 / 8 + CT - 1) / CT;  // vectors of eight words in one go: K <= 11008
     const uint32_t nv = K / 8;
     const bool norm = op.norm_w != nullptr;
-    constexpr int NWV = 2;  // vectors per thread whose norm weights are requested early (K <= 7680: every norm op of the model shapes)
-    float4 nw[NWV][2];
-    if (norm) {  // the norm weights depend on nothing: request them before the polls, which can spin for a while
+    float4 nw[2][2];  // the norm weights depend on nothing: the first two vectors' are requested before the polls, which can spin for a while
+    if (norm) {
 #pragma unroll
-      for (int j = 0; j < NWV; ++j) {
+      for (int j = 0; j < 2; ++j) {
         const uint32_t i = tid + j * CT;
         if (i < nv) {
           nw[j][0] = ldg_f4_ordered(reinterpret_cast<const float4 *>(op.norm_w) + 2 * i);
@@ -441,214 +566,211 @@ __device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global,
         }
       }
     }
-    {
-      // the first loads together (one memory round trip when the producers are done), then the tag checks
-      constexpr int LFIRST = (11008 / 8 + CT - 1) / CT;  // K <= 11008 (the largest input of the model shapes) in one round trip
-      uint4 la[LFIRST], lb[LFIRST];
+    // EPI_ADD: this thread's residual word, so that its memory round trip is not on the path to the stream or the results
+    if (t_row < op.N && (op.epi == EPI_ADD || (TP && op.epi == EPI_REDUCE))) rw = ld_vol_u32(op.out_ll[0] + t_row);
+    float sq = 0.f;
+#pragma unroll 1
+    for (uint32_t i0 = tid; i0 < nv; i0 += NV * CT) {
+      uint4 a[NV], b8[NV];
+      c.template ll_gather<NV>(op.in + 8 * i0, 8 * CT, (nv - i0 + CT - 1) / CT, tag_in, a, b8);
 #pragma unroll
-      for (int j = 0; j < LFIRST; ++j) {
-        const uint32_t i = tid + j * CT;
-        if (i < nv) {
-          la[j] = ld_vol_v4(op.in + 8 * i);
-          lb[j] = ld_vol_v4(op.in + 8 * i + 4);
-        }
-      }
+      for (int j = 0; j < NV; ++j) {
+        const uint32_t i = i0 + j * CT;
+        if (i >= nv) continue;
+        const uint4 v = ll_pack8(a[j], b8[j]);
+        *reinterpret_cast<uint4 *>(xs + 8 * i) = v;
+        if (norm) {
+          float f[8];
+          unpack8(v, f);
 #pragma unroll
-      for (int j = 0; j < MAXV; ++j) {
-        const uint32_t i = tid + j * CT;
-        v[j] = make_uint4(0, 0, 0, 0);
-        if (i < nv) {
-          if (j < LFIRST)
-            v[j] = c.ll_wait8(op.in + 8 * i, la[j], lb[j], tag_in);
-          else
-            v[j] = c.ll_wait8(op.in + 8 * i, ld_vol_v4(op.in + 8 * i), ld_vol_v4(op.in + 8 * i + 4), tag_in);
+          for (int e = 0; e < 8; e += 2) sq += f[e] * f[e] + f[e + 1] * f[e + 1];
         }
       }
     }
-    for (uint32_t i = tid; i < tl * NCW * 32; i += CT) red[i] = 0.f;  // warps that get no unit of a tile leave zeros
     float alpha = 1.f;
     if (norm) {
-      float s = 0.f;
-#pragma unroll
-      for (int j = 0; j < MAXV; ++j) {
-        const __half2 *h = reinterpret_cast<const __half2 *>(&v[j]);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = __half22float2(h[e]);
-          s += f.x * f.x + f.y * f.y;
-        }
-      }
-      s = warp_sum(s);
-      if (lane == 0) ssum[warp] = s;
+      sq = warp_sum(sq);
+      if (lane == 0) ssum[warp] = sq;
       cons_sync();
       float tot = 0.f;
 #pragma unroll
       for (int w = 0; w < NCW; ++w) tot += ssum[w];
       alpha = 1.0f / sqrtf(tot / (float)K + op.eps);
     }
-#pragma unroll
-    for (int j = 0; j < MAXV; ++j) {
-      const uint32_t i = tid + j * CT;
+    // this thread's vectors again: the norm, and 128 * the sum of every block of 32 inputs = 4 consecutive lanes' vectors
+#pragma unroll 1
+    for (uint32_t i = tid; i - tid < nv; i += CT) {
       float bs = 0.f;
       if (i < nv) {
-        uint4 ov = v[j];
+        uint4 v = *reinterpret_cast<const uint4 *>(xs + 8 * i);
+        float f[8];
+        unpack8(v, f);
         if (norm) {
-          const float4 w0 = j < NWV ? nw[j][0] : __ldg(reinterpret_cast<const float4 *>(op.norm_w) + 2 * i);
-          const float4 w1 = j < NWV ? nw[j][1] : __ldg(reinterpret_cast<const float4 *>(op.norm_w) + 2 * i + 1);
-          const __half2 *h = reinterpret_cast<const __half2 *>(&v[j]);
-          const float2 a = __half22float2(h[0]), b = __half22float2(h[1]), cc = __half22float2(h[2]), d = __half22float2(h[3]);
+          const float w[8] = {nw[0][0].x, nw[0][0].y, nw[0][0].z, nw[0][0].w, nw[0][1].x, nw[0][1].y, nw[0][1].z, nw[0][1].w};
           __half2 o[4];
-          o[0] = __halves2half2(__float2half_rn(a.x * w0.x * alpha), __float2half_rn(a.y * w0.y * alpha));
-          o[1] = __halves2half2(__float2half_rn(b.x * w0.z * alpha), __float2half_rn(b.y * w0.w * alpha));
-          o[2] = __halves2half2(__float2half_rn(cc.x * w1.x * alpha), __float2half_rn(cc.y * w1.y * alpha));
-          o[3] = __halves2half2(__float2half_rn(d.x * w1.z * alpha), __float2half_rn(d.y * w1.w * alpha));
-          ov = *reinterpret_cast<uint4 *>(o);
-        }
-        *reinterpret_cast<uint4 *>(xs + 8 * i) = ov;
-        const __half2 *h = reinterpret_cast<const __half2 *>(&ov);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = __half22float2(h[e]);
-          bs += f.x + f.y;
+          for (int e = 0; e < 4; ++e) o[e] = __halves2half2(__float2half_rn(f[2 * e] * w[2 * e] * alpha), __float2half_rn(f[2 * e + 1] * w[2 * e + 1] * alpha));
+          v = *reinterpret_cast<uint4 *>(o);
+          *reinterpret_cast<uint4 *>(xs + 8 * i) = v;
+          unpack8(v, f);
+          nw[0][0] = nw[1][0];
+          nw[0][1] = nw[1][1];
+          if (i + 2 * CT < nv) {
+            nw[1][0] = __ldg(reinterpret_cast<const float4 *>(op.norm_w) + 2 * (i + 2 * CT));
+            nw[1][1] = __ldg(reinterpret_cast<const float4 *>(op.norm_w) + 2 * (i + 2 * CT) + 1);
+          }
         }
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) bs += f[e] + f[e + 1];
       }
-      // a block of 32 inputs = 4 consecutive vectors = 4 consecutive lanes
       bs += __shfl_xor_sync(0xffffffffu, bs, 1);
       bs += __shfl_xor_sync(0xffffffffu, bs, 2);
       if ((lane & 3) == 0 && i < nv) xbias[i >> 2] = 128.0f * bs;
     }
     cons_sync();
   }
-  // EPI_ADD: this thread's residual value, requested now so that its memory round trip is not
-  // on the path between the end of the stream and the publication of the results
-  float resid = 0.f;
-  if ((op.epi == EPI_ADD || op.epi == EPI_REDUCE) && tid < tl * 32) {
-    const uint32_t n = (tile0 + (tid >> 5) * G) * 32 + (tid & 31);
-    if (n < op.N) resid = __half2float(ll_half(c.ll_wait1(op.out_ll[0] + n, tag_res)));  // (its tag is checked: the word may come from another CTA)
-  }
+  if (t_row < op.N && (op.epi == EPI_ADD || (TP && op.epi == EPI_REDUCE)) && (rw >> 16) != tag_res) rw = c.ll_wait1(op.out_ll[0] + t_row, tag_res);  // (the word may come from another CTA)
+  const float resid = __half2float(ll_half(rw));
   if (TIMED && tw) tw[1] = clock64();
   VKL_TRACE(1);
 
-  // ---- stream this CTA's tiles. Every stage holds UPW units per consumer warp; a unit is one
-  // block (32 columns) of a 32-row tile: two 16-row halves, each the A operand of two m16n8k16
-  // MMAs. Stages run on across tile boundaries, so a warp's partial sums of a tile go to the
-  // warp's own slot in shared memory when its units move on to the next tile, and nothing
-  // synchronises until the op's single reduction at the end.
+  // ---- stream this warp's share of the CTA's tiles: consecutive units, piece by piece. A unit is one block (32 columns) of
+  // a 32-row tile: two 16-row halves, each the A operand of two m16n8k16 MMAs. The sums of a tile go to a place of this warp's
+  // own in shared memory when its units move on to the next tile, and nothing synchronises until the op's single reduction.
   {
-    uint32_t cur = 0xffffffffu;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};  // lanes t == 0: rows g, g + 8, 16 + g, 24 + g of the tile
+    uint32_t slotp = s32(red) + (warp * rspan * 32 + g) * 4;  // the warp's first tile, then its second, ...
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};                      // lanes t == 0: rows g, g + 8, 16 + g, 24 + g of the tile
     auto flush = [&]() {
-      if (cur != 0xffffffffu && t == 0) {
-        float *slotp = red + ((size_t)cur * NCW + warp) * 32;
-        slotp[g] = acc[0];
-        slotp[g + 8] = acc[1];
-        slotp[16 + g] = acc[2];
-        slotp[24 + g] = acc[3];
+      if (t == 0) {
+        stsf(slotp, acc[0]);
+        stsf(slotp + 32, acc[1]);
+        stsf(slotp + 64, acc[2]);
+        stsf(slotp + 96, acc[3]);
       }
     };
-    const __half *xbase = g == 0 ? xs + t * 8 : zero16;  // column 0 of B = the input, the other columns zeros
-    const uint32_t xstep = g == 0 ? 32u : 0u;
-    for (uint32_t sidx = 0; sidx < nstages; ++sidx) {
-      unsigned long long w0 = 0;
-      if (TIMED && tw) w0 = clock64();
-      const bool ok = (DBG && (c.p.timing_mode & 128u)) ? true : c.wait(s32(&full[slot]), ph, 1);
-      if (TIMED && tw) tw[0] += (clock64() - w0) * 1000ull / c.p.sm_mhz;  // SM cycles -> ns at the SM clock the host measured
-      if (DBG && (c.p.timing_mode & 64u)) {  // diagnostic: handshake only
-        __syncwarp();
-        if (lane == 0 && !(c.p.timing_mode & 128u)) mbar_arrive(s32(&empty[slot]));
-        ++it;
-        if (++slot == NST) {
-          slot = 0;
-          ph ^= 1u;
-        }
-        continue;
-      }
-      // the stage's place in the op (tile, first block, run lengths) is in the producer's
-      // table entry, which the producer wrote before it armed the stage's barrier
-      const uint4 meta = *reinterpret_cast<const uint4 *>(&tabs[it & 127].n0);
-      const uint32_t n0 = meta.x, n1 = meta.y, tm = meta.z, kg = meta.w;
-      const unsigned char *st = ring + (size_t)slot * STAGE_BYTES;
-      uint4 wa[UPW], wb[UPW];
-      uint2 dsc[UPW];
-      bool have[UPW];
+    const uint32_t wofs = lane * 16, dofs = UNIT_CODES + g * 8, xaddr = s32(xs) + t * 16, baddr = s32(xbias);
+    uint4 X[SU];  // column 0 of B = the input (lanes g == 0); the other columns' lanes are never loaded and stay zero
 #pragma unroll
-      for (int q = 0; q < UPW; ++q) {
-        const uint32_t u = warp * UPW + q;
-        have[q] = ok && u < n0 + n1;
-        if (have[q]) {
-          wa[q] = *reinterpret_cast<const uint4 *>(st + u * UNIT_BYTES + lane * 16);        // rows g, g + 8 of the tile
-          wb[q] = *reinterpret_cast<const uint4 *>(st + u * UNIT_BYTES + 512 + lane * 16);  // rows 16 + g, 24 + g
-          dsc[q] = *reinterpret_cast<const uint2 *>(st + u * UNIT_BYTES + UNIT_CODES + g * 8);  // their four block scales
-        }
-      }
-      __syncwarp();
-      if (lane == 0 && ok) mbar_arrive(s32(&empty[slot]));  // this warp has read all it needs from the stage
-#pragma unroll
-      for (int q = 0; q < UPW; ++q) {
-        if (!have[q]) continue;
-        const uint32_t u = warp * UPW + q;
-        const uint32_t mt = u < n0 ? tm : tm + 1, b = u < n0 ? kg + u : u - n0;
-        if (mt != cur) {
-          flush();
-          cur = mt;
-          acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
-        }
-        if (DBG && (c.p.timing_mode & 4u)) {  // diagnostic: ring traffic without arithmetic
-          acc[0] += __uint_as_float(wa[q].x ^ wb[q].w ^ dsc[q].x);
+    for (int q = 0; q < SU; ++q) X[q] = make_uint4(0, 0, 0, 0);
+    auto scale = [&](const float (&ca)[4], const float (&cb)[4], const uint2 &dsc, float xb) {
+      const float2 d0 = __half22float2(*reinterpret_cast<const __half2 *>(&dsc.x));  // rows g, g + 8
+      const float2 d1 = __half22float2(*reinterpret_cast<const __half2 *>(&dsc.y));  // rows 16 + g, 24 + g
+      acc[0] = fmaf(fmaf(ca[0], 16777216.f, -xb), d0.x, acc[0]);
+      acc[1] = fmaf(fmaf(ca[2], 16777216.f, -xb), d0.y, acc[1]);
+      acc[2] = fmaf(fmaf(cb[0], 16777216.f, -xb), d1.x, acc[2]);
+      acc[3] = fmaf(fmaf(cb[2], 16777216.f, -xb), d1.y, acc[3]);
+    };
+    auto next_tile = [&]() {
+      flush();
+      slotp += 128;
+      b = 0;
+      acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
+    };
+    // (after a wait that ran out the warp multiplies whatever lies in the ring: the results are discarded)
+#pragma unroll 1
+    while (u < u1) {
+      if (b == blocks) next_tile();
+      // whole pieces within the tile: straight-line code, the units' chains run side by side
+      uint32_t whole = min(u1 - u, blocks - b) / SU;
+      u += whole * SU;
+#pragma unroll 1
+      for (; whole; --whole) {
+        unsigned long long w0 = 0;
+        if (TIMED && tw) w0 = clock64();
+        ring_take<DBG>(c, ring);
+        if (TIMED && tw) tw[0] += (clock64() - w0) * 1000ull / c.p.sm_mhz;  // SM cycles -> ns at the SM clock the host measured
+        const uint32_t st = ring.piece;
+        if (DBG && (c.p.timing_mode & (4u | 64u))) {  // diagnostic: handshake only, or ring traffic without arithmetic
+          if (c.p.timing_mode & 4u) acc[0] += ldsf(st + wofs);
+          b += SU;
+          ring_give<DBG>(c, tab, ring, warp);
           continue;
         }
-        const uint4 X = *reinterpret_cast<const uint4 *>(xbase + b * xstep);
-        const float xb = xbias[b];
-        float ca[4] = {0.f, 0.f, 0.f, 0.f}, cb[4] = {0.f, 0.f, 0.f, 0.f};
-        mma16816(ca, codes_sub_h2(wa[q].x, false), codes_sub_h2(wa[q].z, false), codes_sub_h2(wa[q].x, true), codes_sub_h2(wa[q].z, true), X.x, X.y);
-        mma16816(cb, codes_sub_h2(wb[q].x, false), codes_sub_h2(wb[q].z, false), codes_sub_h2(wb[q].x, true), codes_sub_h2(wb[q].z, true), X.x, X.y);
-        mma16816(ca, codes_sub_h2(wa[q].y, false), codes_sub_h2(wa[q].w, false), codes_sub_h2(wa[q].y, true), codes_sub_h2(wa[q].w, true), X.z, X.w);
-        mma16816(cb, codes_sub_h2(wb[q].y, false), codes_sub_h2(wb[q].w, false), codes_sub_h2(wb[q].y, true), codes_sub_h2(wb[q].w, true), X.z, X.w);
-        const float2 d0 = __half22float2(*reinterpret_cast<const __half2 *>(&dsc[q].x));  // rows g, g + 8
-        const float2 d1 = __half22float2(*reinterpret_cast<const __half2 *>(&dsc[q].y));  // rows 16 + g, 24 + g
-        acc[0] = fmaf(fmaf(ca[0], 16777216.f, -xb), d0.x, acc[0]);
-        acc[1] = fmaf(fmaf(ca[2], 16777216.f, -xb), d0.y, acc[1]);
-        acc[2] = fmaf(fmaf(cb[0], 16777216.f, -xb), d1.x, acc[2]);
-        acc[3] = fmaf(fmaf(cb[2], 16777216.f, -xb), d1.y, acc[3]);
+        uint4 wa[SU], wb[SU];
+        uint2 dsc[SU];
+        float xb[SU], ca[SU][4], cb[SU][4];
+#pragma unroll
+        for (int q = 0; q < SU; ++q) {
+          wa[q] = lds128(st + wofs + q * UNIT_BYTES);        // rows g, g + 8 of the tile
+          wb[q] = lds128(st + wofs + q * UNIT_BYTES + 512);  // rows 16 + g, 24 + g
+          dsc[q] = lds64(st + dofs + q * UNIT_BYTES);        // their four block scales
+          lds_if(X[q], xaddr + b * XB_BYTES + q * XB_BYTES, g == 0);
+          xb[q] = ldsf(baddr + b * 4 + q * 4);
+        }
+#pragma unroll
+        for (int q = 0; q < SU; ++q) {
+          mma_first(ca[q], codes_sub_h2(wa[q].x, false), codes_sub_h2(wa[q].z, false), codes_sub_h2(wa[q].x, true), codes_sub_h2(wa[q].z, true), X[q].x, X[q].y);
+          mma_first(cb[q], codes_sub_h2(wb[q].x, false), codes_sub_h2(wb[q].z, false), codes_sub_h2(wb[q].x, true), codes_sub_h2(wb[q].z, true), X[q].x, X[q].y);
+        }
+#pragma unroll
+        for (int q = 0; q < SU; ++q) {
+          mma_next(ca[q], codes_sub_h2(wa[q].y, false), codes_sub_h2(wa[q].w, false), codes_sub_h2(wa[q].y, true), codes_sub_h2(wa[q].w, true), X[q].z, X[q].w);
+          mma_next(cb[q], codes_sub_h2(wb[q].y, false), codes_sub_h2(wb[q].w, false), codes_sub_h2(wb[q].y, true), codes_sub_h2(wb[q].w, true), X[q].z, X[q].w);
+        }
+#pragma unroll
+        for (int q = 0; q < SU; ++q) scale(ca[q], cb[q], dsc[q], xb[q]);
+        b += SU;
+        ring_give<DBG>(c, tab, ring, warp);
       }
-      ++it;
-      if (++slot == NST) {
-        slot = 0;
-        ph ^= 1u;
+      if (u == u1 || b == blocks) continue;
+      // a piece that a tile or the share ends in
+      const uint32_t n = min((uint32_t)SU, u1 - u);
+      u += n;
+      ring_take<DBG>(c, ring);
+#pragma unroll 1
+      for (uint32_t q = 0; q < n; ++q) {
+        if (b == blocks) next_tile();
+        const uint32_t su = ring.piece + q * UNIT_BYTES;
+        const uint4 wa = lds128(su + wofs), wb = lds128(su + 512 + wofs);
+        lds_if(X[0], xaddr + b * XB_BYTES, g == 0);
+        float ca[4], cb[4];
+        mma_first(ca, codes_sub_h2(wa.x, false), codes_sub_h2(wa.z, false), codes_sub_h2(wa.x, true), codes_sub_h2(wa.z, true), X[0].x, X[0].y);
+        mma_first(cb, codes_sub_h2(wb.x, false), codes_sub_h2(wb.z, false), codes_sub_h2(wb.x, true), codes_sub_h2(wb.z, true), X[0].x, X[0].y);
+        mma_next(ca, codes_sub_h2(wa.y, false), codes_sub_h2(wa.w, false), codes_sub_h2(wa.y, true), codes_sub_h2(wa.w, true), X[0].z, X[0].w);
+        mma_next(cb, codes_sub_h2(wb.y, false), codes_sub_h2(wb.w, false), codes_sub_h2(wb.y, true), codes_sub_h2(wb.w, true), X[0].z, X[0].w);
+        scale(ca, cb, lds64(su + dofs), ldsf(baddr + b * 4));
+        ++b;
       }
+      ring_give<DBG>(c, tab, ring, warp);
     }
-    flush();
+    flush();  // (an empty share: zeros)
   }
   // ---- one fixed-order reduction over the warps and the epilogue for all tiles
   VKL_TRACE(2);
   if (TIMED && tw) {
     tw[2] = clock64();
-    if (c.p.timing_mode & 32u) tw[0] = (((tw[2] - tw[1]) * 1000ull / c.p.sm_mhz) << 16) | (uint64_t)min(nstages, 65535u);
+    if (c.p.timing_mode & 32u) tw[0] = (((tw[2] - tw[1]) * 1000ull / c.p.sm_mhz) << 16) | (uint64_t)min((units / NCW + SU - 1) / SU, 65535u);
   }
+  uint32_t *const out0 = t_m == 0 ? op.out_ll[0] : t_m == 1 ? op.out_ll[1] : op.out_ll[2];
   cons_sync();
   VKL_TRACE(3);
-  const uint32_t tpm = (op.N + 31) / 32;  // tiles per matrix (nmat = 3)
+#pragma unroll 1
   for (uint32_t idx = tid; idx < tl * 32; idx += CT) {  // tl * 32 is a multiple of the warp size: whole warps
-    const uint32_t lt = idx >> 5, r = idx & 31;
-    const uint32_t gt = tile0 + lt * G;
-    const float *sp = red + ((size_t)lt * NCW) * 32 + r;
-    float sum = 0.f;
+    const uint32_t r = idx & 31;
+    if (idx != tid) {  // a CTA with more tiles than warps
+      touching(idx >> 5, t_at, t_n);
+      row_of(idx >> 5, r, t_m, t_row);
+    }
+    const uint32_t n = t_row, m = t_m;
+    float part[NCW];
+    const float *sp = red + (size_t)((t_n >> 16) + 1) * rspan * 32 + r;
+    float sum = red[t_at + r];
 #pragma unroll
-    for (int w = 0; w < NCW; ++w) sum += sp[w * 32];
+    for (int w = 0; w < NCW - 1; ++w) part[w] = w < (t_n & 0xffffu) ? sp[w * rspan * 32] : 0.f;
+#pragma unroll
+    for (int w = 0; w < NCW - 1; ++w) sum += part[w];
     if (op.epi == EPI_SWIGLU) {
       // rows 0..15 of the tile are gate rows, rows 16..31 the up rows of the same outputs
       const float up = __shfl_down_sync(0xffffffffu, sum, 16);
-      const uint32_t n = gt * 16 + r;
-      if (r < 16 && n < op.N && !c.aborted()) op.out_ll[0][n] = ll_pack(__float2half_rn(sum / (1.0f + expf(-sum)) * up), tag_out);
+      if (r < 16 && n < op.N) out0[n] = ll_pack(__float2half_rn(sum / (1.0f + expf(-sum)) * up), tag_out);
       continue;
     }
-    const uint32_t m = op.nmat == 3 ? gt / tpm : 0u;
-    const uint32_t n = (op.nmat == 3 ? gt % tpm : gt) * 32 + r;
-    if (n < op.N && !c.aborted()) {
+    // (After an abort what is published is not looked at any more; another rank must not get it, though.)
+    if (n < op.N && !(TP && c.aborted())) {
       if (op.epi == EPI_ADD) {
         const float res = idx == tid ? resid : __half2float(ll_half(c.ll_wait1(op.out_ll[0] + n, tag_res)));
-        op.out_ll[0][n] = ll_pack(__float2half_rn(round_h(sum) + res), tag_out);
-      } else if (op.epi == EPI_REDUCE) {
+        out0[n] = ll_pack(__float2half_rn(round_h(sum) + res), tag_out);
+      } else if (TP && op.epi == EPI_REDUCE) {
         // this rank's share of a row-split projection, reduced in place: the row's raw fp32 sum and the all-reduce's
         // sequence number go as one 8-byte word into slot [parity][my rank] of every OTHER rank's exchange buffer
         // (plain peer stores over NVLink; the word is its own arrival flag); then this thread polls (bounded, all
@@ -692,7 +814,7 @@ __device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global,
             if (r < tp) s += part[r];
           op.out_ll[0][n] = ll_pack(__float2half_rn(round_h(s) + res), tag_out);
         }
-      } else if (op.epi == EPI_PARTIAL) {
+      } else if (TP && op.epi == EPI_PARTIAL) {
         // this rank's share of a row-split projection: the raw fp32 sum and the all-reduce's
         // sequence number go, as one 8-byte word, into slot [parity][my rank] of every rank's
         // exchange buffer (plain peer stores over NVLink; the word is its own arrival flag)
@@ -703,7 +825,7 @@ __device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global,
         }
       } else {
         const __half h0 = __float2half_rn(sum);
-        uint32_t *o = m == 0 ? op.out_ll[0] : m == 1 ? op.out_ll[1] : op.out_ll[2];
+        uint32_t *o = idx == tid ? out0 : m == 0 ? op.out_ll[0] : m == 1 ? op.out_ll[1] : op.out_ll[2];
         if (o) {
           o[n] = ll_pack(h0, tag_out);
         } else {
@@ -725,180 +847,181 @@ __device__ __forceinline__ void rope_pair(float x0, float x1, float cs, float sn
   o1 = __float2half_rn(x0 * sn + x1 * cs);
 }
 
-// One (head, split) per CTA: RoPE(q), RoPE(k) + cache append by the split that
-// owns the new column, scores over its column range, partial softmax and P.V.
-// Same arithmetic as attention_kernel<true> (attention.cu). The cached K and V rows of the
-// split come through the weight ring: they do not depend on this token (only the row of the
-// new position does, and that one is taken from the fresh projections), so the producer warp
-// has copied them into shared memory before q, k and v arrive.
-__device__ __forceinline__ void attn_part_op(const Ctx &c, const MegaOp &op, float *sm, uint32_t pos0, uint32_t S, uint32_t tag_in,
-                                             uint32_t tag_out, uint32_t &slot, uint32_t &ph, const unsigned char *ring, uint64_t *full,
-                                             uint64_t *empty) {
-  const MegaParams &p = c.p;
-  const uint32_t cta = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (cta >= p.heads * S) return;
-  const uint32_t h = cta / S, split = cta % S, D = p.head_dim, NST = p.nst;
-  float *q_s = sm, *kn_s = sm + D, *red_s = sm + 3 * D, *s_s = sm + (3 + NCW / 2) * D + 2 * NCW + 32;
-  uint32_t *vn_s = reinterpret_cast<uint32_t *>(sm + 2 * D);  // the new V row as packed half pairs
-  const uint32_t L = min(pos0 + 1, p.maxlen);
-  uint32_t c0, c1;
-  mega_kv_range(L, S, split, c0, c1);
-  const uint32_t jn = pos0 % p.maxlen;
-  const bool owns = jn >= c0 && jn < c1;
-  const size_t row = (size_t)h * D;
-  __half *kcache = op.kcache, *vcache = op.vcache;
-  if (2 * tid < D) {
-    const size_t fi = (size_t)pos0 * (D / 2) + tid;
-    const float cs = p.freqc[fi], sn = p.freqs[fi];  // requested with the polls below: one round trip
-    __half r0, r1;
-    // q, k, v of this head come from the projection op before: request this thread's pairs of
-    // tagged words together (one memory round trip when they are there), then poll what is missing
-    const uint32_t *qp = p.q + row + 2 * tid, *kp = p.k + row + 2 * tid, *vp = p.v + row + 2 * tid;
-    uint2 qw = ld_vol_v2(qp), kw = make_uint2(0, 0), vw = make_uint2(0, 0);
-    if (owns) {
-      kw = ld_vol_v2(kp);
-      vw = ld_vol_v2(vp);
-    }
-    qw = c.ll_wait2(qp, qw, tag_in);
-    rope_pair(__half2float(ll_half(qw.x)), __half2float(ll_half(qw.y)), cs, sn, r0, r1);
-    q_s[2 * tid] = __half2float(r0);
-    q_s[2 * tid + 1] = __half2float(r1);
-    if (owns) {
-      kw = c.ll_wait2(kp, kw, tag_in);
-      vw = c.ll_wait2(vp, vw, tag_in);
-      rope_pair(__half2float(ll_half(kw.x)), __half2float(ll_half(kw.y)), cs, sn, r0, r1);
-      kn_s[2 * tid] = __half2float(r0);
-      kn_s[2 * tid + 1] = __half2float(r1);
-      const size_t dst = ((size_t)h * p.maxlen + jn) * D + 2 * tid;
-      kcache[dst] = r0;
-      kcache[dst + 1] = r1;
-      vcache[dst] = ll_half(vw.x);
-      vcache[dst + 1] = ll_half(vw.y);
-      vn_s[tid] = (vw.x & 0xffffu) | (vw.y << 16);  // the new row, for this CTA's P.V
-    }
+// RoPE of four pairs of neighbours (eight packed halves), rounded to fp16.
+__device__ __forceinline__ uint4 rope8(const uint4 &v, const float4 &cs, const float4 &sn) {
+  float f[8];
+  unpack8(v, f);
+  const float cc[4] = {cs.x, cs.y, cs.z, cs.w}, ss[4] = {sn.x, sn.y, sn.z, sn.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    __half a, b;
+    rope_pair(f[2 * e], f[2 * e + 1], cc[e], ss[e], a, b);
+    o[e] = (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16);
   }
-  cons_sync();
-  const float scale = 1.0f / sqrtf((float)D);
-  const uint32_t rps = mega_kv_rows_per_stage(D), rows = c1 - c0;
-  // ---- scores: 16 lanes per cached row (8 dims each), two rows per warp and step
-  {
-    const uint32_t sub = lane & 15, hi = lane >> 4;
-    const bool act = sub * 8 < D;
-    float qv[8];
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// One (head, split) per CTA: RoPE(q), RoPE(k) + cache append, scores over the split's rows, partial softmax and P.V (the
+// arithmetic of attention_kernel, attention.cu, with a running maximum). Every warp takes its share of the rows through its
+// ring, a piece of K rows and the piece of the same V rows behind it: cached rows do not depend on this token, only the row of
+// the new position does; the warp whose share it is in takes it from the fresh projections, puts it into the pieces and into
+// the caches. Up to 16 rows' scores come from the tensor cores (rows x dims, the query as column 0; fp16 products, fp32 sums),
+// P.V stays in fp32: 4, 8 or 16 lanes hold a V row's 16-byte parts. Warps meet once, to add their results in order.
+// The kernel's time depends on its code size (beyond the instruction caches a phase's code comes from memory behind the
+// weight stream), hence loops where a few registers more would have allowed straight-line code.
+template <bool DBG>
+__device__ __forceinline__ void attn_part_op(const Ctx &c, const MegaOp &op, float *sm, uint32_t pos0, const KvPlan &kv, uint32_t tag_in,
+                                             uint32_t tag_out, const RunTable &tab, Ring &ring) {
+  const MegaParams &p = c.p;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const uint32_t h = kv.head, split = kv.split, S = kv.S, D = p.head_dim;
+  if (h >= p.heads) return;
+  const uint32_t lanes_log = kv_lanes_log(D), per_step = 32u >> lanes_log, per_piece = kv.per_piece;
+  const uint32_t r0 = kv.share[warp].r0, r1 = r0 + kv.share[warp].rows;
+  const uint32_t jn = pos0 < p.maxlen ? pos0 : pos0 % p.maxlen;
+  const size_t row = (size_t)h * D;
+  const uint32_t sub = lane & ((1u << lanes_log) - 1u), hi = lane >> lanes_log;
+  const bool act = sub * 8 < D, owns = jn >= r0 && jn < r1;
+  float m = -INFINITY, l = 0.f, acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  // (A split without rows waits for its queries too, with warp 0: it must not arrive at the merge of a later layer first.)
+  if (r0 < r1 || warp == 0) {
+    // The query lands where this warp's sums will lie; the new K and V rows behind all of them. The upper lanes fetch the
+    // key while the lower ones fetch the query (from buffers that follow each other), then the lower ones the value.
+    const uint32_t q_s = s32(sm + warp * D), n_s = s32(sm + NCW * D), part = lane & 15u, upper = lane >> 4;
+    const size_t fi = (size_t)pos0 * (D / 2) + part * 4, cell = ((size_t)h * p.maxlen + jn) * D + part * 8;
+#pragma unroll 1
+    for (uint32_t pass = 0; pass < (owns ? 2u : 1u); ++pass) {
+      if (part * 8 >= D || (upper && (pass || !owns))) continue;
+      const uint32_t *src = (pass ? p.v : upper ? p.k : p.q) + row + part * 8;
+      float4 cs, sn;
+      if (!pass) {
+        cs = ldg_f4_ordered(reinterpret_cast<const float4 *>(p.freqc + fi));
+        sn = ldg_f4_ordered(reinterpret_cast<const float4 *>(p.freqs + fi));
+      }
+      uint4 v = c.ll_wait8(src, ld_vol_v4(src), ld_vol_v4(src + 4), tag_in);
+      if (!pass) v = rope8(v, cs, sn);
+      if (pass || upper) *reinterpret_cast<uint4 *>((pass ? op.vcache : op.kcache) + cell) = v;
+      sts128((pass ? n_s + D * 2 : upper ? n_s : q_s) + part * 16, v);
+    }
+    __syncwarp();
+    uint4 Q[4];  // B fragments: of every 32 dims lane t has 8 t .. 8 t + 7, for the A fragments the same; column 0 only
 #pragma unroll
-    for (int e = 0; e < 8; ++e) qv[e] = act ? q_s[sub * 8 + e] : 0.f;
-    for (uint32_t r0 = 0; r0 < rows; r0 += rps) {
-      const bool ok = (p.timing_mode & 128u) ? true : c.wait(s32(&full[slot]), ph, 1);
-      const uint32_t nr = min(rps, rows - r0);
-      const unsigned char *ks = ring + (size_t)slot * STAGE_BYTES;
-      for (uint32_t rb = warp * 2; rb < nr; rb += NCW * 2) {
-        const uint32_t r = rb + hi, j = c0 + r0 + r;
-        float a = 0.f;
-        if (ok && act && r < nr) {
-          if (owns && j == jn) {
+    for (int i = 0; i < 4; ++i) {
+      Q[i] = make_uint4(0, 0, 0, 0);
+      lds_if(Q[i], q_s + (i * 4 + t) * 16, g == 0 && (i * 4 + t) * 8 < D);
+    }
+    float s0 = 0.f, s1 = 0.f;  // scores, then probabilities, of rows g and g + 8 of the piece
+    bool values = false;
+#pragma unroll 1
+    for (uint32_t r = r0; r < r1;) {
+      const uint32_t nr = min(per_piece, r1 - r);
+      const uint32_t piece = ring.piece;
+      ring_take<DBG>(c, ring);
+      if (owns && jn - r < nr) {  // the new row
+        if (part * 8 < D && !upper) sts128(piece + (jn - r) * D * 2 + part * 16, lds128(n_s + (values ? D * 2 : 0) + part * 16));
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before the copy that will take the piece's place
+        __syncwarp();
+      }
+      if (!values) {
+        float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};  // lanes t == 0: rows g, g + 8 in [0], [2]
+        const uint32_t ra = piece + (min(g, nr - 1) * D + t * 8) * 2, rb = piece + (min(g + 8, nr - 1) * D + t * 8) * 2;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) a = fmaf(qv[e], kn_s[sub * 8 + e], a);
-          } else {
-            const uint4 kv = *reinterpret_cast<const uint4 *>(ks + ((size_t)r * D + sub * 8) * 2);
-            const float2 k0 = __half22float2(*reinterpret_cast<const __half2 *>(&kv.x));
-            const float2 k1 = __half22float2(*reinterpret_cast<const __half2 *>(&kv.y));
-            const float2 k2 = __half22float2(*reinterpret_cast<const __half2 *>(&kv.z));
-            const float2 k3 = __half22float2(*reinterpret_cast<const __half2 *>(&kv.w));
-            a = fmaf(qv[0], k0.x, a); a = fmaf(qv[1], k0.y, a); a = fmaf(qv[2], k1.x, a); a = fmaf(qv[3], k1.y, a);
-            a = fmaf(qv[4], k2.x, a); a = fmaf(qv[5], k2.y, a); a = fmaf(qv[6], k3.x, a); a = fmaf(qv[7], k3.y, a);
+        for (int i = 0; i < 4; ++i) {
+          if (i * 32 >= D) break;
+          uint4 A = make_uint4(0, 0, 0, 0), B = A;
+          if ((i * 4 + t) * 8 < D) {
+            A = lds128(ra + i * 64);
+            B = lds128(rb + i * 64);
+          }
+          mma_next(c0, A.x, B.x, A.y, B.y, Q[i].x, Q[i].y);
+          mma_next(c1, A.z, B.z, A.w, B.w, Q[i].z, Q[i].w);
+        }
+        s0 = __shfl_sync(0xffffffffu, c0[0] + c1[0], lane & 28);
+        s1 = __shfl_sync(0xffffffffu, c0[2] + c1[2], lane & 28);
+        s0 = g < nr ? round_h(s0 * p.attn_scale) : -INFINITY;
+        s1 = g + 8 < nr ? round_h(s1 * p.attn_scale) : -INFINITY;
+        float mx = fmaxf(m, fmaxf(s0, s1));
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float base = mx == -INFINITY ? 0.f : mx;  // (rows of minus infinity so far: weights of 0, not NaN)
+        const float keep = expf(m - base);
+        s0 = expf(s0 - base);
+        s1 = expf(s1 - base);
+        m = mx;
+        l = l * keep + (s0 + s1);  // this quad's rows
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] *= keep;
+      } else {
+#pragma unroll 1
+        for (uint32_t a0 = 0; a0 < nr; a0 += 4 * per_step) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t first = a0 + i * per_step, at = first + hi;  // (a step's rows are all among the first eight or among the others)
+            const float pj = __shfl_sync(0xffffffffu, first < 8 ? s0 : s1, (at & 7u) * 4);
+            uint4 vv = make_uint4(0, 0, 0, 0);
+            if (act && at < nr) vv = lds128(piece + (at * D + sub * 8) * 2);
+            float f[8];
+            unpack8(vv, f);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[e] = fmaf(pj, f[e], acc[e]);
           }
         }
-        a += __shfl_xor_sync(0xffffffffu, a, 8);
-        a += __shfl_xor_sync(0xffffffffu, a, 4);
-        a += __shfl_xor_sync(0xffffffffu, a, 2);
-        a += __shfl_xor_sync(0xffffffffu, a, 1);
-        if (sub == 0 && r < nr) s_s[r0 + r] = round_h(a * scale);
+        r += nr;
       }
-      __syncwarp();
-      if (lane == 0 && ok && !(p.timing_mode & 128u)) mbar_arrive(s32(&empty[slot]));
-      if (++slot == NST) {
-        slot = 0;
-        ph ^= 1u;
-      }
+      values = !values;
+      ring_give<DBG>(c, tab, ring, warp);
     }
-  }
-  cons_sync();
-  float lmax = -INFINITY;
-  for (uint32_t i = tid; i < rows; i += CT) lmax = fmaxf(lmax, s_s[i]);
-  lmax = warp_max(lmax);
-  if (lane == 0) red_s[warp] = lmax;
-  cons_sync();
-  float mloc = red_s[0];
 #pragma unroll
-  for (int w = 1; w < NCW; ++w) mloc = fmaxf(mloc, red_s[w]);
-  float lsum = 0.f;
-  for (uint32_t i = tid; i < rows; i += CT) {
-    const float pj = expf(s_s[i] - mloc);
-    s_s[i] = pj;
-    lsum += pj;
-  }
-  lsum = warp_sum(lsum);
-  if (lane == 0) red_s[NCW + warp] = lsum;
-  cons_sync();
-  float lloc = 0.f;
+    for (int o = 4; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+#pragma unroll 1
+    for (uint32_t o = 1u << lanes_log; o < 32; o <<= 1) {
 #pragma unroll
-  for (int w = 0; w < NCW; ++w) lloc += red_s[NCW + w];
-  // P.V: CT/64 row groups x up to 64 dim pairs, rows of a group in ascending order
-  const uint32_t npair = D / 2, grp = tid / 64, dp = tid % 64;
-  constexpr uint32_t NG = CT / 64;  // threads beyond NG*64 sit this part out
-  float2 acc = make_float2(0.f, 0.f);
-  {
-    const bool act = dp < npair && grp < NG;
-    uint32_t rnext = grp;  // this thread's next row of the split (rows grp, grp + NG, ...)
-    for (uint32_t r0 = 0; r0 < rows; r0 += rps) {
-      const bool ok = (p.timing_mode & 128u) ? true : c.wait(s32(&full[slot]), ph, 1);
-      const uint32_t nr = min(rps, rows - r0);
-      const unsigned char *vs = ring + (size_t)slot * STAGE_BYTES;
-      if (ok && act) {
-        for (; rnext < r0 + nr; rnext += NG) {
-          const uint32_t j = c0 + rnext;
-          const uint32_t raw = (owns && j == jn) ? vn_s[dp] : *reinterpret_cast<const uint32_t *>(vs + ((size_t)(rnext - r0) * D + 2 * dp) * 2);
-          const float2 vv = __half22float2(*reinterpret_cast<const __half2 *>(&raw));
-          const float pj = s_s[rnext];
-          acc.x = fmaf(pj, vv.x, acc.x);
-          acc.y = fmaf(pj, vv.y, acc.y);
-        }
-      }
-      __syncwarp();
-      if (lane == 0 && ok) mbar_arrive(s32(&empty[slot]));
-      if (++slot == NST) {
-        slot = 0;
-        ph ^= 1u;
-      }
+      for (int e = 0; e < 8; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
     }
+    __syncwarp();  // the query has been read
   }
-  cons_sync();
-  float *pv = red_s + 2 * NCW;  // [CT/64 groups][D]
-  if (dp < npair && grp < CT / 64) {
-    pv[grp * D + 2 * dp] = acc.x;
-    pv[grp * D + 2 * dp + 1] = acc.y;
+  // [warp][D] sums, the new rows, then [warp] maxima, then [warp] denominators
+  float *wm = sm + (NCW + 1) * D, *wl = wm + NCW;
+  if (act && hi == 0) {
+#pragma unroll
+    for (int e = 0; e < 8; e += 4) *reinterpret_cast<float4 *>(sm + warp * D + sub * 8 + e) = make_float4(acc[e], acc[e + 1], acc[e + 2], acc[e + 3]);
+  }
+  if (lane == 0) {
+    wm[warp] = m;
+    wl[warp] = l;
   }
   cons_sync();
   float *part = p.attn_scratch + ((size_t)h * p.splits + split) * (D + 4);
-  if (tid < D) {
+  if ((tid & ~31u) < D) {
+    // lane w < NCW: warp w's weight
+    const float mw = lane < NCW ? wm[lane] : -INFINITY, lw = lane < NCW ? wl[lane] : 0.f;
+    const float mloc = warp_max(mw);
+    const float e = lw != 0.f ? expf(mw - mloc) : 0.f;  // (NaN counts)
+    const float lloc = warp_sum(lw * e);
     float s = 0.f;
 #pragma unroll
-    for (int gq = 0; gq < CT / 64; ++gq) s += pv[gq * D + tid];
-    if (S == 1)
-      p.ao[row + tid] = ll_pack(__float2half_rn(s / lloc), tag_out);  // whole row in this CTA: no combine phase
-    else
-      part[tid] = s;
-  }
-  if (tid == 0) {
-    part[D] = mloc;
-    part[D + 1] = lloc;
+    for (int w = 0; w < NCW; ++w) {
+      const float ew = __shfl_sync(0xffffffffu, e, w);
+      if (ew != 0.f) s = fmaf(sm[w * D + min(tid, D - 1)], ew, s);
+    }
+    if (tid < D) {
+      if (S == 1)
+        p.ao[row + tid] = ll_pack(__float2half_rn(s / lloc), tag_out);  // whole row in this CTA: no combine phase
+      else
+        part[tid] = s;
+    }
+    if (tid == 0) {
+      part[D] = mloc;
+      part[D + 1] = lloc;
+    }
   }
   if (S > 1 && p.attn_counters) {
     // The split that finishes last merges the head's partials (in split order, so the result
     // does not depend on who is last): no separate combine op and no grid barrier before it.
     __threadfence();  // this thread's partial results before the CTA's arrival below
     cons_sync();
-    volatile uint32_t *last_s = reinterpret_cast<volatile uint32_t *>(red_s);
+    volatile uint32_t *last_s = reinterpret_cast<volatile uint32_t *>(wl + NCW);
     if (tid == 0) {
       uint32_t old;
       asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(p.attn_counters + h) : "memory");
@@ -910,8 +1033,10 @@ __device__ __forceinline__ void attn_part_op(const Ctx &c, const MegaOp &op, flo
     if (*last_s && tid < D) {
       const float *base = p.attn_scratch + (size_t)h * p.splits * (D + 4);
       float M = -INFINITY;
+#pragma unroll 1
       for (uint32_t sp = 0; sp < S; ++sp) M = fmaxf(M, __ldcg(base + sp * (D + 4) + D));
       float den = 0.f, num = 0.f;
+#pragma unroll 1
       for (uint32_t sp = 0; sp < S; ++sp) {
         const float ms = __ldcg(base + sp * (D + 4) + D), ls = __ldcg(base + sp * (D + 4) + D + 1);
         if (ls > 0.f) {
@@ -932,8 +1057,10 @@ __device__ VKL_SLOW void attn_combine_op(const Ctx &c, uint32_t tag_out) {
   if (h >= p.heads || tid >= D) return;
   const float *base = p.attn_scratch + (size_t)h * p.splits * (D + 4);
   float M = -INFINITY;
+#pragma unroll 1
   for (uint32_t s = 0; s < p.splits; ++s) M = fmaxf(M, __ldcg(base + s * (D + 4) + D));
   float den = 0.f, num = 0.f;
+#pragma unroll 1
   for (uint32_t s = 0; s < p.splits; ++s) {
     const float ms = __ldcg(base + s * (D + 4) + D), ls = __ldcg(base + s * (D + 4) + D + 1);
     if (ls > 0.f) {
@@ -963,12 +1090,14 @@ __device__ VKL_SLOW void embed_op(const Ctx &c, uint32_t tok, uint32_t tag_out) 
 
 // CTA 0: best of the per-CTA candidates (lowest index on ties), then publish the id,
 // feed it back and advance position, step and launch epoch.
+template <bool TP>
 __device__ VKL_SLOW void argmax_final_op(const Ctx &c, float *sm, uint32_t pos0, uint64_t rounds_done, uint32_t ar_done,
                                                 uint32_t next_ebase) {
   const MegaParams &p = c.p;
   if (blockIdx.x != 0) return;
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   Best b = {0.f, 0xffffffffu};
+#pragma unroll 1
   for (uint32_t i = tid; i < gridDim.x; i += CT) {
     const float v = __ldcg(p.arg_scratch + 2 * i);
     const uint32_t ix = __float_as_uint(__ldcg(p.arg_scratch + 2 * i + 1));
@@ -993,12 +1122,13 @@ __device__ VKL_SLOW void argmax_final_op(const Ctx &c, float *sm, uint32_t pos0,
   }
   cons_sync();
   if (tid == 0) {
+#pragma unroll 1
     for (int w = 1; w < NCW; ++w)
       if (si[w] != 0xffffffffu && better(sm[32 + w], si[w], b)) {
         b.v = sm[32 + w];
         b.i = si[w];
       }
-    if (p.tp_size > 1 && !c.aborted()) {
+    if (TP && p.tp_size > 1 && !c.aborted()) {
       // vocabulary-split lm head: exchange (value, global index) candidates with all ranks
       const uint32_t tp = p.tp_size, aseq = p.state[4] + 1;
       b.i += p.tp_rank * p.vocab;
@@ -1097,57 +1227,72 @@ __device__ VKL_SLOW void allreduce_op(const Ctx &c, const MegaOp &op, uint32_t s
   }
 }
 
-template <bool TIMED, bool DBG>
+template <bool TIMED, bool DBG, bool TP>
 __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_constant__ MegaParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t NST = p.nst;
-  unsigned char *ring = smem;
-  unsigned char *xq = smem + (size_t)NST * STAGE_BYTES;  // quantised input vector; attention scratch
+  unsigned char *rings = smem;
+  unsigned char *xq = smem + (size_t)NCW * NST * PIECE_BYTES;  // input vector; attention scratch
   float *red = reinterpret_cast<float *>(xq + p.xs_bytes);
   float *ssum = red + (size_t)p.red_slots * NCW * 32;  // [64]
-  const __half *zero16 = reinterpret_cast<const __half *>(ssum + 64);  // 16 zero bytes
-  MegaStage *tabs = reinterpret_cast<MegaStage *>(ssum + 68);  // [128], 16-byte aligned
-  uint64_t *full = reinterpret_cast<uint64_t *>(tabs + 128);
-  uint64_t *empty = full + MAX_NST;
-  volatile uint32_t *abort_s = reinterpret_cast<volatile uint32_t *>(empty + MAX_NST);
+  MegaRun *runs = reinterpret_cast<MegaRun *>(ssum + 64);  // [run_stride], 16-byte aligned
+  KvPlan *kvp = reinterpret_cast<KvPlan *>(runs + p.run_stride);
+  uint64_t *full = reinterpret_cast<uint64_t *>(kvp + 1);
+  volatile uint32_t *abort_s = reinterpret_cast<volatile uint32_t *>(full + NCW * MAX_NST);
   // The op table lives in global memory; reading an entry there costs a chain of L2 round trips
   // (kind, then the fields, then what they point to) at the start of every op. Three entries are
   // kept in shared memory instead: the running op, the next one (looked at when this one ends)
   // and the one after, which is copied in asynchronously while this op runs.
-  MegaOp *opbuf = reinterpret_cast<MegaOp *>(reinterpret_cast<unsigned char *>(empty + MAX_NST) + 16);
+  MegaOp *opbuf = reinterpret_cast<MegaOp *>(reinterpret_cast<unsigned char *>(full + NCW * MAX_NST) + 16);
   constexpr uint32_t OPV = sizeof(MegaOp) / 16;
   static_assert(sizeof(MegaOp) % 16 == 0, "MegaOp is copied in 16-byte pieces");
   if (threadIdx.x < 2 * OPV && threadIdx.x / OPV < p.nops)
     reinterpret_cast<uint4 *>(opbuf)[threadIdx.x] = reinterpret_cast<const uint4 *>(p.ops)[threadIdx.x];
 
+  const uint32_t nruns = p.run_count[blockIdx.x];
+#pragma unroll 1
+  for (uint32_t i = threadIdx.x; i < nruns; i += CT) runs[i] = p.runs[(size_t)blockIdx.x * p.run_stride + i];
+  const uint32_t pos0 = p.state[0], tok = p.tok[0];
+  if ((threadIdx.x & 31) == 0) {
+    const uint32_t warp = threadIdx.x >> 5;
+#pragma unroll 1
+    for (uint32_t i = 0; i < NST; ++i) mbar_init(s32(&full[warp * NST + i]), 1);
+    kv_plan(p, *kvp, pos0, warp);
+  }
   if (threadIdx.x == 0) {
-    for (uint32_t i = 0; i < NST; ++i) {
-      mbar_init(s32(&full[i]), 1);
-      mbar_init(s32(&empty[i]), NCW);
-    }
     abort_s[0] = 0;
     abort_s[1] = 0;
-    *reinterpret_cast<uint4 *>(ssum + 64) = make_uint4(0, 0, 0, 0);
+  }
+  if ((threadIdx.x & 31) == 0) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
   const Ctx c{p, abort_s};
-
-  if (threadIdx.x >= CT) {  // producer warp
-    producer(c, ring, full, empty, tabs);
-    return;
+  const RunTable tab{runs, nruns, kvp};
+  Ring ring;
+  {
+    const uint32_t warp = threadIdx.x >> 5;
+    ring.piece = s32(rings + (size_t)warp * NST * PIECE_BYTES);
+    ring.bar = s32(full + warp * NST);
+    ring.last = ring.bar + (NST - 1) * 8;
+    ring.ph = ring.whole = ring.rest = ring.next = ring.asked = 0;
+    ring.lead = (threadIdx.x & 31) == 0 && (!DBG || !(p.timing_mode & 128u));
+    ring.second = false;
+    ring.src = nullptr;
+    ring.to_v = 0;
+    if (ring.lead)
+#pragma unroll 1
+      for (uint32_t i = 0; i < NST; ++i) ring_request<DBG>(p, tab, ring, ring.piece + i * PIECE_BYTES, ring.bar + i * 8, warp);
+    __syncwarp();
   }
+  const uint32_t S_eff = kvp->S;
 
   const uint32_t G = gridDim.x;
-  const uint32_t pos0 = p.state[0], tok = p.tok[0];
   const uint64_t base_rounds = p.bar[1];  // barrier rounds completed by earlier launches
   uint64_t rounds = 0;
   const uint32_t seq0 = p.state[3];  // all-reduces completed by earlier launches
   uint32_t ar_i = 0;
-  const uint32_t Lnow = min(pos0 + 1, p.maxlen);
-  const uint32_t S_eff = mega_splits(Lnow, p.splits, p.split_rows);
-  uint32_t it = 0, slot = 0, ph = 0;  // ring position, carried across the ops of the token
   const uint32_t ebase = p.state[7];  // sequence number of this launch's first op; op oi tags its results with ebase + oi
   auto tag = [&](uint32_t op_index) { return (ebase + op_index) & 0xffffu; };
   Best best = {0.f, 0xffffffffu};
@@ -1171,21 +1316,21 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
     VKL_TRACE(0);
     switch (op.kind) {
       case MK_EMBED: embed_op(c, tok, tag(oi)); break;
-      case MK_MATVEC: matvec_op<TIMED, DBG>(c, op, it, slot, ph, ring, full, empty, tabs, reinterpret_cast<__half *>(xq), reinterpret_cast<float *>(xq + (size_t)p.xmax_blocks * XB_BYTES), zero16, red, ssum, best, (TIMED && timed) ? twait : nullptr, seq0 + ar_i + 1,
+      case MK_MATVEC: matvec_op<TIMED, DBG, TP>(c, op, tab, ring, reinterpret_cast<__half *>(xq), reinterpret_cast<float *>(xq + (size_t)p.xmax_blocks * XB_BYTES), red, ssum, best, (TIMED && timed) ? twait : nullptr, seq0 + ar_i + 1,
                          tag(op.src_op), tag(oi), tag(op.res_op), trace);
         if (op.epi == EPI_REDUCE) ++ar_i;  // (every CTA counts it, with or without a tile of the op)
         break;
       case MK_ATTN_PART:
-        attn_part_op(c, op, reinterpret_cast<float *>(xq), pos0, S_eff, tag(op.src_op), tag(op.tag_op), slot, ph, ring, full, empty);
-        if (blockIdx.x < p.heads * p.splits) ++it;  // this CTA's KV entry of the stage table
+        attn_part_op<DBG>(c, op, reinterpret_cast<float *>(xq), pos0, *kvp, tag(op.src_op), tag(op.tag_op), tab, ring);
         break;
       case MK_ATTN_COMBINE: attn_combine_op(c, tag(oi)); break;
       case MK_ALLREDUCE:
+        if (!TP) break;
         ++ar_i;
         allreduce_op(c, op, seq0 + ar_i, tag(oi), tag(op.res_op));
         break;
       case MK_ARGMAX:
-        argmax_final_op(c, reinterpret_cast<float *>(xq), pos0, base_rounds + rounds, seq0 + ar_i, ebase + p.nops);
+        argmax_final_op<TP>(c, reinterpret_cast<float *>(xq), pos0, base_rounds + rounds, seq0 + ar_i, ebase + p.nops);
         break;
     }
     if (op.kind == MK_MATVEC && op.track_argmax) {
@@ -1208,6 +1353,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
       }
       cons_sync();
       if (threadIdx.x == 0) {
+#pragma unroll 1
         for (int w = 1; w < NCW; ++w) {
           const uint32_t wi = __float_as_uint(cand[NCW + w]);
           if (wi != 0xffffffffu && better(cand[w], wi, bb)) {
@@ -1230,6 +1376,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
       const MegaOp &nx = opbuf[(oi + 1) % 3];
       if (nx.kind == MK_MATVEC) {
         if (nx.norm_w)
+#pragma unroll 1
           for (uint32_t i = threadIdx.x * 32; i < nx.K; i += CT * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx.norm_w + i));
       }
       asm volatile("cp.async.wait_all;" ::: "memory");  // entry oi + 2 has landed; the barrier below publishes it
@@ -1255,21 +1402,22 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
       t0 = t2;
     }
   }
+  if ((threadIdx.x & 31) == 0 && !ring.lead && (!DBG || !(p.timing_mode & 128u))) ring_drain(p, ring);
 }
 
 }  // namespace
 
-size_t decode_mega_xs_bytes(uint32_t max_blocks, uint32_t head_dim, uint32_t maxlen, uint32_t splits, uint32_t split_rows) {
-  size_t x = (size_t)max_blocks * (XB_BYTES + 4);  // fp16 input + one fp32 bias term per block of 32 inputs
-  // most rows a split can get: all splits at the full context, or one of fewer splits of split_rows rows
-  uint32_t chunk = ((maxlen + splits - 1) / splits + 31) & ~31u;
-  if (split_rows) chunk = std::max(chunk, (std::min(maxlen, split_rows) + 31) & ~31u);
-  size_t a = (size_t)((3 + NCW / 2) * head_dim + 2 * NCW + 32 + chunk + 32) * 4;
-  size_t b = x > a ? x : a;
-  return (b + 127) / 128 * 128;
+size_t decode_mega_xs_bytes(uint32_t max_blocks, uint32_t head_dim) {
+  const size_t x = (size_t)max_blocks * (XB_BYTES + 4);  // fp16 input + one fp32 bias term per block of 32 inputs
+  const size_t a = (size_t)(NCW * (head_dim + 2) + 4 + head_dim) * 4;  // attention: every warp's sums, maximum and denominator; the new K and V rows
+  return (std::max(x, a) + 127) / 128 * 128;
 }
-size_t decode_mega_smem(size_t xs_bytes, uint32_t nst, uint32_t red_slots) {
-  return (size_t)nst * STAGE_BYTES + xs_bytes + ((size_t)red_slots * NCW * 32 + 68) * 4 + 128 * sizeof(MegaStage) + 2 * MAX_NST * 8 + 16 + 3 * sizeof(MegaOp) + 64;
+size_t decode_mega_smem(size_t xs_bytes, uint32_t nst, uint32_t red_slots, uint32_t runs) {
+  return (size_t)NCW * nst * PIECE_BYTES + xs_bytes + ((size_t)red_slots * NCW * 32 + 64) * 4 + runs * sizeof(MegaRun) + sizeof(KvPlan) + NCW * MAX_NST * 8 + 16 + 3 * sizeof(MegaOp) + 64;
+}
+uint32_t decode_mega_red_slots(uint32_t tiles, uint32_t blocks, uint32_t grid) {
+  const uint32_t tl = (tiles + grid - 1) / grid, share = (tl * blocks + NCW - 1) / NCW;
+  return std::min(tl, (share + blocks - 2) / blocks + 1);
 }
 int decode_mega_max_k() { return 16384; }
 int decode_mega_max_stages() { return MAX_NST; }
@@ -1328,10 +1476,12 @@ cudaError_t launch_mega_pack(const uint8_t *const planes[3], uint32_t nmat, int 
 
 cudaError_t launch_decode_mega(const MegaParams &p, int grid, cudaStream_t s) {
   if (p.nst < 2 || p.nst > (uint32_t)MAX_NST) return cudaErrorInvalidValue;
-  const size_t smem = decode_mega_smem(p.xs_bytes, p.nst, p.red_slots);
+  const size_t smem = decode_mega_smem(p.xs_bytes, p.nst, p.red_slots, p.run_stride);
   // the diagnostic switches (no weight copies, no arithmetic) are compiled into separate instances
   const bool dbg = (p.timing_mode & (2u | 4u | 16u | 64u | 128u)) != 0;  // (16: the diagnostic instance with nothing switched off, its own baseline)
-  auto kern = p.timing ? decode_mega_kernel<true, true> : dbg ? decode_mega_kernel<false, true> : decode_mega_kernel<false, false>;
+  auto kern = p.timing ? (dbg || p.tp_size > 1 ? decode_mega_kernel<true, true, true> : decode_mega_kernel<true, false, false>)
+              : dbg    ? decode_mega_kernel<false, true, true>
+              : p.tp_size > 1 ? decode_mega_kernel<false, false, true> : decode_mega_kernel<false, false, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   void *args[] = {(void *)&p};
@@ -1339,9 +1489,9 @@ cudaError_t launch_decode_mega(const MegaParams &p, int grid, cudaStream_t s) {
 }
 
 cudaError_t decode_mega_occupancy(size_t smem, int *blocks_per_sm) {
-  cudaError_t e = cudaFuncSetAttribute(decode_mega_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(decode_mega_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, decode_mega_kernel<false, false>, THREADS, smem);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, decode_mega_kernel<false, false, true>, THREADS, smem);
 }
 
 }  // namespace vkl

@@ -169,7 +169,6 @@ struct alignas(16) MegaOp {
   const float *norm_w;  // fused RMSNorm of the input, or null
   float eps;
   uint32_t track_argmax;  // lm head: keep a per-CTA (max, index) candidate
-  const uint32_t *stages_per_cta;  // [grid]: ring stages of this op per CTA
   // Activations that cross CTAs inside a token live in "tagged" buffers: one 32-bit word per
   // element, fp16 value in the low half and the low 16 bits of the producing op's sequence
   // number in the high half. A reader that knows which op produced its input polls the words
@@ -184,18 +183,13 @@ struct alignas(16) MegaOp {
   float *out_f32;
   __half *kcache, *vcache;  // MK_ATTN_PART
 };
-// One ring stage of the persistent kernel: up to MEGA_SU consecutive units (one Q8_0 block x
-// 32 rows each) of a CTA's weight stream, one range of memory: the tail of one tile (n0 units)
-// and, when that ends inside the stage, the head of the CTA's next tile (n1 units).
-//
-// An entry with n0 == MEGA_KV_MARK stands for the K and V rows of an attention op instead:
-// src / src2 are the layer's K / V cache. How many ring stages it becomes depends on the
-// token's KV length: producer and consumers both derive this CTA's (head, split) row range from
-// the position and cut it into stages of mega_kv_rows_per_stage() rows, all K stages first.
-struct MegaStage {
-  const uint8_t *src, *src2;
-  uint32_t n0, n1;  // units of the first and of the second tile
-  uint32_t tm, kg;  // consumers' view: local tile and first block of the n0 units; the n1 units start at block 0 of local tile tm + 1
+// What one CTA reads of one op, in the order of the ops: its tiles' units, one range of memory, which the CTA's warps share
+// out evenly. Or, with units == MEGA_KV_MARK, the K and V rows of an attention op: src is the layer's K cache, the V cache
+// lies to_v * 256 bytes behind it, and the rows follow from the token's position.
+struct alignas(16) MegaRun {
+  const uint8_t *src;
+  uint32_t units;
+  int32_t to_v;
 };
 constexpr uint32_t MEGA_KV_MARK = 0xffffffffu;
 // Where tile t of an op (of `tiles` tiles, dealt to a grid of `grid` CTAs as tile0 + lt * grid) sits in the
@@ -205,18 +199,16 @@ __host__ __device__ inline uint32_t mega_stream_tile(uint32_t t, uint32_t tiles,
   return tile0 * q + (tile0 < r ? tile0 : r) + lt;
 }
 constexpr uint32_t MEGA_UNIT_CODES = 1024, MEGA_UNIT_SCALES = 64;  // 32 rows x 32 codes, 32 fp16 scales
-#ifndef VKL_MEGA_UPW
-#define VKL_MEGA_UPW 2
+#ifndef VKL_MEGA_SU
+#define VKL_MEGA_SU 4
 #endif
-constexpr uint32_t MEGA_UPW = VKL_MEGA_UPW;       // units per consumer warp and stage
 #ifndef VKL_MEGA_NCW
 #define VKL_MEGA_NCW 11
 #endif
-constexpr uint32_t MEGA_NCW = VKL_MEGA_NCW;       // consumer warps of the kernel
-constexpr uint32_t MEGA_SU = MEGA_NCW * MEGA_UPW; // units per stage
-constexpr uint32_t MEGA_STAGE_BYTES = MEGA_SU * (MEGA_UNIT_CODES + MEGA_UNIT_SCALES);
-// Cache rows (head_dim fp16 values each) of one KV ring stage: whole rows, a multiple of 8.
-__host__ __device__ inline uint32_t mega_kv_rows_per_stage(uint32_t head_dim) { return (MEGA_STAGE_BYTES / (head_dim * 2u)) & ~7u; }
+constexpr uint32_t MEGA_NCW = VKL_MEGA_NCW;  // warps of the kernel
+constexpr uint32_t MEGA_SU = VKL_MEGA_SU;    // units per piece, the step of a warp's ring
+constexpr uint32_t MEGA_MAX_NST = 8;         // pieces of a ring, at most
+constexpr uint32_t MEGA_PIECE_BYTES = MEGA_SU * (MEGA_UNIT_CODES + MEGA_UNIT_SCALES);
 // Splits per head at KV length L: as few as keep a split within `split_rows` cache rows. With one
 // split a head needs no merge step between CTAs; more splits only pay when the rows of a head no
 // longer stream through one SM fast enough.
@@ -232,9 +224,9 @@ __host__ __device__ inline void mega_kv_range(uint32_t L, uint32_t S, uint32_t s
   c0 = split * chunk < L ? split * chunk : L;
   c1 = c0 + chunk < L ? c0 + chunk : L;
 }
-// How a stage that starts at block `kg` of a tile of `blocks` blocks is cut: n0 units of this
-// tile, then n1 of the next one (if the op has one for this CTA). Host and device walk the
-// stream with the same rule.
+// A piece that starts at block `kg` of a tile of `blocks` blocks, as far as the end of the next tile (if the CTA has one): n0
+// units of this tile, then n1 of the next. Units follow each other in memory, so pieces need no table; the host-side check of
+// the stream's order walks it with this rule.
 struct MegaCut {
   uint32_t n0, n1;
 };
@@ -259,9 +251,9 @@ __host__ __device__ inline void mega_stage_advance(const MegaCut &c, uint32_t bl
 }
 struct MegaParams {
   const MegaOp *ops;
-  const MegaStage *stages;       // [grid][stage_stride]: every CTA's stages in consumer order
-  const uint32_t *stage_count;   // [grid]
-  uint32_t stage_stride;
+  const MegaRun *runs;           // [grid][run_stride]: what every CTA reads, op by op
+  const uint32_t *run_count;     // [grid]
+  uint32_t run_stride;
   uint32_t nops, nbarriers;
   uint32_t *state;    // [0] position, [1] step, [2] picked id, [3] all-reduces done, [4] arg-max exchanges done,
                       // [5] number of forced (prompt) tokens, [6] prefill GEMM error, [7] sequence number of the next launch's first op
@@ -273,6 +265,7 @@ struct MegaParams {
   uint32_t embd_rows;
   uint32_t *x, *q, *k, *v, *ao;  // tagged words (see MegaOp)
   const float *freqc, *freqs;
+  float attn_scale;         // 1 / sqrt(head_dim)
   float *attn_scratch;      // heads*splits*(head_dim+4): per (head, split) the un-normalised P.V row, its max and its sum
   uint32_t attn_merge;      // how a head's split partials are merged: 0 combine op, 1 last-arriving split
   uint32_t *attn_counters;  // [heads] arrivals of a head's splits (the last one merges them), or null: separate combine op
@@ -288,8 +281,8 @@ struct MegaParams {
   // arg candidates [16][2].
   uint32_t tp_rank, tp_size, tp_flag_off;
   void *tp_peer[8];
-  uint32_t nst;               // ring stages (as many as fit beside the input and reduction areas)
-  uint32_t red_slots;         // reduction slots: the most tiles one CTA gets of any op
+  uint32_t nst;               // pieces of a warp's ring (as many as fit beside the input and reduction areas)
+  uint32_t red_slots;         // the most tiles that one warp's share of any op touches
   uint32_t split_rows;        // cache rows one attention split should hold: a token at KV length L uses min(splits, ceil(L / split_rows)) splits per head (0: always `splits`)
   uint32_t barrier_pollers;   // warps whose lane 0 polls the grid barrier counter, staggered in time
   // Optional timeline of CTA 0: per op, nanoseconds of work and of barrier wait.
@@ -298,12 +291,14 @@ struct MegaParams {
   uint32_t sm_mhz;       // SM clock for the timeline's cycle counts (measured by the host before a profiled launch)
   uint32_t wait_limit;   // polls after which any wait of the kernel gives up and raises *error
 };
-size_t decode_mega_xs_bytes(uint32_t max_blocks, uint32_t head_dim, uint32_t maxlen, uint32_t splits, uint32_t split_rows);
+size_t decode_mega_xs_bytes(uint32_t max_blocks, uint32_t head_dim);
 // Packs up to three Q8_0 matrices (tiled planes) that share an input into one op's weight stream
 // (layout and row rules at MegaOp). tiles = the stream's 32-row tiles.
 cudaError_t launch_mega_pack(const uint8_t *const planes[3], uint32_t nmat, int swiglu, uint32_t N, uint32_t K, uint32_t tiles,
                              uint32_t grid, uint8_t *stream, cudaStream_t s);
-size_t decode_mega_smem(size_t xs_bytes, uint32_t nst, uint32_t red_slots);
+size_t decode_mega_smem(size_t xs_bytes, uint32_t nst, uint32_t red_slots, uint32_t runs);
+// The most tiles that one warp's share of an op of `tiles` tiles touches.
+uint32_t decode_mega_red_slots(uint32_t tiles, uint32_t blocks, uint32_t grid);
 int decode_mega_max_k();
 int decode_mega_max_stages();
 cudaError_t decode_mega_occupancy(size_t smem_bytes, int *blocks_per_sm);

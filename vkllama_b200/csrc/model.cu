@@ -52,7 +52,7 @@ int ensure_rows(vkl_model *m, uint32_t T) {
   VKL_CUDA(cudaStreamSynchronize(m->stream));
   m->cap_T = 0;  // an allocation that fails below leaves buffers missing: the next call makes them anew
   if (m->mega_tried) {  // the op table of the persistent kernel holds the old buffers too
-    for (vkl_tensor **t : {&m->mega_ops, &m->mega_sync, &m->mega_arg, &m->mega_attn, &m->mega_stages, &m->mega_counts, &m->mega_ll}) {
+    for (vkl_tensor **t : {&m->mega_ops, &m->mega_sync, &m->mega_arg, &m->mega_attn, &m->mega_runs, &m->mega_counts, &m->mega_ll}) {
       vkl_tensor_release(*t);
       *t = nullptr;
     }
@@ -312,21 +312,22 @@ int build_mega(vkl_model *m) {
     if (splits > cap) splits = cap;
   }
   const uint32_t max_blocks = std::max({c.dim, m->dim_l, m->ffn_l}) / 32;
-  // Rows per attention split (VKLLAMA_SPLIT_ROWS; 0 = always all splits). Short contexts run one CTA
-  // per head and skip the merge between CTAs; the default keeps a split's K rows within three ring stages.
+  // Rows per attention split (VKLLAMA_SPLIT_ROWS; 0 = always all splits). Short contexts run one CTA per head and skip
+  // the merge between CTAs. Measured, us per call of four blocks with 192 / 384 rows: 16 heads at position 300 167 / 161 and
+  // at 1500 160 / 149, 32 heads at 3500 308 / 308 (all splits either way), 40 heads at 745 384 / 402.
   const char *sr_env = getenv("VKLLAMA_SPLIT_ROWS");
   const uint32_t split_rows = sr_env ? (uint32_t)atoi(sr_env) : 384u;
-  const size_t xs_bytes = decode_mega_xs_bytes(max_blocks, m->head_dim, c.maxlen, splits, split_rows);
-  // every tile a CTA gets of an op needs a reduction slot: QKV = 3 matrices of 32-row tiles, gate/up = one
-  // tile per 16 outputs, the others one tile per 32 rows
-  auto slots = [&](uint32_t tiles) { return (tiles + G - 1) / G; };
-  const uint32_t red_slots = std::max({slots(3 * ((m->dim_l + 31) / 32)), slots((c.dim + 31) / 32), slots((m->ffn_l + 15) / 16), slots((m->vocab_l + 31) / 32)});
-  uint32_t nst = (uint32_t)decode_mega_max_stages();  // as many ring stages as fit
+  const size_t xs_bytes = decode_mega_xs_bytes(max_blocks, m->head_dim);
+  auto slots = [&](uint32_t tiles, uint32_t k) { return decode_mega_red_slots(tiles, k / 32, (uint32_t)G); };
+  const uint32_t red_slots = std::max({slots(3 * ((m->dim_l + 31) / 32), c.dim), slots((c.dim + 31) / 32, m->dim_l), slots((m->ffn_l + 15) / 16, c.dim),
+                                       slots((c.dim + 31) / 32, m->ffn_l), slots((m->vocab_l + 31) / 32, c.dim)});
+  const uint32_t max_runs = 5 * c.layers + 1;  // four matrices and an attention op per block, the output layer
+  uint32_t nst = (uint32_t)decode_mega_max_stages();  // as many pieces per ring as fit
   if (const char *rs = getenv("VKLLAMA_RING_STAGES")) nst = std::min(nst, std::max(2u, (uint32_t)atoi(rs)));  // experiments: a shallower ring
-  while (nst >= 2 && decode_mega_smem(xs_bytes, nst, red_slots) > (size_t)m->dev->prop.sharedMemPerBlockOptin) --nst;
+  while (nst >= 2 && decode_mega_smem(xs_bytes, nst, red_slots, max_runs) > (size_t)m->dev->prop.sharedMemPerBlockOptin) --nst;
   if (nst < 2) return VKL_OK;
   int occ = 0;
-  VKL_CUDA(decode_mega_occupancy(decode_mega_smem(xs_bytes, nst, red_slots), &occ));
+  VKL_CUDA(decode_mega_occupancy(decode_mega_smem(xs_bytes, nst, red_slots, max_runs), &occ));
   if (occ < 1) return VKL_OK;
   VKL_OKAY(ensure_rows(m, 1));
 
@@ -455,67 +456,29 @@ int build_mega(vkl_model *m) {
   ops.push_back(am);
 
   if (pack_status != VKL_OK) return pack_status;
-  // Stage tables: every CTA's ring stages for one token, in the order its consumers walk them
-  // (the same cutting rule as the kernel: mega_stage_cut / mega_stage_advance).
-  std::vector<std::vector<MegaStage>> per_cta(G);
-  std::vector<uint32_t> op_stages;  // [mat-vec op][cta]
-  std::vector<size_t> op_index;     // index into `ops` of every mat-vec op
-  for (size_t oi = 0; oi < ops.size(); ++oi) {
-    const MegaOp &o = ops[oi];
+  // Every CTA's runs of one token, in the order its warps walk them.
+  std::vector<MegaRun> runs((size_t)G * max_runs);
+  std::vector<uint32_t> counts(G, 0);
+  for (const MegaOp &o : ops) {
     if (o.kind == MK_ATTN_PART) {
-      // the cached K and V rows of every (head, split) CTA go through the ring too: one marker
-      // entry, which the kernel turns into as many stages as the token's KV length needs
-      for (uint32_t cta = 0; cta < m->heads_l * splits; ++cta) {
-        MegaStage e = {};
-        e.n0 = MEGA_KV_MARK;
-        e.src = (const uint8_t *)o.kcache;
-        e.src2 = (const uint8_t *)o.vcache;
-        per_cta[cta].push_back(e);
+      const ptrdiff_t to_v = (const uint8_t *)o.vcache - (const uint8_t *)o.kcache;
+      if (to_v % 256 || to_v / 256 != (int32_t)(to_v / 256)) return fail(VKL_INTERNAL, "decode kernel: caches are not on 256-byte boundaries");
+      for (uint32_t cta = 0; cta < m->heads_l * splits; ++cta) runs[(size_t)cta * max_runs + counts[cta]++] = {(const uint8_t *)o.kcache, MEGA_KV_MARK, (int32_t)(to_v / 256)};
+    } else if (o.kind == MK_MATVEC) {
+      for (uint32_t cta = 0; cta < (uint32_t)G; ++cta) {
+        const uint32_t tile0 = (cta + G - (o.rot % G)) % G;
+        if (tile0 >= o.tiles) continue;
+        // the CTA's units of the op are consecutive in the packed stream (mega_stream_tile)
+        const uint32_t tl = (o.tiles - tile0 + G - 1) / G;
+        const size_t unit = (size_t)mega_stream_tile(tile0, o.tiles, (uint32_t)G) * o.blocks;
+        runs[(size_t)cta * max_runs + counts[cta]++] = {o.codes + unit * (MEGA_UNIT_CODES + MEGA_UNIT_SCALES), tl * o.blocks, 0};
       }
-      continue;
-    }
-    if (o.kind != MK_MATVEC) continue;
-    op_index.push_back(oi);
-    for (int cta = 0; cta < G; ++cta) {
-      const size_t before = per_cta[cta].size();
-      const uint32_t tile0 = ((uint32_t)cta + G - (o.rot % G)) % G;
-      const uint32_t tl = tile0 < o.tiles ? (o.tiles - tile0 + G - 1) / G : 0u;
-      // the CTA's units of the op are consecutive in the packed stream (mega_stream_tile): a stage is one range
-      auto run = [&](uint32_t lt, uint32_t kg) {
-        const size_t unit = (size_t)mega_stream_tile(tile0 + lt * (uint32_t)G, o.tiles, (uint32_t)G) * o.blocks + kg;
-        return o.codes + unit * (MEGA_UNIT_CODES + MEGA_UNIT_SCALES);
-      };
-      uint32_t tm = 0, kg = 0;
-      while (tm < tl) {
-        const MegaCut cut = mega_stage_cut(kg, o.blocks, tm + 1 < tl);
-        MegaStage e = {};
-        e.n0 = cut.n0;
-        e.n1 = cut.n1;
-        e.tm = tm;
-        e.kg = kg;
-        e.src = run(tm, kg);
-        if (cut.n1 && run(tm + 1, 0) != e.src + (size_t)cut.n0 * (MEGA_UNIT_CODES + MEGA_UNIT_SCALES))
-          return fail(VKL_INTERNAL, "decode kernel: a stage's two runs are not consecutive");
-        per_cta[cta].push_back(e);
-        mega_stage_advance(cut, o.blocks, tm, kg);
-      }
-      op_stages.push_back((uint32_t)(per_cta[cta].size() - before));
     }
   }
-  size_t stride = 0;
-  for (auto &v : per_cta) stride = std::max(stride, v.size());
-  std::vector<MegaStage> flat((size_t)G * stride);
-  std::vector<uint32_t> counts(G);
-  for (int cta = 0; cta < G; ++cta) {
-    counts[cta] = (uint32_t)per_cta[cta].size();
-    std::copy(per_cta[cta].begin(), per_cta[cta].end(), flat.begin() + (size_t)cta * stride);
-  }
-  VKL_OKAY(tensor_new(m->dev, 1, 1, flat.size() * sizeof(MegaStage) / 4, VKL_UINT32, &m->mega_stages));
-  VKL_OKAY(tensor_new(m->dev, 1, 1, (size_t)G + op_stages.size(), VKL_UINT32, &m->mega_counts));  // totals, then per op
-  VKL_CUDA(cudaMemcpyAsync(m->mega_stages->data(), flat.data(), flat.size() * sizeof(MegaStage), cudaMemcpyHostToDevice, m->stream));
+  VKL_OKAY(tensor_new(m->dev, 1, 1, runs.size() * sizeof(MegaRun) / 4, VKL_UINT32, &m->mega_runs));
+  VKL_OKAY(tensor_new(m->dev, 1, 1, (size_t)G, VKL_UINT32, &m->mega_counts));
+  VKL_CUDA(cudaMemcpyAsync(m->mega_runs->data(), runs.data(), runs.size() * sizeof(MegaRun), cudaMemcpyHostToDevice, m->stream));
   VKL_CUDA(cudaMemcpyAsync(m->mega_counts->data(), counts.data(), (size_t)G * 4, cudaMemcpyHostToDevice, m->stream));
-  VKL_CUDA(cudaMemcpyAsync((uint32_t *)m->mega_counts->data() + G, op_stages.data(), op_stages.size() * 4, cudaMemcpyHostToDevice, m->stream));
-  for (size_t k = 0; k < op_index.size(); ++k) ops[op_index[k]].stages_per_cta = (const uint32_t *)m->mega_counts->data() + G + k * (size_t)G;
   VKL_CUDA(cudaStreamSynchronize(m->stream));
 
   const size_t ob = ops.size() * sizeof(MegaOp);
@@ -529,9 +492,9 @@ int build_mega(vkl_model *m) {
   MegaParams &p = m->mp;
   p = MegaParams{};
   p.ops = (const MegaOp *)m->mega_ops->data();
-  p.stages = (const MegaStage *)m->mega_stages->data();
-  p.stage_count = (const uint32_t *)m->mega_counts->data();
-  p.stage_stride = (uint32_t)stride;
+  p.runs = (const MegaRun *)m->mega_runs->data();
+  p.run_count = (const uint32_t *)m->mega_counts->data();
+  p.run_stride = max_runs;
   p.nops = (uint32_t)ops.size();
   p.nbarriers = p.nops - 1;
   p.state = (uint32_t *)m->state->data();
@@ -548,6 +511,7 @@ int build_mega(vkl_model *m) {
   p.x = x; p.q = qb; p.k = kb; p.v = vb; p.ao = ao;  // tagged words
   p.freqc = (const float *)m->fc->data();
   p.freqs = (const float *)m->fs->data();
+  p.attn_scale = 1.0f / sqrtf((float)m->head_dim);
   p.attn_scratch = (float *)m->mega_attn->data();
   {
     const char *cenv = getenv("VKLLAMA_DECODE_COMBINE");
@@ -880,7 +844,7 @@ static void drop_packed(vkl_model *m) {
   cudaStreamSynchronize(m->stream);
   for (vkl_tensor *t : m->mega_packed) vkl_tensor_release(t);
   m->mega_packed.clear();
-  for (vkl_tensor **t : {&m->mega_ops, &m->mega_sync, &m->mega_arg, &m->mega_attn, &m->mega_stages, &m->mega_counts, &m->mega_ll}) {
+  for (vkl_tensor **t : {&m->mega_ops, &m->mega_sync, &m->mega_arg, &m->mega_attn, &m->mega_runs, &m->mega_counts, &m->mega_ll}) {
     vkl_tensor_release(*t);
     *t = nullptr;
   }
