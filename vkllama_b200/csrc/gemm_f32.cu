@@ -15,8 +15,9 @@
 //
 // Bound: tensor cores at three MMAs per product, or L2 -> shared memory traffic (three A tiles and one W tile,
 // 64 KB per 64-wide K step and CTA). One CTA computes 128 x BN with the warps of gemm_tcgen05.cu: TMA producer, MMA
-// lane, four epilogue warps, here working through the whole K loop: while the tensor core fills one
-// of two accumulators, they add the other one to their 32 x BN sums (BN registers per thread).
+// lane, eight epilogue warps, here working through the whole K loop: while the tensor core fills one
+// of two accumulators, they add the other one to their 32 x BN / 2 sums (BN / 2 registers per thread; with four warps
+// and BN sums each a launch of 128 columns took 86 us on average in the 300-token prompt, with eight 71).
 #include "rows.cuh"
 #include "tcgen05.cuh"
 
@@ -24,7 +25,8 @@ namespace vkl {
 namespace {
 
 constexpr int kParts = 3, kBuffers = 2;
-constexpr int kThreads = 192;
+constexpr int kHalves = 2;  // epilogue warps per 32 rows, each with half of the columns
+constexpr int kThreads = 64 + 128 * kHalves;
 
 template <int BN> struct SplitCfg {
   static constexpr uint32_t W_TILE_BYTES = BN * BK * 2;
@@ -76,7 +78,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ __align__(8) uint64_t full[C::STAGES];       // TMA bytes of the stage have landed
   __shared__ __align__(8) uint64_t empty[C::STAGES];      // the MMAs have read the stage
   __shared__ __align__(8) uint64_t acc_full[kBuffers];    // a stage's sums are in the accumulator
-  __shared__ __align__(8) uint64_t acc_empty[kBuffers];   // the four epilogue warps have taken them
+  __shared__ __align__(8) uint64_t acc_empty[kBuffers];   // the epilogue warps have taken them
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile uint32_t failed_s;
 
@@ -97,7 +99,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     for (int b = 0; b < kBuffers; ++b) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sa(&acc_full[b])) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(sa(&acc_empty[b])) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sa(&acc_empty[b])), "n"(4 * kHalves) : "memory");
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     failed_s = 0;
@@ -147,9 +149,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else {
     const uint32_t quad = warp & 3u, row = m0 + quad * 32 + lane;
-    float sum[BN];
+    constexpr int COLS = BN / kHalves;
+    const uint32_t c0 = (warp - 2) / 4 * COLS;
+    float sum[COLS];
 #pragma unroll
-    for (int j = 0; j < BN; ++j) sum[j] = 0.f;
+    for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
     bool done = true;
     for (uint32_t kb = 0; kb < nkb; ++kb) {
       const uint32_t b = kb % kBuffers, buse = kb / kBuffers;
@@ -164,9 +168,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-      for (int cc = 0; cc < BN; cc += 32) {
+      for (int cc = 0; cc < COLS; cc += 32) {
         uint32_t r[32];
-        tmem_ld32(tmem_acc + ((quad * 32u) << 16) + b * BN + cc, r);
+        tmem_ld32(tmem_acc + ((quad * 32u) << 16) + b * BN + c0 + cc, r);
 #pragma unroll
         for (int j = 0; j < 32; ++j) sum[cc + j] += __uint_as_float(r[j]);
       }
@@ -176,12 +180,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     if (done && row < p.M) {
 #pragma unroll
-      for (int cc = 0; cc < BN; cc += 32) {
-        if (n0 + cc >= p.N) break;  // N is a multiple of 32
+      for (int cc = 0; cc < COLS; cc += 32) {
+        if (n0 + c0 + cc >= p.N) break;  // N is a multiple of 32
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = sum[cc + j];
-        rows_chunk<float>(p.out, row, n0 + cc, v);
+        rows_chunk<float>(p.out, row, n0 + c0 + cc, v);
       }
     }
   }

@@ -7,7 +7,7 @@
 // the same ring of stages, and of two accumulators in TMEM one is stored while the next tile fills the other.
 //   warp 0    producer (both CTAs): TMA copies of its A rows and its half of W; both complete on the leader's barrier.
 //   warp 1    MMA (leader): four tcgen05.mma (M256 N{BN} K16) per stage; commits give the stage back in both CTAs.
-//   warps 2-5 epilogue (both CTAs): their 128 rows of the tile, then they give the accumulator back to the leader.
+//   the others epilogue (both CTAs): their 128 rows of the tile, one, two or four warps per 32 rows, then they give the accumulator back to the leader.
 // With SwiGLU the leader's half of a W tile is gate rows and the other CTA's the up rows of the same outputs.
 // 2048 rows, 4096 x 11008: 167 us with one CTA per tile and a slow MMA lane, 149 with the present one, 139 in pairs (1330
 // TFLOP/s, 0.84 of the cuBLAS burst rate); 777 x 17152 x 2048 79 -> 56. What is left is the last wave and the power limit.
@@ -19,7 +19,12 @@
 namespace vkl {
 namespace {
 
-constexpr int kThreads = 192;
+// Epilogue warps per 32 rows, each with its share of the columns. A warp executes some thousand dependent instructions per 32 x 32
+// chunk of an epilogue with activations in it: with one warp per 32 rows a 777 x 13856 tile grid of K = 2048 waited for its
+// epilogues (27 us per tile, the products of a tile take 9). us per launch with 1 / 2 / 4: layer-list in-projection of 777 rows 81.7 /
+// 56.6 / 45.9, 2048 rows 142.8 / 108.7 / 103.5, SwiGLU of 509 rows 81.3 / 77.8 / -; a plain rounding: 2048 x 4096 gained nothing.
+__host__ __device__ constexpr uint32_t epilogue_parts(bool rows, bool swiglu) { return rows ? 4 : swiglu ? 2 : 1; }
+__host__ __device__ constexpr int pair_threads(bool rows, bool swiglu) { return 64 + 128 * (int)epilogue_parts(rows, swiglu); }
 constexpr uint32_t kTmemColumns = 512;  // all of them: the two CTAs' accumulators lie at the same address
 
 template <int BN> struct PairCfg {
@@ -53,10 +58,11 @@ __device__ __forceinline__ void tma_load_pair(uint32_t dst, const CUtensorMap *m
 }
 
 template <int BN, bool ROWS, bool SWIGLU>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(ROWS, SWIGLU), 1)
     gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ WeightMaps maps, const typename PairArgs<ROWS>::Type p, const PairGrid g) {
   using C = PairCfg<BN>;
   constexpr uint32_t OUT = SWIGLU ? BN / 2 : BN;  // output columns of a tile
+  constexpr uint32_t kParts = epilogue_parts(ROWS, SWIGLU);
   extern __shared__ unsigned char smem_raw[];
   unsigned char *stages = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t full[C::STAGES];   // leader: the TMA bytes of both CTAs have landed
@@ -85,7 +91,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     }
     for (int b = 0; b < 2; ++b) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sa(&acc_full[b])) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(sa(&acc_empty[b])) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sa(&acc_empty[b])), "n"(8 * kParts) : "memory");
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     failed_s = 0;
@@ -173,7 +179,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-      for (uint32_t cc = 0; cc < OUT; cc += 32) {
+      for (uint32_t cc = (warp - 2) / 4 * 32; cc < OUT; cc += 32 * kParts) {
         if (n0 + cc >= p.N) break;  // uniform over the warp
         uint32_t r[32];
         float v[32];
@@ -231,7 +237,7 @@ template <int BN, bool ROWS, bool SWIGLU> cudaError_t launch_pair(const typename
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PairCfg<BN>::SMEM);
   if (e != cudaSuccess) return e;
   const size_t tiles = (size_t)g.mtiles * g.ntiles, pairs = sm_count() / 2;
-  kern<<<(unsigned)(2 * (tiles < pairs ? tiles : pairs)), kThreads, PairCfg<BN>::SMEM, s>>>(ma, mw, p, g);
+  kern<<<(unsigned)(2 * (tiles < pairs ? tiles : pairs)), pair_threads(ROWS, SWIGLU), PairCfg<BN>::SMEM, s>>>(ma, mw, p, g);
   return cudaGetLastError();
 }
 

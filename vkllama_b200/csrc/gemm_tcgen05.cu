@@ -22,7 +22,7 @@
 //             stage and issues four tcgen05.mma (M128 N{BN} K16, kind::f16) on shared-memory
 //             descriptors; tcgen05.commit arrives on the stage's "empty" mbarrier when the
 //             tensor core has read the stage, and on "acc_ready" after the last K block.
-//   warps 2-5 epilogue: each reads its 32 TMEM lanes (= 32 output rows) with tcgen05.ld,
+//   warps 2-5, or more with 16-bit weights, epilogue: each reads its 32 TMEM lanes (= 32 output rows) with tcgen05.ld,
 //             applies the op's rounding (scale, bias, SiLU, residual add) and stores fp16 or
 //             raw fp32 rows with 128-bit stores.
 // Every mbarrier wait is bounded; on a time-out the kernel raises the error word, lets
@@ -37,7 +37,10 @@
 namespace vkl {
 namespace {
 
-constexpr int GEMM_THREADS = 192;          // FP16 weights: TMA producer, MMA, four epilogue warps
+// 16-bit weights: TMA producer, MMA, and one, two or four epilogue warps per 32 rows, each with its share of the columns (why:
+// gemm_pair.cu). Experts of 777 tokens, us per gate/up launch with 1 / 2 / 4: 72.6 / 60.7 / 55.0.
+__host__ __device__ constexpr int epilogue_parts(bool rows, bool swiglu) { return rows ? 4 : swiglu ? 2 : 1; }
+__host__ __device__ constexpr int gemm_threads(bool rows, bool swiglu) { return 64 + 128 * epilogue_parts(rows, swiglu); }
 #ifndef VKL_GEMM_NDW
 #define VKL_GEMM_NDW 16
 #endif
@@ -97,7 +100,7 @@ template <int KIND> struct GemmArgs { using Type = GemmParams; };
 template <> struct GemmArgs<GK_ROWS> { using Type = GemmRows; };
 
 template <int BN, int KIND>
-__global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS, 1)
+__global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : gemm_threads(KIND == GK_ROWS, true), 1)
     gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ WeightMaps maps, const typename GemmArgs<KIND>::Type p) {
   constexpr bool Q8 = KIND == GK_Q8;
   using C = Cfg<BN, Q8>;
@@ -286,7 +289,7 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
       }
       if (ok) mma_commit(sa(&acc_ready));
     }
-  } else if (warp >= 2 && warp < 6) {
+  } else if (!Q8 || warp < 6) {
     // ---------------------------------------------------------------- epilogue
     // a warp may only touch TMEM lanes 32*(warp % 4) .. +31
     const uint32_t quad = warp & 3u;
@@ -312,7 +315,7 @@ __global__ void __launch_bounds__(KIND == GK_Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS
       };
       const uint32_t cols = swiglu ? BN / 2 : BN;
 #pragma unroll 1
-      for (uint32_t cc = 0; cc < cols; cc += 32) {
+      for (uint32_t cc = Q8 ? 0 : (warp - 2) / 4 * 32; cc < cols; cc += Q8 ? 32 : (blockDim.x - 64) / 4) {
         if (n0 + cc >= p.N) break;  // uniform over the warp
         float acc[32];
         take(cc, acc);
@@ -350,6 +353,7 @@ template <int BN, int KIND> cudaError_t launch_bn(const typename GemmArgs<KIND>:
   CUtensorMap ma;
   WeightMaps mw = {};  // unused with Q8_0: the W tile is written by the dequantising warps
   uint32_t a_rows = p.M, ny = (p.N + BN - 1) / BN;
+  int threads = Q8 ? GEMM_THREADS_Q8 : gemm_threads(KIND == GK_ROWS, false);
   if constexpr (KIND == GK_ROWS) {
     a_rows *= p.n2 ? 2 : 1;
     if (!make_map(&mw.w[0], p.w, w_rows, p.K, BN, true)) return cudaErrorInvalidValue;
@@ -357,12 +361,13 @@ template <int BN, int KIND> cudaError_t launch_bn(const typename GemmArgs<KIND>:
     for (uint32_t i = 0; i < p.nmat && !Q8; ++i)
       if (!make_map(&mw.w[i], p.w[i], w_rows, p.K, p.swiglu ? BN / 2 : BN)) return cudaErrorInvalidValue;
     ny = p.swiglu ? (p.N + BN / 2 - 1) / (BN / 2) : ny * p.nmat;
+    if (!Q8) threads = gemm_threads(false, p.swiglu);
   }
   if (!make_map(&ma, p.a, a_rows, p.K, BM, KIND == GK_ROWS)) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<BN, Q8>::SMEM);
   if (e != cudaSuccess) return e;
   // x = row tile, so that the CTAs sharing one tile of W run together and W crosses HBM once
-  gemm_tcgen05_kernel<BN, KIND><<<dim3((p.M + BM - 1) / BM, ny), Q8 ? GEMM_THREADS_Q8 : GEMM_THREADS, Cfg<BN, Q8>::SMEM, s>>>(ma, mw, p);
+  gemm_tcgen05_kernel<BN, KIND><<<dim3((p.M + BM - 1) / BM, ny), threads, Cfg<BN, Q8>::SMEM, s>>>(ma, mw, p);
   return cudaGetLastError();
 }
 
