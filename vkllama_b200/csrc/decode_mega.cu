@@ -831,7 +831,10 @@ __device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global,
         } else {
           op.out[0][n] = h0;
         }
-        if (op.out_f32) op.out_f32[n] = __half2float(h0);
+        if (op.out_f32) {
+          op.out_f32[n] = __half2float(h0);
+          if (c.p.host_logits) c.p.host_logits[n] = __half2float(h0);
+        }
         if (op.track_argmax && better(__half2float(h0), n, best)) {
           best.v = __half2float(h0);
           best.i = n;
@@ -1166,7 +1169,8 @@ __device__ VKL_SLOW void argmax_final_op(const Ctx &c, float *sm, uint32_t pos0,
       p.state[4] = aseq;
     }
     if (!c.aborted()) {
-      const uint32_t step = p.state[1], n_forced = p.state[5];
+      const uint32_t step = p.with_token ? 0u : p.state[1], n_forced = p.with_token ? 0u : p.state[5];
+      if (p.with_token) p.state[5] = 0;
       p.state[2] = b.i;
       if (pos0 + 1 < n_forced) {
         p.tok[0] = p.forced[pos0 + 1];  // still inside the prompt: feed the next prompt token
@@ -1179,6 +1183,8 @@ __device__ VKL_SLOW void argmax_final_op(const Ctx &c, float *sm, uint32_t pos0,
       p.state[3] = ar_done;
       p.state[7] = next_ebase;
       p.bar[1] = rounds_done;
+      // (every CTA has passed the grid barrier: none of them can raise an error any more)
+      if (p.host_logits) reinterpret_cast<uint32_t *>(p.host_logits)[p.vocab] = 0u;
     }
   }
 }
@@ -1252,7 +1258,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
   const uint32_t nruns = p.run_count[blockIdx.x];
 #pragma unroll 1
   for (uint32_t i = threadIdx.x; i < nruns; i += CT) runs[i] = p.runs[(size_t)blockIdx.x * p.run_stride + i];
-  const uint32_t pos0 = p.state[0], tok = p.tok[0];
+  const uint32_t pos0 = p.with_token ? p.call_pos : p.state[0], tok = p.with_token ? p.call_tok : p.tok[0];
   if ((threadIdx.x & 31) == 0) {
     const uint32_t warp = threadIdx.x >> 5;
 #pragma unroll 1

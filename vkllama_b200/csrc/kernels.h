@@ -259,6 +259,10 @@ struct MegaParams {
                       // [5] number of forced (prompt) tokens, [6] prefill GEMM error, [7] sequence number of the next launch's first op
   const uint32_t *forced;  // prompt ids: while position+1 < state[5] the next input is forced[position+1]
   uint32_t *tok;      // current token id
+  // A one-token call of a host-driven loop: position and token come with the launch (instead of state[0] and tok), and the output
+  // layer writes its fp32 logits to page-locked host memory as well, one word behind which the launch ends with a 0.
+  uint32_t with_token, call_pos, call_tok;
+  float *host_logits;
   uint32_t *out_ids;
   uint32_t out_cap;
   const uint8_t *embd;  // token embedding, Q8_0 tiled planes

@@ -545,13 +545,24 @@ int build_mega(vkl_model *m) {
 
 __global__ void bump_sequence_kernel(uint32_t *seq, uint32_t by) { *seq += by; }
 
-// Start of a one-token call: position, step counter, no forced tokens, the token itself (one launch instead of
-// three small copies).
-__global__ void begin_token_kernel(uint32_t *state, uint32_t *tok, uint32_t pos, uint32_t id) {
-  state[0] = pos;
-  state[1] = 0;
-  state[5] = 0;
-  tok[0] = id;
+// Start of a call: position, step counter, no forced tokens, the ids (read from page-locked host memory): one launch instead of
+// a copy each.
+__global__ void begin_call_kernel(uint32_t *state, uint32_t *toks, const uint32_t *ids, uint32_t n, uint32_t pos) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) toks[i] = ids[i];
+  if (i == 0) {
+    state[0] = pos;
+    state[1] = 0;
+    state[5] = 0;
+  }
+}
+// End of a call: logits and error words to page-locked host memory, one launch instead of a copy each (11 us of a prompt's call).
+__global__ void __launch_bounds__(256) end_call_kernel(const float *logits, uint32_t n, float *host, const uint32_t *err0, const uint32_t *err1) {
+  for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) host[i] = logits[i];
+  if (blockIdx.x == 0 && threadIdx.x < 2) {
+    const uint32_t *e = threadIdx.x ? err1 : err0;
+    reinterpret_cast<uint32_t *>(host)[n + threadIdx.x] = e ? *e : 0u;
+  }
 }
 
 // SM cycles and nanoseconds of one thread spinning for about 50 us: the SM clock a profiled
@@ -605,11 +616,25 @@ int check_gemm(vkl_model *m) {
   return VKL_OK;
 }
 
-// The error words of the decode kernel and of the bounded waits in prompt kernels come back through pinned memory behind the
+int ensure_pin(vkl_model *m) {
+  if (m->pin) return VKL_OK;
+  VKL_CUDA(cudaHostAlloc((void **)&m->pin, ((size_t)m->vocab_l + 4 + m->cfg.maxlen) * 4, cudaHostAllocMapped));
+  VKL_CUDA(cudaHostGetDevicePointer((void **)&m->pin_dev, m->pin, 0));
+  return VKL_OK;
+}
+int begin_call(vkl_model *m, const uint32_t *toks, uint32_t n, uint32_t pos) {
+  VKL_OKAY(ensure_pin(m));
+  const size_t at = ((size_t)m->vocab_l + 4) * 4;
+  memcpy(m->pin + at, toks, (size_t)n * 4);  // (the last call that read it has been synchronised with)
+  begin_call_kernel<<<(n + 255) / 256, 256, 0, m->stream>>>((uint32_t *)m->state->data(), (uint32_t *)m->toks->data(), (const uint32_t *)(m->pin_dev + at), n, pos);
+  VKL_LAUNCH(1, cudaGetLastError());
+  return VKL_OK;
+}
+// The error words of the decode kernel and of the bounded waits in prompt kernels come back through page-locked memory behind the
 // synchronisation that the caller's results need anyway; each took a copy and a synchronisation of its own (8 us).
 int queue_errors(vkl_model *m, bool decoded) {
   const size_t lb = (size_t)m->vocab_l * 4;
-  if (!m->pin) VKL_CUDA(cudaHostAlloc((void **)&m->pin, lb + 16, cudaHostAllocDefault));
+  VKL_OKAY(ensure_pin(m));
   uint32_t *w = (uint32_t *)(m->pin + lb);
   w[0] = w[1] = 0;
   if (decoded && m->mega_ready) VKL_CUDA(cudaMemcpyAsync(w, m->mp.error, 4, cudaMemcpyDeviceToHost, m->stream));
@@ -624,12 +649,34 @@ int check_errors(vkl_model *m) {  // the stream has been synchronised since; a w
 }
 // The pass's logits, behind one synchronisation.
 int fetch_logits(vkl_model *m, float *logits_out, bool decoded) {
-  VKL_OKAY(queue_errors(m, decoded));
-  const size_t lb = (size_t)m->vocab_l * 4;
-  VKL_CUDA(cudaMemcpyAsync(m->pin, m->logits32->data(), lb, cudaMemcpyDeviceToHost, m->stream));
+  VKL_OKAY(ensure_pin(m));
+  const uint32_t n = m->vocab_l;
+  end_call_kernel<<<std::min((n + 255) / 256, 64u), 256, 0, m->stream>>>((const float *)m->logits32->data(), n, (float *)m->pin_dev, decoded && m->mega_ready ? m->mp.error : nullptr,
+                                                                         m->gemm_used ? (const uint32_t *)m->state->data() + 6 : nullptr);
+  VKL_LAUNCH(1, cudaGetLastError());
   VKL_CUDA(cudaStreamSynchronize(m->stream));
-  memcpy(logits_out, m->pin, lb);
+  memcpy(logits_out, m->pin, (size_t)n * 4);
   return check_errors(m);
+}
+
+// One token through the persistent decode kernel, logits to the host: one launch and one synchronisation.
+int decode_call(vkl_model *m, uint32_t tok, uint32_t pos, float *logits_out) {
+  VKL_OKAY(ensure_pin(m));
+  volatile uint32_t *left = (volatile uint32_t *)m->pin + m->vocab_l;
+  *left = 1;
+  MegaParams p = m->mp;
+  p.with_token = 1;
+  p.call_pos = pos;
+  p.call_tok = tok;
+  p.host_logits = (float *)m->pin_dev;
+  VKL_LAUNCH(1, launch_decode_mega(p, m->mega_grid, m->stream));
+  VKL_CUDA(cudaStreamSynchronize(m->stream));
+  if (*left) {  // the launch gave up: its error word says where
+    VKL_OKAY(check_mega(m));
+    return fail(VKL_INTERNAL, "decode kernel: the launch did not end");
+  }
+  memcpy(logits_out, m->pin, (size_t)m->vocab_l * 4);
+  return VKL_OK;
 }
 
 int build_decode_graph(vkl_model *m);
@@ -988,20 +1035,18 @@ int vkl_model_forward(vkl_model *m, const uint32_t *toks, size_t n, size_t offse
     return check_mega(m);
   }
   if (n == 1) {
-    // The per-token call of a host-driven loop: one small launch sets the step up, the logits and the decode
-    // kernel's error word come back through pinned memory behind one synchronisation.
-    begin_token_kernel<<<1, 1, 0, m->stream>>>((uint32_t *)m->state->data(), (uint32_t *)m->toks->data(), (uint32_t)offset, toks[0]);
-    VKL_LAUNCH(1, cudaGetLastError());
+    if (m->mega_ready && !m->tp_failed) return decode_call(m, toks[0], (uint32_t)offset, logits_out);
+    VKL_OKAY(begin_call(m, toks, 1, (uint32_t)offset));
     VKL_OKAY(decode_step(m));
     VKL_OKAY(fetch_logits(m, logits_out, true));
     if (m->dec) decoder_end(m, offset + 1);
     return VKL_OK;
   }
-  VKL_CUDA(cudaMemsetAsync((uint32_t *)m->state->data() + 5, 0, 4, m->stream));
-  const uint32_t st[2] = {(uint32_t)offset, 0};
-  VKL_CUDA(cudaMemcpyAsync(m->state->data(), st, 8, cudaMemcpyHostToDevice, m->stream));
-  VKL_CUDA(cudaMemcpyAsync(m->toks->data(), toks, n * 4, cudaMemcpyHostToDevice, m->stream));
-  VKL_OKAY(run_tokens(m, (uint32_t)n, false));
+  VKL_OKAY(begin_call(m, toks, (uint32_t)n, (uint32_t)offset));
+  if (const int st = run_tokens(m, (uint32_t)n, false)) {
+    cudaStreamSynchronize(m->stream);  // nothing may still be reading the ids when the next call writes its own
+    return st;
+  }
   VKL_OKAY(fetch_logits(m, logits_out, false));
   if (m->dec) decoder_end(m, offset + n);
   return VKL_OK;

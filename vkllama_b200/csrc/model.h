@@ -80,7 +80,8 @@ struct vkl_model {
   uint32_t sm_mhz = 0;  // measured SM clock, for the profiled launches' cycle counts
   uint32_t wait_limit = 0;  // polls a wait of the decode kernel may spin (0: the default of build_mega)
   bool tp_failed = false;   // a wait on another rank ran out: the ranks' sequence counters are out of step until they reconnect
-  unsigned char *pin = nullptr;  // pinned host staging: this rank's fp32 logits, then the error words (queue_errors)
+  unsigned char *pin = nullptr;  // page-locked host memory: this rank's fp32 logits, then four words (errors), then the token ids of a call
+  unsigned char *pin_dev = nullptr;  // the same as kernels see it
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
   uint32_t *pos_dev() { return (uint32_t *)state->data(); }
   uint32_t *step_dev() { return (uint32_t *)state->data() + 1; }
