@@ -10,7 +10,8 @@ from util import LOGITS_MAX_ABS, load_from_oracle
 pytestmark = pytest.mark.gpu
 
 
-# width, heads, feed-forward, vocabulary, cached rows before the calls
+# weights; width, heads, feed-forward, vocabulary, cached rows before the calls
+@pytest.mark.parametrize("f16", [False, True])
 @pytest.mark.parametrize("dim,heads,ffn,vocab,pos", [
     (32, 2, 32, 20000, 3),     # one block per row: one unit per tile, empty shares
     (64, 8, 96, 61000, 20),    # heads of 8; 13 tiles of the output layer per CTA, two units each
@@ -21,10 +22,10 @@ pytestmark = pytest.mark.gpu
     (160, 2, 416, 997, 30),    # heads of 80: half-filled lanes
     (480, 5, 1280, 997, 30),   # heads of 96
 ])
-def test_one_token_calls_match_the_oracle(dev, dim, heads, ffn, vocab, pos):
+def test_one_token_calls_match_the_oracle(dev, f16, dim, heads, ffn, vocab, pos):
     cfg = dict(dim=dim, heads=heads, ffn=ffn, vocab=vocab, layers=2, maxlen=512)
-    om = O.Model(seed=91, **cfg)
-    dm = vk.Model(dev, dim, heads, ffn, vocab, 2, 512)
+    om = O.Model(seed=91, fp16=f16, **cfg)
+    dm = vk.Model(dev, dim, heads, ffn, vocab, 2, 512, weight_dtype=vk.FP16 if f16 else vk.Q8_0)
     load_from_oracle(dm, om)
     text = O.synth_tokens(91, 1000, pos + 3, vocab)
     om.forward(text[:pos], 0)

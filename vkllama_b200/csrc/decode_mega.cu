@@ -52,6 +52,9 @@ constexpr uint32_t UNIT_CODES = MEGA_UNIT_CODES, UNIT_SCALES = MEGA_UNIT_SCALES;
 constexpr uint32_t UNIT_BYTES = UNIT_CODES + UNIT_SCALES;  // a unit's codes, then its 32 scales
 constexpr uint32_t PIECE_BYTES = SU * UNIT_BYTES;
 static_assert(PIECE_BYTES == MEGA_PIECE_BYTES, "host and device agree on the size of a piece");
+template <bool F16> struct Unit {  // bytes; columns of a unit
+  static constexpr uint32_t BYTES = F16 ? MEGA_UNIT_CODES : UNIT_BYTES, COLUMNS = F16 ? 16 : 32;
+};
 constexpr uint32_t XB_BYTES = 64;      // the input vector in shared memory: fp16, 64 bytes per block of 32 inputs
 constexpr int MAX_NST = (int)MEGA_MAX_NST;  // a ring's pieces are a launch parameter (whatever fits), at most this many
 // Every wait of the kernel is bounded by MegaParams::wait_limit polls (about half a microsecond each): the host
@@ -318,13 +321,14 @@ struct Ring {
   bool second;          // cache run: the K piece has been requested, its V piece comes next
 };
 // Lane 0: requests the next piece into the place `piece`.
-template <bool DBG>
+template <bool DBG, bool F16>
 __device__ __forceinline__ void ring_request(const MegaParams &p, const RunTable &tab, Ring &r, uint32_t piece, uint32_t bar, uint32_t warp) {
-  uint32_t bytes = PIECE_BYTES;
+  constexpr uint32_t UB = Unit<F16>::BYTES;
+  uint32_t bytes = SU * UB;
   const uint8_t *src = r.src;
   if (r.whole) {  // most requests
     --r.whole;
-    r.src += PIECE_BYTES;
+    r.src += SU * UB;
   } else {
 #pragma unroll 1
     while (r.rest == 0) {  // on to the next run that has something for this warp
@@ -337,9 +341,9 @@ __device__ __forceinline__ void ring_request(const MegaParams &p, const RunTable
         r.rest = sh.rows * p.head_dim * 2u;
       } else {
         const uint32_t u0 = share_begin(e.units, warp), n = share_begin(e.units, warp + 1) - u0;
-        r.src = e.src + (size_t)u0 * UNIT_BYTES;
+        r.src = e.src + (size_t)u0 * UB;
         r.whole = n / SU;
-        r.rest = n % SU * UNIT_BYTES;
+        r.rest = n % SU * UB;
         if (r.whole) break;
       }
     }
@@ -354,7 +358,7 @@ __device__ __forceinline__ void ring_request(const MegaParams &p, const RunTable
       r.second = !r.second;
     } else if (r.whole) {
       --r.whole;
-      r.src += PIECE_BYTES;
+      r.src += SU * UB;
     } else {
       bytes = r.rest;
       r.rest = 0;
@@ -376,10 +380,10 @@ __device__ __forceinline__ void ring_take(const Ctx &c, Ring &r) {
   if (c.aborted() || !slow_mbar_wait(c.abort_s, c.p.error, c.p.wait_limit, r.bar, r.ph, 1, 0)) r.lead = false;
 }
 // The warp has read what it needs of the piece: request the one that takes its place, and on to the next.
-template <bool DBG>
+template <bool DBG, bool F16>
 __device__ __forceinline__ void ring_give(const Ctx &c, const RunTable &tab, Ring &r, uint32_t warp) {
   __syncwarp();
-  if (r.lead) ring_request<DBG>(c.p, tab, r, r.piece, r.bar, warp);
+  if (r.lead) ring_request<DBG, F16>(c.p, tab, r, r.piece, r.bar, warp);
   r.piece += PIECE_BYTES;
   r.bar += 8;
   if (r.bar > r.last) {
@@ -492,6 +496,10 @@ __device__ __forceinline__ void lds_if(uint4 &v, uint32_t addr, bool take) {  //
                : "memory");
 }
 
+__device__ __forceinline__ void lds64_if(uint32_t &x, uint32_t &y, uint32_t addr, bool take) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p ld.shared.v2.u32 {%0,%1}, [%2];\n}" : "+r"(x), "+r"(y) : "r"(addr), "r"((uint32_t)take) : "memory");
+}
+
 // One mat-vec op of the token: y = W . x for the op's packed weight stream (MegaOp).
 //
 // Arithmetic. The stored codes u = q + 128 go into the tensor core as fp16 subnormals u * 2^-24
@@ -501,7 +509,7 @@ __device__ __forceinline__ void lds_if(uint4 &v, uint32_t addr, bool take) {  //
 // the reference does (matmul_b0_fp16_x_q8_0.comp:99-133). The input is column 0 of the B operand,
 // the other columns read zeros. (An integer path, dp4a on three byte planes of the input, was
 // measured 30 % slower: dp4a issues at about 16 lanes per clock and SM on this GPU.)
-template <bool TIMED, bool DBG, bool TP>
+template <bool TIMED, bool DBG, bool TP, bool F16>
 __device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global, const RunTable &tab, Ring &ring, __half *xs, float *xbias,
                                           float *red, float *ssum, Best &best, unsigned long long *tw, uint32_t ar_seq,
                                           uint32_t tag_in, uint32_t tag_out, uint32_t tag_res, unsigned long long *trace) {
@@ -597,9 +605,9 @@ __device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global,
       for (int w = 0; w < NCW; ++w) tot += ssum[w];
       alpha = 1.0f / sqrtf(tot / (float)K + op.eps);
     }
-    // this thread's vectors again: the norm, and 128 * the sum of every block of 32 inputs = 4 consecutive lanes' vectors
+    // this thread's vectors again: the norm, and for Q8_0 codes (biased) 128 * the sum of every block of 32 inputs = 4 consecutive lanes' vectors
 #pragma unroll 1
-    for (uint32_t i = tid; i - tid < nv; i += CT) {
+    for (uint32_t i = tid; i - tid < nv && (norm || !F16); i += CT) {
       float bs = 0.f;
       if (i < nv) {
         uint4 v = *reinterpret_cast<const uint4 *>(xs + 8 * i);
@@ -623,6 +631,7 @@ __device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global,
 #pragma unroll
         for (int e = 0; e < 8; e += 2) bs += f[e] + f[e + 1];
       }
+      if (F16) continue;
       bs += __shfl_xor_sync(0xffffffffu, bs, 1);
       bs += __shfl_xor_sync(0xffffffffu, bs, 2);
       if ((lane & 3) == 0 && i < nv) xbias[i >> 2] = 128.0f * bs;
@@ -640,7 +649,16 @@ __device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global,
   {
     uint32_t slotp = s32(red) + (warp * rspan * 32 + g) * 4;  // the warp's first tile, then its second, ...
     float acc[4] = {0.f, 0.f, 0.f, 0.f};                      // lanes t == 0: rows g, g + 8, 16 + g, 24 + g of the tile
+    float even_a[4] = {0.f, 0.f, 0.f, 0.f}, even_b[4] = {0.f, 0.f, 0.f, 0.f}, odd_a[4] = {0.f, 0.f, 0.f, 0.f}, odd_b[4] = {0.f, 0.f, 0.f, 0.f};  // FP16
     auto flush = [&]() {
+      if (F16) {
+        acc[0] = even_a[0] + odd_a[0];
+        acc[1] = even_a[2] + odd_a[2];
+        acc[2] = even_b[0] + odd_b[0];
+        acc[3] = even_b[2] + odd_b[2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) even_a[i] = even_b[i] = odd_a[i] = odd_b[i] = 0.f;
+      }
       if (t == 0) {
         stsf(slotp, acc[0]);
         stsf(slotp + 32, acc[1]);
@@ -648,7 +666,8 @@ __device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global,
         stsf(slotp + 96, acc[3]);
       }
     };
-    const uint32_t wofs = lane * 16, dofs = UNIT_CODES + g * 8, xaddr = s32(xs) + t * 16, baddr = s32(xbias);
+    constexpr uint32_t UB = Unit<F16>::BYTES, XB = Unit<F16>::COLUMNS * 2;  // of the weights, of the input
+    const uint32_t wofs = lane * 16, dofs = UNIT_CODES + g * 8, xaddr = s32(xs) + t * (F16 ? 8 : 16), baddr = s32(xbias);
     uint4 X[SU];  // column 0 of B = the input (lanes g == 0); the other columns' lanes are never loaded and stay zero
 #pragma unroll
     for (int q = 0; q < SU; ++q) X[q] = make_uint4(0, 0, 0, 0);
@@ -683,18 +702,32 @@ __device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global,
         if (DBG && (c.p.timing_mode & (4u | 64u))) {  // diagnostic: handshake only, or ring traffic without arithmetic
           if (c.p.timing_mode & 4u) acc[0] += ldsf(st + wofs);
           b += SU;
-          ring_give<DBG>(c, tab, ring, warp);
+          ring_give<DBG, F16>(c, tab, ring, warp);
           continue;
         }
+        if constexpr (F16) {
+          uint4 wa[SU], wb[SU];
+#pragma unroll
+          for (int q = 0; q < SU; ++q) {
+            wa[q] = lds128(st + wofs + q * UB);        // rows g, g + 8 of the tile: columns 4 t, 4 t + 1, then the next two
+            wb[q] = lds128(st + wofs + q * UB + 512);  // rows 16 + g, 24 + g
+            lds64_if(X[q].x, X[q].y, xaddr + b * XB + q * XB, g == 0);
+          }
+#pragma unroll
+          for (int q = 0; q < SU; ++q) {  // two chains per half tile
+            mma_next(q & 1 ? odd_a : even_a, wa[q].x, wa[q].y, wa[q].z, wa[q].w, X[q].x, X[q].y);
+            mma_next(q & 1 ? odd_b : even_b, wb[q].x, wb[q].y, wb[q].z, wb[q].w, X[q].x, X[q].y);
+          }
+        } else {
         uint4 wa[SU], wb[SU];
         uint2 dsc[SU];
         float xb[SU], ca[SU][4], cb[SU][4];
 #pragma unroll
         for (int q = 0; q < SU; ++q) {
-          wa[q] = lds128(st + wofs + q * UNIT_BYTES);        // rows g, g + 8 of the tile
-          wb[q] = lds128(st + wofs + q * UNIT_BYTES + 512);  // rows 16 + g, 24 + g
-          dsc[q] = lds64(st + dofs + q * UNIT_BYTES);        // their four block scales
-          lds_if(X[q], xaddr + b * XB_BYTES + q * XB_BYTES, g == 0);
+          wa[q] = lds128(st + wofs + q * UB);        // rows g, g + 8 of the tile
+          wb[q] = lds128(st + wofs + q * UB + 512);  // rows 16 + g, 24 + g
+          dsc[q] = lds64(st + dofs + q * UB);        // their four block scales
+          lds_if(X[q], xaddr + b * XB + q * XB, g == 0);
           xb[q] = ldsf(baddr + b * 4 + q * 4);
         }
 #pragma unroll
@@ -709,8 +742,9 @@ __device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global,
         }
 #pragma unroll
         for (int q = 0; q < SU; ++q) scale(ca[q], cb[q], dsc[q], xb[q]);
+        }
         b += SU;
-        ring_give<DBG>(c, tab, ring, warp);
+        ring_give<DBG, F16>(c, tab, ring, warp);
       }
       if (u == u1 || b == blocks) continue;
       // a piece that a tile or the share ends in
@@ -720,18 +754,24 @@ __device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global,
 #pragma unroll 1
       for (uint32_t q = 0; q < n; ++q) {
         if (b == blocks) next_tile();
-        const uint32_t su = ring.piece + q * UNIT_BYTES;
+        const uint32_t su = ring.piece + q * UB;
         const uint4 wa = lds128(su + wofs), wb = lds128(su + 512 + wofs);
-        lds_if(X[0], xaddr + b * XB_BYTES, g == 0);
-        float ca[4], cb[4];
-        mma_first(ca, codes_sub_h2(wa.x, false), codes_sub_h2(wa.z, false), codes_sub_h2(wa.x, true), codes_sub_h2(wa.z, true), X[0].x, X[0].y);
-        mma_first(cb, codes_sub_h2(wb.x, false), codes_sub_h2(wb.z, false), codes_sub_h2(wb.x, true), codes_sub_h2(wb.z, true), X[0].x, X[0].y);
-        mma_next(ca, codes_sub_h2(wa.y, false), codes_sub_h2(wa.w, false), codes_sub_h2(wa.y, true), codes_sub_h2(wa.w, true), X[0].z, X[0].w);
-        mma_next(cb, codes_sub_h2(wb.y, false), codes_sub_h2(wb.w, false), codes_sub_h2(wb.y, true), codes_sub_h2(wb.w, true), X[0].z, X[0].w);
-        scale(ca, cb, lds64(su + dofs), ldsf(baddr + b * 4));
+        if constexpr (F16) {
+          lds64_if(X[0].x, X[0].y, xaddr + b * XB, g == 0);
+          mma_next(even_a, wa.x, wa.y, wa.z, wa.w, X[0].x, X[0].y);
+          mma_next(even_b, wb.x, wb.y, wb.z, wb.w, X[0].x, X[0].y);
+        } else {
+          lds_if(X[0], xaddr + b * XB, g == 0);
+          float ca[4], cb[4];
+          mma_first(ca, codes_sub_h2(wa.x, false), codes_sub_h2(wa.z, false), codes_sub_h2(wa.x, true), codes_sub_h2(wa.z, true), X[0].x, X[0].y);
+          mma_first(cb, codes_sub_h2(wb.x, false), codes_sub_h2(wb.z, false), codes_sub_h2(wb.x, true), codes_sub_h2(wb.z, true), X[0].x, X[0].y);
+          mma_next(ca, codes_sub_h2(wa.y, false), codes_sub_h2(wa.w, false), codes_sub_h2(wa.y, true), codes_sub_h2(wa.w, true), X[0].z, X[0].w);
+          mma_next(cb, codes_sub_h2(wb.y, false), codes_sub_h2(wb.w, false), codes_sub_h2(wb.y, true), codes_sub_h2(wb.w, true), X[0].z, X[0].w);
+          scale(ca, cb, lds64(su + dofs), ldsf(baddr + b * 4));
+        }
         ++b;
       }
-      ring_give<DBG>(c, tab, ring, warp);
+      ring_give<DBG, F16>(c, tab, ring, warp);
     }
     flush();  // (an empty share: zeros)
   }
@@ -873,7 +913,7 @@ __device__ __forceinline__ uint4 rope8(const uint4 &v, const float4 &cs, const f
 // P.V stays in fp32: 4, 8 or 16 lanes hold a V row's 16-byte parts. Warps meet once, to add their results in order.
 // The kernel's time depends on its code size (beyond the instruction caches a phase's code comes from memory behind the
 // weight stream), hence loops where a few registers more would have allowed straight-line code.
-template <bool DBG>
+template <bool DBG, bool F16>
 __device__ __forceinline__ void attn_part_op(const Ctx &c, const MegaOp &op, float *sm, uint32_t pos0, const KvPlan &kv, uint32_t tag_in,
                                              uint32_t tag_out, const RunTable &tab, Ring &ring) {
   const MegaParams &p = c.p;
@@ -973,7 +1013,7 @@ __device__ __forceinline__ void attn_part_op(const Ctx &c, const MegaOp &op, flo
         r += nr;
       }
       values = !values;
-      ring_give<DBG>(c, tab, ring, warp);
+      ring_give<DBG, F16>(c, tab, ring, warp);
     }
 #pragma unroll
     for (int o = 4; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
@@ -1076,12 +1116,17 @@ __device__ VKL_SLOW void attn_combine_op(const Ctx &c, uint32_t tag_out) {
 }
 
 // Embedding gather + dequantisation of the current token (embedding_q8_0.comp:39-85).
+template <bool F16>
 __device__ VKL_SLOW void embed_op(const Ctx &c, uint32_t tok, uint32_t tag_out) {
   const MegaParams &p = c.p;
   const uint32_t per = (p.dim + gridDim.x - 1) / gridDim.x;
   const uint32_t k = blockIdx.x * per + threadIdx.x;
   if (threadIdx.x >= per || k >= p.dim) return;
   if (tok >= p.embd_rows) tok = 0;  // UNK = 0 (models/llama2.h:455-458)
+  if (F16) {
+    p.x[k] = ll_pack(reinterpret_cast<const __half *>(p.embd)[(size_t)tok * p.dim + k], tag_out);
+    return;
+  }
   const Q8Layout L = q8_layout(p.embd_rows, p.dim);
   const uint32_t tile = tok >> 4, r = tok & 15, g = r & 7, half = r >> 3;
   const uint32_t b = k >> 5, t = (k >> 3) & 3, i = k & 7;
@@ -1233,7 +1278,7 @@ __device__ VKL_SLOW void allreduce_op(const Ctx &c, const MegaOp &op, uint32_t s
   }
 }
 
-template <bool TIMED, bool DBG, bool TP>
+template <bool TIMED, bool DBG, bool TP, bool F16>
 __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_constant__ MegaParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t NST = p.nst;
@@ -1289,7 +1334,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
     ring.to_v = 0;
     if (ring.lead)
 #pragma unroll 1
-      for (uint32_t i = 0; i < NST; ++i) ring_request<DBG>(p, tab, ring, ring.piece + i * PIECE_BYTES, ring.bar + i * 8, warp);
+      for (uint32_t i = 0; i < NST; ++i) ring_request<DBG, F16>(p, tab, ring, ring.piece + i * PIECE_BYTES, ring.bar + i * 8, warp);
     __syncwarp();
   }
   const uint32_t S_eff = kvp->S;
@@ -1321,13 +1366,13 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
     unsigned long long *trace = (tracing && threadIdx.x == 0) ? p.timing + ((size_t)oi * gridDim.x + blockIdx.x) * 8 : nullptr;
     VKL_TRACE(0);
     switch (op.kind) {
-      case MK_EMBED: embed_op(c, tok, tag(oi)); break;
-      case MK_MATVEC: matvec_op<TIMED, DBG, TP>(c, op, tab, ring, reinterpret_cast<__half *>(xq), reinterpret_cast<float *>(xq + (size_t)p.xmax_blocks * XB_BYTES), red, ssum, best, (TIMED && timed) ? twait : nullptr, seq0 + ar_i + 1,
+      case MK_EMBED: embed_op<F16>(c, tok, tag(oi)); break;
+      case MK_MATVEC: matvec_op<TIMED, DBG, TP, F16>(c, op, tab, ring, reinterpret_cast<__half *>(xq), reinterpret_cast<float *>(xq + (size_t)p.xmax_blocks * XB_BYTES), red, ssum, best, (TIMED && timed) ? twait : nullptr, seq0 + ar_i + 1,
                          tag(op.src_op), tag(oi), tag(op.res_op), trace);
         if (op.epi == EPI_REDUCE) ++ar_i;  // (every CTA counts it, with or without a tile of the op)
         break;
       case MK_ATTN_PART:
-        attn_part_op<DBG>(c, op, reinterpret_cast<float *>(xq), pos0, *kvp, tag(op.src_op), tag(op.tag_op), tab, ring);
+        attn_part_op<DBG, F16>(c, op, reinterpret_cast<float *>(xq), pos0, *kvp, tag(op.src_op), tag(op.tag_op), tab, ring);
         break;
       case MK_ATTN_COMBINE: attn_combine_op(c, tag(oi)); break;
       case MK_ALLREDUCE:
@@ -1480,14 +1525,43 @@ cudaError_t launch_mega_pack(const uint8_t *const planes[3], uint32_t nmat, int 
   return cudaGetLastError();
 }
 
+// The same for FP16 matrices [N, K]: a unit is 32 rows x 16 columns, 512 bytes per 16 rows: lane (g, t) has columns 4 t and 4 t + 1 of
+// rows g and g + 8, then columns 4 t + 2 and 4 t + 3 of both, the A fragment of one m16n8k16 whose k runs through the columns
+// in this order (for the input the same).
+namespace {
+// A CTA packs eight blocks of a tile, a warp each, so that it reads whole lines.
+__global__ void __launch_bounds__(256) mega_pack_f16_kernel(const __half *p0, const __half *p1, const __half *p2, uint32_t nmat, int swiglu, uint32_t N, uint32_t K, uint32_t tiles,
+                                                            uint32_t grid, uint8_t *stream) {
+  const uint32_t b = blockIdx.x * 8 + (threadIdx.x >> 5), t = blockIdx.y, blocks = K / 16, lane = threadIdx.x & 31, g = lane >> 2, c = b * 16 + (lane & 3) * 4;
+  if (b >= blocks) return;
+  const uint32_t tpm = (N + 31) / 32;
+  uint4 *dst = reinterpret_cast<uint4 *>(stream + ((size_t)mega_stream_tile(t, tiles, grid) * blocks + b) * MEGA_UNIT_CODES) + lane;
+#pragma unroll
+  for (uint32_t half = 0; half < 2; ++half) {
+    const uint32_t m = swiglu ? half : nmat == 3 ? t / tpm : 0u, row = swiglu ? t * 16 + g : (nmat == 3 ? t % tpm : t) * 32 + half * 16 + g;
+    const __half *src = m == 0 ? p0 : m == 1 ? p1 : p2;
+    uint2 lo = make_uint2(0, 0), hi = lo;
+    if (row < N) lo = __ldcs(reinterpret_cast<const uint2 *>(src + (size_t)row * K + c));
+    if (row + 8 < N) hi = __ldcs(reinterpret_cast<const uint2 *>(src + (size_t)(row + 8) * K + c));
+    dst[half * 32] = make_uint4(lo.x, hi.x, lo.y, hi.y);
+  }
+}
+}  // namespace
+cudaError_t launch_mega_pack_f16(const __half *const w[3], uint32_t nmat, int swiglu, uint32_t N, uint32_t K, uint32_t tiles, uint32_t grid, uint8_t *stream, cudaStream_t s) {
+  if (K % 16 || tiles == 0 || tiles > 65535u || grid == 0) return cudaErrorInvalidValue;
+  mega_pack_f16_kernel<<<dim3((K / 16 + 7) / 8, tiles), 256, 0, s>>>(w[0], w[1], w[2], nmat, swiglu, N, K, tiles, grid, stream);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_decode_mega(const MegaParams &p, int grid, cudaStream_t s) {
   if (p.nst < 2 || p.nst > (uint32_t)MAX_NST) return cudaErrorInvalidValue;
   const size_t smem = decode_mega_smem(p.xs_bytes, p.nst, p.red_slots, p.run_stride);
   // the diagnostic switches (no weight copies, no arithmetic) are compiled into separate instances
   const bool dbg = (p.timing_mode & (2u | 4u | 16u | 64u | 128u)) != 0;  // (16: the diagnostic instance with nothing switched off, its own baseline)
-  auto kern = p.timing ? (dbg || p.tp_size > 1 ? decode_mega_kernel<true, true, true> : decode_mega_kernel<true, false, false>)
-              : dbg    ? decode_mega_kernel<false, true, true>
-              : p.tp_size > 1 ? decode_mega_kernel<false, false, true> : decode_mega_kernel<false, false, false>;
+  auto kern = p.f16 ? (p.timing ? decode_mega_kernel<true, false, false, true> : decode_mega_kernel<false, false, false, true>)
+              : p.timing ? (dbg || p.tp_size > 1 ? decode_mega_kernel<true, true, true, false> : decode_mega_kernel<true, false, false, false>)
+              : dbg      ? decode_mega_kernel<false, true, true, false>
+              : p.tp_size > 1 ? decode_mega_kernel<false, false, true, false> : decode_mega_kernel<false, false, false, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   void *args[] = {(void *)&p};
@@ -1495,9 +1569,9 @@ cudaError_t launch_decode_mega(const MegaParams &p, int grid, cudaStream_t s) {
 }
 
 cudaError_t decode_mega_occupancy(size_t smem, int *blocks_per_sm) {
-  cudaError_t e = cudaFuncSetAttribute(decode_mega_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(decode_mega_kernel<false, false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, decode_mega_kernel<false, false, true>, THREADS, smem);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, decode_mega_kernel<false, false, true, false>, THREADS, smem);
 }
 
 }  // namespace vkl

@@ -265,7 +265,8 @@ struct MegaParams {
   float *host_logits;
   uint32_t *out_ids;
   uint32_t out_cap;
-  const uint8_t *embd;  // token embedding, Q8_0 tiled planes
+  uint32_t f16;         // FP16 weights: units of 32 rows x 16 columns without scales (mega_pack_f16), embedding rows of halves
+  const uint8_t *embd;  // token embedding, Q8_0 tiled planes (or rows of halves)
   uint32_t embd_rows;
   uint32_t *x, *q, *k, *v, *ao;  // tagged words (see MegaOp)
   const float *freqc, *freqs;
@@ -300,6 +301,7 @@ size_t decode_mega_xs_bytes(uint32_t max_blocks, uint32_t head_dim);
 // (layout and row rules at MegaOp). tiles = the stream's 32-row tiles.
 cudaError_t launch_mega_pack(const uint8_t *const planes[3], uint32_t nmat, int swiglu, uint32_t N, uint32_t K, uint32_t tiles,
                              uint32_t grid, uint8_t *stream, cudaStream_t s);
+cudaError_t launch_mega_pack_f16(const __half *const w[3], uint32_t nmat, int swiglu, uint32_t N, uint32_t K, uint32_t tiles, uint32_t grid, uint8_t *stream, cudaStream_t s);
 size_t decode_mega_smem(size_t xs_bytes, uint32_t nst, uint32_t red_slots, uint32_t runs);
 // The most tiles that one warp's share of an op of `tiles` tiles touches.
 uint32_t decode_mega_red_slots(uint32_t tiles, uint32_t blocks, uint32_t grid);

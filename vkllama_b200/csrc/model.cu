@@ -285,14 +285,19 @@ int launch_advance(vkl_model *m, uint32_t pos_inc) {
   return VKL_OK;
 }
 
-// Builds the op table of the persistent decode kernel. Q8_0 weights, one GPU.
+// Builds the op table of the persistent decode kernel. Q8_0 weights, on any number of GPUs, or FP16 weights. Four 7B blocks of FP16
+// weights, ms for a 17-token prompt and 32 tokens: 14.3 with five kernels per block in a graph, 11.6 here (a new model's
+// first call, packing included, 14.8 and 12.8).
 // VKLLAMA_DECODE=graph keeps the multi-kernel CUDA-graph step instead.
 int build_mega(vkl_model *m) {
   if (m->mega_tried) return VKL_OK;
   m->mega_tried = true;
   const char *env = getenv("VKLLAMA_DECODE");
   if (env && !strcmp(env, "graph")) return VKL_OK;
-  if (!q8(m) || m->tok_embd->dtype != VKL_Q8_0) return VKL_OK;
+  if (m->dec) return VKL_OK;  // the layer-list decoders have kernels of their own
+  const bool f16 = !q8(m);
+  if (m->tok_embd->dtype != (f16 ? VKL_FP16 : VKL_Q8_0)) return VKL_OK;
+  const uint32_t columns = f16 ? 16 : 32, unit_bytes = MEGA_UNIT_CODES + (f16 ? 0 : MEGA_UNIT_SCALES);
   const uint32_t tp = m->cfg.tp_size;
   if (tp > 1 && !m->tp_connected) return fail(VKL_FAILED_PRECONDITION, "model: tensor-parallel ranks are not connected (vkl_model_tp_connect)");
   const vkl_model_config &c = m->cfg;
@@ -318,7 +323,7 @@ int build_mega(vkl_model *m) {
   const char *sr_env = getenv("VKLLAMA_SPLIT_ROWS");
   const uint32_t split_rows = sr_env ? (uint32_t)atoi(sr_env) : 384u;
   const size_t xs_bytes = decode_mega_xs_bytes(max_blocks, m->head_dim);
-  auto slots = [&](uint32_t tiles, uint32_t k) { return decode_mega_red_slots(tiles, k / 32, (uint32_t)G); };
+  auto slots = [&](uint32_t tiles, uint32_t k) { return decode_mega_red_slots(tiles, k / columns, (uint32_t)G); };
   const uint32_t red_slots = std::max({slots(3 * ((m->dim_l + 31) / 32), c.dim), slots((c.dim + 31) / 32, m->dim_l), slots((m->ffn_l + 15) / 16, c.dim),
                                        slots((c.dim + 31) / 32, m->ffn_l), slots((m->vocab_l + 31) / 32, c.dim)});
   const uint32_t max_runs = 5 * c.layers + 1;  // four matrices and an attention op per block, the output layer
@@ -330,6 +335,22 @@ int build_mega(vkl_model *m) {
   VKL_CUDA(decode_mega_occupancy(decode_mega_smem(xs_bytes, nst, red_slots, max_runs), &occ));
   if (occ < 1) return VKL_OK;
   VKL_OKAY(ensure_rows(m, 1));
+  // The kernel reads a second copy of the matrices, all of it in one allocation (one per matrix took the first token of four 7B
+  // blocks 6 ms).
+  const bool packed = m->mega_packed != nullptr;  // an earlier build of the tables made it already
+  auto stream_bytes = [&](size_t tiles, size_t k) { return (tiles * (k / columns) * unit_bytes + 255) / 256 * 256; };
+  if (!packed) {
+    const size_t need = (size_t)c.layers * (stream_bytes(3 * (size_t)((m->dim_l + 31) / 32), c.dim) + stream_bytes((c.dim + 31) / 32, m->dim_l) +
+                                            stream_bytes((m->ffn_l + 15) / 16, c.dim) + stream_bytes((c.dim + 31) / 32, m->ffn_l)) +
+                        stream_bytes((m->vocab_l + 31) / 32, c.dim);
+    if (f16) {  // where memory is short the graph reads the first
+      size_t left = 0, total = 0;
+      VKL_CUDA(cudaMemGetInfo(&left, &total));
+      if (left < 2 * need) return VKL_OK;
+    }
+    if (const int st = tensor_new(m->dev, 1, 1, need / 4, VKL_UINT32, &m->mega_packed)) return f16 && st == VKL_RESOURCE_EXHAUSTED ? VKL_OK : st;
+  }
+  size_t packed_at = 0;
 
   std::vector<MegaOp> ops;
   uint32_t rot = 0;
@@ -345,7 +366,6 @@ int build_mega(vkl_model *m) {
   uint32_t *x = (uint32_t *)m->mega_ll->data(), *kb = x + c.dim, *qb = kb + m->dim_l, *vb = qb + m->dim_l, *ao = vb + m->dim_l, *tb = ao + m->dim_l;
   uint32_t x_writer = 0;  // index of the op that last wrote the residual stream x
   int pack_status = VKL_OK;
-  size_t pack_index = 0;
   auto matvec = [&](std::initializer_list<const vkl_tensor *> ws, const float *norm, float eps, const uint32_t *in, uint32_t src_op,
                     std::initializer_list<uint32_t *> outs, int epi) {
     MegaOp o = {};
@@ -354,7 +374,7 @@ int build_mega(vkl_model *m) {
     const vkl_tensor *w0 = *ws.begin();
     o.N = (uint32_t)w0->h;
     o.K = (uint32_t)w0->w;
-    o.blocks = o.K / 32;
+    o.blocks = o.K / columns;
     o.nmat = (uint32_t)ws.size();
     const bool swiglu = epi == EPI_SWIGLU;
     o.tiles = swiglu ? (o.N + 15) / 16 : o.nmat * ((o.N + 31) / 32);
@@ -364,20 +384,12 @@ int build_mega(vkl_model *m) {
       const uint8_t *planes[3] = {nullptr, nullptr, nullptr};
       int j = 0;
       for (const vkl_tensor *w : ws) planes[j++] = w->data();
-      const size_t units = (size_t)o.tiles * o.blocks;
-      const bool packed = pack_index < m->mega_packed.size();  // an earlier build of the tables packed it already
-      vkl_tensor *pk = packed ? m->mega_packed[pack_index] : nullptr;
+      uint8_t *codes = m->mega_packed->data() + packed_at;
+      packed_at += stream_bytes(o.tiles, o.K);
       if (!packed) {
-        if (int st = tensor_new(m->dev, 1, 1, units * (MEGA_UNIT_CODES + MEGA_UNIT_SCALES) / 4, VKL_UINT32, &pk)) {
-          pack_status = st;
-          return 0u;
-        }
-        m->mega_packed.push_back(pk);
-      }
-      ++pack_index;
-      uint8_t *codes = pk->data();
-      if (!packed) {
-        cudaError_t pe = launch_mega_pack(planes, o.nmat, swiglu ? 1 : 0, o.N, o.K, o.tiles, (uint32_t)G, codes, m->stream);
+        const __half *halves[3] = {(const __half *)planes[0], (const __half *)planes[1], (const __half *)planes[2]};
+        cudaError_t pe = f16 ? launch_mega_pack_f16(halves, o.nmat, swiglu ? 1 : 0, o.N, o.K, o.tiles, (uint32_t)G, codes, m->stream)
+                             : launch_mega_pack(planes, o.nmat, swiglu ? 1 : 0, o.N, o.K, o.tiles, (uint32_t)G, codes, m->stream);
         count_launches(1);
         if (pe != cudaSuccess && pack_status == VKL_OK) pack_status = fail(VKL_INTERNAL, "decode kernel: packing the weights failed: %s", cudaGetErrorString(pe));
       }
@@ -471,7 +483,7 @@ int build_mega(vkl_model *m) {
         // the CTA's units of the op are consecutive in the packed stream (mega_stream_tile)
         const uint32_t tl = (o.tiles - tile0 + G - 1) / G;
         const size_t unit = (size_t)mega_stream_tile(tile0, o.tiles, (uint32_t)G) * o.blocks;
-        runs[(size_t)cta * max_runs + counts[cta]++] = {o.codes + unit * (MEGA_UNIT_CODES + MEGA_UNIT_SCALES), tl * o.blocks, 0};
+        runs[(size_t)cta * max_runs + counts[cta]++] = {o.codes + unit * unit_bytes, tl * o.blocks, 0};
       }
     }
   }
@@ -506,6 +518,7 @@ int build_mega(vkl_model *m) {
   p.tok = (uint32_t *)m->toks->data();
   p.out_ids = (uint32_t *)m->out_ids->data();
   p.out_cap = m->out_cap;
+  p.f16 = f16;
   p.embd = m->tok_embd->data();
   p.embd_rows = (uint32_t)m->tok_embd->h;
   p.x = x; p.q = qb; p.k = kb; p.v = vb; p.ao = ao;  // tagged words
@@ -887,10 +900,10 @@ int vkl_model_destroy(vkl_model *m) {
 
 // New weights: the decode kernel's packed copies and tables, if already built, are stale.
 static void drop_packed(vkl_model *m) {
-  if (m->mega_packed.empty() && !m->mega_tried) return;
+  if (!m->mega_packed && !m->mega_tried) return;
   cudaStreamSynchronize(m->stream);
-  for (vkl_tensor *t : m->mega_packed) vkl_tensor_release(t);
-  m->mega_packed.clear();
+  vkl_tensor_release(m->mega_packed);
+  m->mega_packed = nullptr;
   for (vkl_tensor **t : {&m->mega_ops, &m->mega_sync, &m->mega_arg, &m->mega_attn, &m->mega_runs, &m->mega_counts, &m->mega_ll}) {
     vkl_tensor_release(*t);
     *t = nullptr;

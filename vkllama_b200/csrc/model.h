@@ -74,7 +74,7 @@ struct vkl_model {
   bool mega_ready = false, mega_tried = false;
   int mega_grid = 0;
   vkl_tensor *mega_ops = nullptr, *mega_sync = nullptr, *mega_arg = nullptr, *mega_attn = nullptr, *mega_runs = nullptr, *mega_counts = nullptr, *mega_ll = nullptr;
-  std::vector<vkl_tensor *> mega_packed;  // the ops' weight streams in the persistent kernel's layout
+  vkl_tensor *mega_packed = nullptr;  // the ops' weight streams in the persistent kernel's layout, one behind the other
   vkl::MegaParams mp;
   uint32_t mega_launches_per_token = 1;
   uint32_t sm_mhz = 0;  // measured SM clock, for the profiled launches' cycle counts
@@ -93,8 +93,7 @@ struct vkl_model {
     if (pin) cudaFreeHost(pin);
     for (auto &l : L)
       for (vkl_tensor *p : {l.attn_norm, l.ffn_norm, l.wq, l.wk, l.wv, l.wo, l.gate, l.up, l.down, l.kcache, l.vcache, l.state, l.ring}) vkl_tensor_release(p);
-    for (vkl_tensor *p : mega_packed) vkl_tensor_release(p);
-    for (vkl_tensor *p : {wide, tok_embd, output_norm, output, fc, fs, x, xn, q, k, v, ao, t, logits16, logits32, toks, state, out_ids, forced, argpart, attn_scratch, attn_counters, mega_ops, mega_sync, mega_arg, mega_attn, mega_runs, mega_counts, mega_ll})
+    for (vkl_tensor *p : {mega_packed, wide, tok_embd, output_norm, output, fc, fs, x, xn, q, k, v, ao, t, logits16, logits32, toks, state, out_ids, forced, argpart, attn_scratch, attn_counters, mega_ops, mega_sync, mega_arg, mega_attn, mega_runs, mega_counts, mega_ll})
       vkl_tensor_release(p);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
