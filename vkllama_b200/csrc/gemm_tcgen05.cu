@@ -444,21 +444,26 @@ cudaError_t launch_gemm_f16_tcgen05(const GemmParams &p, cudaStream_t s) {
 }
 
 namespace {
+struct WidenArgs {
+  const uint8_t *codes[3], *scales[3];
+  __half *out;
+};
 // Tiled planes -> row-major fp16(q * d), the values that the dequantising warps write. A thread turns eight codes each of two
 // rows; bound by memory (4096 x 11008: 24 us, 138 MB).
-__global__ void __launch_bounds__(256) widen_kernel(const uint8_t *__restrict__ codes, const uint8_t *__restrict__ scales, __half *__restrict__ out, Q8Layout L) {
+__device__ __forceinline__ void widen_rows(const uint8_t *__restrict__ codes, const uint8_t *__restrict__ scales, __half *__restrict__ out, const Q8Layout &L) {
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;  // (row tile, block, lane)
   const uint32_t lane = i & 31, g = lane >> 2, t = lane & 3, per = L.groups * 4;
-  const uint32_t tile = (uint32_t)((i >> 5) / per), b = (uint32_t)((i >> 5) % per), k = b * 32 + t * 8, row = tile * 16 + g;
+  const uint32_t unit = (uint32_t)(i >> 5), tile = unit / per, b = unit - tile * per, k = b * 32 + t * 8, row = tile * 16 + g;
   if (tile >= L.tiles || k >= L.K) return;
   const uint4 w = ldg_stream(codes + i * 16);
   const __half *d = reinterpret_cast<const __half *>(scales) + (((size_t)tile * L.groups + (b >> 2)) * 8 + g) * 8 + (b & 3);
+  const __half sc[2] = {d[0], d[4]};
   const uint32_t c[2][4] = {{codes_to_h2(w.x, false), codes_to_h2(w.x, true), codes_to_h2(w.y, false), codes_to_h2(w.y, true)},
                             {codes_to_h2(w.z, false), codes_to_h2(w.z, true), codes_to_h2(w.w, false), codes_to_h2(w.w, true)}};
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     if (row + 8 * r >= L.N) break;
-    const __half2 s = __half2half2(d[4 * r]);
+    const __half2 s = __half2half2(sc[r]);
     uint32_t v[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -468,11 +473,17 @@ __global__ void __launch_bounds__(256) widen_kernel(const uint8_t *__restrict__ 
     *reinterpret_cast<uint4 *>(out + (size_t)(row + 8 * r) * L.K + k) = make_uint4(v[0], v[1], v[2], v[3]);
   }
 }
+// Grid y: the matrices of one GEMM. A prompt of 509 rows through four 7B blocks took 1321 us with a launch per matrix and 64-bit
+// divisions, 1277 this way (and 1476 where the compiler could not see that stores and scales do not alias).
+__global__ void __launch_bounds__(256) widen_kernel(const WidenArgs a, Q8Layout L) {
+  const uint32_t m = blockIdx.y;
+  widen_rows(m == 0 ? a.codes[0] : m == 1 ? a.codes[1] : a.codes[2], m == 0 ? a.scales[0] : m == 1 ? a.scales[1] : a.scales[2], a.out + (size_t)m * L.N * L.K, L);
+}
 }  // namespace
 
 // A 128-row tile dequantises the whole matrix for itself, at the pace of its dequantising warps (0.67 us per K step of 128
 // columns); widened once, the matrix runs on the fp16 GEMM's tiles. A prompt through four 7B blocks, us, dequantised in the tiles /
-// widened: 128 rows 989 / 1139, 129 1361 / 1186, 256 1387 / 1207, 257 1613 / 1302, 509 2046 / 1385, 900 3386 / 1816, 2048 6639 / 3102.
+// widened: 100 rows 937 / -, 128 rows 989 / 1077, 129 1361 / 1077, 256 1387 / 1117, 509 2046 / 1277, 900 3386 / 1716, 2048 6639 / 3015.
 // Only vkl_model keeps the room (GemmParams::wide); the operator classes dequantise in the tiles at any number of rows.
 constexpr uint32_t kWideRows = 129;
 bool gemm_q8_wide(uint32_t M) {
@@ -487,13 +498,15 @@ cudaError_t launch_gemm_q8_tcgen05(const GemmParams &p, cudaStream_t s) {
     const Q8Layout L = q8_layout(p.N, p.K);
     const size_t threads = (size_t)L.tiles * L.groups * 4 * 32;
     GemmParams h = p;
+    WidenArgs a = {{}, {}, p.wide};
     for (uint32_t i = 0; i < p.nmat; ++i) {
-      __half *w = p.wide + (size_t)i * p.N * p.K;
-      widen_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(p.w_codes[i], p.w_scales[i], w, L);
-      cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) return e;
-      h.w[i] = w;
+      a.codes[i] = p.w_codes[i];
+      a.scales[i] = p.w_scales[i];
+      h.w[i] = p.wide + (size_t)i * p.N * p.K;
     }
+    widen_kernel<<<dim3((unsigned)((threads + 255) / 256), p.nmat), 256, 0, s>>>(a, L);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
     return launch_gemm_f16_tcgen05(h, s);
   }
   switch (pick_bn_q8(p.M, p.N, p.nmat, p.swiglu)) {

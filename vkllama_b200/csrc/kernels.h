@@ -340,7 +340,7 @@ constexpr uint32_t GEMM_Q8_MIN_ROWS = 64;  // below this launch_matvec, whose ke
 cudaError_t launch_gemm_q8_tcgen05(const GemmParams &p, cudaStream_t s);
 // Whether the Q8_0 matrices are turned into fp16 once, in GemmParams::wide, and multiplied as such.
 bool gemm_q8_wide(uint32_t M);
-inline uint32_t gemm_launches(const GemmParams &p) { return !p.w[0] && p.wide && gemm_q8_wide(p.M) ? p.nmat + 1 : 1; }
+inline uint32_t gemm_launches(const GemmParams &p) { return !p.w[0] && p.wide && gemm_q8_wide(p.M) ? 2 : 1; }
 // Rows from which a weight of this kind goes to the tensor-core GEMM.
 inline uint32_t gemm_min_rows(bool q8) { return q8 ? GEMM_Q8_MIN_ROWS : GEMM_MIN_ROWS; }
 // Dispatch on the weight kind: w[0] set = FP16 weights, else w_codes / w_scales = Q8_0.
