@@ -21,8 +21,11 @@ pytestmark = pytest.mark.gpu
     (640, 5, 1696, 500, 383),  # heads of 128, the last row of one split, then two
     (160, 2, 416, 997, 30),    # heads of 80: half-filled lanes
     (480, 5, 1280, 997, 30),   # heads of 96
+    (120, 5, 200, 997, 30),    # FP16 widths that are no multiples of 32: the graph
 ])
 def test_one_token_calls_match_the_oracle(dev, f16, dim, heads, ffn, vocab, pos):
+    if dim % 32 and not f16:
+        pytest.skip("Q8_0 rows are whole blocks")
     cfg = dict(dim=dim, heads=heads, ffn=ffn, vocab=vocab, layers=2, maxlen=512)
     om = O.Model(seed=91, fp16=f16, **cfg)
     dm = vk.Model(dev, dim, heads, ffn, vocab, 2, 512, weight_dtype=vk.FP16 if f16 else vk.Q8_0)

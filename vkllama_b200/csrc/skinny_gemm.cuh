@@ -10,8 +10,9 @@
 // weights) by TMA tensor copies, Q8_0 planes by bulk copies, a few large ones per chunk, since issuing a copy takes a
 // warp some 60 cycles (a copy per row of X was twice as slow as the mat-vec kernel). Sixteen warps: each takes a pair of 16-row
 // tiles (with SwiGLU a gate and an up tile) and one 32-column block of the chunk, so that an X fragment serves two
-// tiles. The warps' K shares are added in a fixed order at the end. 64 to 128 registers; at the cap of 128 (one CTA per SM) some of those of 33 rows and more
-// spill 8 to 52 bytes.
+// tiles. The warps' K shares are added in a fixed order at the end. 62 to 128 registers; at the cap of 128 (one CTA per SM) some of those of 33 rows and more
+// spill 4 to 16 bytes (12 to 52 with 64-bit shared addresses). MMAs whose order the scheduler may choose and 32-bit shared addresses, us per call of
+// four 13B blocks before / now: FP16 17 rows 916 / 848, 45 858 / 836, Q8_0 17 rows 848 / 823, 45 977 / 955 (about 10 of each are the call's).
 //
 // Included by skinny_gemm.cu (Q8_0, and the rule) and skinny_gemm_f16.cu. In one file the 48 kernels with their line tables were 10 MB, from which
 // size on nvcc compresses device code: a process's first launch took 9.3 ms to unpack and load them, 3.2 (Q8_0) and 3.6 ms (FP16) now.
@@ -46,13 +47,30 @@ template <int MT, bool Q8, int PAIRS> struct SkinnyCfg {
 __device__ __forceinline__ uint32_t swap3(uint32_t g) { return (g & 1u) << 2 | g >> 1; }
 __device__ __forceinline__ uint32_t unswap3(uint32_t r) { return (r & 3u) << 1 | r >> 2; }
 
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ __half lds_half(uint32_t a) {
+  unsigned short v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
+  return __ushort_as_half(v);
+}
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
+// (Not volatile, the order is the scheduler's to choose.)
 __device__ __forceinline__ void mma16816_zero(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+
+__device__ __forceinline__ void mma16816_onto(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 template <int MT, int EPI, bool Q8, int PAIRS>
@@ -88,6 +106,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int mt = 0; mt < MT; ++mt) acc[i][mt][0] = acc[i][mt][1] = acc[i][mt][2] = acc[i][mt][3] = 0.f;
   const uint32_t pair = warp / C::KQ, kq = warp % C::KQ, sub = kq >> 1;
   const uint32_t row = swap3(g), piece = ((((kq & 1u) << 2) + t) ^ row) * 16;
+  // this lane's pieces of a stage: inputs, weights (of the pair's first tile), scales
+  const uint32_t x_at = sa(smem) + sub * (MT * 1024) + row * 128 + piece;
+  const uint32_t w_at = sa(smem) + C::X_BYTES + pair * 2 * C::TILE + (Q8 ? kq * 512 + lane * 16 : sub * 2048 + row * 128 + piece);
+  const uint32_t d_at = sa(smem) + C::X_BYTES + pair * 2 * C::TILE + C::CODES + (kq >> 2) * 128 + g * 16 + (kq & 3) * 2;
   uint32_t tiles_here = 0;
   for (uint32_t i = 0; i < C::TILES; ++i) tiles_here += tile_of(i) < ntiles ? 1u : 0u;
 
@@ -136,15 +158,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       break;
     }
     if (c * C::KQ + kq < blocks) {  // uniform over the warp; the last chunk may be short. Rows beyond N hold anything and are not stored
-      const unsigned char *xs = smem + s * C::STAGE + sub * (MT * 1024) + row * 128 + piece;
-      const unsigned char *ws = smem + s * C::STAGE + C::X_BYTES + pair * 2 * C::TILE;
+      const uint32_t xs = x_at + s * C::STAGE, ws = w_at + s * C::STAGE;
       uint32_t A0[2][4], A1[2][4];
       float d_lo[2], d_hi[2];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const unsigned char *w = ws + i * C::TILE;
         if constexpr (Q8) {
-          const uint4 cw = *reinterpret_cast<const uint4 *>(w + kq * 512 + lane * 16);
+          const uint4 cw = lds128(ws + i * C::TILE);
           A0[i][0] = codes_to_h2(cw.x, false);
           A0[i][1] = codes_to_h2(cw.z, false);
           A0[i][2] = codes_to_h2(cw.x, true);
@@ -153,12 +173,11 @@ __global__ void __launch_bounds__(kThreads, 1)
           A1[i][1] = codes_to_h2(cw.w, false);
           A1[i][2] = codes_to_h2(cw.y, true);
           A1[i][3] = codes_to_h2(cw.w, true);
-          const __half *d = reinterpret_cast<const __half *>(w + C::CODES + (kq >> 2) * 128 + g * 16) + (kq & 3);
-          d_lo[i] = __half2float(d[0]);
-          d_hi[i] = __half2float(d[4]);
+          const uint32_t d = d_at + s * C::STAGE + i * C::TILE;
+          d_lo[i] = __half2float(lds_half(d));
+          d_hi[i] = __half2float(lds_half(d + 8));
         } else {
-          const unsigned char *f = w + sub * 2048 + row * 128 + piece;
-          const uint4 r0 = *reinterpret_cast<const uint4 *>(f), r8 = *reinterpret_cast<const uint4 *>(f + 1024);
+          const uint4 r0 = lds128(ws + i * C::TILE), r8 = lds128(ws + i * C::TILE + 1024);
           A0[i][0] = r0.x; A0[i][1] = r8.x; A0[i][2] = r0.y; A0[i][3] = r8.y;
           A1[i][0] = r0.z; A1[i][1] = r8.z; A1[i][2] = r0.w; A1[i][3] = r8.w;
           d_lo[i] = d_hi[i] = 1.f;
@@ -166,21 +185,25 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
-        const uint4 X = *reinterpret_cast<const uint4 *>(xs + mt * 1024);
+        const uint4 X = lds128(xs + mt * 1024);
+        if constexpr (Q8) {
+          float v[2][4];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          if constexpr (Q8) {
-            float v[4];
-            mma16816_zero(v, A0[i][0], A0[i][1], A0[i][2], A0[i][3], X.x, X.y);
-            mma16816(v, A1[i][0], A1[i][1], A1[i][2], A1[i][3], X.z, X.w);
-            acc[i][mt][0] = fmaf(v[0], d_lo[i], acc[i][mt][0]);
-            acc[i][mt][1] = fmaf(v[1], d_lo[i], acc[i][mt][1]);
-            acc[i][mt][2] = fmaf(v[2], d_hi[i], acc[i][mt][2]);
-            acc[i][mt][3] = fmaf(v[3], d_hi[i], acc[i][mt][3]);
-          } else {
-            mma16816(acc[i][mt], A0[i][0], A0[i][1], A0[i][2], A0[i][3], X.x, X.y);
-            mma16816(acc[i][mt], A1[i][0], A1[i][1], A1[i][2], A1[i][3], X.z, X.w);
+          for (int i = 0; i < 2; ++i) mma16816_zero(v[i], A0[i][0], A0[i][1], A0[i][2], A0[i][3], X.x, X.y);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) mma16816_onto(v[i], A1[i][0], A1[i][1], A1[i][2], A1[i][3], X.z, X.w);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            acc[i][mt][0] = fmaf(v[i][0], d_lo[i], acc[i][mt][0]);
+            acc[i][mt][1] = fmaf(v[i][1], d_lo[i], acc[i][mt][1]);
+            acc[i][mt][2] = fmaf(v[i][2], d_hi[i], acc[i][mt][2]);
+            acc[i][mt][3] = fmaf(v[i][3], d_hi[i], acc[i][mt][3]);
           }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 2; ++i) mma16816_onto(acc[i][mt], A0[i][0], A0[i][1], A0[i][2], A0[i][3], X.x, X.y);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) mma16816_onto(acc[i][mt], A1[i][0], A1[i][1], A1[i][2], A1[i][3], X.z, X.w);
         }
       }
     }
