@@ -303,10 +303,10 @@ const char *vkl_model_architectures(void);
  * cannot reach `far`. */
 int vkl_distance_bucket(uint32_t n, uint32_t rows, uint32_t far);
 /* llama2_infer's loop (app/llama2_infer.cpp:141-210) with the greedy pick kept
- * on the device: prefill `prompt`, then n_gen - 1 one-token steps. With Q8_0 weights a
- * step is one launch of the persistent decode kernel (all ops of the token in one
- * cooperative launch); with FP16 weights, or under VKLLAMA_DECODE=graph, it is one replay
- * of a captured CUDA graph of five kernels per layer. out_ids receives n_gen ids.
+ * on the device: prefill `prompt`, then n_gen - 1 one-token steps. A step is one launch of
+ * the persistent decode kernel (all ops of the token in one cooperative launch); under
+ * VKLLAMA_DECODE=graph, and with FP16 weights whose second copy the device has no room for,
+ * it is one replay of a captured CUDA graph of five kernels per layer. out_ids receives n_gen ids.
  * prefill_ms / decode_ms, when not NULL, receive the device time of the two phases. */
 int vkl_model_generate(vkl_model *m, const uint32_t *prompt, size_t n_prompt, size_t n_gen,
                        uint32_t *out_ids, float *prefill_ms, float *decode_ms);

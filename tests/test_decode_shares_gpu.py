@@ -21,11 +21,8 @@ pytestmark = pytest.mark.gpu
     (640, 5, 1696, 500, 383),  # heads of 128, the last row of one split, then two
     (160, 2, 416, 997, 30),    # heads of 80: half-filled lanes
     (480, 5, 1280, 997, 30),   # heads of 96
-    (120, 5, 200, 997, 30),    # FP16 widths that are no multiples of 32: the graph
 ])
 def test_one_token_calls_match_the_oracle(dev, f16, dim, heads, ffn, vocab, pos):
-    if dim % 32 and not f16:
-        pytest.skip("Q8_0 rows are whole blocks")
     cfg = dict(dim=dim, heads=heads, ffn=ffn, vocab=vocab, layers=2, maxlen=512)
     om = O.Model(seed=91, fp16=f16, **cfg)
     dm = vk.Model(dev, dim, heads, ffn, vocab, 2, 512, weight_dtype=vk.FP16 if f16 else vk.Q8_0)
@@ -36,4 +33,19 @@ def test_one_token_calls_match_the_oracle(dev, f16, dim, heads, ffn, vocab, pos)
     for i in range(pos, pos + 3):
         want, got = om.forward(text[i:i + 1], i), dm(text[i:i + 1], i)
         assert np.abs(got - want).max() <= LOGITS_MAX_ABS, i
+    dm.close()
+
+
+def test_fp16_decode_without_the_persistent_kernel(dev, monkeypatch):
+    """The plan that a model falls back to where the device has no room for the decode kernel's copy of its weights."""
+    cfg = dict(dim=256, heads=4, ffn=512, vocab=997, layers=2, maxlen=64)
+    om = O.Model(seed=92, fp16=True, **cfg)
+    text = O.synth_tokens(92, 1000, 12, 997)
+    monkeypatch.setenv("VKLLAMA_DECODE", "graph")
+    dm = vk.Model(dev, 256, 4, 512, 997, 2, 64, weight_dtype=vk.FP16)
+    load_from_oracle(dm, om)
+    om.forward(text[:9], 0)
+    dm(text[:9], 0)
+    for i in range(9, 12):
+        assert np.abs(dm(text[i:i + 1], i) - om.forward(text[i:i + 1], i)).max() <= LOGITS_MAX_ABS, i
     dm.close()

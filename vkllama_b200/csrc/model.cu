@@ -286,8 +286,8 @@ int launch_advance(vkl_model *m, uint32_t pos_inc) {
 }
 
 // Builds the op table of the persistent decode kernel. Q8_0 weights, on any number of GPUs, or FP16 weights. Four 7B blocks of FP16
-// weights, ms for a 17-token prompt and 32 tokens: 14.3 with five kernels per block in a graph, 11.6 here (a new model's
-// first call, packing included, 14.8 and 12.8).
+// weights, ms for a 17-token prompt and 32 tokens: 14.3 with five kernels per block in a graph, 11.6 here (a new
+// model's first call, packing included, 14.8 and 12.8; 15.0 and 16.5 where the copy's 1.9 GB come from the device and not from the pool).
 // VKLLAMA_DECODE=graph keeps the multi-kernel CUDA-graph step instead.
 int build_mega(vkl_model *m) {
   if (m->mega_tried) return VKL_OK;
