@@ -1,0 +1,51 @@
+"""Which plan a one-token call takes, and what it does where the persistent decode kernel's tables cannot be built, its waits run
+out, or the device has little memory left for the second copy of the weights."""
+import numpy as np
+import pytest
+
+import vkllama_b200 as vk
+from oracle import oracle as O
+from test_model_gpu import fill
+
+pytestmark = pytest.mark.gpu
+
+
+def launches(call):
+    before = vk.kernel_launches()
+    out = call()
+    return out, vk.kernel_launches() - before
+
+
+def model(dev, dims, f16, seed):
+    dm = vk.Model(dev, *dims, weight_dtype=vk.FP16 if f16 else vk.Q8_0)
+    dm.synth_weights(seed)
+    return dm
+
+
+def test_tables_that_could_not_be_built_are_not_taken_for_built(dev):
+    """The decode kernel's copy of the weights gets its 128 MiB, the small buffer after it gets nothing: the call fails. Once there
+    is room, a call of more rows has the tables built again, and the copy must be filled then."""
+    dims = (4096, 32, 4096, 500, 1, 64)
+    prompt, tok = O.synth_tokens(51, 1000, 20, 500), np.array([7], np.uint32)
+    room = vk.Tensor(1, 4, 1 << 23, dev, vk.FP32)
+    roomy = model(dev, dims, False, 51)
+    roomy(prompt, 0)
+    want = roomy(tok, 20)
+    roomy.close()
+    dm = model(dev, dims, False, 51)
+    dm(prompt[:8], 0)
+    filler = fill(dev, 8)
+    try:
+        with pytest.raises(vk.VklError):
+            while True:
+                filler.append(vk.Tensor(1, 1, 24 << 10, dev, vk.FP32))  # as large as the small buffer
+        del room  # the pool keeps it, for a request of its size
+        with pytest.raises(vk.VklError) as e:
+            dm(tok, 8)
+        assert e.value.code == 8
+    finally:
+        del filler
+    dm(prompt, 0)
+    got, n = launches(lambda: dm(tok, 20))
+    assert (got == want).all() and n == 6  # five streams packed, one launch for the token
+    dm.close()

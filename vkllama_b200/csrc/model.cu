@@ -44,6 +44,20 @@ namespace {
 
 bool q8(const vkl_model *m) { return m->cfg.weight_dtype == VKL_Q8_0; }
 
+// The tables of the persistent decode kernel hold pointers to the activations and to the weights. Its copy of the weights does
+// not depend on the activations: `copy` gives that back too. (Nothing of the model is in flight.)
+void release_mega(vkl_model *m, bool copy) {
+  for (vkl_tensor **t : {&m->mega_ops, &m->mega_sync, &m->mega_arg, &m->mega_attn, &m->mega_runs, &m->mega_counts, &m->mega_ll}) {
+    vkl_tensor_release(*t);
+    *t = nullptr;
+  }
+  if (copy) {
+    vkl_tensor_release(m->mega_packed);
+    m->mega_packed = nullptr;
+  }
+  m->mega_ready = false;
+}
+
 bool use_gemm(const vkl_model *m, uint32_t rows);
 int ensure_rows(vkl_model *m, uint32_t T) {
   if (T <= m->cap_T) return VKL_OK;
@@ -51,13 +65,8 @@ int ensure_rows(vkl_model *m, uint32_t T) {
   model_drop_graph(m);  // the graph holds the old buffers
   VKL_CUDA(cudaStreamSynchronize(m->stream));
   m->cap_T = 0;  // an allocation that fails below leaves buffers missing: the next call makes them anew
-  if (m->mega_tried) {  // the op table of the persistent kernel holds the old buffers too
-    for (vkl_tensor **t : {&m->mega_ops, &m->mega_sync, &m->mega_arg, &m->mega_attn, &m->mega_runs, &m->mega_counts, &m->mega_ll}) {
-      vkl_tensor_release(*t);
-      *t = nullptr;
-    }
-    m->mega_ready = m->mega_tried = false;  // the packed weight streams (mega_packed) do not depend on the row count: kept
-  }
+  release_mega(m, false);
+  m->mega_tried = false;
   const size_t D = m->cfg.dim;
   VKL_OKAY(ensure_tensor(m->dev, &m->x, 1, T, D, VKL_FP16));
   VKL_OKAY(ensure_tensor(m->dev, &m->xn, 1, T, D, VKL_FP16));
@@ -289,9 +298,7 @@ int launch_advance(vkl_model *m, uint32_t pos_inc) {
 // weights, ms for a 17-token prompt and 32 tokens: 14.3 with five kernels per block in a graph, 11.6 here (a new
 // model's first call, packing included, 14.8 and 12.8; 15.0 and 16.5 where the copy's 1.9 GB come from the device and not from the pool).
 // VKLLAMA_DECODE=graph keeps the multi-kernel CUDA-graph step instead.
-int build_mega(vkl_model *m) {
-  if (m->mega_tried) return VKL_OK;
-  m->mega_tried = true;
+int make_mega(vkl_model *m) {
   const char *env = getenv("VKLLAMA_DECODE");
   if (env && !strcmp(env, "graph")) return VKL_OK;
   if (m->dec) return VKL_OK;  // the layer-list decoders have kernels of their own
@@ -337,7 +344,7 @@ int build_mega(vkl_model *m) {
   VKL_OKAY(ensure_rows(m, 1));
   // The kernel reads a second copy of the matrices, all of it in one allocation (one per matrix took the first token of four 7B
   // blocks 6 ms).
-  const bool packed = m->mega_packed != nullptr;  // an earlier build of the tables made it already
+  const bool packed = m->mega_packed != nullptr;  // an earlier build of the tables, which succeeded, made it already
   auto stream_bytes = [&](size_t tiles, size_t k) { return (tiles * (k / columns) * unit_bytes + 255) / 256 * 256; };
   if (!packed) {
     const size_t need = (size_t)c.layers * (stream_bytes(3 * (size_t)((m->dim_l + 31) / 32), c.dim) + stream_bytes((c.dim + 31) / 32, m->dim_l) +
@@ -554,6 +561,16 @@ int build_mega(vkl_model *m) {
   m->mega_grid = G;
   m->mega_ready = true;
   return VKL_OK;
+}
+int build_mega(vkl_model *m) {
+  if (m->mega_tried) return VKL_OK;
+  m->mega_tried = true;
+  const int st = make_mega(m);
+  if (!m->mega_ready) {  // a copy that was allocated is not one that was filled: the next build starts from nothing
+    cudaStreamSynchronize(m->stream);
+    release_mega(m, true);
+  }
+  return st;
 }
 
 __global__ void bump_sequence_kernel(uint32_t *seq, uint32_t by) { *seq += by; }
@@ -902,13 +919,8 @@ int vkl_model_destroy(vkl_model *m) {
 static void drop_packed(vkl_model *m) {
   if (!m->mega_packed && !m->mega_tried) return;
   cudaStreamSynchronize(m->stream);
-  vkl_tensor_release(m->mega_packed);
-  m->mega_packed = nullptr;
-  for (vkl_tensor **t : {&m->mega_ops, &m->mega_sync, &m->mega_arg, &m->mega_attn, &m->mega_runs, &m->mega_counts, &m->mega_ll}) {
-    vkl_tensor_release(*t);
-    *t = nullptr;
-  }
-  m->mega_ready = m->mega_tried = false;
+  release_mega(m, true);
+  m->mega_tried = false;
 }
 
 int vkl_model_set_weight(vkl_model *m, const char *name, int dtype, const void *data, size_t bytes) {
