@@ -1,5 +1,5 @@
-"""Which plan a one-token call takes, and what it does where the persistent decode kernel's tables cannot be built, its waits run
-out, or the device has little memory left for the second copy of the weights."""
+"""Which plan a one-token call takes, and what it does where the persistent decode kernel's tables cannot be built or
+the device has little memory left for the second copy of the weights."""
 import numpy as np
 import pytest
 

@@ -1,5 +1,5 @@
 """What the host does with the word that a kernel raises when one of its bounded waits has run out. The word is set from the
-host (tests/cpp/error_word.cu reaches it); no wait runs out on the GPU."""
+host (tests/cpp/error_word.cu reaches it), or the decode kernel's bound made so short that healthy waits run out."""
 import ctypes as C
 import os
 import subprocess
@@ -20,8 +20,10 @@ def words(tmp_path_factory):
     so = str(tmp_path_factory.mktemp("words") / "error_word.so")
     subprocess.check_call([B.NVCC] + B.FLAGS + ["-shared", "-I", B.CSRC, os.path.join(ROOT, "tests", "cpp", "error_word.cu"), "-o", so])
     L = C.CDLL(so)
-    for f in (L.raise_model_word, L.command_is_watched, L.raise_command_word):
+    for f in (L.raise_model_word, L.command_is_watched, L.raise_command_word, L.decode_word):
         f.argtypes = [C.c_void_p]
+    L.decode_word.restype = C.c_uint32
+    L.set_polls.argtypes = [C.c_void_p, C.c_uint32]
     return L
 
 
@@ -44,6 +46,30 @@ def test_model_calls_report_their_own_waits(dev, words):
         dm(np.arange(33, dtype=np.uint32), 0)
     assert e.value.code == 13
     dm(np.arange(33, dtype=np.uint32), 0)
+    dm.close()
+
+
+def test_a_decode_wait_that_ran_out_on_any_sm_is_reported(dev, words):
+    """CTA 0 has the only tile of the output layer (148 tiles lie before it), so the others wait for it at the end, and it for nobody.
+    With a bound of a few dozen polls some of them give up there while it ends the launch. A call that succeeds leaves no word
+    behind for a later call."""
+    dm = vk.Model(dev, 256, 4, 544, 32, 2, 64)
+    dm.synth_weights(73)
+    tok = np.array([7], np.uint32)
+    dm(tok, 0)
+    want = dm(tok, 1)
+    failed = 0
+    for polls in list(range(20, 84)) * 3:
+        words.set_polls(dm.h, polls)
+        try:
+            assert (dm(tok, 1) == want).all(), polls
+        except vk.VklError as e:
+            assert e.code == 13 and "bounded wait ran out" in e.message
+            failed += 1
+        assert words.decode_word(dm.h) == 0, polls
+    assert failed
+    dm.set_wait_limit(0)
+    assert (dm(tok, 1) == want).all()
     dm.close()
 
 

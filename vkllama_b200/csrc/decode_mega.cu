@@ -1228,7 +1228,6 @@ __device__ VKL_SLOW void argmax_final_op(const Ctx &c, float *sm, uint32_t pos0,
       p.state[3] = ar_done;
       p.state[7] = next_ebase;
       p.bar[1] = rounds_done;
-      // (every CTA has passed the grid barrier: none of them can raise an error any more)
       if (p.host_logits) reinterpret_cast<uint32_t *>(p.host_logits)[p.vocab] = 0u;
     }
   }
@@ -1454,6 +1453,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
     }
   }
   if ((threadIdx.x & 31) == 0 && !ring.lead && (!DBG || !(p.timing_mode & 128u))) ring_drain(p, ring);
+  // A CTA that gave up has published words computed from whatever it had, and CTA 0 may have ended the launch with them all the
+  // same. (Its threads have met since it gave up, in the last op's barrier; CTA 0's own late waits are this thread's.)
+  if (threadIdx.x == 0 && p.host_logits && c.aborted()) reinterpret_cast<uint32_t *>(p.host_logits)[p.vocab + 1] = 1u;
 }
 
 }  // namespace

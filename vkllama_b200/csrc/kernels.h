@@ -260,7 +260,8 @@ struct MegaParams {
   const uint32_t *forced;  // prompt ids: while position+1 < state[5] the next input is forced[position+1]
   uint32_t *tok;      // current token id
   // A one-token call of a host-driven loop: position and token come with the launch (instead of state[0] and tok), and the output
-  // layer writes its fp32 logits to page-locked host memory as well, one word behind which the launch ends with a 0.
+  // layer writes its fp32 logits to page-locked host memory as well. Of the two words behind them CTA 0 sets the first to 0 when it
+  // ends the launch, and any CTA with a wait that ran out sets the second to 1.
   uint32_t with_token, call_pos, call_tok;
   float *host_logits;
   uint32_t *out_ids;

@@ -692,8 +692,9 @@ int fetch_logits(vkl_model *m, float *logits_out, bool decoded) {
 // One token through the persistent decode kernel, logits to the host: one launch and one synchronisation.
 int decode_call(vkl_model *m, uint32_t tok, uint32_t pos, float *logits_out) {
   VKL_OKAY(ensure_pin(m));
-  volatile uint32_t *left = (volatile uint32_t *)m->pin + m->vocab_l;
-  *left = 1;
+  volatile uint32_t *word = (volatile uint32_t *)m->pin + m->vocab_l;
+  word[0] = 1;  // CTA 0 clears it at the end
+  word[1] = 0;  // a CTA with a wait that ran out sets it
   MegaParams p = m->mp;
   p.with_token = 1;
   p.call_pos = pos;
@@ -701,7 +702,7 @@ int decode_call(vkl_model *m, uint32_t tok, uint32_t pos, float *logits_out) {
   p.host_logits = (float *)m->pin_dev;
   VKL_LAUNCH(1, launch_decode_mega(p, m->mega_grid, m->stream));
   VKL_CUDA(cudaStreamSynchronize(m->stream));
-  if (*left) {  // the launch gave up: its error word says where
+  if (word[0] || word[1]) {  // the error word says where the launch gave up
     VKL_OKAY(check_mega(m));
     return fail(VKL_INTERNAL, "decode kernel: the launch did not end");
   }
