@@ -6,6 +6,7 @@ import pytest
 import vkllama_b200 as vk
 from oracle import oracle as O
 from test_model_gpu import fill
+from util import LOGITS_MAX_ABS, load_from_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -48,4 +49,22 @@ def test_tables_that_could_not_be_built_are_not_taken_for_built(dev):
     dm(prompt, 0)
     got, n = launches(lambda: dm(tok, 20))
     assert (got == want).all() and n == 6  # five streams packed, one launch for the token
+    dm.close()
+
+
+@pytest.mark.parametrize("f16", [False, True])
+def test_separate_merge_leaves_out_splits_of_a_longer_sequence(dev, monkeypatch, f16):
+    """Four splits per head, then a shorter sequence with two: the merge must not add what the first sequence left in the others."""
+    monkeypatch.setenv("VKLLAMA_DECODE_COMBINE", "separate")
+    monkeypatch.setenv("VKLLAMA_SPLIT_ROWS", "32")
+    cfg = dict(dim=256, heads=4, ffn=512, vocab=997, layers=2, maxlen=256)
+    om = O.Model(seed=52, fp16=f16, **cfg)
+    dm = vk.Model(dev, 256, 4, 512, 997, 2, 256, weight_dtype=vk.FP16 if f16 else vk.Q8_0)
+    load_from_oracle(dm, om)
+    for seed, n in ((52, 120), (53, 50)):
+        text = O.synth_tokens(seed, 1000, n + 2, 997)
+        om.forward(text[:n], 0)
+        dm(text[:n], 0)
+        for i in (n, n + 1):
+            assert np.abs(dm(text[i:i + 1], i) - om.forward(text[i:i + 1], i)).max() <= LOGITS_MAX_ABS, (n, i)
     dm.close()

@@ -1093,18 +1093,18 @@ __device__ __forceinline__ void attn_part_op(const Ctx &c, const MegaOp &op, flo
   }
 }
 
-// One head per CTA: merge the split partials in split order.
-__device__ VKL_SLOW void attn_combine_op(const Ctx &c, uint32_t tag_out) {
+// One head per CTA: merge the partials of the token's S splits in split order (the places of further splits hold an earlier token's).
+__device__ VKL_SLOW void attn_combine_op(const Ctx &c, uint32_t S, uint32_t tag_out) {
   const MegaParams &p = c.p;
   const uint32_t h = blockIdx.x, tid = threadIdx.x, D = p.head_dim;
   if (h >= p.heads || tid >= D) return;
   const float *base = p.attn_scratch + (size_t)h * p.splits * (D + 4);
   float M = -INFINITY;
 #pragma unroll 1
-  for (uint32_t s = 0; s < p.splits; ++s) M = fmaxf(M, __ldcg(base + s * (D + 4) + D));
+  for (uint32_t s = 0; s < S; ++s) M = fmaxf(M, __ldcg(base + s * (D + 4) + D));
   float den = 0.f, num = 0.f;
 #pragma unroll 1
-  for (uint32_t s = 0; s < p.splits; ++s) {
+  for (uint32_t s = 0; s < S; ++s) {
     const float ms = __ldcg(base + s * (D + 4) + D), ls = __ldcg(base + s * (D + 4) + D + 1);
     if (ls > 0.f) {
       const float w = expf(ms - M);
@@ -1373,7 +1373,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
       case MK_ATTN_PART:
         attn_part_op<DBG, F16>(c, op, reinterpret_cast<float *>(xq), pos0, *kvp, tag(op.src_op), tag(op.tag_op), tab, ring);
         break;
-      case MK_ATTN_COMBINE: attn_combine_op(c, tag(oi)); break;
+      case MK_ATTN_COMBINE: attn_combine_op(c, S_eff, tag(oi)); break;
       case MK_ALLREDUCE:
         if (!TP) break;
         ++ar_i;
