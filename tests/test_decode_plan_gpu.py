@@ -68,3 +68,20 @@ def test_separate_merge_leaves_out_splits_of_a_longer_sequence(dev, monkeypatch,
         for i in (n, n + 1):
             assert np.abs(dm(text[i:i + 1], i) - om.forward(text[i:i + 1], i)).max() <= LOGITS_MAX_ABS, (n, i)
     dm.close()
+
+
+@pytest.mark.parametrize("f16", [False, True])
+def test_output_layers_beyond_a_grid_dimension(dev, monkeypatch, f16):
+    """A vocabulary of more than 65535 tiles of 32 rows."""
+    dims = (64, 2, 64, 2097300, 1, 64)
+    tok = np.array([2097299], np.uint32)
+    monkeypatch.setenv("VKLLAMA_DECODE", "graph")
+    graph = model(dev, dims, f16, 54)
+    want = graph(tok, 0)
+    graph.close()
+    monkeypatch.delenv("VKLLAMA_DECODE")
+    dm = model(dev, dims, f16, 54)
+    dm(tok, 0)
+    got, n = launches(lambda: dm(tok, 0))
+    assert n == 1 and np.abs(got - want).max() <= LOGITS_MAX_ABS
+    dm.close()

@@ -1482,9 +1482,10 @@ int decode_mega_max_stages() { return MAX_NST; }
 // read them. Tiles are stored in the order the decode kernel's CTAs take them (mega_stream_tile), so
 // that every CTA reads one consecutive range of the op.
 namespace {
+constexpr uint32_t kGridY = 65535;  // tiles of a launch: a vocabulary of 2.1 million rows has more
 __global__ void __launch_bounds__(64) mega_pack_kernel(const uint8_t *p0, const uint8_t *p1, const uint8_t *p2, uint32_t nmat, int swiglu, uint32_t N,
-                                                       uint32_t K, uint32_t tiles, uint32_t grid, uint8_t *stream) {
-  const uint32_t b = blockIdx.x, t = blockIdx.y, blocks = K / 32;
+                                                       uint32_t K, uint32_t tile0, uint32_t tiles, uint32_t grid, uint8_t *stream) {
+  const uint32_t b = blockIdx.x, t = tile0 + blockIdx.y, blocks = K / 32;
   const uint32_t half = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t tpm = (N + 31) / 32;
   // the 16-row plane tile behind this half of the 32-row tile
@@ -1522,8 +1523,9 @@ __global__ void __launch_bounds__(64) mega_pack_kernel(const uint8_t *p0, const 
 
 cudaError_t launch_mega_pack(const uint8_t *const planes[3], uint32_t nmat, int swiglu, uint32_t N, uint32_t K, uint32_t tiles, uint32_t grid,
                              uint8_t *stream, cudaStream_t s) {
-  if (K % 32 || tiles == 0 || tiles > 65535u || grid == 0) return cudaErrorInvalidValue;
-  mega_pack_kernel<<<dim3(K / 32, tiles), 64, 0, s>>>(planes[0], planes[1], planes[2], nmat, swiglu, N, K, tiles, grid, stream);
+  if (K % 32 || tiles == 0 || grid == 0) return cudaErrorInvalidValue;
+  for (uint32_t t = 0; t < tiles; t += kGridY)
+    mega_pack_kernel<<<dim3(K / 32, std::min(tiles - t, kGridY)), 64, 0, s>>>(planes[0], planes[1], planes[2], nmat, swiglu, N, K, t, tiles, grid, stream);
   return cudaGetLastError();
 }
 
@@ -1532,9 +1534,9 @@ cudaError_t launch_mega_pack(const uint8_t *const planes[3], uint32_t nmat, int 
 // in this order (for the input the same).
 namespace {
 // A CTA packs eight blocks of a tile, a warp each, so that it reads whole lines.
-__global__ void __launch_bounds__(256) mega_pack_f16_kernel(const __half *p0, const __half *p1, const __half *p2, uint32_t nmat, int swiglu, uint32_t N, uint32_t K, uint32_t tiles,
-                                                            uint32_t grid, uint8_t *stream) {
-  const uint32_t b = blockIdx.x * 8 + (threadIdx.x >> 5), t = blockIdx.y, blocks = K / 16, lane = threadIdx.x & 31, g = lane >> 2, c = b * 16 + (lane & 3) * 4;
+__global__ void __launch_bounds__(256) mega_pack_f16_kernel(const __half *p0, const __half *p1, const __half *p2, uint32_t nmat, int swiglu, uint32_t N, uint32_t K, uint32_t tile0,
+                                                            uint32_t tiles, uint32_t grid, uint8_t *stream) {
+  const uint32_t b = blockIdx.x * 8 + (threadIdx.x >> 5), t = tile0 + blockIdx.y, blocks = K / 16, lane = threadIdx.x & 31, g = lane >> 2, c = b * 16 + (lane & 3) * 4;
   if (b >= blocks) return;
   const uint32_t tpm = (N + 31) / 32;
   uint4 *dst = reinterpret_cast<uint4 *>(stream + ((size_t)mega_stream_tile(t, tiles, grid) * blocks + b) * MEGA_UNIT_CODES) + lane;
@@ -1550,8 +1552,9 @@ __global__ void __launch_bounds__(256) mega_pack_f16_kernel(const __half *p0, co
 }
 }  // namespace
 cudaError_t launch_mega_pack_f16(const __half *const w[3], uint32_t nmat, int swiglu, uint32_t N, uint32_t K, uint32_t tiles, uint32_t grid, uint8_t *stream, cudaStream_t s) {
-  if (K % 16 || tiles == 0 || tiles > 65535u || grid == 0) return cudaErrorInvalidValue;
-  mega_pack_f16_kernel<<<dim3((K / 16 + 7) / 8, tiles), 256, 0, s>>>(w[0], w[1], w[2], nmat, swiglu, N, K, tiles, grid, stream);
+  if (K % 16 || tiles == 0 || grid == 0) return cudaErrorInvalidValue;
+  for (uint32_t t = 0; t < tiles; t += kGridY)
+    mega_pack_f16_kernel<<<dim3((K / 16 + 7) / 8, std::min(tiles - t, kGridY)), 256, 0, s>>>(w[0], w[1], w[2], nmat, swiglu, N, K, t, tiles, grid, stream);
   return cudaGetLastError();
 }
 
