@@ -2,6 +2,7 @@
 the device has little memory left for the second copy of the weights."""
 import numpy as np
 import pytest
+import torch
 
 import vkllama_b200 as vk
 from oracle import oracle as O
@@ -84,4 +85,20 @@ def test_output_layers_beyond_a_grid_dimension(dev, monkeypatch, f16):
     dm(tok, 0)
     got, n = launches(lambda: dm(tok, 0))
     assert n == 1 and np.abs(got - want).max() <= LOGITS_MAX_ABS
+    dm.close()
+
+
+F16_DIMS = (4096, 32, 4096, 500, 1, 4096)  # the decode kernel's copy of these weights takes 256 MiB
+
+
+def test_a_single_generated_id_has_no_use_for_the_copy(dev):
+    dm = model(dev, F16_DIMS, True, 57)
+    prompt = O.synth_tokens(57, 1000, 20, 500)
+    dm(prompt, 0)
+    fill(dev, 1 << 20)  # (empties the pool, fills nothing)
+    free = [torch.cuda.mem_get_info()[0]]
+    for n in (1, 2):
+        dm.generate(prompt, n)
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] - free[1] < 64 << 20 < 200 << 20 < free[1] - free[2]
     dm.close()

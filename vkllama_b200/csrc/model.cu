@@ -1197,15 +1197,16 @@ int vkl_model_generate(vkl_model *m, const uint32_t *prompt, size_t n_prompt, si
   VKL_CUDA(cudaSetDevice(m->dev->ordinal));
   if (m->dec) VKL_OKAY(decoder_begin(m, 0));
   VKL_OKAY(ensure_rows(m, (uint32_t)n_prompt));
-  VKL_OKAY(prepare_decode(m));
-  const uint32_t st[2] = {0, 0};
-  VKL_CUDA(cudaMemcpyAsync(m->state->data(), st, 8, cudaMemcpyHostToDevice, m->stream));
-  VKL_CUDA(cudaMemcpyAsync(m->toks->data(), prompt, n_prompt * 4, cudaMemcpyHostToDevice, m->stream));
   // Tensor-parallel models (and VKLLAMA_PREFILL=sequential) prefill token by token through
   // the persistent decode kernel: while the position is inside the prompt the kernel feeds
   // itself the next prompt id instead of its arg-max.
   const char *pf = getenv("VKLLAMA_PREFILL");
   const bool by_token = pf && !strcmp(pf, "sequential");
+  // A prompt's first id takes no decode step: nor does it wait for the decode kernel's copy of the weights to be made.
+  if (n_gen > 1 || n_prompt == 1 || m->cfg.tp_size > 1 || by_token) VKL_OKAY(prepare_decode(m));
+  const uint32_t st[2] = {0, 0};
+  VKL_CUDA(cudaMemcpyAsync(m->state->data(), st, 8, cudaMemcpyHostToDevice, m->stream));
+  VKL_CUDA(cudaMemcpyAsync(m->toks->data(), prompt, n_prompt * 4, cudaMemcpyHostToDevice, m->stream));
   const bool sequential = m->mega_ready && n_prompt > 1 && (m->cfg.tp_size > 1 || by_token);
   if (m->cfg.tp_size > 1 && !m->mega_ready) return fail(VKL_UNIMPLEMENTED, "model_generate: tensor-parallel models need the persistent decode kernel");
   if (m->tp_failed) return decode_step(m);  // reports the state
