@@ -91,6 +91,37 @@ def test_output_layers_beyond_a_grid_dimension(dev, monkeypatch, f16):
 F16_DIMS = (4096, 32, 4096, 500, 1, 4096)  # the decode kernel's copy of these weights takes 256 MiB
 
 
+def test_fp16_copy_where_memory_is_short_and_where_the_pool_has_it(dev):
+    """No copy where less than twice its size is free (the graph then reads the weights as they are); blocks that the library's own
+    pool holds count as free."""
+    tok = np.array([7], np.uint32)
+    dm = model(dev, F16_DIMS, True, 55)
+    one = dm(tok, 0)
+    want, n = launches(lambda: dm(tok, 1))
+    assert n == 1
+    dm.close()
+    dm = model(dev, F16_DIMS, True, 55)
+    filler = fill(dev, 300)
+    try:
+        assert np.abs(dm(tok, 0) - one).max() <= LOGITS_MAX_ABS
+        got, n = launches(lambda: dm(tok, 1))
+    finally:
+        del filler
+    assert n > 5 and np.abs(got - want).max() <= LOGITS_MAX_ABS
+    dm.close()
+    dm = model(dev, F16_DIMS, True, 55)
+    pooled = vk.Tensor(1, 16, 1 << 23, dev, vk.FP32)
+    filler = fill(dev, 60)
+    try:
+        del pooled
+        dm(tok, 0)
+        got, n = launches(lambda: dm(tok, 1))
+    finally:
+        del filler
+    assert n == 1 and (got == want).all()
+    dm.close()
+
+
 def test_a_single_generated_id_has_no_use_for_the_copy(dev):
     dm = model(dev, F16_DIMS, True, 57)
     prompt = O.synth_tokens(57, 1000, 20, 500)

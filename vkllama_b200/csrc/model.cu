@@ -350,10 +350,10 @@ int make_mega(vkl_model *m) {
     const size_t need = (size_t)c.layers * (stream_bytes(3 * (size_t)((m->dim_l + 31) / 32), c.dim) + stream_bytes((c.dim + 31) / 32, m->dim_l) +
                                             stream_bytes((m->ffn_l + 15) / 16, c.dim) + stream_bytes((c.dim + 31) / 32, m->ffn_l)) +
                         stream_bytes((m->vocab_l + 31) / 32, c.dim);
-    if (f16) {  // where memory is short the graph reads the first
+    if (f16) {  // where memory is short the graph reads the first. (What the pool holds goes back to the driver when it is needed.)
       size_t left = 0, total = 0;
       VKL_CUDA(cudaMemGetInfo(&left, &total));
-      if (left < 2 * need) return VKL_OK;
+      if (left + m->dev->pool_bytes() < 2 * vkl_device::size_class(need)) return VKL_OK;
     }
     if (const int st = tensor_new(m->dev, 1, 1, need / 4, VKL_UINT32, &m->mega_packed)) return f16 && st == VKL_RESOURCE_EXHAUSTED ? VKL_OK : st;
   }
