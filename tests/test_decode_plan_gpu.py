@@ -122,6 +122,26 @@ def test_fp16_copy_where_memory_is_short_and_where_the_pool_has_it(dev):
     dm.close()
 
 
+def test_fp16_copy_makes_way_for_the_rows_of_a_call(dev):
+    prompt, tok = O.synth_tokens(56, 1000, 4000, 500), np.array([7], np.uint32)
+    dm = model(dev, F16_DIMS, True, 56)
+    want = dm(prompt, 0)
+    one = dm(tok, 4000)
+    dm.close()
+    dm = model(dev, F16_DIMS, True, 56)
+    dm(prompt[:20], 0)
+    dm(tok, 20)
+    assert launches(lambda: dm(tok, 21))[1] == 1
+    filler = fill(dev, 64)  # the rows need 230 MiB
+    try:
+        assert (dm(prompt, 0) == want).all()
+        got, n = launches(lambda: dm(tok, 4000))
+    finally:
+        del filler
+    assert n > 5 and np.abs(got - one).max() <= LOGITS_MAX_ABS
+    dm.close()
+
+
 def test_a_single_generated_id_has_no_use_for_the_copy(dev):
     dm = model(dev, F16_DIMS, True, 57)
     prompt = O.synth_tokens(57, 1000, 20, 500)

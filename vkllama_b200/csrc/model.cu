@@ -59,9 +59,7 @@ void release_mega(vkl_model *m, bool copy) {
 }
 
 bool use_gemm(const vkl_model *m, uint32_t rows);
-int ensure_rows(vkl_model *m, uint32_t T) {
-  if (T <= m->cap_T) return VKL_OK;
-  if (m->dec) return decoder_ensure_rows(m, T);
+int grow_rows(vkl_model *m, uint32_t T) {
   model_drop_graph(m);  // the graph holds the old buffers
   VKL_CUDA(cudaStreamSynchronize(m->stream));
   m->cap_T = 0;  // an allocation that fails below leaves buffers missing: the next call makes them anew
@@ -86,6 +84,16 @@ int ensure_rows(vkl_model *m, uint32_t T) {
   }
   m->cap_T = T;
   return VKL_OK;
+}
+int ensure_rows(vkl_model *m, uint32_t T) {
+  if (T <= m->cap_T) return VKL_OK;
+  if (m->dec) return decoder_ensure_rows(m, T);
+  int st = grow_rows(m, T);
+  if (st == VKL_RESOURCE_EXHAUSTED && !q8(m) && m->mega_packed) {  // FP16 weights decode without the second copy, too
+    release_mega(m, true);
+    st = grow_rows(m, T);
+  }
+  return st;
 }
 
 MvParams mv(const vkl_model *m, const vkl_tensor *w, const __half *x, __half *out, uint32_t M) {
@@ -355,7 +363,7 @@ int make_mega(vkl_model *m) {
       VKL_CUDA(cudaMemGetInfo(&left, &total));
       if (left + m->dev->pool_bytes() < 2 * vkl_device::size_class(need)) return VKL_OK;
     }
-    if (const int st = tensor_new(m->dev, 1, 1, need / 4, VKL_UINT32, &m->mega_packed)) return f16 && st == VKL_RESOURCE_EXHAUSTED ? VKL_OK : st;
+    VKL_OKAY(tensor_new(m->dev, 1, 1, need / 4, VKL_UINT32, &m->mega_packed));
   }
   size_t packed_at = 0;
 
@@ -570,7 +578,7 @@ int build_mega(vkl_model *m) {
     cudaStreamSynchronize(m->stream);
     release_mega(m, true);
   }
-  return st;
+  return st == VKL_RESOURCE_EXHAUSTED && !q8(m) ? VKL_OK : st;  // (the graph needs none of it)
 }
 
 __global__ void bump_sequence_kernel(uint32_t *seq, uint32_t by) { *seq += by; }
