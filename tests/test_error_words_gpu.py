@@ -9,6 +9,7 @@ import pytest
 
 import vkllama_b200 as vk
 from oracle import oracle as O
+from util import LOGITS_MAX_ABS, load_from_oracle
 from vkllama_b200 import build as B
 
 pytestmark = pytest.mark.gpu
@@ -23,7 +24,7 @@ def words(tmp_path_factory):
     for f in (L.raise_model_word, L.command_is_watched, L.raise_command_word, L.decode_word):
         f.argtypes = [C.c_void_p]
     L.decode_word.restype = C.c_uint32
-    L.set_polls.argtypes = [C.c_void_p, C.c_uint32]
+    L.set_polls.argtypes = L.shift_v_cache.argtypes = [C.c_void_p, C.c_uint32]
     return L
 
 
@@ -70,6 +71,21 @@ def test_a_decode_wait_that_ran_out_on_any_sm_is_reported(dev, words):
     assert failed
     dm.set_wait_limit(0)
     assert (dm(tok, 1) == want).all()
+    dm.close()
+
+
+def test_caches_that_the_decode_kernel_cannot_address_are_left_to_the_graph(dev, words):
+    """It names the V cache by its distance from the K cache, in 256 bytes."""
+    cfg = dict(dim=256, heads=4, ffn=512, vocab=1000, layers=2, maxlen=64)
+    om = O.Model(seed=74, **cfg)
+    dm = vk.Model(dev, 256, 4, 512, 1000, 2, 64)
+    load_from_oracle(dm, om)
+    assert words.shift_v_cache(dm.h, 1) == 0
+    text = O.synth_tokens(74, 1000, 4, 1000)
+    for i in range(4):
+        before = vk.kernel_launches()
+        assert np.abs(dm(text[i:i + 1], i) - om.forward(text[i:i + 1], i)).max() <= LOGITS_MAX_ABS, i
+        assert vk.kernel_launches() - before > 10
     dm.close()
 
 

@@ -320,6 +320,10 @@ int make_mega(vkl_model *m) {
   int coop = 0;
   VKL_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->dev->ordinal));
   if (!coop) return VKL_OK;
+  for (const Layer &y : m->L) {  // MegaRun::to_v: the graph has no such limit
+    const ptrdiff_t to_v = y.vcache->data() - y.kcache->data();
+    if (to_v % 256 || to_v / 256 != (int32_t)(to_v / 256)) return VKL_OK;
+  }
   const int G = m->dev->prop.multiProcessorCount;
   uint32_t splits = (uint32_t)G / m->heads_l;
   if (splits < 1) return VKL_OK;  // more heads than SMs: keep the graph path
@@ -489,7 +493,6 @@ int make_mega(vkl_model *m) {
   for (const MegaOp &o : ops) {
     if (o.kind == MK_ATTN_PART) {
       const ptrdiff_t to_v = (const uint8_t *)o.vcache - (const uint8_t *)o.kcache;
-      if (to_v % 256 || to_v / 256 != (int32_t)(to_v / 256)) return fail(VKL_INTERNAL, "decode kernel: caches are not on 256-byte boundaries");
       for (uint32_t cta = 0; cta < m->heads_l * splits; ++cta) runs[(size_t)cta * max_runs + counts[cta]++] = {(const uint8_t *)o.kcache, MEGA_KV_MARK, (int32_t)(to_v / 256)};
     } else if (o.kind == MK_MATVEC) {
       for (uint32_t cta = 0; cta < (uint32_t)G; ++cta) {
