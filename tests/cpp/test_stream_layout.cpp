@@ -1,6 +1,6 @@
 // Host-side check of the decode kernel's weight-stream bookkeeping (csrc/kernels.h): the tile order of the packed
-// stream is a permutation in which every CTA's tiles are consecutive, and cutting a CTA's units into ring stages
-// covers every unit exactly once, in order, with the two tiles of a stage adjacent in memory. No GPU involved.
+// stream is a permutation in which every CTA's tiles are consecutive, the warps' shares cover a CTA's units and a split's
+// cache rows exactly once, in order, and the reduction asks the warps that hold a tile's sums. No GPU involved.
 #include <cstdio>
 #include <vector>
 
@@ -18,28 +18,34 @@ static int check(uint32_t tiles, uint32_t grid, uint32_t blocks) {
     const uint32_t tl = (tiles - tile0 + grid - 1) / grid;
     for (uint32_t lt = 1; lt < tl; ++lt)  // a CTA's tiles follow each other
       if (mega_stream_tile(tile0 + lt * grid, tiles, grid) != mega_stream_tile(tile0, tiles, grid) + lt) return 2;
-    // stage cutting: every unit once, in order
-    uint32_t tm = 0, kg = 0;
-    uint64_t next_unit = 0;  // position in the CTA's own unit sequence
-    uint32_t stages = 0;
-    while (tm < tl) {
-      const MegaCut cut = mega_stage_cut(kg, blocks, tm + 1 < tl);
-      if (cut.n0 == 0 || cut.n0 + cut.n1 > MEGA_SU) return 3;
-      if ((uint64_t)tm * blocks + kg != next_unit) return 4;
-      if (cut.n1 && kg + cut.n0 != blocks) return 5;  // the second tile's units start where the first tile ends
-      next_unit += cut.n0 + cut.n1;
-      mega_stage_advance(cut, blocks, tm, kg);
-      if (++stages > 1000000) return 6;
+    // the warps' shares: every unit once, in order, and as many places for its tiles as a warp needs
+    const uint32_t units = tl * blocks, slots = mega_red_slots(tiles, blocks, grid);
+    std::vector<uint32_t> owner(units, MEGA_NCW);
+    for (uint32_t w = 0; w < MEGA_NCW; ++w) {
+      const uint32_t u0 = mega_share_begin(units, w), u1 = mega_share_begin(units, w + 1);
+      if (u0 > u1 || u1 > units) return 3;
+      for (uint32_t u = u0; u < u1; ++u) owner[u] = w;
+      if (u0 < u1 && (u1 - 1) / blocks - u0 / blocks + 1 > slots) return 4;
     }
-    if (next_unit != (uint64_t)tl * blocks) return 7;
+    if (slots < 1 || mega_share_begin(units, 0) != 0 || mega_share_begin(units, MEGA_NCW) != units) return 5;
+    // the warps that the reduction of a tile asks are those with units of it, and it finds the tile's place
+    for (uint32_t lt = 0; lt < tl; ++lt) {
+      const MegaTileShares ts = mega_tile_shares(units, blocks, lt);
+      if (ts.first != owner[lt * blocks] || ts.first + ts.more != owner[lt * blocks + blocks - 1]) return 6;
+      if (ts.place != lt - mega_share_begin(units, ts.first) / blocks || ts.place >= slots) return 7;
+      for (uint32_t w = ts.first + 1; w <= ts.first + ts.more; ++w) {
+        const uint32_t u0 = mega_share_begin(units, w), u1 = mega_share_begin(units, w + 1);
+        if (u0 < u1 && u0 / blocks != lt) return 8;  // their first place is this tile's
+      }
+    }
   }
   return 0;
 }
 
 int main() {
   const uint32_t grids[] = {1, 2, 7, 132, 148};
-  const uint32_t tile_counts[] = {1, 3, 128, 147, 148, 149, 160, 384, 480, 688, 864, 1000};
-  const uint32_t block_counts[] = {1, 2, 29, 30, 31, 40, 128, 160, 344, 432};
+  const uint32_t tile_counts[] = {1, 3, 128, 147, 148, 149, 160, 384, 480, 688, 864, 1000, 1907};
+  const uint32_t block_counts[] = {1, 2, 3, 5, 10, 11, 12, 29, 30, 31, 40, 128, 160, 344, 432, 864};
   for (uint32_t g : grids)
     for (uint32_t t : tile_counts)
       for (uint32_t b : block_counts)
@@ -62,6 +68,20 @@ int main() {
           mega_kv_range(L, S, s, c0, c1);
           if (c0 != at || c1 < c0) {
             std::printf("FAIL kv range L=%u S=%u s=%u\n", L, S, s);
+            return 1;
+          }
+          uint32_t row = c0;
+          for (uint32_t w = 0; w < MEGA_NCW; ++w) {
+            uint32_t r0, rows;
+            mega_kv_share(c0, c1, w, r0, rows);
+            if (rows && r0 != row) {
+              std::printf("FAIL kv share L=%u S=%u s=%u w=%u\n", L, S, s, w);
+              return 1;
+            }
+            row += rows;
+          }
+          if (row != c1) {
+            std::printf("FAIL kv shares L=%u S=%u s=%u\n", L, S, s);
             return 1;
           }
           at = c1;

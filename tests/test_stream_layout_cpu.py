@@ -1,5 +1,5 @@
-"""Host-side bookkeeping of the persistent decode kernel (tile order of the packed weight stream, stage
-cutting, attention split ranges), compiled from csrc/kernels.h with the host compiler and run on the CPU."""
+"""Host-side bookkeeping of the persistent decode kernel (tile order of the packed weight stream, warps'
+shares of it and of the cache rows, attention split ranges), compiled from csrc/kernels.h with the host compiler and run on the CPU."""
 import os
 import shutil
 import subprocess
@@ -9,7 +9,7 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-def test_stream_layout_and_stage_cuts(tmp_path):
+def test_stream_layout_and_shares(tmp_path):
     cuda_inc = "/usr/local/cuda/include"
     if not shutil.which("g++") or not os.path.isdir(cuda_inc):
         pytest.skip("needs g++ and the CUDA headers")

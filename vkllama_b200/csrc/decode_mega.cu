@@ -266,7 +266,6 @@ struct Ctx {
 // requested into the place of the one that the warp has just taken, so nothing but the copy's own barrier is needed: the
 // reads of the old bytes come before the request in program order (__syncwarp between them). The requests sit between a
 // warp's loads and its arithmetic, so what they need is worked out beforehand: no divisions, nothing from global memory.
-__device__ __forceinline__ uint32_t share_begin(uint32_t units, uint32_t w) { return units * w / NCW; }
 // The cached rows that a warp takes of every attention op of the token.
 struct alignas(16) KvShare {
   unsigned long long off;  // bytes from the start of a cache to the first of them
@@ -287,9 +286,7 @@ __device__ __forceinline__ void kv_plan(const MegaParams &p, KvPlan &k, uint32_t
   if (head < p.heads) {
     uint32_t c0, c1;
     mega_kv_range(L, S, split, c0, c1);
-    const uint32_t each = (c1 - c0 + NCW - 1) / NCW;
-    sh.r0 = min(c0 + warp * each, c1);
-    sh.rows = min(each, c1 - sh.r0);
+    mega_kv_share(c0, c1, warp, sh.r0, sh.rows);
     sh.off = ((unsigned long long)head * p.maxlen + sh.r0) * rowb;
   }
   k.share[warp] = sh;
@@ -340,7 +337,7 @@ __device__ __forceinline__ void ring_request(const MegaParams &p, const RunTable
         r.src = e.src + sh.off;
         r.rest = sh.rows * p.head_dim * 2u;
       } else {
-        const uint32_t u0 = share_begin(e.units, warp), n = share_begin(e.units, warp + 1) - u0;
+        const uint32_t u0 = mega_share_begin(e.units, warp), n = mega_share_begin(e.units, warp + 1) - u0;
         r.src = e.src + (size_t)u0 * UB;
         r.whole = n / SU;
         r.rest = n % SU * UB;
@@ -524,16 +521,14 @@ __device__ __forceinline__ void matvec_op(const Ctx &c, const MegaOp &op_global,
   // No tile here: nothing to read either. (It must not wait for the input: nobody waits for this
   // CTA's results, so by the time it looked the producers of a later op may have re-tagged the words.)
   if (tl == 0) return;
-  // This warp's share of the CTA's units, and, for the reduction, the warps w0..w1 whose shares touch this thread's tile: their
-  // sums of it lie in the first of their places, but for w0, whose share may have begun tiles before.
+  // This warp's share of the CTA's units, and, for the reduction, the warps whose shares touch this thread's tile.
   const uint32_t units = tl * blocks, rspan = c.p.red_slots;
-  uint32_t u = share_begin(units, warp), b = u % blocks;
-  const uint32_t u1 = share_begin(units, warp + 1);
+  uint32_t u = mega_share_begin(units, warp), b = u % blocks;
+  const uint32_t u1 = mega_share_begin(units, warp + 1);
   auto touching = [&](uint32_t lt, uint32_t &at, uint32_t &n) {
-    const uint32_t ub = lt * blocks, w0 = (NCW * (ub + 1) - 1) / units;
-    n = (NCW * (ub + blocks) - 1) / units - w0;
-    at = (w0 * rspan + lt - share_begin(units, w0) / blocks) * 32;
-    n |= w0 << 16;
+    const MegaTileShares ts = mega_tile_shares(units, blocks, lt);
+    at = (ts.first * rspan + ts.place) * 32;
+    n = ts.more | ts.first << 16;
   };
   // row r of tile lt: which matrix and which of its rows
   auto row_of = [&](uint32_t lt, uint32_t r, uint32_t &m, uint32_t &n) {
@@ -1467,10 +1462,6 @@ size_t decode_mega_xs_bytes(uint32_t max_blocks, uint32_t head_dim) {
 }
 size_t decode_mega_smem(size_t xs_bytes, uint32_t nst, uint32_t red_slots, uint32_t runs) {
   return (size_t)NCW * nst * PIECE_BYTES + xs_bytes + ((size_t)red_slots * NCW * 32 + 64) * 4 + runs * sizeof(MegaRun) + sizeof(KvPlan) + NCW * MAX_NST * 8 + 16 + 3 * sizeof(MegaOp) + 64;
-}
-uint32_t decode_mega_red_slots(uint32_t tiles, uint32_t blocks, uint32_t grid) {
-  const uint32_t tl = (tiles + grid - 1) / grid, share = (tl * blocks + NCW - 1) / NCW;
-  return std::min(tl, (share + blocks - 2) / blocks + 1);
 }
 int decode_mega_max_k() { return 16384; }
 int decode_mega_max_stages() { return MAX_NST; }

@@ -224,30 +224,29 @@ __host__ __device__ inline void mega_kv_range(uint32_t L, uint32_t S, uint32_t s
   c0 = split * chunk < L ? split * chunk : L;
   c1 = c0 + chunk < L ? c0 + chunk : L;
 }
-// A piece that starts at block `kg` of a tile of `blocks` blocks, as far as the end of the next tile (if the CTA has one): n0
-// units of this tile, then n1 of the next. Units follow each other in memory, so pieces need no table; the host-side check of
-// the stream's order walks it with this rule.
-struct MegaCut {
-  uint32_t n0, n1;
+// Shares. The `units` units that a CTA reads of an op (its tiles of `blocks` blocks, one behind the other) go to the warps in equal
+// consecutive parts: warp w has those from mega_share_begin(units, w) to mega_share_begin(units, w + 1).
+__host__ __device__ inline uint32_t mega_share_begin(uint32_t units, uint32_t w) { return units * w / MEGA_NCW; }
+// A warp adds up each tile of its share by itself, in a place of its own per tile. The warps whose shares touch tile lt are first ..
+// first + more (warps with an empty share among them count: their first place holds zeros), and the tile is the place-th that warp `first`
+// touches and the first that the others do.
+struct MegaTileShares {
+  uint32_t first, more, place;
 };
-__host__ __device__ inline MegaCut mega_stage_cut(uint32_t kg, uint32_t blocks, bool has_next) {
-  MegaCut c;
-  c.n0 = blocks - kg < MEGA_SU ? blocks - kg : MEGA_SU;
-  const uint32_t rem = MEGA_SU - c.n0;
-  c.n1 = has_next ? (rem < blocks ? rem : blocks) : 0u;
-  return c;
+__host__ __device__ inline MegaTileShares mega_tile_shares(uint32_t units, uint32_t blocks, uint32_t lt) {
+  const uint32_t ub = lt * blocks, first = (MEGA_NCW * (ub + 1) - 1) / units;
+  return {first, (MEGA_NCW * (ub + blocks) - 1) / units - first, lt - mega_share_begin(units, first) / blocks};
 }
-__host__ __device__ inline void mega_stage_advance(const MegaCut &c, uint32_t blocks, uint32_t &tm, uint32_t &kg) {
-  if (c.n1) {
-    tm += 1;
-    kg = c.n1;
-  } else {
-    kg += c.n0;
-  }
-  if (kg >= blocks) {
-    kg = 0;
-    tm += 1;
-  }
+// The most places that a warp needs of an op of `tiles` tiles.
+__host__ __device__ inline uint32_t mega_red_slots(uint32_t tiles, uint32_t blocks, uint32_t grid) {
+  const uint32_t tl = (tiles + grid - 1) / grid, share = (tl * blocks + MEGA_NCW - 1) / MEGA_NCW, most = (share + blocks - 2) / blocks + 1;
+  return tl < most ? tl : most;
+}
+// The cached rows [r0, r0 + rows) of a split's [c0, c1) that warp w takes.
+__host__ __device__ inline void mega_kv_share(uint32_t c0, uint32_t c1, uint32_t w, uint32_t &r0, uint32_t &rows) {
+  const uint32_t each = (c1 - c0 + MEGA_NCW - 1) / MEGA_NCW, at = c0 + w * each;
+  r0 = at < c1 ? at : c1;
+  rows = each < c1 - r0 ? each : c1 - r0;
 }
 struct MegaParams {
   const MegaOp *ops;
@@ -304,8 +303,6 @@ cudaError_t launch_mega_pack(const uint8_t *const planes[3], uint32_t nmat, int 
                              uint32_t grid, uint8_t *stream, cudaStream_t s);
 cudaError_t launch_mega_pack_f16(const __half *const w[3], uint32_t nmat, int swiglu, uint32_t N, uint32_t K, uint32_t tiles, uint32_t grid, uint8_t *stream, cudaStream_t s);
 size_t decode_mega_smem(size_t xs_bytes, uint32_t nst, uint32_t red_slots, uint32_t runs);
-// The most tiles that one warp's share of an op of `tiles` tiles touches.
-uint32_t decode_mega_red_slots(uint32_t tiles, uint32_t blocks, uint32_t grid);
 int decode_mega_max_k();
 int decode_mega_max_stages();
 cudaError_t decode_mega_occupancy(size_t smem_bytes, int *blocks_per_sm);

@@ -342,7 +342,7 @@ int make_mega(vkl_model *m) {
   const char *sr_env = getenv("VKLLAMA_SPLIT_ROWS");
   const uint32_t split_rows = sr_env ? (uint32_t)atoi(sr_env) : 384u;
   const size_t xs_bytes = decode_mega_xs_bytes(max_blocks, m->head_dim);
-  auto slots = [&](uint32_t tiles, uint32_t k) { return decode_mega_red_slots(tiles, k / columns, (uint32_t)G); };
+  auto slots = [&](uint32_t tiles, uint32_t k) { return mega_red_slots(tiles, k / columns, (uint32_t)G); };
   const uint32_t red_slots = std::max({slots(3 * ((m->dim_l + 31) / 32), c.dim), slots((c.dim + 31) / 32, m->dim_l), slots((m->ffn_l + 15) / 16, c.dim),
                                        slots((c.dim + 31) / 32, m->ffn_l), slots((m->vocab_l + 31) / 32, c.dim)});
   const uint32_t max_runs = 5 * c.layers + 1;  // four matrices and an attention op per block, the output layer
