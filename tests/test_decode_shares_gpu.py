@@ -31,8 +31,10 @@ def test_one_token_calls_match_the_oracle(dev, f16, dim, heads, ffn, vocab, pos)
     om.forward(text[:pos], 0)
     dm(text[:pos], 0)
     for i in range(pos, pos + 3):
-        want, got = om.forward(text[i:i + 1], i), dm(text[i:i + 1], i)
+        want, before = om.forward(text[i:i + 1], i), vk.kernel_launches()
+        got = dm(text[i:i + 1], i)
         assert np.abs(got - want).max() <= LOGITS_MAX_ABS, i
+        assert i == pos or vk.kernel_launches() - before == 1  # the persistent kernel (before its first launch the weights are packed)
     dm.close()
 
 
@@ -47,5 +49,7 @@ def test_fp16_decode_without_the_persistent_kernel(dev, monkeypatch):
     om.forward(text[:9], 0)
     dm(text[:9], 0)
     for i in range(9, 12):
+        before = vk.kernel_launches()
         assert np.abs(dm(text[i:i + 1], i) - om.forward(text[i:i + 1], i)).max() <= LOGITS_MAX_ABS, i
+        assert vk.kernel_launches() - before > 5 * 2
     dm.close()
