@@ -360,11 +360,11 @@ int vkl_model_decode_trace(vkl_model *m, uint32_t token, size_t offset, unsigned
  * output layer. vkl_model_forward returns this rank's slice of the logits. */
 int vkl_model_tp_buffer(vkl_model *m, void **local_ptr, size_t *bytes);
 /* Failure detection (the reference's counterpart is the 60 s fence time-out of
- * src/core/command.h:389-395). Every wait inside the persistent decode kernel (weight
- * stage, ring slot, tagged input, grid barrier, tensor-parallel all-reduce and arg-max
+ * src/core/command.h:389-395). Every wait inside the persistent decode kernel (weights
+ * or cache rows, tagged input, grid barrier, tensor-parallel all-reduce and arg-max
  * exchange) gives up after `polls` polls of about half a microsecond each: the kernel
  * then leaves through its normal path and the call returns VKL_INTERNAL naming the wait
- * (code 1 weight stage, 2 ring slot, 3 grid barrier, 4 all-reduce, 5 arg-max exchange,
+ * (code 1 weights or cache rows, 3 grid barrier, 4 all-reduce, 5 arg-max exchange,
  * 6 tagged input). The device context stays usable. Default (polls = 0): 2^21, and 2^24
  * for tensor-parallel models, the same bound for every wait so that none gives up while
  * another it depends on is still waiting; ranks may start a step up to that much apart.

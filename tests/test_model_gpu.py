@@ -472,7 +472,7 @@ def test_wait_that_runs_out_returns_an_error_and_leaves_the_device_usable(dev):
 
 def test_short_wait_bound_on_a_healthy_model_is_reported_not_hung(dev):
     """With a bound far below what a step needs, the first wait that cannot be met reports its code
-    (a weight stage, a ring slot or a tagged input); restoring the default bound makes the same
+    (weights or cache rows, the grid barrier or a tagged input); restoring the default bound makes the same
     model work again and give the oracle's ids."""
     om, dm, cfg = small_pair(dev, seed=43)
     prompt = O.synth_tokens(43, 1000, 5, cfg["vocab"])

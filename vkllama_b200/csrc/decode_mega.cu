@@ -1,4 +1,4 @@
-// One persistent kernel per decode token (Q8_0 weights, batch 1).
+// One persistent kernel per decode token (Q8_0 or FP16 weights, batch 1).
 //
 // The reference records 19 Vulkan dispatches per layer per token
 // (models/llama2.h:160-213, src/ops/multiheadattention_v2.cpp:190-319) and stalls
@@ -10,7 +10,7 @@
 //     (cp.async.bulk + mbarrier): as soon as it has used a piece (MEGA_SU units), its lane 0 requests the piece
 //     that takes its place, across op boundaries. Weights never depend on activations, so HBM stays busy while
 //     the warps sit in a norm, an attention op or a wait;
-//   * a unit is one Q8_0 block x 32 rows: the codes go into the tensor cores as fp16 subnormals (exact, one
+//   * a unit is one Q8_0 block x 32 rows (FP16: 16 columns x 32 rows, MMA operands as they are): the codes go into the tensor cores as fp16 subnormals (exact, one
 //     byte permute per pair; m16n8k16, fp32 accumulate), block scales are applied in fp32, the warps' sums of
 //     a tile are added in fixed order and the fused epilogue runs (RMSNorm prologue, residual add, SwiGLU, fp32
 //     logits, running arg-max);
@@ -23,7 +23,7 @@
 // What bounds it: not HBM (7B: 1.45 ms per token against 1.07 at the measured copy rate) and not the tensor pipe (12 %), but
 // what a warp executes one instruction after the other: with three warps per scheduler and dependent instructions four to six
 // cycles apart, a branch costs 50 to 100 cycles of a warp's time and even an empty turn of the stream loop took 400. With no
-// weight copies at all a 7B token of the version before took 1.49 of its 1.53 ms. Hence: no producer warp and no barrier pair
+// weight copies at all a 7B token of this form's first version took 1.49 of its 1.53 ms. Hence: no producer warp and no barrier pair
 // per stage between warps (its handshake, table entry and two units per stage and warp bounded the earlier form: 1.60 ms);
 // straight-line code for whole pieces; divisions, addresses and residuals worked out before the input arrives; and little code
 // and no spills, because both come from memory behind the weight stream when they miss (150 KB of code 1.68 ms, 123 KB
@@ -44,7 +44,7 @@
 namespace vkl {
 namespace {
 
-constexpr int NCW = (int)MEGA_NCW;     // warps, 184 registers each
+constexpr int NCW = (int)MEGA_NCW;     // warps: at most 184 registers per thread (160 to 168 are used)
 constexpr int CT = NCW * 32;
 constexpr int THREADS = CT;
 constexpr int SU = (int)MEGA_SU;       // units per piece, the step of a warp's ring
@@ -158,10 +158,9 @@ __device__ __forceinline__ unsigned long long gtime() {
 // words through local memory and registers to be saved around every wait.
 struct Ctx;
 #define VKL_SLOW __forceinline__
-__device__ VKL_SLOW bool slow_mbar_wait(volatile uint32_t *abort_s, uint32_t *error, uint32_t limit, uint32_t bar, uint32_t parity, uint32_t code, uint32_t sleep_ns) {
+__device__ VKL_SLOW bool slow_mbar_wait(volatile uint32_t *abort_s, uint32_t *error, uint32_t limit, uint32_t bar, uint32_t parity, uint32_t code) {
 #pragma unroll 1
   for (uint32_t i = 0; i < limit; ++i) {
-    if (sleep_ns) __nanosleep(sleep_ns);  // keep a waiting warp off the shared-memory pipe the working warps need
     if (mbar_try(bar, parity)) return true;
     if ((i & 255u) == 255u && (*(volatile uint32_t *)error != 0u || *abort_s != 0)) {
       *abort_s = 1;
@@ -374,7 +373,7 @@ template <bool DBG>
 __device__ __forceinline__ void ring_take(const Ctx &c, Ring &r) {
   if (DBG && (c.p.timing_mode & 128u)) return;
   if (mbar_try(r.bar, r.ph)) return;
-  if (c.aborted() || !slow_mbar_wait(c.abort_s, c.p.error, c.p.wait_limit, r.bar, r.ph, 1, 0)) r.lead = false;
+  if (c.aborted() || !slow_mbar_wait(c.abort_s, c.p.error, c.p.wait_limit, r.bar, r.ph, 1)) r.lead = false;
 }
 // The warp has read what it needs of the piece: request the one that takes its place, and on to the next.
 template <bool DBG, bool F16>
@@ -1552,7 +1551,7 @@ cudaError_t launch_mega_pack_f16(const __half *const w[3], uint32_t nmat, int sw
 cudaError_t launch_decode_mega(const MegaParams &p, int grid, cudaStream_t s) {
   if (p.nst < 2 || p.nst > (uint32_t)MAX_NST) return cudaErrorInvalidValue;
   const size_t smem = decode_mega_smem(p.xs_bytes, p.nst, p.red_slots, p.run_stride);
-  // the diagnostic switches (no weight copies, no arithmetic) are compiled into separate instances
+  // the diagnostic switches (no weight copies, no arithmetic) are compiled into separate instances, for Q8_0 weights only
   const bool dbg = (p.timing_mode & (2u | 4u | 16u | 64u | 128u)) != 0;  // (16: the diagnostic instance with nothing switched off, its own baseline)
   auto kern = p.f16 ? (p.timing ? decode_mega_kernel<true, false, false, true> : decode_mega_kernel<false, false, false, true>)
               : p.timing ? (dbg || p.tp_size > 1 ? decode_mega_kernel<true, true, true, false> : decode_mega_kernel<true, false, false, false>)
@@ -1564,10 +1563,11 @@ cudaError_t launch_decode_mega(const MegaParams &p, int grid, cudaStream_t s) {
   return cudaLaunchCooperativeKernel((void *)kern, dim3(grid), dim3(THREADS), args, smem, s);
 }
 
-cudaError_t decode_mega_occupancy(size_t smem, int *blocks_per_sm) {
-  cudaError_t e = cudaFuncSetAttribute(decode_mega_kernel<false, false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+cudaError_t decode_mega_occupancy(size_t smem, bool f16, bool tp, int *blocks_per_sm) {
+  auto kern = f16 ? decode_mega_kernel<false, false, false, true> : tp ? decode_mega_kernel<false, false, true, false> : decode_mega_kernel<false, false, false, false>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, decode_mega_kernel<false, false, true, false>, THREADS, smem);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, THREADS, smem);
 }
 
 }  // namespace vkl

@@ -155,11 +155,11 @@ enum MegaKind { MK_EMBED = 0, MK_MATVEC = 1, MK_ATTN_PART = 2, MK_ATTN_COMBINE =
 struct alignas(16) MegaOp {
   uint32_t kind, epi, nmat, rot;
   uint32_t N, K;          // rows of one matrix, columns
-  uint32_t tiles, blocks; // 32-row tiles of the op's packed weight stream, Q8_0 blocks per row (K / 32)
+  uint32_t tiles, blocks; // 32-row tiles of the op's packed weight stream, units per tile (K / 32; FP16 weights K / 16)
   // The op's weights, packed for the kernel (mega_pack): per 32-row tile and block one unit of
   // MEGA_UNIT_CODES + MEGA_UNIT_SCALES bytes. Codes: the two 512-byte (16 rows x 32 columns) units of the
   // library's tiled planes (common.cuh) that hold the tile's rows, as they are: MMA A-fragment order, biased
-  // by +128. Then the unit's scales: [g 0..7][rows g, g + 8, 16 + g, 24 + g] fp16. Units of a tile follow each
+  // by +128. Then the unit's scales: [g 0..7][rows g, g + 8, 16 + g, 24 + g] fp16. (FP16 weights: mega_pack_f16.) Units of a tile follow each
   // other block by block, tiles in the order of mega_stream_tile: everything one CTA reads of the op is one
   // consecutive range. Which matrix row a tile row is:
   //   one matrix         tile t, row r = matrix row 32 t + r
@@ -305,7 +305,7 @@ cudaError_t launch_mega_pack_f16(const __half *const w[3], uint32_t nmat, int sw
 size_t decode_mega_smem(size_t xs_bytes, uint32_t nst, uint32_t red_slots, uint32_t runs);
 int decode_mega_max_k();
 int decode_mega_max_stages();
-cudaError_t decode_mega_occupancy(size_t smem_bytes, int *blocks_per_sm);
+cudaError_t decode_mega_occupancy(size_t smem_bytes, bool f16, bool tp, int *blocks_per_sm);  // of the instance that a launch takes
 cudaError_t launch_decode_mega(const MegaParams &p, int grid, cudaStream_t s);
 
 // ---- dense FP16 GEMM on tcgen05 tensor cores: C[M,N] = A[M,K] . W[N,K]^T (gemm_tcgen05.cu) ----

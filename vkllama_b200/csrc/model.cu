@@ -303,9 +303,9 @@ int launch_advance(vkl_model *m, uint32_t pos_inc) {
 }
 
 // Builds the op table of the persistent decode kernel. Q8_0 weights, on any number of GPUs, or FP16 weights. Four 7B blocks of FP16
-// weights, ms for a 17-token prompt and 32 tokens: 14.3 with five kernels per block in a graph, 11.6 here (a new
-// model's first call, packing included, 14.8 and 12.8; 15.0 and 16.5 where the copy's 1.9 GB come from the device and not from the pool).
-// VKLLAMA_DECODE=graph keeps the multi-kernel CUDA-graph step instead.
+// weights, ms for a 17-token prompt and 32 tokens: 13.8 with five kernels per block in a graph, 11.3 here. A new model's first call
+// makes the second copy (1.9 GB: 0.9 ms to pack, 0.8 to 2.9 ms for the device to allocate), graph / here: 8 tokens 4.5 / 5.5, 32
+// tokens 14.8 / 13.8, 64 tokens 28.5 / 24.7. VKLLAMA_DECODE=graph keeps the multi-kernel CUDA-graph step, and one copy, instead.
 int make_mega(vkl_model *m) {
   const char *env = getenv("VKLLAMA_DECODE");
   if (env && !strcmp(env, "graph")) return VKL_OK;
@@ -351,7 +351,7 @@ int make_mega(vkl_model *m) {
   while (nst >= 2 && decode_mega_smem(xs_bytes, nst, red_slots, max_runs) > (size_t)m->dev->prop.sharedMemPerBlockOptin) --nst;
   if (nst < 2) return VKL_OK;
   int occ = 0;
-  VKL_CUDA(decode_mega_occupancy(decode_mega_smem(xs_bytes, nst, red_slots, max_runs), &occ));
+  VKL_CUDA(decode_mega_occupancy(decode_mega_smem(xs_bytes, nst, red_slots, max_runs), f16, tp > 1, &occ));
   if (occ < 1) return VKL_OK;
   VKL_OKAY(ensure_rows(m, 1));
   // The kernel reads a second copy of the matrices, all of it in one allocation (one per matrix took the first token of four 7B
@@ -362,7 +362,7 @@ int make_mega(vkl_model *m) {
     const size_t need = (size_t)c.layers * (stream_bytes(3 * (size_t)((m->dim_l + 31) / 32), c.dim) + stream_bytes((c.dim + 31) / 32, m->dim_l) +
                                             stream_bytes((m->ffn_l + 15) / 16, c.dim) + stream_bytes((c.dim + 31) / 32, m->ffn_l)) +
                         stream_bytes((m->vocab_l + 31) / 32, c.dim);
-    if (f16) {  // where memory is short the graph reads the first. (What the pool holds goes back to the driver when it is needed.)
+    if (f16) {  // where memory is short the graph reads the first (its sums run in another order: the low bits differ). (What the pool holds goes back to the driver when it is needed.)
       size_t left = 0, total = 0;
       VKL_CUDA(cudaMemGetInfo(&left, &total));
       if (left + m->dev->pool_bytes() < 2 * vkl_device::size_class(need)) return VKL_OK;
@@ -635,7 +635,7 @@ int check_mega(vkl_model *m) {
     // sequence numbers, words already pushed under the number a retry would expect): the model refuses
     // further steps until every rank has called vkl_model_tp_connect again, between two host barriers.
     if (m->cfg.tp_size > 1) m->tp_failed = true;
-    return fail(VKL_INTERNAL, "decode kernel: a bounded wait ran out (code %u: 1 weight stage, 2 ring slot, 3 grid barrier, 4 all-reduce, 5 arg-max exchange, 6 tagged input)", err);
+    return fail(VKL_INTERNAL, "decode kernel: a bounded wait ran out (code %u: 1 weights or cache rows, 3 grid barrier, 4 all-reduce, 5 arg-max exchange, 6 tagged input)", err);
   }
   return VKL_OK;
 }
